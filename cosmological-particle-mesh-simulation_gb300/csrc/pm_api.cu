@@ -10,14 +10,14 @@ struct pm_ctx {
   int n = 0;
   Tables tab;
   SortBufs sort;
-  DBuf d_sim, d_prefix, d_err, d_maps;
+  DBuf d_sim, d_work, d_err, d_maps;
   DBuf tile_next;  // tile counter of the fused deposit
   const void* maps_for = nullptr;     // spectrum the device tensor maps describe
   DBuf row_start, spec, phi, rho;     // scratch grids
   DBuf hpos, hvel;                    // device copies for pm_step_host
   DBuf pk_partial, pk_out;            // power spectrum scratch
-  DBuf row_count, row_cursor, scan_sums;  // counting sort of row keys
-  DBuf spos, svel;                        // the state in row order (drop-in step)
+  DBuf row_count, scan_sums;              // row counts of a call, block sums of their scan
+  DBuf rec;                               // cell records in row order, then the forces
   // spectral gradient: spectra and force grids of the y and z axes (x uses spec and phi), the
   // three descriptors of the inverse passes and their work tables and tensor maps
   DBuf gspec[2], ggrid[2], d_sim3, d_prefix3, d_maps3;
@@ -29,8 +29,6 @@ struct pm_ctx {
 };
 
 namespace {
-
-enum Phase { PH_KEYS = 0, PH_DEP, PH_KICK, PH_X, PH_LINE, PH_COUNT };
 
 int fail(pm_ctx* c, int code, const std::string& msg) {
   if (c) c->err = msg;
@@ -48,11 +46,10 @@ int cuda_fail(pm_ctx* c, cudaError_t e, const char* where) {
     if (e_ != cudaSuccess) return cuda_fail(c, e_, where);   \
   } while (0)
 
-// Host image of the single-simulation descriptor + its work prefixes.
+// Host image of the single-simulation descriptor + its work table.
 struct Call {
   Sim sim{};
-  int prefix[PH_COUNT][2]{};
-  Parts parts{};
+  CallWork work{};
 };
 
 Sim base_sim(pm_ctx* c, long long np) {
@@ -77,31 +74,32 @@ Sim base_sim(pm_ctx* c, long long np) {
   return s;
 }
 
-void set_prefix(Call& k, long long np, int n) {
-  k.prefix[PH_KEYS][1] = (int)((np + 255) / 256);
-  k.prefix[PH_DEP][1] = (n / TILE_Y) * (n / TILE_Z);
-  k.prefix[PH_KICK][1] = (int)((np + KICK_UNIT - 1) / KICK_UNIT);
-  k.prefix[PH_X][1] = (int)spectral_units(SPEC_X_R2C, n);
-  k.prefix[PH_LINE][1] = (int)spectral_units(SPEC_Y_FWD, n);
+void set_work(Call& k, long long np, int n) {
+  k.work.prefix[CALL_KEYS][1] = (int)((np + 255) / 256);
+  k.work.prefix[CALL_DEP][1] = (n / TILE_Y) * (n / TILE_Z);
+  k.work.prefix[CALL_X][1] = (int)spectral_units(SPEC_X_R2C, n);
+  k.work.prefix[CALL_LINE][1] = (int)spectral_units(SPEC_Y_FWD, n);
 }
 
-Work work(pm_ctx* c, const Call& k, Phase ph) {
+Work work(pm_ctx* c, const Call& k, CallPhase ph) {
   Work w;
-  w.prefix = c->d_prefix.as<int>() + 2 * ph;
+  w.prefix = c->d_work.as<CallWork>()->prefix[ph];
   w.nsims = 1;
-  w.total = k.prefix[ph][1];
+  w.total = k.work.prefix[ph][1];
   return w;
 }
 
-Parts abs_parts(float* pos, float* vel, long long np) {
+Parts abs_parts(const float* pos, long long np) {
   Parts p{};
-  p.x = pos;
-  p.y = pos ? pos + np : nullptr;
-  p.z = pos ? pos + 2 * np : nullptr;
-  p.vx = vel;
-  p.vy = vel ? vel + np : nullptr;
-  p.vz = vel ? vel + 2 * np : nullptr;
-  p.id = nullptr;
+  p.x = const_cast<float*>(pos);
+  p.y = p.x + np;
+  p.z = p.x + 2 * np;
+  return p;
+}
+
+Parts record_parts(pm_ctx* c) {
+  Parts p{};
+  p.rec = c->rec.as<uint4>();
   return p;
 }
 
@@ -111,20 +109,19 @@ int check_np(pm_ctx* c, long long np) {
   return PM_OK;
 }
 
-int upload(pm_ctx* c, Call& k, cudaStream_t st) {
-  PM_CK(cudaMemcpyAsync(c->d_sim.p, &k.sim, sizeof(Sim), cudaMemcpyHostToDevice, st), "upload sim");
-  PM_CK(cudaMemcpyAsync(c->d_prefix.p, k.prefix, sizeof(k.prefix), cudaMemcpyHostToDevice, st),
-        "upload work");
+// The call's descriptor and work table on the device; zero (optional): bytes cleared with them.
+int begin(pm_ctx* c, const Call& k, cudaStream_t st, void* zero = nullptr, size_t zero_bytes = 0) {
+  PM_CK(launch_call_begin(c->d_sim.as<Sim>(), c->d_work.as<CallWork>(), k.sim, k.work, zero, zero_bytes, st), "begin");
   return PM_OK;
 }
 
 // keys -> sort -> row starts for absolute positions; leaves perm / sorted keys pointers.
-int sort_particles(pm_ctx* c, Call& k, cudaStream_t st, unsigned** perm, unsigned** skeys) {
+int sort_particles(pm_ctx* c, Call& k, const float* positions, cudaStream_t st, unsigned** perm, unsigned** skeys) {
   const long long np = k.sim.np;
   PM_CK(c->sort.ensure(np), "alloc sort");
   const Sim* ds = c->d_sim.as<Sim>();
-  PM_CK(launch_keys_abs(ds, work(c, k, PH_KEYS), k.parts, c->sort.keys.as<unsigned>(), nullptr,
-                        c->d_err.as<int>(), grid_for(k.prefix[PH_KEYS][1], c->sms, 16), st),
+  PM_CK(launch_keys_abs(ds, work(c, k, CALL_KEYS), abs_parts(positions, np), c->sort.keys.as<unsigned>(), nullptr,
+                        c->d_err.as<int>(), grid_for(k.work.prefix[CALL_KEYS][1], c->sms, 16), st),
         "keys");
   const long long nrows = (long long)c->n * c->n;
   const int bits = ceil_log2(nrows) + k.sim.xbits;
@@ -137,34 +134,33 @@ int sort_particles(pm_ctx* c, Call& k, cudaStream_t st, unsigned** perm, unsigne
   return PM_OK;
 }
 
-// keys (x-row numbers: k.sim.xbits must be 0) -> counting sort: row starts in c->row_start
-// and the permutation to row order.  The deposit and the kick need the particles grouped
-// by row only; their results do not depend on the order inside a row.
-int group_particles(pm_ctx* c, Call& k, cudaStream_t st, unsigned** perm, unsigned* inv = nullptr,
-                    float* pos_copy = nullptr) {
+// Writes the call's descriptor and groups the particles by x-row: row starts in c->row_start,
+// cell records in row order in c->rec, and each particle's place there in c->sort.keys.  The
+// deposit and the force need the particles grouped by row only; their results do not depend
+// on the order inside a row.  Work enqueued here reads `positions` once more after the
+// first kernel: pos_copy (optional) receives a device copy in that first read.
+int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy, cudaStream_t st) {
   const long long np = k.sim.np;
   const unsigned nrows = (unsigned)((long long)c->n * c->n);
   PM_CK(c->sort.ensure(np), "alloc sort");
+  PM_CK(c->rec.ensure((size_t)np * sizeof(uint4)), "alloc records");
   PM_CK(c->row_start.ensure(((size_t)nrows + 1) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->row_count.ensure((size_t)nrows * sizeof(unsigned)), "alloc rows");
-  PM_CK(c->row_cursor.ensure((size_t)nrows * sizeof(unsigned)), "alloc rows");
   PM_CK(c->scan_sums.ensure(row_sort_block_sums(nrows) * sizeof(unsigned)), "alloc rows");
-  PM_CK(launch_keys_abs(c->d_sim.as<Sim>(), work(c, k, PH_KEYS), k.parts, c->sort.keys.as<unsigned>(), nullptr,
-                        c->d_err.as<int>(), grid_for(k.prefix[PH_KEYS][1], c->sms, 16), st,
-                        pos_copy ? abs_parts(pos_copy, nullptr, np) : Parts{}),
-        "keys");
-  *perm = c->sort.vals.as<unsigned>();
-  PM_CK(row_counting_sort(c->sort.keys.as<unsigned>(), np, nrows, c->row_count.as<unsigned>(),
-                          c->row_start.as<unsigned>(), c->row_cursor.as<unsigned>(), c->scan_sums.as<unsigned>(),
-                          *perm, c->d_err.as<int>(), c->sms, st, inv),
-        "sort");
+  unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
+  unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
+  if (int r = begin(c, k, st, count, (size_t)nrows * sizeof(unsigned))) return r;
+  PM_CK(launch_row_rank(positions, np, c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, st), "row ranks");
+  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), st), "row starts");
+  PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, c->n, start, ranks, place, c->rec.as<uint4>(), st),
+        "row order");
   return PM_OK;
 }
 
-int deposit(pm_ctx* c, Call& k, unsigned* perm, cudaStream_t st) {
-  PM_CK(launch_deposit(c->d_sim.as<Sim>(), work(c, k, PH_DEP), k.parts, perm, c->row_start.as<unsigned>(),
-                       POS_ABS, c->d_err.as<int>(), grid_for(k.prefix[PH_DEP][1], c->sms, 8),
-                       deposit_smem_bytes(c->n, TILE_Y, TILE_Z), st),
+int deposit(pm_ctx* c, Call& k, cudaStream_t st) {
+  PM_CK(launch_deposit(c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
+                       c->row_start.as<unsigned>(), POS_DISP, c->d_err.as<int>(),
+                       grid_for(k.work.prefix[CALL_DEP][1], c->sms, 8), deposit_smem_bytes(c->n, TILE_Y, TILE_Z), st),
         "deposit");
   return PM_OK;
 }
@@ -174,16 +170,16 @@ int gradient_solve(pm_ctx* c, Call& k, cudaStream_t st);
 int spectral(pm_ctx* c, Call& k, bool table, cudaStream_t st, bool skip_r2c = false, bool gradient = false) {
   const Sim* ds = c->d_sim.as<Sim>();
   const int n = c->n;
-  const int gx = grid_for(k.prefix[PH_X][1], c->sms, 8), gl = grid_for(k.prefix[PH_LINE][1], c->sms, 8);
+  const int gx = grid_for(k.work.prefix[CALL_X][1], c->sms, 8), gl = grid_for(k.work.prefix[CALL_LINE][1], c->sms, 8);
   const CUtensorMap* maps = c->maps_for ? c->d_maps.as<CUtensorMap>() : nullptr;
   int* err = c->d_err.as<int>();
-  if (!skip_r2c) PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, PH_X), gx, st, maps, err), "x r2c");
-  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, PH_LINE), gl, st, maps, err), "y fwd");
+  if (!skip_r2c) PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, CALL_X), gx, st, maps, err), "x r2c");
+  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "y fwd");
   if (gradient) return gradient_solve(c, k, st);
-  PM_CK(spectral_dispatch(table ? SPEC_Z_TABLE : SPEC_Z_GREEN, n, ds, work(c, k, PH_LINE), gl, st, maps, err),
+  PM_CK(spectral_dispatch(table ? SPEC_Z_TABLE : SPEC_Z_GREEN, n, ds, work(c, k, CALL_LINE), gl, st, maps, err),
         "z green");
-  PM_CK(spectral_dispatch(SPEC_Y_INV, n, ds, work(c, k, PH_LINE), gl, st, maps, err), "y inv");
-  PM_CK(spectral_dispatch(SPEC_X_C2R, n, ds, work(c, k, PH_X), gx, st, maps, err), "x c2r");
+  PM_CK(spectral_dispatch(SPEC_Y_INV, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "y inv");
+  PM_CK(spectral_dispatch(SPEC_X_C2R, n, ds, work(c, k, CALL_X), gx, st, maps, err), "x c2r");
   return PM_OK;
 }
 
@@ -273,9 +269,16 @@ double f_step(pm_ctx* c, double a, double da) {
   return cosmo_f(a + da, slot, c->cfg.omega_lambda0, c->cfg.omega_k0);
 }
 
-int kick(pm_ctx* c, Call& k, unsigned* perm, cudaStream_t st) {
-  PM_CK(launch_kick(c->d_sim.as<Sim>(), work(c, k, PH_KICK), k.parts, k.parts, perm, nullptr, POS_ABS,
-                    c->d_err.as<int>(), grid_for(k.prefix[PH_KICK][1], c->sms, 16), st),
+// The force of c->rec's particles and the kick and drift of the caller's state.
+int force(pm_ctx* c, const Call& k, cudaStream_t st) {
+  PM_CK(launch_force(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(), c->sms, st), "force");
+  return PM_OK;
+}
+
+int advance(pm_ctx* c, const Call& k, const float* pos, const float* vel, float* pos_out, float* vel_out,
+            cudaStream_t st) {
+  PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(), c->sort.keys.as<unsigned>(), pos, vel, pos_out,
+                       vel_out, c->d_err.as<int>(), st),
         "kick");
   return PM_OK;
 }
@@ -301,7 +304,7 @@ int pm_ctx_create(const pm_config* cfg, int device, pm_ctx** out) {
   if (!e) c->sms = sm_count(device);
   if (!e) e = c->tab.build(c->n);
   if (!e) e = c->d_sim.ensure(sizeof(Sim));
-  if (!e) e = c->d_prefix.ensure(sizeof(int) * 2 * PH_COUNT);
+  if (!e) e = c->d_work.ensure(sizeof(CallWork));
   if (!e) e = c->d_err.ensure(sizeof(int));
   if (!e) e = c->tile_next.ensure(sizeof(unsigned));
   if (!e) e = cudaMemset(c->d_err.p, 0, sizeof(int));
@@ -319,7 +322,7 @@ void pm_ctx_destroy(pm_ctx* c) {
   c->tab.release();
   c->sort.release();
   c->d_sim.release();
-  c->d_prefix.release();
+  c->d_work.release();
   c->d_err.release();
   c->tile_next.release();
   c->d_maps.release();
@@ -332,12 +335,10 @@ void pm_ctx_destroy(pm_ctx* c) {
   c->pk_partial.release();
   c->pk_out.release();
   c->row_count.release();
-  c->spos.release();
-  c->svel.release();
+  c->rec.release();
   if (c->side) cudaStreamDestroy(c->side);
   if (c->ev_start) cudaEventDestroy(c->ev_start);
   if (c->ev_vel) cudaEventDestroy(c->ev_vel);
-  c->row_cursor.release();
   c->scan_sums.release();
   for (int i = 0; i < 2; ++i) { c->gspec[i].release(); c->ggrid[i].release(); }
   c->d_sim3.release();
@@ -369,16 +370,9 @@ int pm_density(pm_ctx* c, const float* positions, long long np, double mass, flo
   k.sim.xbits = 0;  // row keys
   k.sim.rho = rho;
   k.sim.mass_scale = (float)(mass / (double)(1u << PM_FIX_BITS));
-  set_prefix(k, np, c->n);
-  k.parts = abs_parts(const_cast<float*>(positions), nullptr, np);
-  if (int r = upload(c, k, st)) return r;
-  unsigned* perm = nullptr;
-  if (int r = group_particles(c, k, st, &perm)) return r;
-  // deposit from a row-ordered copy of the positions (sequential reads of each row)
-  PM_CK(c->spos.ensure((size_t)3 * np * sizeof(float)), "alloc state");
-  PM_CK(launch_gather_state(positions, nullptr, np, perm, c->spos.as<float>(), nullptr, c->sms, st), "gather");
-  k.parts = abs_parts(c->spos.as<float>(), nullptr, np);
-  return deposit(c, k, nullptr, st);
+  set_work(k, np, c->n);
+  if (int r = place_particles(c, k, positions, nullptr, st)) return r;
+  return deposit(c, k, st);
 }
 
 int pm_fourier_grid(pm_ctx* c, float* fgrid, void* stream) {
@@ -388,7 +382,7 @@ int pm_fourier_grid(pm_ctx* c, float* fgrid, void* stream) {
   Call k;
   k.sim = base_sim(c, 1);
   k.sim.rho = fgrid;
-  if (int r = upload(c, k, st)) return r;
+  if (int r = begin(c, k, st)) return r;
   PM_CK(launch_fourier_grid(c->d_sim.as<Sim>(), c->sms * 8, st), "fourier grid");
   return PM_OK;
 }
@@ -404,9 +398,9 @@ int pm_potential(pm_ctx* c, const float* rho, const float* fgrid, double a, floa
   k.sim.phi = phi;
   k.sim.fgrid = fgrid;
   set_green(c, k.sim, a);
-  set_prefix(k, 1, c->n);
+  set_work(k, 1, c->n);
   if (int r = prepare_spectral(c, k)) return r;
-  if (int r = upload(c, k, st)) return r;
+  if (int r = begin(c, k, st)) return r;
   return spectral(c, k, fgrid != nullptr, st);
 }
 
@@ -418,15 +412,13 @@ int pm_integrate(pm_ctx* c, float* positions, float* velocities, long long np, d
   cudaStream_t st = (cudaStream_t)stream;
   Call k;
   k.sim = base_sim(c, np);
-  k.sim.xbits = 0;  // row keys: the kick reads the particles grouped by row (locality)
+  k.sim.xbits = 0;  // row keys: the force is read with the particles grouped by row (locality)
   k.sim.phi = const_cast<float*>(phi);
   set_kick(k.sim, a, f_a1, da);
-  set_prefix(k, np, c->n);
-  k.parts = abs_parts(positions, velocities, np);
-  if (int r = upload(c, k, st)) return r;
-  unsigned* perm = nullptr;
-  if (int r = group_particles(c, k, st, &perm)) return r;
-  return kick(c, k, perm, st);
+  set_work(k, np, c->n);
+  if (int r = place_particles(c, k, positions, nullptr, st)) return r;
+  if (int r = force(c, k, st)) return r;
+  return advance(c, k, positions, velocities, positions, velocities, st);
 }
 
 int pm_advance_time(pm_ctx* c, const float* rho, float* positions, float* velocities, long long np,
@@ -447,23 +439,23 @@ namespace {
 
 // Where a step reads and writes the caller's state.
 struct StepIO {
-  const float* pos_in;    // read once by the keys kernel (device-accessible: device or pinned host)
-  float* pos_copy;        // device copy the keys kernel leaves (null: pos_in is device memory)
+  const float* pos_in;    // device memory, or pinned host memory with a pos_copy
+  float* pos_copy;        // device copy left by the kernel that reads pos_in first (null: pos_in is device memory)
   const float* vel_in;    // device
   cudaEvent_t vel_ready;  // vel_in complete (null: already)
   float* pos_out;         // result in particle order (device or pinned host)
   float* vel_out;
-  // pinned host velocities: copied to vel_in on `side` once the keys kernel has read the
-  // positions (the two transfers would share the link)
+  // pinned host velocities: copied to vel_in on `side` once the positions have been read (the
+  // two transfers would share the link)
   const float* vel_host = nullptr;
   cudaStream_t side = nullptr;
-  cudaEvent_t keys_done = nullptr;
+  cudaEvent_t pos_read = nullptr;
 };
 
-// src/pmesh.py:60-61 on absolute positions: keys -> counting sort by row -> row-ordered copy
-// of the state (the caller's arrays are in particle order, which scatters every row across
-// memory) -> deposit (fused with the x R2C when the density is not requested) -> Poisson
-// solve -> kick/drift in row order -> gathered back into particle order.
+// src/pmesh.py:60-61 on absolute positions: cell records in row order (the caller's arrays are
+// in particle order, which scatters every row across memory) -> deposit (fused with the x R2C
+// when the density is not requested) -> Poisson solve -> force in row order -> kick and drift
+// in particle order.
 int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, double da, float* rho_out,
               cudaStream_t st) {
   const bool gradient = (c->cfg.flags & PM_FLAG_SPECTRAL_GRADIENT) != 0;
@@ -482,48 +474,33 @@ int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, 
   k.sim.mass_scale = (float)(mass / (double)(1u << PM_FIX_BITS));
   set_green(c, k.sim, a);
   set_kick(k.sim, a, f_step(c, a, da), da);
-  set_prefix(k, np, c->n);
-  k.parts = abs_parts(const_cast<float*>(io.pos_in), nullptr, np);
+  set_work(k, np, c->n);
   if (int r = prepare_spectral(c, k)) return r;
-  if (int r = upload(c, k, st)) return r;
-  const size_t pb = (size_t)3 * np * sizeof(float);
-  PM_CK(c->spos.ensure(pb), "alloc state");
-  PM_CK(c->svel.ensure(pb), "alloc state");
-  PM_CK(c->sort.ensure(np), "alloc sort");
-  unsigned* perm = nullptr;
-  unsigned* inv = c->sort.vals_alt.as<unsigned>();
-  if (int r = group_particles(c, k, st, &perm, inv, io.pos_copy)) return r;
+  if (int r = place_particles(c, k, io.pos_in, io.pos_copy, st)) return r;
   if (io.vel_host) {
-    PM_CK(cudaEventRecord(io.keys_done, st), "event");
-    PM_CK(cudaStreamWaitEvent(io.side, io.keys_done, 0), "event");
-    PM_CK(cudaMemcpyAsync(const_cast<float*>(io.vel_in), io.vel_host, pb, cudaMemcpyHostToDevice, io.side),
+    PM_CK(cudaEventRecord(io.pos_read, st), "event");
+    PM_CK(cudaStreamWaitEvent(io.side, io.pos_read, 0), "event");
+    PM_CK(cudaMemcpyAsync(const_cast<float*>(io.vel_in), io.vel_host, (size_t)3 * np * sizeof(float),
+                          cudaMemcpyHostToDevice, io.side),
           "h2d velocities");
     PM_CK(cudaEventRecord(io.vel_ready, io.side), "event");
   }
-  PM_CK(launch_gather_state(io.pos_copy ? io.pos_copy : io.pos_in, nullptr, np, perm, c->spos.as<float>(), nullptr,
-                            c->sms, st),
-        "gather");
-  Parts sp = abs_parts(c->spos.as<float>(), c->svel.as<float>(), np);
-  k.parts = sp;
   if (!rho_out && deposit_r2c_supported(c->n)) {
     // the density is not requested: deposit straight into the x-transformed spectrum
-    PM_CK(deposit_r2c_dispatch(c->n, c->d_sim.as<Sim>(), work(c, k, PH_DEP), sp, nullptr,
-                               c->row_start.as<unsigned>(), POS_ABS, c->d_err.as<int>(), c->tile_next.as<unsigned>(),
-                               nullptr, grid_for(k.prefix[PH_DEP][1], c->sms, deposit_r2c_ctas_per_sm(c->n)), st),
+    PM_CK(deposit_r2c_dispatch(c->n, c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
+                               c->row_start.as<unsigned>(), c->d_err.as<int>(), c->tile_next.as<unsigned>(), nullptr,
+                               grid_for(k.work.prefix[CALL_DEP][1], c->sms, deposit_r2c_ctas_per_sm(c->n)), st),
           "fused deposit");
     if (int r = spectral(c, k, false, st, true, gradient)) return r;
   } else {
-    if (int r = deposit(c, k, nullptr, st)) return r;
+    if (int r = deposit(c, k, st)) return r;
     if (int r = spectral(c, k, false, st, false, gradient)) return r;
   }
-  if (gradient)  // the kick's descriptor now names the three force grids
-    PM_CK(cudaMemcpyAsync(c->d_sim.p, &k.sim, sizeof(Sim), cudaMemcpyHostToDevice, st), "upload sim");
+  if (gradient)  // the force's descriptor now names the three force grids
+    if (int r = begin(c, k, st)) return r;
+  if (int r = force(c, k, st)) return r;
   if (io.vel_ready) PM_CK(cudaStreamWaitEvent(st, io.vel_ready, 0), "wait velocities");
-  PM_CK(launch_gather_state(io.vel_in, nullptr, np, perm, c->svel.as<float>(), nullptr, c->sms, st), "gather");
-  if (int r = kick(c, k, nullptr, st)) return r;
-  PM_CK(launch_gather_state(c->spos.as<float>(), c->svel.as<float>(), np, inv, io.pos_out, io.vel_out, c->sms, st),
-        "gather back");
-  return PM_OK;
+  return advance(c, k, io.pos_copy ? io.pos_copy : io.pos_in, io.vel_in, io.pos_out, io.vel_out, st);
 }
 
 bool pinned_host(const void* p) {
@@ -560,10 +537,10 @@ int pm_step_host(pm_ctx* c, float* h_positions, float* h_velocities, long long n
   PM_CK(c->hpos.ensure(pb), "alloc positions");
   PM_CK(c->hvel.ensure(pb), "alloc velocities");
   if (pinned_host(h_positions) && pinned_host(h_velocities)) {
-    // Pinned arrays: the keys kernel reads the positions over the host link and leaves a
-    // device copy; the velocities then cross on a copy engine while the deposit and the
-    // solve run (the kick needs them first); the result is gathered back straight into the
-    // host arrays.
+    // Pinned arrays: the first kernel reads the positions over the host link and leaves a
+    // device copy; the velocities then cross on a copy engine while the deposit, the solve
+    // and the force run (the kick needs them first), and the kick writes the result straight
+    // into the host arrays.
     if (!c->side) {
       PM_CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking), "side stream");
       PM_CK(cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming), "event");
@@ -572,7 +549,7 @@ int pm_step_host(pm_ctx* c, float* h_positions, float* h_velocities, long long n
     StepIO io{h_positions, c->hpos.as<float>(), c->hvel.as<float>(), c->ev_vel, h_positions, h_velocities};
     io.vel_host = h_velocities;
     io.side = c->side;
-    io.keys_done = c->ev_start;
+    io.pos_read = c->ev_start;
     if (int r = step_core(c, io, np, mass, a, da, nullptr, st)) return r;
   } else {  // pageable: copy engines both ways
     PM_CK(cudaMemcpyAsync(c->hpos.p, h_positions, pb, cudaMemcpyHostToDevice, st), "h2d positions");
@@ -594,17 +571,15 @@ int pm_sort_keys(pm_ctx* c, const float* positions, long long np, unsigned* keys
   cudaStream_t st = (cudaStream_t)stream;
   Call k;
   k.sim = base_sim(c, np);
-  set_prefix(k, np, c->n);
-  k.parts = abs_parts(const_cast<float*>(positions), nullptr, np);
-  if (int r = upload(c, k, st)) return r;
-  PM_CK(c->sort.ensure(np), "alloc sort");
+  set_work(k, np, c->n);
+  if (int r = begin(c, k, st)) return r;
   if (keys_out) {
-    PM_CK(launch_keys_abs(c->d_sim.as<Sim>(), work(c, k, PH_KEYS), k.parts, keys_out, nullptr,
-                          c->d_err.as<int>(), grid_for(k.prefix[PH_KEYS][1], c->sms, 16), st),
+    PM_CK(launch_keys_abs(c->d_sim.as<Sim>(), work(c, k, CALL_KEYS), abs_parts(positions, np), keys_out, nullptr,
+                          c->d_err.as<int>(), grid_for(k.work.prefix[CALL_KEYS][1], c->sms, 16), st),
           "keys");
   }
   unsigned *perm = nullptr, *skeys = nullptr;
-  if (int r = sort_particles(c, k, st, &perm, &skeys)) return r;
+  if (int r = sort_particles(c, k, positions, st, &perm, &skeys)) return r;
   const size_t b = (size_t)np * sizeof(unsigned);
   if (sorted_keys) PM_CK(cudaMemcpyAsync(sorted_keys, skeys, b, cudaMemcpyDeviceToDevice, st), "copy keys");
   if (perm_out) PM_CK(cudaMemcpyAsync(perm_out, perm, b, cudaMemcpyDeviceToDevice, st), "copy perm");
@@ -633,16 +608,16 @@ int pm_power_spectrum(pm_ctx* c, const float* rho, double box_size, int nbins, d
   Call k;
   k.sim = base_sim(c, 1);
   k.sim.rho = const_cast<float*>(rho);
-  set_prefix(k, 1, n);
+  set_work(k, 1, n);
   if (int r = prepare_spectral(c, k)) return r;
-  if (int r = upload(c, k, st)) return r;
+  if (int r = begin(c, k, st)) return r;
   const Sim* ds = c->d_sim.as<Sim>();
-  const int gx = grid_for(k.prefix[PH_X][1], c->sms, 8), gl = grid_for(k.prefix[PH_LINE][1], c->sms, 8);
+  const int gx = grid_for(k.work.prefix[CALL_X][1], c->sms, 8), gl = grid_for(k.work.prefix[CALL_LINE][1], c->sms, 8);
   const CUtensorMap* maps = c->maps_for ? c->d_maps.as<CUtensorMap>() : nullptr;
   int* err = c->d_err.as<int>();
-  PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, PH_X), gx, st, maps, err), "x r2c");
-  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, PH_LINE), gl, st, maps, err), "y fwd");
-  PM_CK(spectral_dispatch(SPEC_Z_FWD, n, ds, work(c, k, PH_LINE), gl, st, maps, err), "z fwd");
+  PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, CALL_X), gx, st, maps, err), "x r2c");
+  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "y fwd");
+  PM_CK(spectral_dispatch(SPEC_Z_FWD, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "z fwd");
   const int nb = nbins - 1;
   PM_CK(c->pk_partial.ensure(pk_partial_doubles(nbins) * sizeof(double)), "alloc pk");
   PM_CK(c->pk_out.ensure((size_t)3 * nb * sizeof(double)), "alloc pk");

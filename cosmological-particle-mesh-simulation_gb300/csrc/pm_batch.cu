@@ -475,7 +475,7 @@ int build_plan(pm_batch* b, cudaStream_t st) {
   for (size_t g = 0; g < P.sizes.size(); ++g) {
     PB_CK(spectral_dispatch(SPEC_PREPARE, P.sizes[g], nullptr, Work(), 0, st), "prepare");
     if (P.fused[g])
-      PB_CK(deposit_r2c_dispatch(P.sizes[g], nullptr, Work(), Parts(), nullptr, nullptr, POS_DISP, nullptr, nullptr,
+      PB_CK(deposit_r2c_dispatch(P.sizes[g], nullptr, Work(), Parts(), nullptr, nullptr, nullptr, nullptr,
                                  nullptr, 0, st),
             "prepare fused deposit");
   }
@@ -533,7 +533,7 @@ int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigne
   }
   if (sh.dep == DEP_FUSED_DENSE_FIRST)
     PB_CK(launch_tile_order(ds, wg, b->row_start.as<unsigned>(), order, next + 2, b->sms, st), "tile order");
-  PB_CK(deposit_r2c_dispatch(n, ds, wg, in, perm, b->row_start.as<unsigned>(), POS_DISP, err, next,
+  PB_CK(deposit_r2c_dispatch(n, ds, wg, in, perm, b->row_start.as<unsigned>(), err, next,
                              sh.dep == DEP_FUSED_DENSE_FIRST ? order : nullptr,
                              grid_for(tot, b->sms, sh.dep_cps ? sh.dep_cps : deposit_r2c_ctas_per_sm(n)), st),
         "fused deposit");
@@ -554,7 +554,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   // (the row histogram of the keys was made by the previous kick, or by ensure_keys)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, nullptr, true),
+                          perm, err, b->sms, st, true),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
@@ -604,7 +604,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   // the kick writes the next keys and counts them per row for the next step's sort
   PB_CK(cudaMemsetAsync(b->row_count.p, 0, sizeof(unsigned) * (size_t)P.rows, st), "count reset");
   PB_CK(launch_kick(ds, work_of(b, PH_KICK, P.fixed_total[PH_KICK]), in, out, perm, b->sort.keys.as<unsigned>(),
-                    POS_DISP, err, grid_for(P.fixed_total[PH_KICK], b->sms, P.kick_cps), st,
+                    err, grid_for(P.fixed_total[PH_KICK], b->sms, P.kick_cps), st,
                     b->row_count.as<unsigned>()),
         "kick");
   PB_CK(mark(1 + PP_KICK), "event");
@@ -668,7 +668,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
   // the row starts and permutation of the current keys (the step recomputes the same)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, nullptr, true),
+                          perm, err, b->sms, st, true),
         "sort");
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   PB_CK(cudaEventCreate(&e0), "event");
@@ -747,7 +747,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
     for (int cps : {4, 8, 16, 32}) {
       float ms = 0.f;
       rc = time3([&]() -> int {
-        PB_CK(launch_kick(ds, wk, in, out, perm, b->sort.vals_alt.as<unsigned>(), POS_DISP, err,
+        PB_CK(launch_kick(ds, wk, in, out, perm, b->sort.vals_alt.as<unsigned>(), err,
                           grid_for(wk.total, b->sms, cps), st, b->row_cursor.as<unsigned>()),
               "kick");
         return PM_OK;
@@ -1176,7 +1176,7 @@ int pm_batch_density(pm_batch* b, int sim_id, float* rho, void* stream) {
   PB_CK(cudaStreamWaitEvent(st, b->last_step, 0), "wait");
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, nullptr, true),
+                          perm, err, b->sms, st, true),
         "sort");
   // this simulation's descriptor with the caller's grid as the deposit's output
   Sim s{};

@@ -115,6 +115,12 @@ struct Work {
   int total;          // prefix[nsims]
 };
 
+// Work table of a drop-in call (one simulation): (0, units) of each phase.
+enum CallPhase : int { CALL_KEYS = 0, CALL_DEP, CALL_X, CALL_LINE, CALL_PHASES };
+struct CallWork {
+  int prefix[CALL_PHASES][2];
+};
+
 // Particle arrays of a batch (structure of arrays, indexed by slot).
 struct Parts {
   float* x; float* y; float* z;       // positions (POS_ABS) or displacements (POS_DISP)
@@ -172,13 +178,13 @@ cudaError_t launch_fourier_grid(const Sim* sims, int ctas, cudaStream_t st);
 // take them (launch_tile_order).
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
-                               int mode, int* err, unsigned* next_tile, const unsigned* order, int ctas,
+                               int* err, unsigned* next_tile, const unsigned* order, int ctas,
                                cudaStream_t st);
 bool deposit_r2c_supported(int n);
 bool xrow_supported(int n);  // the x passes of size n transform rows in registers (their grid is tunable)
 int deposit_r2c_ctas_per_sm(int n);  // resident CTAs per SM of the fused deposit
 cudaError_t deposit_r2c_dispatch(int n, const Sim* sims, Work w, Parts p, const unsigned* perm,
-                                 const unsigned* row_start, int mode, int* err, unsigned* next_tile,
+                                 const unsigned* row_start, int* err, unsigned* next_tile,
                                  const unsigned* order, int ctas, cudaStream_t st);
 
 // sum of the first n_slices planes of an n^3 grid, float64 n^2 output (pm_diagnostics.cu)
@@ -192,7 +198,7 @@ cudaError_t launch_power_spectrum(const float2* spec, int n, int pitch, int nbin
 
 // particle kernels
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                            int* err, int ctas, cudaStream_t st, Parts copy = Parts{});
+                            int* err, int ctas, cudaStream_t st);
 cudaError_t launch_keys_disp(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
                              int* err, int ctas, cudaStream_t st);
 cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsigned nrows,
@@ -201,15 +207,24 @@ cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsign
                            const unsigned* row_start, int mode, int* err, int ctas, size_t smem,
                            cudaStream_t st);
 constexpr int KICK_UNIT = 512;  // particles per work unit of the kick
-// row_count (displacement mode, with keys_next): the kick also counts the next keys per row
+// resident kick: the state in row order (through perm), the next keys and their row histogram
 cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, const unsigned* perm,
-                        unsigned* keys_next, int mode, int* err, int ctas, cudaStream_t st,
-                        unsigned* row_count = nullptr);
+                        unsigned* keys_next, int* err, int ctas, cudaStream_t st, unsigned* row_count);
+// ---- drop-in step on (3, np) arrays in the caller's order (see pm_particles.cu) ----
+// descriptor and work table of one call (from kernel arguments); zero_bytes: a multiple of 16
+cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
+                              size_t zero_bytes, cudaStream_t st);
+// row key and rank inside its row of every particle; count (zero before) ends as the row counts
+cudaError_t launch_row_rank(const float* pos, long long np, int n, unsigned* count, unsigned* keys, unsigned* ranks,
+                            int* err, float* copy, cudaStream_t st);
+// cell records in row order; place: in the keys, out each particle's place in row order
+cudaError_t launch_row_place(const float* pos, long long np, int n, const unsigned* row_start, const unsigned* ranks,
+                             unsigned* place, uint4* rec, cudaStream_t st);
+// rec: in the cell records, out the forces (3 floats in the first words of each entry)
+cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cudaStream_t st);
+cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place, const float* pos,
+                           const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st);
 cudaError_t launch_coef(Sim* sims, int nsims, int advance, cudaStream_t st);
-// dst[k][j] = src[k][idx[j]] for the three rows of (3, np) positions (and velocities unless
-// vel is null)
-cudaError_t launch_gather_state(const float* pos, const float* vel, long long np, const unsigned* idx, float* spos,
-                                float* svel, int sms, cudaStream_t st);
 cudaError_t deposit_prepare();  // sets kernel attributes of the current device (call before graph capture)
 // order of the fused deposit's tiles (dense tiles first); counts: 2 device words of scratch
 cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* row_start, unsigned* order,
@@ -245,11 +260,13 @@ cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bi
 // counts) and perm[j] = index of the j-th key in row order (order inside a row not
 // specified).  Scratch: count and cursor (nrows each), block_sums (row_sort_block_sums).
 size_t row_sort_block_sums(unsigned nrows);
-// inv (optional): inv[i] = sorted position of key i.  counted: count already holds the
-// row histogram of keys (else it is zeroed and computed here).
+// counted: count already holds the row histogram of keys (else it is zeroed and computed here).
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, unsigned* inv = nullptr, bool counted = false);
+                              int sms, cudaStream_t st, bool counted = false);
+// row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows entries
+cudaError_t row_scan(const unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
+                     cudaStream_t st);
 // count[r] = number of keys equal to r (count zeroed first)
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
                           cudaStream_t st);

@@ -23,12 +23,10 @@ constexpr int KEY_NT = 256;
 // ---------------------------------------------------------------------------------
 // keys
 // ---------------------------------------------------------------------------------
-// copy (POS_ABS, optional): the positions are also written there (the keys kernel reads
-// them once, e.g. from host memory, and leaves a device copy)
 template <int MODE>
 __global__ void __launch_bounds__(KEY_NT) k_keys(const Sim* __restrict__ sims, Work w, Parts p,
                                                  unsigned* __restrict__ keys,
-                                                 unsigned* __restrict__ vals, int* err, Parts copy) {
+                                                 unsigned* __restrict__ vals, int* err) {
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
     const int si = locate_sim(w, unit);
     const Sim& S = sims[si];
@@ -38,13 +36,7 @@ __global__ void __launch_bounds__(KEY_NT) k_keys(const Sim* __restrict__ sims, W
     // from the state itself (the cell records, if any, are written here)
     Cell c;
     if (MODE == POS_ABS) {
-      const float x = p.x[slot], y = p.y[slot], z = p.z[slot];
-      if (copy.x) {
-        copy.x[slot] = x;
-        copy.y[slot] = y;
-        copy.z[slot] = z;
-      }
-      c = cell_abs(x, y, z, S.n);
+      c = cell_abs(p.x[slot], p.y[slot], p.z[slot], S.n);
     } else {
       c = cell_disp(S, p.id[slot], p.x[slot], p.y[slot], p.z[slot]);
       if (p.rec) store_cell_record(p, slot, c);
@@ -114,10 +106,9 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
 // x_a += drift * v_a (integrate.py:94-95).  All three axes use the cell and weights
 // of the position before the step, as the reference's three sweeps do.
 //
-// POS_ABS: absolute positions, updated in place at their slot (drop-in layout),
-//          wrapped into [0, n).
-// POS_DISP: displacements; the particle that is i-th in sorted order is written to
+// Resident (k_kick): displacements; the particle that is i-th in sorted order is written to
 //          output slot sort_off + i, together with its cell key for the next step.
+// Drop-in: k_force in row order, k_advance in the caller's order (below).
 // ---------------------------------------------------------------------------------
 // Potential rows around a particle, read from global memory: row(oy, oz) is the x-row at
 // (y + oy, z + oz) (periodic), oy, oz in {-1, 0, 1, 2}.  The taps are scalar loads: at one
@@ -210,48 +201,8 @@ __device__ __forceinline__ void gather_grad(const Sim& S, const Cell& c, float g
   }
 }
 
-// Kick/drift of one particle whose state and force are in registers; writes it out and
-// returns its next key (resident mode with keys_next; else 0xffffffff).
-template <int MODE>
-__device__ __forceinline__ unsigned kick_store(const Sim& S, const Parts& out, long long sp, long long slot, float px,
-                                           float py, float pz, float vx, float vy, float vz, unsigned id,
-                                           const float (&g)[3], unsigned* __restrict__ keys_next, int* err) {
-  const float kk = S.kick, dr = S.drift;
-  vx = fmaf(kk, g[0], vx);
-  vy = fmaf(kk, g[1], vy);
-  vz = fmaf(kk, g[2], vz);
-  if (MODE == POS_ABS) {
-    // positions may arrive as exactly n: drift the canonical value and wrap
-    const float fn = (float)S.n;
-    const float nx = canon(fmaf(dr, vx, canon(px, fn)), fn);
-    const float ny = canon(fmaf(dr, vy, canon(py, fn)), fn);
-    const float nz = canon(fmaf(dr, vz, canon(pz, fn)), fn);
-    if (!(isfinite(nx) && isfinite(ny) && isfinite(nz) && isfinite(vx) && isfinite(vy) && isfinite(vz)))
-      set_error(err, ERR_NONFINITE);
-    out.x[slot] = nx; out.y[slot] = ny; out.z[slot] = nz;
-    out.vx[slot] = vx; out.vy[slot] = vy; out.vz[slot] = vz;
-  } else {
-    const float nx = fmaf(dr, vx, px), ny = fmaf(dr, vy, py), nz = fmaf(dr, vz, pz);
-    if (!(isfinite(nx) && isfinite(ny) && isfinite(nz) && isfinite(vx) && isfinite(vy) && isfinite(vz)))
-      set_error(err, ERR_NONFINITE);
-    out.x[sp] = nx; out.y[sp] = ny; out.z[sp] = nz;
-    out.vx[sp] = vx; out.vy[sp] = vy; out.vz[sp] = vz;
-    out.id[sp] = id;
-    if (keys_next) {
-      Cell cn = cell_disp(S, id, nx, ny, nz);
-      if (out.rec) store_cell_record(out, sp, cn);
-      if (!cn.ok) { set_error(err, ERR_CELL_RANGE); cn.x = cn.y = cn.z = 0; }
-      const unsigned key = cell_key(S, cn);
-      keys_next[sp] = key;
-      return key;
-    }
-  }
-  return 0xffffffffu;
-}
-
 // Each thread advances KICK_PPT particles, KICK_NT apart: all their loads (state, then the
 // 32 potential taps each) are issued before any store, so that they overlap.
-template <int MODE>
 // row_count (optional, with keys_next): histogram of the next keys, for the next step's
 // counting sort
 __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sims, Work w, Parts in, Parts out,
@@ -269,27 +220,23 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sim
 #pragma unroll
     for (int q = 0; q < KICK_PPT; ++q) {
       const long long i = i0 + q * KICK_NT;
-      sp[q] = S.part_off + i;  // position in sorted order (or slot without perm)
-      slot[q] = i < S.np ? (perm ? (long long)__ldg(&perm[sp[q]]) : sp[q]) : -1;
+      sp[q] = S.part_off + i;  // position in sorted order
+      slot[q] = i < S.np ? (long long)__ldg(&perm[sp[q]]) : -1;
     }
 #pragma unroll
     for (int q = 0; q < KICK_PPT; ++q) {
       const long long sl = slot[q] >= 0 ? slot[q] : 0;
       px[q] = in.x[sl]; py[q] = in.y[sl]; pz[q] = in.z[sl];
       vx[q] = in.vx[sl]; vy[q] = in.vy[sl]; vz[q] = in.vz[sl];
-      id[q] = MODE == POS_DISP ? in.id[sl] : 0u;
+      id[q] = in.id[sl];
     }
 #pragma unroll
-    for (int q = 0; q < KICK_PPT; ++q)
-      c[q] = MODE == POS_ABS ? cell_abs(px[q], py[q], pz[q], S.n) : cell_disp(S, id[q], px[q], py[q], pz[q]);
+    for (int q = 0; q < KICK_PPT; ++q) c[q] = cell_disp(S, id[q], px[q], py[q], pz[q]);
     float g[KICK_PPT][3];
 #pragma unroll
     for (int q = 0; q < KICK_PPT; ++q) {
       g[q][0] = g[q][1] = g[q][2] = 0.f;
-      if (slot[q] >= 0 && c[q].ok) {
-        if (S.grad[0]) gather_grad(S, c[q], g[q]);  // spectral gradient: three force grids
-        else gather_force(S.phi, S.n, c[q], g[q]);
-      }
+      if (slot[q] >= 0 && c[q].ok) gather_force(S.phi, S.n, c[q], g[q]);
     }
     unsigned key[KICK_PPT];
 #pragma unroll
@@ -297,10 +244,21 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sim
       key[q] = 0xffffffffu;
       if (slot[q] < 0) continue;
       if (!c[q].ok) set_error(err, ERR_CELL_RANGE);
-      key[q] = kick_store<MODE>(S, out, sp[q], slot[q], px[q], py[q], pz[q], vx[q], vy[q], vz[q], id[q], g[q],
-                                keys_next, err);
+      const float nvx = fmaf(S.kick, g[q][0], vx[q]), nvy = fmaf(S.kick, g[q][1], vy[q]),
+                  nvz = fmaf(S.kick, g[q][2], vz[q]);
+      const float nx = fmaf(S.drift, nvx, px[q]), ny = fmaf(S.drift, nvy, py[q]), nz = fmaf(S.drift, nvz, pz[q]);
+      if (!(isfinite(nx) && isfinite(ny) && isfinite(nz) && isfinite(nvx) && isfinite(nvy) && isfinite(nvz)))
+        set_error(err, ERR_NONFINITE);
+      out.x[sp[q]] = nx; out.y[sp[q]] = ny; out.z[sp[q]] = nz;
+      out.vx[sp[q]] = nvx; out.vy[sp[q]] = nvy; out.vz[sp[q]] = nvz;
+      out.id[sp[q]] = id[q];
+      Cell cn = cell_disp(S, id[q], nx, ny, nz);
+      store_cell_record(out, sp[q], cn);
+      if (!cn.ok) { set_error(err, ERR_CELL_RANGE); cn.x = cn.y = cn.z = 0; }
+      key[q] = cell_key(S, cn);
+      keys_next[sp[q]] = key[q];
     }
-    if (row_count) {  // the whole warp takes part: equal keys are counted once per warp
+    {  // the whole warp takes part: equal keys are counted once per warp
       const int lane = threadIdx.x & 31;
 #pragma unroll
       for (int q = 0; q < KICK_PPT; ++q) {
@@ -309,6 +267,174 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sim
       }
     }
   }
+}
+
+// ---------------------------------------------------------------------------------
+// drop-in step on absolute positions in the caller's order
+//
+// The caller's arrays are in particle order (the slowest particle index is x, the fastest grid
+// axis), which scatters every grid row over memory.  Each particle crosses between the two
+// orders twice, as one 16-byte word each time:
+//   k_row_rank  (particle order) row key, and the particle's rank in its row from the returning
+//               atomic that counts the row -- no second atomic pass is needed to place it;
+//   (scan of the counts: row starts)
+//   k_row_place (particle order) writes the particle's cell record to its place in row order
+//               and keeps the place;
+//   deposit and k_force work on the records in row order (k_force leaves the force in the
+//               record's own word);
+//   k_advance   (particle order) reads the force back and kicks and drifts the caller's state,
+//               which is read and written in its own order only.
+// Both crossings are bound by the rate of 32-byte sectors in L2 (the lines being filled or
+// read are the rows' current ends, a few MB).  Measured on 256^3 particles, 512^3 cells: see
+// the launchers.
+// ---------------------------------------------------------------------------------
+constexpr int ORD_NT = 256;
+constexpr int ORD_PPT = 4;  // particles per thread, ORD_NT apart: their loads and atomics overlap
+
+// copy (optional): the positions are also written there (they are read once, e.g. from host
+// memory, and leave a device copy)
+__global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ pos, long long np, int n,
+                                                     unsigned* __restrict__ count, unsigned* __restrict__ keys,
+                                                     unsigned* __restrict__ ranks, int* err,
+                                                     float* __restrict__ copy) {
+  const int lane = threadIdx.x & 31;
+  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
+  float x[ORD_PPT], y[ORD_PPT], z[ORD_PPT];
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    x[q] = y[q] = z[q] = 0.f;
+    if (i < np) { x[q] = pos[i]; y[q] = pos[np + i]; z[q] = pos[2 * np + i]; }
+  }
+  unsigned key[ORD_PPT], grp[ORD_PPT], base[ORD_PPT];
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    key[q] = 0xffffffffu;
+    if (i < np) {
+      if (copy) { copy[i] = x[q]; copy[np + i] = y[q]; copy[2 * np + i] = z[q]; }
+      const Cell c = cell_abs(x[q], y[q], z[q], n);
+      if (!c.ok) set_error(err, ERR_CELL_RANGE);
+      key[q] = c.ok ? row_number(c.y, c.z, n) : 0u;
+    }
+    // equal keys of a warp share one atomic
+    grp[q] = __match_any_sync(FULL, key[q]);
+    base[q] = 0;
+    if (key[q] != 0xffffffffu && lane == __ffs(grp[q]) - 1) base[q] = atomicAdd(&count[key[q]], (unsigned)__popc(grp[q]));
+  }
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    const unsigned b = __shfl_sync(FULL, base[q], __ffs(grp[q]) - 1);
+    if (i < np) {
+      keys[i] = key[q];
+      ranks[i] = b + __popc(grp[q] & ((1u << lane) - 1u));
+    }
+  }
+}
+
+// place: in the row key of each particle, out its place in row order
+__global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ pos, long long np, int n,
+                                                      const unsigned* __restrict__ row_start,
+                                                      const unsigned* __restrict__ ranks, unsigned* __restrict__ place,
+                                                      uint4* __restrict__ rec) {
+  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
+  Parts out{};
+  out.rec = rec;
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    if (i >= np) continue;
+    const Cell c = cell_abs(pos[i], pos[np + i], pos[2 * np + i], n);
+    const unsigned slot = __ldg(&row_start[place[i]]) + ranks[i];
+    store_cell_record(out, slot, c);
+    place[i] = slot;
+  }
+}
+
+// The force (gx, gy, gz) at every record, in row order, over the record's own word.  Two
+// particles per thread, as k_kick.
+__global__ void __launch_bounds__(KICK_NT, 4) k_force(const Sim* __restrict__ sims, uint4* __restrict__ rec) {
+  const Sim& S = sims[0];
+  const long long units = (S.np + KICK_UNIT - 1) / KICK_UNIT;
+  for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    const long long i0 = unit * KICK_UNIT + threadIdx.x;
+    Cell c[KICK_PPT];
+    float g[KICK_PPT][3];
+#pragma unroll
+    for (int q = 0; q < KICK_PPT; ++q) {
+      const long long i = i0 + q * KICK_NT;
+      c[q] = record_cell(i < S.np ? rec[i] : make_uint4(CELL_BAD, 0u, 0u, 0u));
+    }
+#pragma unroll
+    for (int q = 0; q < KICK_PPT; ++q) {
+      g[q][0] = g[q][1] = g[q][2] = 0.f;
+      if (c[q].ok) {
+        if (S.grad[0]) gather_grad(S, c[q], g[q]);  // spectral gradient: three force grids
+        else gather_force(S.phi, S.n, c[q], g[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < KICK_PPT; ++q) {
+      const long long i = i0 + q * KICK_NT;
+      if (i < S.np)
+        rec[i] = make_uint4(__float_as_uint(g[q][0]), __float_as_uint(g[q][1]), __float_as_uint(g[q][2]), 0u);
+    }
+  }
+}
+
+// Kick and drift (integrate.py:94-95) of the caller's state with the forces in row order;
+// positions may arrive as exactly n: the canonical value drifts and is wrapped into [0, n).
+// pos_out / vel_out may be pos / vel, or host memory.
+__global__ void __launch_bounds__(ORD_NT) k_advance(const Sim* __restrict__ sims, const uint4* __restrict__ force,
+                                                    const unsigned* __restrict__ place, const float* pos,
+                                                    const float* vel, float* pos_out, float* vel_out, int* err) {
+  const Sim& S = sims[0];
+  const long long np = S.np;
+  const float kk = S.kick, dr = S.drift, fn = (float)S.n;
+  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
+  uint4 g[ORD_PPT];
+  float p[ORD_PPT][3], v[ORD_PPT][3];
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    if (i < np) g[q] = __ldg(&force[__ldg(&place[i])]);
+  }
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (i < np) { p[q][d] = pos[d * np + i]; v[q][d] = vel[d * np + i]; }
+  }
+#pragma unroll
+  for (int q = 0; q < ORD_PPT; ++q) {
+    const long long i = i0 + q * ORD_NT;
+    if (i >= np) continue;
+    const float f[3] = {__uint_as_float(g[q].x), __uint_as_float(g[q].y), __uint_as_float(g[q].z)};
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float nv = fmaf(kk, f[d], v[q][d]);
+      const float nx = canon(fmaf(dr, nv, canon(p[q][d], fn)), fn);
+      ok = ok && isfinite(nv) && isfinite(nx);
+      pos_out[d * np + i] = nx;
+      vel_out[d * np + i] = nv;
+    }
+    if (!ok) set_error(err, ERR_NONFINITE);
+  }
+}
+
+// Writes a call's descriptor and work table to device memory (they arrive as kernel arguments:
+// no staging of host memory, and the call can be captured) and zeroes `nzero` 16-byte words.
+__global__ void k_call_begin(Sim* __restrict__ dsim, CallWork* __restrict__ dwork, Sim sim, CallWork work,
+                             uint4* __restrict__ zero, long long nzero) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) {
+    *dsim = sim;
+    *dwork = work;
+  }
+  for (long long i = t; i < nzero; i += (long long)gridDim.x * blockDim.x) zero[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // ---------------------------------------------------------------------------------
@@ -437,13 +563,13 @@ cudaError_t deposit_prepare() {
 size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * sizeof(unsigned long long); }
 
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                            int* err, int ctas, cudaStream_t st, Parts copy) {
-  k_keys<POS_ABS><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err, copy);
+                            int* err, int ctas, cudaStream_t st) {
+  k_keys<POS_ABS><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err);
   return cudaGetLastError();
 }
 cudaError_t launch_keys_disp(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
                              int* err, int ctas, cudaStream_t st) {
-  k_keys<POS_DISP><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err, Parts{});
+  k_keys<POS_DISP><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err);
   return cudaGetLastError();
 }
 
@@ -499,29 +625,45 @@ cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsign
 }
 
 cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, const unsigned* perm,
-                        unsigned* keys_next, int mode, int* err, int ctas, cudaStream_t st, unsigned* row_count) {
-  if (mode == POS_ABS) k_kick<POS_ABS><<<ctas, KICK_NT, 0, st>>>(sims, w, in, out, perm, keys_next, err, nullptr);
-  else k_kick<POS_DISP><<<ctas, KICK_NT, 0, st>>>(sims, w, in, out, perm, keys_next, err, row_count);
+                        unsigned* keys_next, int* err, int ctas, cudaStream_t st, unsigned* row_count) {
+  k_kick<<<ctas, KICK_NT, 0, st>>>(sims, w, in, out, perm, keys_next, err, row_count);
   return cudaGetLastError();
 }
 
-// Absolute state in caller order <-> row order (drop-in step): sorted[j] = state[perm[j]],
-// and back, state[i] = sorted[inv[i]] -- gathers, so that the writes stay coalesced.  One
-// array per launch: the randomly read source (np floats) then stays in L2.
-__global__ void k_gather1(const float* __restrict__ src, long long np, const unsigned* __restrict__ idx,
-                          float* __restrict__ dst) {
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < np; j += (long long)gridDim.x * blockDim.x)
-    dst[j] = __ldg(&src[__ldg(&idx[j])]);
+namespace {
+int ord_ctas(long long np) { return (int)((np + ORD_NT * ORD_PPT - 1) / (ORD_NT * ORD_PPT)); }
+}  // namespace
+
+cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
+                              size_t zero_bytes, cudaStream_t st) {
+  const long long nz = (long long)(zero_bytes / sizeof(uint4));
+  const long long want = (nz + 1023) / 1024;  // four words per thread
+  k_call_begin<<<(int)(want < 1 ? 1 : (want > 1024 ? 1024 : want)), 256, 0, st>>>(dsim, dwork, sim, work,
+                                                                                 static_cast<uint4*>(zero), nz);
+  return cudaGetLastError();
 }
 
-cudaError_t launch_gather_state(const float* pos, const float* vel, long long np, const unsigned* idx, float* spos,
-                                float* svel, int sms, cudaStream_t st) {
-  long long b = (np + 255) / 256;
-  if (b > (long long)sms * 16) b = (long long)sms * 16;
-  for (int k = 0; k < 3; ++k) {
-    k_gather1<<<(int)b, 256, 0, st>>>(pos + k * np, np, idx, spos + k * np);
-    if (vel) k_gather1<<<(int)b, 256, 0, st>>>(vel + k * np, np, idx, svel + k * np);
-  }
+cudaError_t launch_row_rank(const float* pos, long long np, int n, unsigned* count, unsigned* keys, unsigned* ranks,
+                            int* err, float* copy, cudaStream_t st) {
+  k_row_rank<<<ord_ctas(np), ORD_NT, 0, st>>>(pos, np, n, count, keys, ranks, err, copy);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_row_place(const float* pos, long long np, int n, const unsigned* row_start, const unsigned* ranks,
+                             unsigned* place, uint4* rec, cudaStream_t st) {
+  k_row_place<<<ord_ctas(np), ORD_NT, 0, st>>>(pos, np, n, row_start, ranks, place, rec);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cudaStream_t st) {
+  const long long units = (np + KICK_UNIT - 1) / KICK_UNIT, cap = (long long)sms * 16;
+  k_force<<<(int)(units < cap ? units : cap), KICK_NT, 0, st>>>(sims, rec);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place, const float* pos,
+                           const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st) {
+  k_advance<<<ord_ctas(np), ORD_NT, 0, st>>>(sims, force, place, pos, vel, pos_out, vel_out, err);
   return cudaGetLastError();
 }
 

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(CS_NT) k_scan_top(unsigned* __restrict__ block
   }
 }
 
-// out[i] = exclusive prefix of in, i < n; out[n] = total; cursor = copy of out[0, n)
+// out[i] = exclusive prefix of in, i < n; out[n] = total; cursor (optional) = copy of out[0, n)
 __global__ void __launch_bounds__(CS_NT) k_scan_apply(const unsigned* __restrict__ in, long long n,
                                                       const unsigned* __restrict__ block_sums,
                                                       unsigned* __restrict__ out, unsigned* __restrict__ cursor) {
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(CS_NT) k_scan_apply(const unsigned* __restrict
     const long long i = base + j;
     if (i < n) {
       out[i] = run;
-      cursor[i] = run;
+      if (cursor) cursor[i] = run;
     }
     run += v[j];
     if (i == n - 1) out[n] = run;
@@ -360,8 +360,7 @@ __global__ void __launch_bounds__(CS_NT) k_scan_apply(const unsigned* __restrict
 constexpr int SCATTER_CHUNK = 1024;
 
 __global__ void __launch_bounds__(CS_NT) k_row_scatter(const unsigned* __restrict__ keys, long long n, unsigned nrows,
-                                                       unsigned* __restrict__ cursor, unsigned* __restrict__ perm,
-                                                       unsigned* __restrict__ inv) {
+                                                       unsigned* __restrict__ cursor, unsigned* __restrict__ perm) {
   const int lane = threadIdx.x & 31;
   const long long nchunks = (n + SCATTER_CHUNK - 1) / SCATTER_CHUNK;
   const long long nwarps = (long long)gridDim.x * (CS_NT / 32);
@@ -390,7 +389,6 @@ __global__ void __launch_bounds__(CS_NT) k_row_scatter(const unsigned* __restric
           const long long i = b + u * 32 + lane;
           const unsigned p = p0 + __popc(grp[u] & ((1u << lane) - 1u));
           perm[p] = (unsigned)i;
-          if (inv) inv[i] = p;
         }
       }
     }
@@ -412,22 +410,28 @@ cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, uns
   return cudaGetLastError();
 }
 
-cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
-                              unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, unsigned* inv, bool counted) {
+cudaError_t row_scan(const unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
+                     cudaStream_t st) {
   if (nrows == 0) return cudaErrorInvalidValue;
-  if (!counted) {
-    cudaError_t e = row_histogram(keys, n, nrows, count, err, sms, st);
-    if (e) return e;
-  }
   const int nb = (int)row_sort_block_sums(nrows);
   k_scan_reduce<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums);
   k_scan_top<<<1, CS_NT, 0, st>>>(block_sums, nb);
   k_scan_apply<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums, row_start, cursor);
+  return cudaGetLastError();
+}
+
+cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
+                              unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
+                              int sms, cudaStream_t st, bool counted) {
+  if (!counted) {
+    cudaError_t e = row_histogram(keys, n, nrows, count, err, sms, st);
+    if (e) return e;
+  }
+  if (cudaError_t e = row_scan(count, nrows, row_start, cursor, block_sums, st)) return e;
   const long long chunks = (n + SCATTER_CHUNK - 1) / SCATTER_CHUNK;
   const long long sblocks = (chunks + CS_NT / 32 - 1) / (CS_NT / 32);
   k_row_scatter<<<(int)(sblocks < (long long)sms * 8 ? (sblocks > 0 ? sblocks : 1) : (long long)sms * 8), CS_NT, 0,
-                  st>>>(keys, n, nrows, cursor, perm, inv);
+                  st>>>(keys, n, nrows, cursor, perm);
   return cudaGetLastError();
 }
 

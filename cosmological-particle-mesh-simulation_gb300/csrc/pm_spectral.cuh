@@ -783,7 +783,7 @@ __host__ __device__ constexpr int dep_tiles(int n) {
   return t;
 }
 
-template <int N, int MODE>
+template <int N>
 __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
     k_deposit_r2c(const Sim* __restrict__ sims, Work w, Parts p, const unsigned* __restrict__ perm,
                   const unsigned* __restrict__ row_start, int* err, unsigned* __restrict__ next_tile,
@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
       {  // the particles of this group's tile (a group without a tile has an empty table)
         int si, y0, z0;
         tile_of(idx + g, si, y0, z0);
-        deposit_tile<MODE, NTT, N>(sims[si], p, perm, row_start, err, y0, z0, lo + g * NL * RS, hi + g * NL * RS, RS,
+        deposit_tile<POS_DISP, NTT, N>(sims[si], p, perm, row_start, err, y0, z0, lo + g * NL * RS, hi + g * NL * RS, RS,
                                 s_begin[g], s_off[g], true, gtid, &s_ts[g], true);
       }
       // the CTA's TPB * NL rows: T lanes per row, rows R = warp * RPW + sub; a row's exchange
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
       int si, y0, z0;
       tile_of(idx, si, y0, z0);
       const Sim& S = sims[si];
-      const TileSum ts = deposit_tile<MODE, NT, N>(S, p, perm, row_start, err, y0, z0, lo, hi, RS, s_begin[0], s_off[0],
+      const TileSum ts = deposit_tile<POS_DISP, NT, N>(S, p, perm, row_start, err, y0, z0, lo, hi, RS, s_begin[0], s_off[0],
                                                 runs_ready);
       runs_ready = false;
       float v[PER];
@@ -955,18 +955,15 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
 
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
-                               int mode, int* err, unsigned* next_tile, const unsigned* order, int ctas,
-                               cudaStream_t st) {
+                               int* err, unsigned* next_tile, const unsigned* order, int ctas, cudaStream_t st) {
   if constexpr (!deposit_r2c_ok(N)) {
     return cudaErrorNotSupported;
   } else {
   static DeviceOnce once;
   const size_t sm = dep_tiles(N) * deposit_r2c_smem_bytes(N);
   const cudaError_t ie = once.run([&]() {
-    cudaError_t e = cudaFuncSetAttribute(k_deposit_r2c<N, POS_ABS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N, POS_DISP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N, POS_ABS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N, POS_DISP>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaError_t e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return e;
   });
   if (ie) return ie;
@@ -978,10 +975,7 @@ cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned*
     const cudaError_t e = cudaMemsetAsync(next_tile, 0, sizeof(unsigned), st);
     if (e) return e;
   }
-  if (mode == POS_ABS)
-    k_deposit_r2c<N, POS_ABS><<<ctas, NT, sm, st>>>(sims, w, p, perm, row_start, err, next_tile, order);
-  else
-    k_deposit_r2c<N, POS_DISP><<<ctas, NT, sm, st>>>(sims, w, p, perm, row_start, err, next_tile, order);
+  k_deposit_r2c<N><<<ctas, NT, sm, st>>>(sims, w, p, perm, row_start, err, next_tile, order);
   return cudaGetLastError();
   }
 }
