@@ -118,7 +118,7 @@ int begin(pm_ctx* c, const Call& k, cudaStream_t st, void* zero = nullptr, size_
 // keys -> sort -> row starts for absolute positions; leaves perm / sorted keys pointers.
 int sort_particles(pm_ctx* c, Call& k, const float* positions, cudaStream_t st, unsigned** perm, unsigned** skeys) {
   const long long np = k.sim.np;
-  PM_CK(c->sort.ensure(np), "alloc sort");
+  PM_CK(c->sort.ensure(np, true), "alloc sort");
   const Sim* ds = c->d_sim.as<Sim>();
   PM_CK(launch_keys_abs(ds, work(c, k, CALL_KEYS), abs_parts(positions, np), c->sort.keys.as<unsigned>(), nullptr,
                         c->d_err.as<int>(), grid_for(k.work.prefix[CALL_KEYS][1], c->sms, 16), st),
@@ -134,14 +134,21 @@ int sort_particles(pm_ctx* c, Call& k, const float* positions, cudaStream_t st, 
   return PM_OK;
 }
 
-// Writes the call's descriptor and groups the particles by x-row: row starts in c->row_start,
+// Particles per side if np is the configuration's whole lattice (the caller's arrays are then
+// taken to be in lattice order; any other order gives the same results, slower), else 0.
+int lattice_side(pm_ctx* c, long long np) {
+  const long long l = c->cfg.n_parts;
+  return l * l * l == np ? (int)l : 0;
+}
+
+// Writes the call's descriptor and groups the particles by row bin: bin starts in c->row_start,
 // cell records in row order in c->rec, and each particle's place there in c->sort.keys.  The
 // deposit and the force need the particles grouped by row only; their results do not depend
 // on the order inside a row.  Work enqueued here reads `positions` once more after the
 // first kernel: pos_copy (optional) receives a device copy in that first read.
 int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy, cudaStream_t st) {
   const long long np = k.sim.np;
-  const unsigned nrows = (unsigned)((long long)c->n * c->n);
+  const unsigned nrows = row_bins(c->n);
   PM_CK(c->sort.ensure(np), "alloc sort");
   PM_CK(c->rec.ensure((size_t)np * sizeof(uint4)), "alloc records");
   PM_CK(c->row_start.ensure(((size_t)nrows + 1) * sizeof(unsigned)), "alloc rows");
@@ -150,9 +157,10 @@ int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy,
   unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
   unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
   if (int r = begin(c, k, st, count, (size_t)nrows * sizeof(unsigned))) return r;
-  PM_CK(launch_row_rank(positions, np, c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, st), "row ranks");
-  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), st), "row starts");
-  PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, c->n, start, ranks, place, c->rec.as<uint4>(), st),
+  PM_CK(launch_row_rank(positions, np, lattice_side(c, np), c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, st), "row ranks");
+  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, st), "row starts");
+  PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, lattice_side(c, np), c->n, start, ranks, place,
+                         c->rec.as<uint4>(), st),
         "row order");
   return PM_OK;
 }
@@ -277,8 +285,8 @@ int force(pm_ctx* c, const Call& k, cudaStream_t st) {
 
 int advance(pm_ctx* c, const Call& k, const float* pos, const float* vel, float* pos_out, float* vel_out,
             cudaStream_t st) {
-  PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(), c->sort.keys.as<unsigned>(), pos, vel, pos_out,
-                       vel_out, c->d_err.as<int>(), st),
+  PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, lattice_side(c, k.sim.np), c->rec.as<uint4>(),
+                       c->sort.keys.as<unsigned>(), pos, vel, pos_out, vel_out, c->d_err.as<int>(), st),
         "kick");
   return PM_OK;
 }
@@ -367,7 +375,7 @@ int pm_density(pm_ctx* c, const float* positions, long long np, double mass, flo
   cudaStream_t st = (cudaStream_t)stream;
   Call k;
   k.sim = base_sim(c, np);
-  k.sim.xbits = 0;  // row keys
+  k.sim.xbits = 0;  // row bins
   k.sim.rho = rho;
   k.sim.mass_scale = (float)(mass / (double)(1u << PM_FIX_BITS));
   set_work(k, np, c->n);
@@ -412,7 +420,7 @@ int pm_integrate(pm_ctx* c, float* positions, float* velocities, long long np, d
   cudaStream_t st = (cudaStream_t)stream;
   Call k;
   k.sim = base_sim(c, np);
-  k.sim.xbits = 0;  // row keys: the force is read with the particles grouped by row (locality)
+  k.sim.xbits = 0;  // row bins
   k.sim.phi = const_cast<float*>(phi);
   set_kick(k.sim, a, f_a1, da);
   set_work(k, np, c->n);
@@ -468,7 +476,7 @@ int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, 
   PM_CK(c->phi.ensure(gb), "alloc phi");
   Call k;
   k.sim = base_sim(c, np);
-  k.sim.xbits = 0;  // row keys
+  k.sim.xbits = 0;  // row bins
   k.sim.rho = rho;
   k.sim.phi = c->phi.as<float>();
   k.sim.mass_scale = (float)(mass / (double)(1u << PM_FIX_BITS));

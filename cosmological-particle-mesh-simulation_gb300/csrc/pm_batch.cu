@@ -4,7 +4,7 @@
 // structure-of-arrays buffers (double buffered), stored as float32 displacements from
 // their Lagrangian lattice point plus the particle index; every step the kick writes
 // the state back in the order of the step's cell-key sort, so that the next step reads
-// it almost in order.  Simulation s owns the x-rows [row_base_s, row_base_s + N_s^2) of the
+// it almost in order.  Simulation s owns row bins [row_base_s, row_base_s + row_bins(N_s)) of the
 // common key space and, in the sorted order (and so in the state a step writes), the range
 // [part_off_s, part_off_s + np_s), in the same order, so one counting sort over the rows
 // serves the whole batch.  Every phase is one launch over all simulations (the spectral
@@ -330,8 +330,8 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     r.part_off = off;
     r.row_base = rows;
     off += r.np;
-    if ((long long)rows + (long long)r.n * r.n >= (1ll << 32)) return bfail(b, PM_ERR_ADMIT, "too many x-rows");
-    rows += (unsigned)((long long)r.n * r.n);
+    if ((long long)rows + row_bins(r.n) >= (1ll << 32)) return bfail(b, PM_ERR_ADMIT, "too many row bins");
+    rows += row_bins(r.n);
     if (std::find(P.sizes.begin(), P.sizes.end(), r.n) == P.sizes.end()) P.sizes.push_back(r.n);
   }
   P.ptot = off;
@@ -551,10 +551,11 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   Parts in = state(b, cur), out = state(b, 1 - cur);
   // group the particles by x-row: row starts and the permutation to row order
   unsigned* perm = b->sort.vals.as<unsigned>();
-  // (the row histogram of the keys was made by the previous kick, or by ensure_keys)
+  // (the row histogram of the keys was made by the previous kick, or by ensure_keys; the scan
+  // clears it for this step's kick)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, true),
+                          perm, err, b->sms, st, true, true),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
@@ -601,8 +602,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
       PB_CK(mark(1 + PP_X_R2C + o), "event");
     }
   }
-  // the kick writes the next keys and counts them per row for the next step's sort
-  PB_CK(cudaMemsetAsync(b->row_count.p, 0, sizeof(unsigned) * (size_t)P.rows, st), "count reset");
+  // the kick writes the next keys and counts them per row bin for the next step's sort
   PB_CK(launch_kick(ds, work_of(b, PH_KICK, P.fixed_total[PH_KICK]), in, out, perm, b->sort.keys.as<unsigned>(),
                     err, grid_for(P.fixed_total[PH_KICK], b->sms, P.kick_cps), st,
                     b->row_count.as<unsigned>()),
@@ -616,9 +616,8 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
 // Kernel launches of one step for the current plan.
 int launches_per_step(pm_batch* b) {
   const Plan& P = b->plan;
-  // counting sort: 3 scan kernels and the scatter (the kick makes the histogram; the count
-  // reset is a memset)
-  int n = 4 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1 + 1;
+  // counting sort: 2 scan kernels and the scatter (the kick makes the histogram)
+  int n = 3 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1 + 1;
   // a fused size replaces its x R2C launch by the fused deposit (with a dense-first tile
   // order, one launch more); a separate one adds its deposit launch
   for (size_t g = 0; g < P.sizes.size(); ++g)
@@ -744,10 +743,13 @@ int autotune(pm_batch* b, cudaStream_t st) {
   if (!rc && !kick_known) {  // the kick's grid; its keys and histogram go to scratch buffers
     const Work wk = work_of(b, PH_KICK, P.fixed_total[PH_KICK]);
     float best_ms = 1e30f;
+    DBuf keys;
+    if (cudaError_t e = keys.ensure(sizeof(unsigned) * (size_t)P.ptot)) rc = bcuda(b, e, "alloc keys");
     for (int cps : {4, 8, 16, 32}) {
+      if (rc) break;
       float ms = 0.f;
       rc = time3([&]() -> int {
-        PB_CK(launch_kick(ds, wk, in, out, perm, b->sort.vals_alt.as<unsigned>(), err,
+        PB_CK(launch_kick(ds, wk, in, out, perm, keys.as<unsigned>(), err,
                           grid_for(wk.total, b->sms, cps), st, b->row_cursor.as<unsigned>()),
               "kick");
         return PM_OK;
@@ -755,6 +757,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
       if (rc) break;
       if (ms < best_ms) { best_ms = ms; P.kick_cps = cps; }
     }
+    keys.release();
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1040,7 +1043,7 @@ int pm_batch_add(pm_batch* b, const pm_config* cfg, const float* positions, cons
   {  // the state is written in row order (the counting sort of the new particles' rows), so that
      // its first step reads it almost in order like every later one (a step sorts the state
      // it writes)
-    const unsigned nrows = (unsigned)((long long)r->n * r->n);
+    const unsigned nrows = row_bins(r->n);
     PB_CK(b->adm_count.ensure_geo(sizeof(unsigned) * nrows), "alloc rows");
     PB_CK(b->adm_start.ensure_geo(sizeof(unsigned) * ((size_t)nrows + 1)), "alloc rows");
     PB_CK(b->adm_cursor.ensure_geo(sizeof(unsigned) * nrows), "alloc rows");

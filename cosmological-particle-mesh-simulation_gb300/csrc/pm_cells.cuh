@@ -147,10 +147,15 @@ __device__ __forceinline__ Cell raw_cell(const Sim& S, const Parts& p, const Raw
   return cell_disp(S, r.w, r.a, r.b, r.c);
 }
 
-// xbits == 0 (resident batches): the key is the x-row number alone
+// Row bin of a cell: its x-row and its block of cells along x.
+__device__ __forceinline__ unsigned row_bin(const Cell& c, int n) {
+  return row_number(c.y, c.z, n) * (unsigned)x_bins(n) + ((unsigned)c.x >> x_shift(n));
+}
+
+// xbits == 0: the key is the row bin
 __device__ __forceinline__ unsigned cell_key(const Sim& S, const Cell& c) {
-  const unsigned row = S.row_base + row_number(c.y, c.z, S.n);
-  return S.xbits ? ((row << S.xbits) | (unsigned)c.x) : row;
+  if (!S.xbits) return S.row_base + row_bin(c, S.n);
+  return ((S.row_base + row_number(c.y, c.z, S.n)) << S.xbits) | (unsigned)c.x;
 }
 
 // The 8 CIC weights in the order of integrate.py:44-51: [ttt, dtt, tdt, ttd, ddt, dtd, tdd, ddd]

@@ -66,6 +66,15 @@ enum : int {
   ERR_TIMEOUT = 8,      // a bounded wait on an asynchronous copy gave up
 };
 
+// Row bins: the drop-in step and the resident engine group particles by x-row and, inside a row, by
+// blocks of 128 cells (256 above 512 cells a side; the last block may be short).  The deposit
+// needs rows only, but the lanes of the kick then read potential taps next to one another:
+// resident kick 516 -> 469 us early and 489 -> 453 us clustered (256^3 on 512^3), for 6 us more in
+// the sort.  Blocks of 64 cells give the kick 2-6 us more and cost the sort 6; 32 cells, 20.
+__host__ __device__ constexpr int x_shift(int n) { return n <= 512 ? 7 : 8; }
+__host__ __device__ constexpr int x_bins(int n) { return ((n - 1) >> x_shift(n)) + 1; }
+__host__ __device__ constexpr unsigned row_bins(int n) { return (unsigned)n * (unsigned)n * (unsigned)x_bins(n); }
+
 enum PosMode : int { POS_ABS = 0, POS_DISP = 1 };
 
 // Device-side description of one simulation.  All pointers are device pointers.
@@ -82,7 +91,7 @@ struct Sim {
                        // state the kick writes: the batch particle arrays after a step)
   long long slot_off;  // first particle slot of this simulation in the state being read by the
                        // keys kernel (differs from part_off right after a retirement)
-  unsigned row_base;   // first global row number of this simulation
+  unsigned row_base;   // first global row (xbits != 0) or row-bin (xbits == 0) of this simulation
   unsigned pad1;
   float* rho;          // density n^3 (output of the deposit)
   float2* spec;        // half spectrum
@@ -214,16 +223,17 @@ cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, con
 // descriptor and work table of one call (from kernel arguments); zero_bytes: a multiple of 16
 cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
                               size_t zero_bytes, cudaStream_t st);
+// np1: particles per side when the particles are in lattice order (np = np1^3), else 0
 // row key and rank inside its row of every particle; count (zero before) ends as the row counts
-cudaError_t launch_row_rank(const float* pos, long long np, int n, unsigned* count, unsigned* keys, unsigned* ranks,
-                            int* err, float* copy, cudaStream_t st);
+cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
+                            unsigned* ranks, int* err, float* copy, cudaStream_t st);
 // cell records in row order; place: in the keys, out each particle's place in row order
-cudaError_t launch_row_place(const float* pos, long long np, int n, const unsigned* row_start, const unsigned* ranks,
-                             unsigned* place, uint4* rec, cudaStream_t st);
+cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
+                             const unsigned* ranks, unsigned* place, uint4* rec, cudaStream_t st);
 // rec: in the cell records, out the forces (3 floats in the first words of each entry)
 cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cudaStream_t st);
-cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place, const float* pos,
-                           const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st);
+cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
+                           const float* pos, const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st);
 cudaError_t launch_coef(Sim* sims, int nsims, int advance, cudaStream_t st);
 cudaError_t deposit_prepare();  // sets kernel attributes of the current device (call before graph capture)
 // order of the fused deposit's tiles (dense tiles first); counts: 2 device words of scratch
@@ -232,7 +242,7 @@ cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* ro
 cudaError_t launch_abs_to_disp(const float* pos, const float* vel, long long np, int np1, int n,
                                const int* q_int, const float* q_frac, Parts out, long long off,
                                cudaStream_t st, const unsigned* order = nullptr);
-// keys[i] = x-row (tile order) of the cell of absolute position i (n^2 rows)
+// keys[i] = row bin (rows in tile order) of the cell of absolute position i
 cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned* keys, cudaStream_t st);
 cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, int n, const int* q_int,
                                const float* q_frac, float* pos, float* vel, cudaStream_t st);
@@ -260,13 +270,15 @@ cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bi
 // counts) and perm[j] = index of the j-th key in row order (order inside a row not
 // specified).  Scratch: count and cursor (nrows each), block_sums (row_sort_block_sums).
 size_t row_sort_block_sums(unsigned nrows);
-// counted: count already holds the row histogram of keys (else it is zeroed and computed here).
+// counted: count already holds the row histogram of keys (else it is zeroed and computed here);
+// zero: count is cleared once read.
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, bool counted = false);
-// row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows entries
-cudaError_t row_scan(const unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
-                     cudaStream_t st);
+                              int sms, cudaStream_t st, bool counted = false, bool zero = false);
+// row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows
+// entries; zero: count is cleared once read.  All arrays 16-byte aligned.
+cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
+                     bool zero, cudaStream_t st);
 // count[r] = number of keys equal to r (count zeroed first)
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
                           cudaStream_t st);

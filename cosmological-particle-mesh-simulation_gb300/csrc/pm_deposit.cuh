@@ -219,9 +219,10 @@ __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __rest
     else if (lane == 1) { r0 = t_zb * (TZ * TY) + (TZ - 1) * TY; nr = TY; }
     else if (lane < 6) { r0 = t_yb * (TZ * TY) + (lane - 2) * TY + TY - 1; nr = 1; }
     else { r0 = t_c * (TZ * TY) + (TZ - 1) * TY + TY - 1; nr = 1; }
-    r0 += S.row_base;
-    v.beg = __ldg(&row_start[r0]);
-    v.cnt = __ldg(&row_start[r0 + nr]) - v.beg;
+    const unsigned per_row = S.xbits ? 1u : (unsigned)x_bins(n);  // entries of row_start per x-row
+    const unsigned* s = row_start + (S.row_base + r0 * per_row);
+    v.beg = __ldg(s);
+    v.cnt = __ldg(s + nr * per_row) - v.beg;
   }
   return v;
 }

@@ -107,20 +107,20 @@ struct Lattice {
   void release() { qi.release(); qf.release(); np1 = n = 0; }
 };
 
-// Sort scratch sized for n elements.
+// Keys and values of n elements, and (radix) the scratch of the radix sort.
 struct SortBufs {
   DBuf keys, vals, keys_alt, vals_alt, hist, digit_tot;
   long long cap = 0;
-  cudaError_t ensure(long long n) {
-    if (n <= cap && keys.p) return cudaSuccess;
+  cudaError_t ensure(long long n, bool radix = false) {
     const size_t b = (size_t)(n > 0 ? n : 1) * sizeof(unsigned);
     cudaError_t e = keys.ensure(b);
     if (!e) e = vals.ensure(b);
-    if (!e) e = keys_alt.ensure(b);
+    if (!radix || e) return e;
+    e = keys_alt.ensure(b);
     if (!e) e = vals_alt.ensure(b);
     if (!e) e = hist.ensure(sort_scratch_hist_entries(n) * sizeof(unsigned));
     if (!e) e = digit_tot.ensure(SORT_DIGIT_TOTALS * sizeof(unsigned));
-    if (!e) cap = n;
+    if (!e && n > cap) cap = n;
     return e;
   }
   SortScratch scratch() const {

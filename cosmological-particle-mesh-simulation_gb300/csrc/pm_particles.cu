@@ -289,33 +289,57 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sim
 // the launchers.
 // ---------------------------------------------------------------------------------
 constexpr int ORD_NT = 256;
-constexpr int ORD_PPT = 4;  // particles per thread, ORD_NT apart: their loads and atomics overlap
+constexpr int ORD_PPT = 4;  // particles per thread: their loads and atomics overlap
+
+// The particle that element q of thread t of block b handles (-1: none).  Particles in lattice
+// order (np1 > 0: np = np1^3, index (ix np1 + iy) np1 + iz) are taken in boxes of 16 iz x 4 iy x
+// 16 ix, boxes along ix first: a box's particles lie in a few neighbouring rows, and the boxes in
+// flight fill whole rows, so the words they write stay in L2 until their lines are full.  Plain
+// order sweeps all rows once per ix plane.  np1 = 0: plain order.
+struct ParticleOrder {
+  long long np;
+  int np1, bx, by;  // boxes per axis ix, iy
+  __host__ __device__ ParticleOrder(long long n, int l) : np(n), np1(l), bx((l + 15) / 16), by((l + 3) / 4) {}
+  __host__ long long blocks() const {
+    return np1 ? (long long)bx * by * bx : (np + ORD_NT * ORD_PPT - 1) / (ORD_NT * ORD_PPT);
+  }
+  __device__ __forceinline__ long long at(int q) const {
+    if (!np1) {
+      const long long i = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + q * ORD_NT + threadIdx.x;
+      return i < np ? i : -1;
+    }
+    const int b = blockIdx.x, x0 = b % bx * 16, y0 = b / bx % by * 4, z0 = b / (bx * by) * 16;
+    const int e = q * ORD_NT + threadIdx.x;
+    const int ix = x0 + (e >> 6), iy = y0 + ((e >> 4) & 3), iz = z0 + (e & 15);
+    return ix < np1 && iy < np1 && iz < np1 ? ((long long)ix * np1 + iy) * np1 + iz : -1;
+  }
+};
 
 // copy (optional): the positions are also written there (they are read once, e.g. from host
 // memory, and leave a device copy)
-__global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ pos, long long np, int n,
+__global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ pos, ParticleOrder ord, int n,
                                                      unsigned* __restrict__ count, unsigned* __restrict__ keys,
                                                      unsigned* __restrict__ ranks, int* err,
                                                      float* __restrict__ copy) {
   const int lane = threadIdx.x & 31;
-  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
+  const long long np = ord.np;
   float x[ORD_PPT], y[ORD_PPT], z[ORD_PPT];
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
+    const long long i = ord.at(q);
     x[q] = y[q] = z[q] = 0.f;
-    if (i < np) { x[q] = pos[i]; y[q] = pos[np + i]; z[q] = pos[2 * np + i]; }
+    if (i >= 0) { x[q] = pos[i]; y[q] = pos[np + i]; z[q] = pos[2 * np + i]; }
   }
   unsigned key[ORD_PPT], grp[ORD_PPT], base[ORD_PPT];
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
+    const long long i = ord.at(q);
     key[q] = 0xffffffffu;
-    if (i < np) {
+    if (i >= 0) {
       if (copy) { copy[i] = x[q]; copy[np + i] = y[q]; copy[2 * np + i] = z[q]; }
       const Cell c = cell_abs(x[q], y[q], z[q], n);
       if (!c.ok) set_error(err, ERR_CELL_RANGE);
-      key[q] = c.ok ? row_number(c.y, c.z, n) : 0u;
+      key[q] = c.ok ? row_bin(c, n) : 0u;
     }
     // equal keys of a warp share one atomic
     grp[q] = __match_any_sync(FULL, key[q]);
@@ -324,9 +348,9 @@ __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ p
   }
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
+    const long long i = ord.at(q);
     const unsigned b = __shfl_sync(FULL, base[q], __ffs(grp[q]) - 1);
-    if (i < np) {
+    if (i >= 0) {
       keys[i] = key[q];
       ranks[i] = b + __popc(grp[q] & ((1u << lane) - 1u));
     }
@@ -334,17 +358,17 @@ __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ p
 }
 
 // place: in the row key of each particle, out its place in row order
-__global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ pos, long long np, int n,
+__global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ pos, ParticleOrder ord, int n,
                                                       const unsigned* __restrict__ row_start,
                                                       const unsigned* __restrict__ ranks, unsigned* __restrict__ place,
                                                       uint4* __restrict__ rec) {
-  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
+  const long long np = ord.np;
   Parts out{};
   out.rec = rec;
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
-    if (i >= np) continue;
+    const long long i = ord.at(q);
+    if (i < 0) continue;
     const Cell c = cell_abs(pos[i], pos[np + i], pos[2 * np + i], n);
     const unsigned slot = __ldg(&row_start[place[i]]) + ranks[i];
     store_cell_record(out, slot, c);
@@ -386,31 +410,31 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_force(const Sim* __restrict__ si
 // Kick and drift (integrate.py:94-95) of the caller's state with the forces in row order;
 // positions may arrive as exactly n: the canonical value drifts and is wrapped into [0, n).
 // pos_out / vel_out may be pos / vel, or host memory.
-__global__ void __launch_bounds__(ORD_NT) k_advance(const Sim* __restrict__ sims, const uint4* __restrict__ force,
+__global__ void __launch_bounds__(ORD_NT) k_advance(const Sim* __restrict__ sims, ParticleOrder ord,
+                                                    const uint4* __restrict__ force,
                                                     const unsigned* __restrict__ place, const float* pos,
                                                     const float* vel, float* pos_out, float* vel_out, int* err) {
   const Sim& S = sims[0];
-  const long long np = S.np;
+  const long long np = ord.np;
   const float kk = S.kick, dr = S.drift, fn = (float)S.n;
-  const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x;
   uint4 g[ORD_PPT];
   float p[ORD_PPT][3], v[ORD_PPT][3];
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
-    if (i < np) g[q] = __ldg(&force[__ldg(&place[i])]);
+    const long long i = ord.at(q);
+    if (i >= 0) g[q] = __ldg(&force[__ldg(&place[i])]);
   }
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
+    const long long i = ord.at(q);
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      if (i < np) { p[q][d] = pos[d * np + i]; v[q][d] = vel[d * np + i]; }
+      if (i >= 0) { p[q][d] = pos[d * np + i]; v[q][d] = vel[d * np + i]; }
   }
 #pragma unroll
   for (int q = 0; q < ORD_PPT; ++q) {
-    const long long i = i0 + q * ORD_NT;
-    if (i >= np) continue;
+    const long long i = ord.at(q);
+    if (i < 0) continue;
     const float f[3] = {__uint_as_float(g[q].x), __uint_as_float(g[q].y), __uint_as_float(g[q].z)};
     bool ok = true;
 #pragma unroll
@@ -462,12 +486,12 @@ __global__ void k_coef(Sim* sims, int nsims, int advance) {
 // resident-state conversion: absolute (3, np) arrays in particle order <-> displacement
 // state at slots [off, off + np)
 // ---------------------------------------------------------------------------------
-// x-row of the cell of every absolute position (the row part of the cell key, tile order)
+// row bin of the cell of every absolute position
 __global__ void k_row_keys_abs(const float* __restrict__ pos, long long np, int n, unsigned* __restrict__ keys) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < np;
        i += (long long)gridDim.x * blockDim.x) {
     const Cell c = cell_abs(pos[i], pos[np + i], pos[2 * np + i], n);
-    keys[i] = c.ok ? row_number(c.y, c.z, n) : 0u;
+    keys[i] = c.ok ? row_bin(c, n) : 0u;
   }
 }
 
@@ -630,10 +654,6 @@ cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, con
   return cudaGetLastError();
 }
 
-namespace {
-int ord_ctas(long long np) { return (int)((np + ORD_NT * ORD_PPT - 1) / (ORD_NT * ORD_PPT)); }
-}  // namespace
-
 cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
                               size_t zero_bytes, cudaStream_t st) {
   const long long nz = (long long)(zero_bytes / sizeof(uint4));
@@ -643,15 +663,17 @@ cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_row_rank(const float* pos, long long np, int n, unsigned* count, unsigned* keys, unsigned* ranks,
-                            int* err, float* copy, cudaStream_t st) {
-  k_row_rank<<<ord_ctas(np), ORD_NT, 0, st>>>(pos, np, n, count, keys, ranks, err, copy);
+cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
+                            unsigned* ranks, int* err, float* copy, cudaStream_t st) {
+  const ParticleOrder o(np, 0);
+  k_row_rank<<<(int)o.blocks(), ORD_NT, 0, st>>>(pos, o, n, count, keys, ranks, err, copy);
   return cudaGetLastError();
 }
 
-cudaError_t launch_row_place(const float* pos, long long np, int n, const unsigned* row_start, const unsigned* ranks,
-                             unsigned* place, uint4* rec, cudaStream_t st) {
-  k_row_place<<<ord_ctas(np), ORD_NT, 0, st>>>(pos, np, n, row_start, ranks, place, rec);
+cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
+                             const unsigned* ranks, unsigned* place, uint4* rec, cudaStream_t st) {
+  const ParticleOrder o(np, np1);
+  k_row_place<<<(int)o.blocks(), ORD_NT, 0, st>>>(pos, o, n, row_start, ranks, place, rec);
   return cudaGetLastError();
 }
 
@@ -661,9 +683,11 @@ cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cud
   return cudaGetLastError();
 }
 
-cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place, const float* pos,
-                           const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st) {
-  k_advance<<<ord_ctas(np), ORD_NT, 0, st>>>(sims, force, place, pos, vel, pos_out, vel_out, err);
+cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
+                           const float* pos, const float* vel, float* pos_out, float* vel_out, int* err,
+                           cudaStream_t st) {
+  const ParticleOrder o(np, 0);
+  k_advance<<<(int)o.blocks(), ORD_NT, 0, st>>>(sims, o, force, place, pos, vel, pos_out, vel_out, err);
   return cudaGetLastError();
 }
 

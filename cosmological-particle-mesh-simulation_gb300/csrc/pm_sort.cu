@@ -294,6 +294,19 @@ __global__ void __launch_bounds__(CS_NT) k_row_hist(const unsigned* __restrict__
   }
 }
 
+// Four consecutive words of v from i on (0 past n; i a multiple of 4, v 16-byte aligned).
+__device__ __forceinline__ uint4 load4(const unsigned* __restrict__ v, long long i, long long n) {
+  if (i + 3 < n) return *reinterpret_cast<const uint4*>(v + i);
+  return make_uint4(i < n ? v[i] : 0u, i + 1 < n ? v[i + 1] : 0u, i + 2 < n ? v[i + 2] : 0u, 0u);
+}
+
+__device__ __forceinline__ void store4(unsigned* __restrict__ v, long long i, long long n, uint4 q) {
+  if (i + 3 < n) { *reinterpret_cast<uint4*>(v + i) = q; return; }
+  if (i < n) v[i] = q.x;
+  if (i + 1 < n) v[i + 1] = q.y;
+  if (i + 2 < n) v[i + 2] = q.z;
+}
+
 // per-block sums of SCAN_TILE entries
 __global__ void __launch_bounds__(CS_NT) k_scan_reduce(const unsigned* __restrict__ in, long long n,
                                                        unsigned* __restrict__ block_sums) {
@@ -301,9 +314,9 @@ __global__ void __launch_bounds__(CS_NT) k_scan_reduce(const unsigned* __restric
   const long long base = (long long)blockIdx.x * SCAN_TILE;
   unsigned s = 0;
 #pragma unroll
-  for (int j = 0; j < SCAN_IPT; ++j) {
-    const long long i = base + j * CS_NT + threadIdx.x;
-    if (i < n) s += __ldg(&in[i]);
+  for (int j = 0; j < SCAN_IPT / 4; ++j) {
+    const uint4 q = load4(in, base + (j * CS_NT + threadIdx.x) * 4, n);
+    s += q.x + q.y + q.z + q.w;
   }
   unsigned total;
   block_exclusive_scan<CS_NT>(s, ws, total);
@@ -325,32 +338,58 @@ __global__ void __launch_bounds__(CS_NT) k_scan_top(unsigned* __restrict__ block
   }
 }
 
-// out[i] = exclusive prefix of in, i < n; out[n] = total; cursor (optional) = copy of out[0, n)
-__global__ void __launch_bounds__(CS_NT) k_scan_apply(const unsigned* __restrict__ in, long long n,
-                                                      const unsigned* __restrict__ block_sums,
+// out[i] = exclusive prefix of in, i < n; out[n] = total; cursor (optional) = copy of out[0, n).
+// A block adds up the sums of the blocks before it (scanned: block_sums holds their prefix
+// already).  zero: the entries of `in` are cleared once read.  A warp takes 512 consecutive
+// entries, four to a lane and load (6.6 -> 4.0 us for the 2.1 M bins of a 512 grid, against
+// 16 strided words per lane on its 262,144 rows).
+__global__ void __launch_bounds__(CS_NT) k_scan_apply(unsigned* __restrict__ in, long long n,
+                                                      const unsigned* __restrict__ block_sums, int scanned, int zero,
                                                       unsigned* __restrict__ out, unsigned* __restrict__ cursor) {
   __shared__ unsigned ws[CS_NT / 32];
-  const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_IPT;
-  unsigned v[SCAN_IPT];
-  unsigned s = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long base = (long long)blockIdx.x * SCAN_TILE + warp * (SCAN_TILE / (CS_NT / 32)) + lane * 4;
+  constexpr int R = SCAN_IPT / 4;
+  uint4 v[R];
+  unsigned ex[R], sum = 0;
 #pragma unroll
-  for (int j = 0; j < SCAN_IPT; ++j) {
-    const long long i = base + j;
-    v[j] = i < n ? __ldg(&in[i]) : 0u;
-    s += v[j];
-  }
-  unsigned total;
-  unsigned run = block_sums[blockIdx.x] + block_exclusive_scan<CS_NT>(s, ws, total);
+  for (int r = 0; r < R; ++r) v[r] = load4(in, base + r * 128, n);
 #pragma unroll
-  for (int j = 0; j < SCAN_IPT; ++j) {
-    const long long i = base + j;
-    if (i < n) {
-      out[i] = run;
-      if (cursor) cursor[i] = run;
+  for (int r = 0; r < R; ++r) {
+    const unsigned s = v[r].x + v[r].y + v[r].z + v[r].w;
+    unsigned x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
-    run += v[j];
-    if (i == n - 1) out[n] = run;
+    ex[r] = sum + x - s;
+    sum += __shfl_sync(0xffffffffu, x, 31);
   }
+  // the sum of the blocks before this one
+  unsigned before = 0;
+  if (scanned) {
+    before = block_sums[blockIdx.x];
+  } else {
+    for (int i = threadIdx.x; i < (int)blockIdx.x; i += CS_NT) before += block_sums[i];
+    unsigned total;
+    block_exclusive_scan<CS_NT>(before, ws, total);
+    before = total;
+  }
+  if (lane == 31) ws[warp] = sum;
+  __syncthreads();
+  unsigned run = before;
+  for (int w = 0; w < warp; ++w) run += ws[w];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const long long i = base + r * 128;
+    const unsigned a = run + ex[r];
+    const uint4 q = make_uint4(a, a + v[r].x, a + v[r].x + v[r].y, a + v[r].x + v[r].y + v[r].z);
+    store4(out, i, n, q);
+    if (cursor) store4(cursor, i, n, q);
+    if (zero) store4(in, i, n, make_uint4(0u, 0u, 0u, 0u));
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == CS_NT - 1) out[n] = run + sum;
 }
 
 // Each warp scatters one chunk of SCATTER_CHUNK consecutive keys, in order: the keys of a
@@ -410,24 +449,27 @@ cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, uns
   return cudaGetLastError();
 }
 
-cudaError_t row_scan(const unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
-                     cudaStream_t st) {
+cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
+                     bool zero, cudaStream_t st) {
   if (nrows == 0) return cudaErrorInvalidValue;
   const int nb = (int)row_sort_block_sums(nrows);
-  k_scan_reduce<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums);
-  k_scan_top<<<1, CS_NT, 0, st>>>(block_sums, nb);
-  k_scan_apply<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums, row_start, cursor);
+  // from 8192 blocks on (33 M bins) adding up the earlier blocks' sums in every block costs more
+  // than a scan of the sums
+  const bool scanned = nb > 8192;
+  if (nb > 1) k_scan_reduce<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums);
+  if (scanned) k_scan_top<<<1, CS_NT, 0, st>>>(block_sums, nb);
+  k_scan_apply<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums, scanned, zero, row_start, cursor);
   return cudaGetLastError();
 }
 
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, bool counted) {
+                              int sms, cudaStream_t st, bool counted, bool zero) {
   if (!counted) {
     cudaError_t e = row_histogram(keys, n, nrows, count, err, sms, st);
     if (e) return e;
   }
-  if (cudaError_t e = row_scan(count, nrows, row_start, cursor, block_sums, st)) return e;
+  if (cudaError_t e = row_scan(count, nrows, row_start, cursor, block_sums, zero, st)) return e;
   const long long chunks = (n + SCATTER_CHUNK - 1) / SCATTER_CHUNK;
   const long long sblocks = (chunks + CS_NT / 32 - 1) / (CS_NT / 32);
   k_row_scatter<<<(int)(sblocks < (long long)sms * 8 ? (sblocks > 0 ? sblocks : 1) : (long long)sms * 8), CS_NT, 0,
