@@ -11,12 +11,11 @@ struct pm_ctx {
   Tables tab;
   SortBufs sort;
   DBuf d_sim, d_work, d_err, d_maps;
-  DBuf tile_next;  // tile counter of the fused deposit
   const void* maps_for = nullptr;     // spectrum the device tensor maps describe
   DBuf row_start, spec, phi, rho;     // scratch grids
   DBuf hpos, hvel;                    // device copies for pm_step_host
   DBuf pk_partial, pk_out;            // power spectrum scratch
-  DBuf row_count, scan_sums;              // row counts of a call, block sums of their scan
+  DBuf row_count, scan_sums;  // row bin counts of a call (then 4 words: tile counter), block sums of their scan
   DBuf rec;                               // cell records in row order, then the forces
   // spectral gradient: spectra and force grids of the y and z axes (x uses spec and phi), the
   // three descriptors of the inverse passes and their work tables and tensor maps
@@ -109,9 +108,14 @@ int check_np(pm_ctx* c, long long np) {
   return PM_OK;
 }
 
+// The caller's stream with small grids' launches chained (pm_launch.cuh).
+Launch chained(pm_ctx* c, cudaStream_t st) { return Launch(st, c->n <= 256); }
+
 // The call's descriptor and work table on the device; zero (optional): bytes cleared with them.
 int begin(pm_ctx* c, const Call& k, cudaStream_t st, void* zero = nullptr, size_t zero_bytes = 0) {
-  PM_CK(launch_call_begin(c->d_sim.as<Sim>(), c->d_work.as<CallWork>(), k.sim, k.work, zero, zero_bytes, st), "begin");
+  PM_CK(launch_call_begin(c->d_sim.as<Sim>(), c->d_work.as<CallWork>(), k.sim, k.work, zero, zero_bytes,
+                          chained(c, st)),
+        "begin");
   return PM_OK;
 }
 
@@ -147,28 +151,30 @@ int lattice_side(pm_ctx* c, long long np) {
 // on the order inside a row.  Work enqueued here reads `positions` once more after the
 // first kernel: pos_copy (optional) receives a device copy in that first read.
 int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy, cudaStream_t st) {
+  const Launch lc = chained(c, st);
   const long long np = k.sim.np;
   const unsigned nrows = row_bins(c->n);
   PM_CK(c->sort.ensure(np), "alloc sort");
   PM_CK(c->rec.ensure((size_t)np * sizeof(uint4)), "alloc records");
   PM_CK(c->row_start.ensure(((size_t)nrows + 1) * sizeof(unsigned)), "alloc rows");
-  PM_CK(c->row_count.ensure((size_t)nrows * sizeof(unsigned)), "alloc rows");
+  PM_CK(c->row_count.ensure(((size_t)nrows + 4) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->scan_sums.ensure(row_sort_block_sums(nrows) * sizeof(unsigned)), "alloc rows");
   unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
   unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
-  if (int r = begin(c, k, st, count, (size_t)nrows * sizeof(unsigned))) return r;
-  PM_CK(launch_row_rank(positions, np, lattice_side(c, np), c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, st), "row ranks");
-  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, st), "row starts");
+  if (int r = begin(c, k, st, count, ((size_t)nrows + 4) * sizeof(unsigned))) return r;
+  PM_CK(launch_row_rank(positions, np, lattice_side(c, np), c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, lc), "row ranks");
+  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, lc), "row starts");
   PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, lattice_side(c, np), c->n, start, ranks, place,
-                         c->rec.as<uint4>(), st),
+                         c->rec.as<uint4>(), lc),
         "row order");
   return PM_OK;
 }
 
 int deposit(pm_ctx* c, Call& k, cudaStream_t st) {
+  const Launch lc = chained(c, st);
   PM_CK(launch_deposit(c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
                        c->row_start.as<unsigned>(), POS_DISP, c->d_err.as<int>(),
-                       grid_for(k.work.prefix[CALL_DEP][1], c->sms, 8), deposit_smem_bytes(c->n, TILE_Y, TILE_Z), st),
+                       grid_for(k.work.prefix[CALL_DEP][1], c->sms, 8), deposit_smem_bytes(c->n, TILE_Y, TILE_Z), lc),
         "deposit");
   return PM_OK;
 }
@@ -176,18 +182,19 @@ int deposit(pm_ctx* c, Call& k, cudaStream_t st) {
 int gradient_solve(pm_ctx* c, Call& k, cudaStream_t st);
 
 int spectral(pm_ctx* c, Call& k, bool table, cudaStream_t st, bool skip_r2c = false, bool gradient = false) {
+  const Launch lc = chained(c, st);
   const Sim* ds = c->d_sim.as<Sim>();
   const int n = c->n;
   const int gx = grid_for(k.work.prefix[CALL_X][1], c->sms, 8), gl = grid_for(k.work.prefix[CALL_LINE][1], c->sms, 8);
   const CUtensorMap* maps = c->maps_for ? c->d_maps.as<CUtensorMap>() : nullptr;
   int* err = c->d_err.as<int>();
-  if (!skip_r2c) PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, CALL_X), gx, st, maps, err), "x r2c");
-  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "y fwd");
+  if (!skip_r2c) PM_CK(spectral_dispatch(SPEC_X_R2C, n, ds, work(c, k, CALL_X), gx, lc, maps, err), "x r2c");
+  PM_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, work(c, k, CALL_LINE), gl, lc, maps, err), "y fwd");
   if (gradient) return gradient_solve(c, k, st);
-  PM_CK(spectral_dispatch(table ? SPEC_Z_TABLE : SPEC_Z_GREEN, n, ds, work(c, k, CALL_LINE), gl, st, maps, err),
+  PM_CK(spectral_dispatch(table ? SPEC_Z_TABLE : SPEC_Z_GREEN, n, ds, work(c, k, CALL_LINE), gl, lc, maps, err),
         "z green");
-  PM_CK(spectral_dispatch(SPEC_Y_INV, n, ds, work(c, k, CALL_LINE), gl, st, maps, err), "y inv");
-  PM_CK(spectral_dispatch(SPEC_X_C2R, n, ds, work(c, k, CALL_X), gx, st, maps, err), "x c2r");
+  PM_CK(spectral_dispatch(SPEC_Y_INV, n, ds, work(c, k, CALL_LINE), gl, lc, maps, err), "y inv");
+  PM_CK(spectral_dispatch(SPEC_X_C2R, n, ds, work(c, k, CALL_X), gx, lc, maps, err), "x c2r");
   return PM_OK;
 }
 
@@ -278,15 +285,15 @@ double f_step(pm_ctx* c, double a, double da) {
 }
 
 // The force of c->rec's particles and the kick and drift of the caller's state.
-int force(pm_ctx* c, const Call& k, cudaStream_t st) {
-  PM_CK(launch_force(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(), c->sms, st), "force");
+int force(pm_ctx* c, const Call& k, Launch l) {
+  PM_CK(launch_force(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(), c->sms, l), "force");
   return PM_OK;
 }
 
 int advance(pm_ctx* c, const Call& k, const float* pos, const float* vel, float* pos_out, float* vel_out,
             cudaStream_t st) {
   PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, lattice_side(c, k.sim.np), c->rec.as<uint4>(),
-                       c->sort.keys.as<unsigned>(), pos, vel, pos_out, vel_out, c->d_err.as<int>(), st),
+                       c->sort.keys.as<unsigned>(), pos, vel, pos_out, vel_out, c->d_err.as<int>(), chained(c, st)),
         "kick");
   return PM_OK;
 }
@@ -314,7 +321,6 @@ int pm_ctx_create(const pm_config* cfg, int device, pm_ctx** out) {
   if (!e) e = c->d_sim.ensure(sizeof(Sim));
   if (!e) e = c->d_work.ensure(sizeof(CallWork));
   if (!e) e = c->d_err.ensure(sizeof(int));
-  if (!e) e = c->tile_next.ensure(sizeof(unsigned));
   if (!e) e = cudaMemset(c->d_err.p, 0, sizeof(int));
   if (!e) e = cudaDeviceSynchronize();
   if (e) {
@@ -332,7 +338,6 @@ void pm_ctx_destroy(pm_ctx* c) {
   c->d_sim.release();
   c->d_work.release();
   c->d_err.release();
-  c->tile_next.release();
   c->d_maps.release();
   c->row_start.release();
   c->spec.release();
@@ -425,7 +430,7 @@ int pm_integrate(pm_ctx* c, float* positions, float* velocities, long long np, d
   set_kick(k.sim, a, f_a1, da);
   set_work(k, np, c->n);
   if (int r = place_particles(c, k, positions, nullptr, st)) return r;
-  if (int r = force(c, k, st)) return r;
+  if (int r = force(c, k, chained(c, st))) return r;
   return advance(c, k, positions, velocities, positions, velocities, st);
 }
 
@@ -496,8 +501,8 @@ int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, 
   if (!rho_out && deposit_r2c_supported(c->n)) {
     // the density is not requested: deposit straight into the x-transformed spectrum
     PM_CK(deposit_r2c_dispatch(c->n, c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
-                               c->row_start.as<unsigned>(), c->d_err.as<int>(), c->tile_next.as<unsigned>(), nullptr,
-                               grid_for(k.work.prefix[CALL_DEP][1], c->sms, deposit_r2c_ctas_per_sm(c->n)), st),
+                               c->row_start.as<unsigned>(), c->d_err.as<int>(), c->row_count.as<unsigned>() + row_bins(c->n), nullptr,
+                               grid_for(k.work.prefix[CALL_DEP][1], c->sms, deposit_r2c_ctas_per_sm(c->n)), chained(c, st)),
           "fused deposit");
     if (int r = spectral(c, k, false, st, true, gradient)) return r;
   } else {
@@ -506,7 +511,7 @@ int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, 
   }
   if (gradient)  // the force's descriptor now names the three force grids
     if (int r = begin(c, k, st)) return r;
-  if (int r = force(c, k, st)) return r;
+  if (int r = force(c, k, st)) return r;  // (not chained: behind the transforms)
   if (io.vel_ready) PM_CK(cudaStreamWaitEvent(st, io.vel_ready, 0), "wait velocities");
   return advance(c, k, io.pos_copy ? io.pos_copy : io.pos_in, io.vel_in, io.pos_out, io.vel_out, st);
 }

@@ -514,9 +514,11 @@ enum ProfPhase { PP_SORT = 0, PP_ROWS, PP_DEPOSIT, PP_X_R2C, PP_Y_FWD, PP_Z_GREE
                  PP_COEF, PP_COUNT };
 
 // The deposit of the simulations of distinct size g that can fuse it with the x R2C, on the
-// schedule `sh` (a separate deposit leaves the x R2C to the spectral phase).
-int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigned* perm, cudaStream_t st) {
+// schedule `sh` (a separate deposit leaves the x R2C to the spectral phase).  The size's words
+// of tile_next are 0 when it starts.
+int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigned* perm, cudaStream_t stream) {
   const Plan& P = b->plan;
+  const Launch st(stream, P.sizes[g] <= 256);  // small grids: chained (pm_launch.cuh)
   const Sim* ds = b->d_sims.as<Sim>();
   int* err = b->d_err.as<int>();
   const int n = P.sizes[g], tot = P.fdep_total[g];
@@ -555,7 +557,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   // clears it for this step's kick)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, true, true),
+                          perm, err, b->sms, Launch(st, P.max_n <= 256), true, true, b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size()),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
@@ -571,7 +573,8 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
     const int ph = PH_FIXED + 3 * g + (xk ? 0 : 1);
     const int tot = xk ? P.x_total[g] : P.line_total[g];
     PB_CK(spectral_dispatch(k, P.sizes[g], ds, work_of(b, ph, tot),
-                            xk ? grid_for(tot, b->sms, P.shape[g].x_cps) : grid_for(tot, b->sms, 8), s,
+                            xk ? grid_for(tot, b->sms, P.shape[g].x_cps) : grid_for(tot, b->sms, 8),
+                            Launch(s, P.sizes[g] <= 256),
                             b->d_maps.as<CUtensorMap>(), err),
           "spectral");
     return PM_OK;
@@ -608,7 +611,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
                     b->row_count.as<unsigned>()),
         "kick");
   PB_CK(mark(1 + PP_KICK), "event");
-  PB_CK(launch_coef(b->d_sims.as<Sim>(), P.nsims, 1, st), "coef");
+  PB_CK(launch_coef(b->d_sims.as<Sim>(), P.nsims, 1, Launch(st, P.max_n <= 256)), "coef");
   PB_CK(mark(1 + PP_COEF), "event");
   return PM_OK;
 }
@@ -704,6 +707,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
       for (const Shape& c : cands) {
         float ms = 0.f;
         rc = time3([&]() -> int {
+          PB_CK(cudaMemsetAsync(b->tile_next.p, 0, 4 * sizeof(unsigned) * P.sizes.size(), st), "clear");
           if (int r = enqueue_deposit(b, (int)g, c, in, perm, st)) return r;
           if (c.dep == DEP_SEPARATE)
             PB_CK(spectral_dispatch(SPEC_X_R2C, n, ds, wx, grid_for(wx.total, b->sms, c.x_cps), st,

@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pm_launch.cuh"
+
 #include <atomic>
 #include <mutex>
 
@@ -168,7 +170,7 @@ enum SpecKind : int { SPEC_X_R2C = 0, SPEC_Y_FWD, SPEC_Z_GREEN, SPEC_Z_TABLE, SP
 // spectral_encode_maps) -- enables the TMA-streamed line passes; nullptr falls back to
 // plain loads.  Every kernel finds its simulation through the work prefix.
 template <int N>
-cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, cudaStream_t st,
+cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, Launch st,
                             const CUtensorMap* maps, int* err);
 // Encodes the y- and z-pass tensor maps of a half spectrum of size n (false if n has no
 // TMA line pass).
@@ -178,23 +180,22 @@ bool spectral_supported(int n);
 long long spectral_units(SpecKind kind, int n);
 // resident CTAs per SM of a spectral pass for size n (for persistent grid sizing)
 int spectral_ctas_per_sm(SpecKind kind, int n);
-cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, cudaStream_t st,
+cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, Launch st,
                               const CUtensorMap* maps = nullptr, int* err = nullptr);
-cudaError_t launch_fourier_grid(const Sim* sims, int ctas, cudaStream_t st);
+cudaError_t launch_fourier_grid(const Sim* sims, int ctas, Launch st);
 // fused deposit + x R2C (the density grid is not written); ctas <= 0 only prepares.
-// next_tile: one device word, the tile counter (zeroed on `st` before the launch); nullptr:
-// CTAs take every ctas-th tile.  order (optional, w.total entries): the tiles in the order to
+// next_tile: one device word, the tile counter, 0 when the kernel starts.  order (optional, w.total entries): the tiles in the order to
 // take them (launch_tile_order).
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
                                int* err, unsigned* next_tile, const unsigned* order, int ctas,
-                               cudaStream_t st);
+                               Launch st);
 bool deposit_r2c_supported(int n);
 bool xrow_supported(int n);  // the x passes of size n transform rows in registers (their grid is tunable)
 int deposit_r2c_ctas_per_sm(int n);  // resident CTAs per SM of the fused deposit
 cudaError_t deposit_r2c_dispatch(int n, const Sim* sims, Work w, Parts p, const unsigned* perm,
                                  const unsigned* row_start, int* err, unsigned* next_tile,
-                                 const unsigned* order, int ctas, cudaStream_t st);
+                                 const unsigned* order, int ctas, Launch st);
 
 // sum of the first n_slices planes of an n^3 grid, float64 n^2 output (pm_diagnostics.cu)
 cudaError_t launch_project(const float* rho, int n, int n_slices, double* out, int ctas, cudaStream_t st);
@@ -207,45 +208,45 @@ cudaError_t launch_power_spectrum(const float2* spec, int n, int pitch, int nbin
 
 // particle kernels
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                            int* err, int ctas, cudaStream_t st);
+                            int* err, int ctas, Launch st);
 cudaError_t launch_keys_disp(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                             int* err, int ctas, cudaStream_t st);
+                             int* err, int ctas, Launch st);
 cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsigned nrows,
-                             unsigned* row_start, cudaStream_t st);
+                             unsigned* row_start, Launch st);
 cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsigned* perm,
                            const unsigned* row_start, int mode, int* err, int ctas, size_t smem,
-                           cudaStream_t st);
+                           Launch st);
 constexpr int KICK_UNIT = 512;  // particles per work unit of the kick
 // resident kick: the state in row order (through perm), the next keys and their row histogram
 cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, const unsigned* perm,
-                        unsigned* keys_next, int* err, int ctas, cudaStream_t st, unsigned* row_count);
+                        unsigned* keys_next, int* err, int ctas, Launch st, unsigned* row_count);
 // ---- drop-in step on (3, np) arrays in the caller's order (see pm_particles.cu) ----
 // descriptor and work table of one call (from kernel arguments); zero_bytes: a multiple of 16
 cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
-                              size_t zero_bytes, cudaStream_t st);
+                              size_t zero_bytes, Launch st);
 // np1: particles per side when the particles are in lattice order (np = np1^3), else 0
 // row key and rank inside its row of every particle; count (zero before) ends as the row counts
 cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
-                            unsigned* ranks, int* err, float* copy, cudaStream_t st);
+                            unsigned* ranks, int* err, float* copy, Launch st);
 // cell records in row order; place: in the keys, out each particle's place in row order
 cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
-                             const unsigned* ranks, unsigned* place, uint4* rec, cudaStream_t st);
+                             const unsigned* ranks, unsigned* place, uint4* rec, Launch st);
 // rec: in the cell records, out the forces (3 floats in the first words of each entry)
-cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cudaStream_t st);
+cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, Launch st);
 cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
-                           const float* pos, const float* vel, float* pos_out, float* vel_out, int* err, cudaStream_t st);
-cudaError_t launch_coef(Sim* sims, int nsims, int advance, cudaStream_t st);
+                           const float* pos, const float* vel, float* pos_out, float* vel_out, int* err, Launch st);
+cudaError_t launch_coef(Sim* sims, int nsims, int advance, Launch st);
 cudaError_t deposit_prepare();  // sets kernel attributes of the current device (call before graph capture)
-// order of the fused deposit's tiles (dense tiles first); counts: 2 device words of scratch
+// order of the fused deposit's tiles (dense tiles first); counts: 2 device words, 0 when the kernel starts
 cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* row_start, unsigned* order,
-                              unsigned* counts, int sms, cudaStream_t st);
+                              unsigned* counts, int sms, Launch st);
 cudaError_t launch_abs_to_disp(const float* pos, const float* vel, long long np, int np1, int n,
                                const int* q_int, const float* q_frac, Parts out, long long off,
-                               cudaStream_t st, const unsigned* order = nullptr);
+                               Launch st, const unsigned* order);
 // keys[i] = row bin (rows in tile order) of the cell of absolute position i
-cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned* keys, cudaStream_t st);
+cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned* keys, Launch st);
 cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, int n, const int* q_int,
-                               const float* q_frac, float* pos, float* vel, cudaStream_t st);
+                               const float* q_frac, float* pos, float* vel, Launch st);
 size_t deposit_smem_bytes(int n, int ty, int tz);
 
 // radix sort of (key, value) pairs, stable, LSD, digits of up to 9 bits
@@ -265,22 +266,23 @@ cudaError_t sort_prepare();
 // *in_alt whether the result sits in the scratch (alt) buffers.  When gen_vals is set,
 // vals are not read on the first pass and the identity 0..n-1 is used instead.
 cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bit, int bits, bool gen_vals,
-                       const SortScratch& s, bool* in_alt, cudaStream_t st);
+                       const SortScratch& s, bool* in_alt, Launch st);
 // Groups n row keys (< nrows) by row: row_start[0..nrows] (exclusive prefix of the row
 // counts) and perm[j] = index of the j-th key in row order (order inside a row not
 // specified).  Scratch: count and cursor (nrows each), block_sums (row_sort_block_sums).
 size_t row_sort_block_sums(unsigned nrows);
 // counted: count already holds the row histogram of keys (else it is zeroed and computed here);
-// zero: count is cleared once read.
+// zero: count is cleared once read; clear: nclear words set to 0.
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, bool counted = false, bool zero = false);
+                              int sms, Launch st, bool counted = false, bool zero = false,
+                              unsigned* clear = nullptr, int nclear = 0);
 // row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows
 // entries; zero: count is cleared once read.  All arrays 16-byte aligned.
 cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
-                     bool zero, cudaStream_t st);
+                     bool zero, Launch st);
 // count[r] = number of keys equal to r (count zeroed first)
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
-                          cudaStream_t st);
+                          Launch st);
 
 }  // namespace pm

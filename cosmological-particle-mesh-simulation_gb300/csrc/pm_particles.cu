@@ -27,6 +27,7 @@ template <int MODE>
 __global__ void __launch_bounds__(KEY_NT) k_keys(const Sim* __restrict__ sims, Work w, Parts p,
                                                  unsigned* __restrict__ keys,
                                                  unsigned* __restrict__ vals, int* err) {
+  chain_begin();
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
     const int si = locate_sim(w, unit);
     const Sim& S = sims[si];
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(KEY_NT) k_keys(const Sim* __restrict__ sims, W
 // ---------------------------------------------------------------------------------
 __global__ void k_row_start(const unsigned* __restrict__ keys, long long n, int xbits, unsigned nrows,
                             unsigned* __restrict__ row_start) {
+  chain_begin();
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s <= n;
        s += (long long)gridDim.x * blockDim.x) {
     long long rp = -1, rc = nrows;
@@ -69,6 +71,7 @@ template <int MODE>
 __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ sims, Work w, Parts p,
                                                        const unsigned* __restrict__ perm,
                                                        const unsigned* __restrict__ row_start, int* err) {
+  chain_begin();
   extern __shared__ uint4 acc_raw[];
   __shared__ unsigned s_begin[NSRC];
   __shared__ unsigned s_off[NSRC + 1];
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(KICK_NT, 4) k_kick(const Sim* __restrict__ sim
                                                   const unsigned* __restrict__ perm,
                                                   unsigned* __restrict__ keys_next, int* err,
                                                   unsigned* __restrict__ row_count) {
+  chain_begin();
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
     const int si = locate_sim(w, unit);
     const Sim& S = sims[si];
@@ -321,6 +325,7 @@ __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ p
                                                      unsigned* __restrict__ count, unsigned* __restrict__ keys,
                                                      unsigned* __restrict__ ranks, int* err,
                                                      float* __restrict__ copy) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long np = ord.np;
   float x[ORD_PPT], y[ORD_PPT], z[ORD_PPT];
@@ -362,6 +367,7 @@ __global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ 
                                                       const unsigned* __restrict__ row_start,
                                                       const unsigned* __restrict__ ranks, unsigned* __restrict__ place,
                                                       uint4* __restrict__ rec) {
+  chain_begin();
   const long long np = ord.np;
   Parts out{};
   out.rec = rec;
@@ -379,6 +385,7 @@ __global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ 
 // The force (gx, gy, gz) at every record, in row order, over the record's own word.  Two
 // particles per thread, as k_kick.
 __global__ void __launch_bounds__(KICK_NT, 4) k_force(const Sim* __restrict__ sims, uint4* __restrict__ rec) {
+  chain_begin();
   const Sim& S = sims[0];
   const long long units = (S.np + KICK_UNIT - 1) / KICK_UNIT;
   for (long long unit = blockIdx.x; unit < units; unit += gridDim.x) {
@@ -414,6 +421,7 @@ __global__ void __launch_bounds__(ORD_NT) k_advance(const Sim* __restrict__ sims
                                                     const uint4* __restrict__ force,
                                                     const unsigned* __restrict__ place, const float* pos,
                                                     const float* vel, float* pos_out, float* vel_out, int* err) {
+  chain_begin();
   const Sim& S = sims[0];
   const long long np = ord.np;
   const float kk = S.kick, dr = S.drift, fn = (float)S.n;
@@ -453,6 +461,7 @@ __global__ void __launch_bounds__(ORD_NT) k_advance(const Sim* __restrict__ sims
 // no staging of host memory, and the call can be captured) and zeroes `nzero` 16-byte words.
 __global__ void k_call_begin(Sim* __restrict__ dsim, CallWork* __restrict__ dwork, Sim sim, CallWork work,
                              uint4* __restrict__ zero, long long nzero) {
+  chain_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0) {
     *dsim = sim;
@@ -465,6 +474,7 @@ __global__ void k_call_begin(Sim* __restrict__ dsim, CallWork* __restrict__ dwor
 // coefficients (one thread per simulation, fp64)
 // ---------------------------------------------------------------------------------
 __global__ void k_coef(Sim* sims, int nsims, int advance) {
+  chain_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsims) return;
   Sim& S = sims[s];
@@ -488,6 +498,7 @@ __global__ void k_coef(Sim* sims, int nsims, int advance) {
 // ---------------------------------------------------------------------------------
 // row bin of the cell of every absolute position
 __global__ void k_row_keys_abs(const float* __restrict__ pos, long long np, int n, unsigned* __restrict__ keys) {
+  chain_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < np;
        i += (long long)gridDim.x * blockDim.x) {
     const Cell c = cell_abs(pos[i], pos[np + i], pos[2 * np + i], n);
@@ -499,6 +510,7 @@ __global__ void k_row_keys_abs(const float* __restrict__ pos, long long np, int 
 __global__ void k_abs_to_disp(const float* __restrict__ pos, const float* __restrict__ vel, long long np,
                               int np1, int n, const int* __restrict__ q_int, const float* __restrict__ q_frac,
                               Parts out, long long off, const unsigned* __restrict__ order) {
+  chain_begin();
   const float fn = (float)n, half = 0.5f * fn;
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < np;
        s += (long long)gridDim.x * blockDim.x) {
@@ -523,6 +535,7 @@ __global__ void k_abs_to_disp(const float* __restrict__ pos, const float* __rest
 __global__ void k_disp_to_abs(Parts in, long long off, long long np, int np1, int n,
                               const int* __restrict__ q_int, const float* __restrict__ q_frac,
                               float* __restrict__ pos, float* __restrict__ vel) {
+  chain_begin();
   const float fn = (float)n;
   for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < np;
        j += (long long)gridDim.x * blockDim.x) {
@@ -549,22 +562,22 @@ __global__ void k_disp_to_abs(Parts in, long long off, long long np, int np1, in
 // ---------------------------------------------------------------------------------
 cudaError_t launch_abs_to_disp(const float* pos, const float* vel, long long np, int np1, int n,
                                const int* q_int, const float* q_frac, Parts out, long long off,
-                               cudaStream_t st, const unsigned* order) {
+                               Launch st, const unsigned* order) {
   long long b = (np + 255) / 256;
   if (b > 152 * 32) b = 152 * 32;
   k_abs_to_disp<<<(int)b, 256, 0, st>>>(pos, vel, np, np1, n, q_int, q_frac, out, off, order);
   return cudaGetLastError();
 }
 
-cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned* keys, cudaStream_t st) {
+cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned* keys, Launch st) {
   long long b = (np + 255) / 256;
   if (b > 152 * 32) b = 152 * 32;
-  k_row_keys_abs<<<(int)(b > 0 ? b : 1), 256, 0, st>>>(pos, np, n, keys);
+  launch_chained(k_row_keys_abs, (int)(b > 0 ? b : 1), 256, 0, st, pos, np, n, keys);
   return cudaGetLastError();
 }
 
 cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, int n, const int* q_int,
-                               const float* q_frac, float* pos, float* vel, cudaStream_t st) {
+                               const float* q_frac, float* pos, float* vel, Launch st) {
   long long b = (np + 255) / 256;
   if (b > 152 * 32) b = 152 * 32;
   k_disp_to_abs<<<(int)b, 256, 0, st>>>(in, off, np, np1, n, q_int, q_frac, pos, vel);
@@ -587,22 +600,22 @@ cudaError_t deposit_prepare() {
 size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * sizeof(unsigned long long); }
 
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                            int* err, int ctas, cudaStream_t st) {
-  k_keys<POS_ABS><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err);
+                            int* err, int ctas, Launch st) {
+  launch_chained(k_keys<POS_ABS>, ctas, KEY_NT, 0, st, sims, w, p, keys, vals, err);
   return cudaGetLastError();
 }
 cudaError_t launch_keys_disp(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
-                             int* err, int ctas, cudaStream_t st) {
-  k_keys<POS_DISP><<<ctas, KEY_NT, 0, st>>>(sims, w, p, keys, vals, err);
+                             int* err, int ctas, Launch st) {
+  launch_chained(k_keys<POS_DISP>, ctas, KEY_NT, 0, st, sims, w, p, keys, vals, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsigned nrows,
-                             unsigned* row_start, cudaStream_t st) {
+                             unsigned* row_start, Launch st) {
   long long work = n + 1;
   int ctas = (int)((work + 255) / 256);
   if (ctas > 152 * 16) ctas = 152 * 16;
-  k_row_start<<<ctas, 256, 0, st>>>(keys, n, xbits, nrows, row_start);
+  launch_chained(k_row_start, ctas, 256, 0, st, keys, n, xbits, nrows, row_start);
   return cudaGetLastError();
 }
 
@@ -613,6 +626,7 @@ cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsig
 // tile's sums do not depend on when it runs).  counts[0], counts[1]: zero at launch.
 __global__ void k_tile_order(const Sim* __restrict__ sims, Work w, const unsigned* __restrict__ row_start,
                              unsigned* __restrict__ order, unsigned* __restrict__ counts) {
+  chain_begin();
   for (int unit = blockIdx.x * blockDim.x + threadIdx.x; unit < w.total; unit += gridDim.x * blockDim.x) {
     const int si = locate_sim(w, unit);
     const Sim& S = sims[si];
@@ -630,69 +644,66 @@ __global__ void k_tile_order(const Sim* __restrict__ sims, Work w, const unsigne
 }
 
 cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* row_start, unsigned* order,
-                              unsigned* counts, int sms, cudaStream_t st) {
+                              unsigned* counts, int sms, Launch st) {
   if (w.total <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned), st);
-  if (e) return e;
   const int ctas = std::min((w.total + 255) / 256, 4 * sms);
-  k_tile_order<<<ctas, 256, 0, st>>>(sims, w, row_start, order, counts);
+  launch_chained(k_tile_order, ctas, 256, 0, st, sims, w, row_start, order, counts);
   return cudaGetLastError();
 }
 
 cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsigned* perm,
                            const unsigned* row_start, int mode, int* err, int ctas, size_t smem,
-                           cudaStream_t st) {
+                           Launch st) {
   if (cudaError_t e = deposit_prepare()) return e;
-  if (mode == POS_ABS) k_deposit<POS_ABS><<<ctas, DEP_NT, smem, st>>>(sims, w, p, perm, row_start, err);
-  else k_deposit<POS_DISP><<<ctas, DEP_NT, smem, st>>>(sims, w, p, perm, row_start, err);
+  if (mode == POS_ABS) launch_chained(k_deposit<POS_ABS>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, err);
+  else launch_chained(k_deposit<POS_DISP>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, const unsigned* perm,
-                        unsigned* keys_next, int* err, int ctas, cudaStream_t st, unsigned* row_count) {
+                        unsigned* keys_next, int* err, int ctas, Launch st, unsigned* row_count) {
   k_kick<<<ctas, KICK_NT, 0, st>>>(sims, w, in, out, perm, keys_next, err, row_count);
   return cudaGetLastError();
 }
 
 cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
-                              size_t zero_bytes, cudaStream_t st) {
+                              size_t zero_bytes, Launch st) {
   const long long nz = (long long)(zero_bytes / sizeof(uint4));
   const long long want = (nz + 1023) / 1024;  // four words per thread
-  k_call_begin<<<(int)(want < 1 ? 1 : (want > 1024 ? 1024 : want)), 256, 0, st>>>(dsim, dwork, sim, work,
-                                                                                 static_cast<uint4*>(zero), nz);
+  launch_chained(k_call_begin, (int)(want < 1 ? 1 : (want > 1024 ? 1024 : want)), 256, 0, st, dsim, dwork, sim, work, static_cast<uint4*>(zero), nz);
   return cudaGetLastError();
 }
 
 cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
-                            unsigned* ranks, int* err, float* copy, cudaStream_t st) {
+                            unsigned* ranks, int* err, float* copy, Launch st) {
   const ParticleOrder o(np, 0);
-  k_row_rank<<<(int)o.blocks(), ORD_NT, 0, st>>>(pos, o, n, count, keys, ranks, err, copy);
+  launch_chained(k_row_rank, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, count, keys, ranks, err, copy);
   return cudaGetLastError();
 }
 
 cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
-                             const unsigned* ranks, unsigned* place, uint4* rec, cudaStream_t st) {
+                             const unsigned* ranks, unsigned* place, uint4* rec, Launch st) {
   const ParticleOrder o(np, np1);
-  k_row_place<<<(int)o.blocks(), ORD_NT, 0, st>>>(pos, o, n, row_start, ranks, place, rec);
+  launch_chained(k_row_place, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, row_start, ranks, place, rec);
   return cudaGetLastError();
 }
 
-cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, cudaStream_t st) {
+cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, Launch st) {
   const long long units = (np + KICK_UNIT - 1) / KICK_UNIT, cap = (long long)sms * 16;
-  k_force<<<(int)(units < cap ? units : cap), KICK_NT, 0, st>>>(sims, rec);
+  launch_chained(k_force, (int)(units < cap ? units : cap), KICK_NT, 0, st, sims, rec);
   return cudaGetLastError();
 }
 
 cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
                            const float* pos, const float* vel, float* pos_out, float* vel_out, int* err,
-                           cudaStream_t st) {
+                           Launch st) {
   const ParticleOrder o(np, 0);
-  k_advance<<<(int)o.blocks(), ORD_NT, 0, st>>>(sims, o, force, place, pos, vel, pos_out, vel_out, err);
+  launch_chained(k_advance, (int)o.blocks(), ORD_NT, 0, st, sims, o, force, place, pos, vel, pos_out, vel_out, err);
   return cudaGetLastError();
 }
 
-cudaError_t launch_coef(Sim* sims, int nsims, int advance, cudaStream_t st) {
-  k_coef<<<(nsims + 127) / 128, 128, 0, st>>>(sims, nsims, advance);
+cudaError_t launch_coef(Sim* sims, int nsims, int advance, Launch st) {
+  launch_chained(k_coef, (nsims + 127) / 128, 128, 0, st, sims, nsims, advance);
   return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@ constexpr int DPT = MAX_RADIX / SORT_NT;  // digits per thread in per-digit loop
 __global__ void __launch_bounds__(SORT_NT) k_sort_upsweep(const unsigned* __restrict__ keys, long long n,
                                                           int shift, int dbits, unsigned* __restrict__ hist,
                                                           int nblocks) {
+  chain_begin();
   __shared__ unsigned h[SORT_WARPS][MAX_RADIX];
   const int warp = threadIdx.x >> 5;
   const unsigned mask = (1u << dbits) - 1u, radix = 1u << dbits;
@@ -80,6 +81,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* w
 
 __global__ void __launch_bounds__(SORT_SCAN_NT) k_sort_scan(unsigned* __restrict__ hist, int nblocks,
                                                             unsigned* __restrict__ digit_tot) {
+  chain_begin();
   __shared__ unsigned ws[32];
   unsigned* row = hist + (long long)blockIdx.x * nblocks;
   unsigned carry = 0;
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(SORT_NT) k_sort_downsweep(const unsigned* __re
                                                             const unsigned* __restrict__ hist,
                                                             const unsigned* __restrict__ digit_tot,
                                                             int nblocks, int gen_vals) {
+  chain_begin();
   extern __shared__ uint4 down_raw[];
   DownSmem& sm = *reinterpret_cast<DownSmem*>(down_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -224,7 +227,7 @@ cudaError_t sort_prepare() {
 int radix_sort_passes(int bits) { return bits <= 0 ? 1 : (bits + MAX_DIGIT_BITS - 1) / MAX_DIGIT_BITS; }
 
 cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bit, int bits, bool gen_vals,
-                       const SortScratch& s, bool* in_alt, cudaStream_t st) {
+                       const SortScratch& s, bool* in_alt, Launch st) {
   *in_alt = false;
   if (n <= 0) return cudaSuccess;
   if (n > s.capacity || n >= (1ll << 32)) return cudaErrorInvalidValue;
@@ -236,11 +239,9 @@ cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bi
   unsigned *ki = keys, *vi = vals, *ko = s.keys_alt, *vo = s.vals_alt;
   for (int p = 0; p < passes; ++p) {
     const int shift = begin_bit + dbits * p;
-    k_sort_upsweep<<<nblocks, SORT_NT, 0, st>>>(ki, n, shift, dbits, s.hist, nblocks);
-    k_sort_scan<<<1 << dbits, SORT_SCAN_NT, 0, st>>>(s.hist, nblocks, s.digit_tot);
-    k_sort_downsweep<<<nblocks, SORT_NT, sizeof(DownSmem), st>>>(ki, vi, ko, vo, n, shift, dbits, s.hist,
-                                                                 s.digit_tot, nblocks,
-                                                                 (p == 0 && gen_vals) ? 1 : 0);
+    launch_chained(k_sort_upsweep, nblocks, SORT_NT, 0, st, ki, n, shift, dbits, s.hist, nblocks);
+    launch_chained(k_sort_scan, 1 << dbits, SORT_SCAN_NT, 0, st, s.hist, nblocks, s.digit_tot);
+    launch_chained(k_sort_downsweep, nblocks, SORT_NT, sizeof(DownSmem), st, ki, vi, ko, vo, n, shift, dbits, s.hist, s.digit_tot, nblocks, (p == 0 && gen_vals) ? 1 : 0);
     cudaError_t e = cudaGetLastError();
     if (e) return e;
     unsigned* t = ki; ki = ko; ko = t;
@@ -273,6 +274,7 @@ constexpr int CS_UNR = 4;
 
 __global__ void __launch_bounds__(CS_NT) k_row_hist(const unsigned* __restrict__ keys, long long n, unsigned nrows,
                                                     unsigned* __restrict__ count, int* err) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)gridDim.x * CS_NT * CS_UNR;
   for (long long b = ((long long)blockIdx.x * CS_NT + (threadIdx.x & ~31)) * CS_UNR; b < n; b += stride) {
@@ -310,6 +312,7 @@ __device__ __forceinline__ void store4(unsigned* __restrict__ v, long long i, lo
 // per-block sums of SCAN_TILE entries
 __global__ void __launch_bounds__(CS_NT) k_scan_reduce(const unsigned* __restrict__ in, long long n,
                                                        unsigned* __restrict__ block_sums) {
+  chain_begin();
   __shared__ unsigned ws[CS_NT / 32];
   const long long base = (long long)blockIdx.x * SCAN_TILE;
   unsigned s = 0;
@@ -325,6 +328,7 @@ __global__ void __launch_bounds__(CS_NT) k_scan_reduce(const unsigned* __restric
 
 // exclusive scan of the block sums in place (one block, chunks of CS_NT with a carry)
 __global__ void __launch_bounds__(CS_NT) k_scan_top(unsigned* __restrict__ block_sums, int nblocks) {
+  chain_begin();
   __shared__ unsigned ws[CS_NT / 32];
   unsigned carry = 0;
   for (int c = 0; c < nblocks; c += CS_NT) {
@@ -346,6 +350,7 @@ __global__ void __launch_bounds__(CS_NT) k_scan_top(unsigned* __restrict__ block
 __global__ void __launch_bounds__(CS_NT) k_scan_apply(unsigned* __restrict__ in, long long n,
                                                       const unsigned* __restrict__ block_sums, int scanned, int zero,
                                                       unsigned* __restrict__ out, unsigned* __restrict__ cursor) {
+  chain_begin();
   __shared__ unsigned ws[CS_NT / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long base = (long long)blockIdx.x * SCAN_TILE + warp * (SCAN_TILE / (CS_NT / 32)) + lane * 4;
@@ -399,7 +404,11 @@ __global__ void __launch_bounds__(CS_NT) k_scan_apply(unsigned* __restrict__ in,
 constexpr int SCATTER_CHUNK = 1024;
 
 __global__ void __launch_bounds__(CS_NT) k_row_scatter(const unsigned* __restrict__ keys, long long n, unsigned nrows,
-                                                       unsigned* __restrict__ cursor, unsigned* __restrict__ perm) {
+                                                       unsigned* __restrict__ cursor, unsigned* __restrict__ perm,
+                                                       unsigned* __restrict__ clear, int nclear) {
+  chain_begin();
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < nclear; i += CS_NT) clear[i] = 0u;
   const int lane = threadIdx.x & 31;
   const long long nchunks = (n + SCATTER_CHUNK - 1) / SCATTER_CHUNK;
   const long long nwarps = (long long)gridDim.x * (CS_NT / 32);
@@ -439,32 +448,32 @@ __global__ void __launch_bounds__(CS_NT) k_row_scatter(const unsigned* __restric
 size_t row_sort_block_sums(unsigned nrows) { return ((size_t)nrows + SCAN_TILE - 1) / SCAN_TILE; }
 
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
-                          cudaStream_t st) {
+                          Launch st) {
   if (nrows == 0) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(count, 0, (size_t)nrows * sizeof(unsigned), st);
   if (e) return e;
   long long want = (n + CS_NT * CS_UNR - 1) / (CS_NT * CS_UNR);
   const int ctas = (int)(want < (long long)sms * 8 ? (want > 0 ? want : 1) : (long long)sms * 8);
-  k_row_hist<<<ctas, CS_NT, 0, st>>>(keys, n, nrows, count, err);
+  launch_chained(k_row_hist, ctas, CS_NT, 0, st, keys, n, nrows, count, err);
   return cudaGetLastError();
 }
 
 cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
-                     bool zero, cudaStream_t st) {
+                     bool zero, Launch st) {
   if (nrows == 0) return cudaErrorInvalidValue;
   const int nb = (int)row_sort_block_sums(nrows);
   // from 8192 blocks on (33 M bins) adding up the earlier blocks' sums in every block costs more
   // than a scan of the sums
   const bool scanned = nb > 8192;
-  if (nb > 1) k_scan_reduce<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums);
-  if (scanned) k_scan_top<<<1, CS_NT, 0, st>>>(block_sums, nb);
-  k_scan_apply<<<nb, CS_NT, 0, st>>>(count, nrows, block_sums, scanned, zero, row_start, cursor);
+  if (nb > 1) launch_chained(k_scan_reduce, nb, CS_NT, 0, st, count, nrows, block_sums);
+  if (scanned) launch_chained(k_scan_top, 1, CS_NT, 0, st, block_sums, nb);
+  launch_chained(k_scan_apply, nb, CS_NT, 0, st, count, nrows, block_sums, scanned, zero, row_start, cursor);
   return cudaGetLastError();
 }
 
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
-                              int sms, cudaStream_t st, bool counted, bool zero) {
+                              int sms, Launch st, bool counted, bool zero, unsigned* clear, int nclear) {
   if (!counted) {
     cudaError_t e = row_histogram(keys, n, nrows, count, err, sms, st);
     if (e) return e;
@@ -472,8 +481,7 @@ cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows,
   if (cudaError_t e = row_scan(count, nrows, row_start, cursor, block_sums, zero, st)) return e;
   const long long chunks = (n + SCATTER_CHUNK - 1) / SCATTER_CHUNK;
   const long long sblocks = (chunks + CS_NT / 32 - 1) / (CS_NT / 32);
-  k_row_scatter<<<(int)(sblocks < (long long)sms * 8 ? (sblocks > 0 ? sblocks : 1) : (long long)sms * 8), CS_NT, 0,
-                  st>>>(keys, n, nrows, cursor, perm);
+  launch_chained(k_row_scatter, (int)(sblocks < (long long)sms * 8 ? (sblocks > 0 ? sblocks : 1) : (long long)sms * 8), CS_NT, 0, st, keys, n, nrows, cursor, perm, clear, nclear);
   return cudaGetLastError();
 }
 

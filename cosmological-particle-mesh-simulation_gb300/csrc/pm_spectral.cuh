@@ -151,6 +151,7 @@ __device__ __forceinline__ void x_r2c_body(const Sim& S, int unit, float2* s) {
 
 template <int N>
 __global__ void __launch_bounds__(SP_NT) k_x_r2c(const Sim* __restrict__ sims, Work w) {
+  chain_begin();
   extern __shared__ float4 smem_f4[];
   float2* s = reinterpret_cast<float2*>(smem_f4);
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
@@ -214,6 +215,7 @@ __device__ __forceinline__ void x_c2r_body(const Sim& S, int unit, float2* s) {
 
 template <int N>
 __global__ void __launch_bounds__(SP_NT) k_x_c2r(const Sim* __restrict__ sims, Work w) {
+  chain_begin();
   extern __shared__ float4 smem_f4[];
   float2* s = reinterpret_cast<float2*>(smem_f4);
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
@@ -303,6 +305,7 @@ __device__ __forceinline__ void line_body(const Sim& S, int unit, float2* s) {
 
 template <int N, bool ZAXIS, bool INV>
 __global__ void __launch_bounds__(SP_NT) k_line_pass(const Sim* __restrict__ sims, Work w) {
+  chain_begin();
   extern __shared__ float4 smem_f4[];
   float2* s = reinterpret_cast<float2*>(smem_f4);
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
@@ -354,6 +357,7 @@ __device__ __forceinline__ void z_body(const Sim& S, int unit, float2* s) {
 
 template <int N, bool TABLE, bool GRAD = false>
 __global__ void __launch_bounds__(SP_NT) k_z_green(const Sim* __restrict__ sims, Work w) {
+  chain_begin();
   extern __shared__ float4 smem_f4[];
   float2* s = reinterpret_cast<float2*>(smem_f4);
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
@@ -422,6 +426,7 @@ __global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(co
     fence_mbar_init();
   }
   __syncthreads();
+  chain_begin();
   auto stage_ptr = [&](int st) { return stg0 + (size_t)st * (STAGE / sizeof(float2)); };
   // unit -> (simulation, first bundle, bundles in the unit)
   auto unit_info = [&](int unit, int& si, int& b0, int& cnt) {
@@ -561,6 +566,7 @@ __device__ __forceinline__ void xrow_untangle_store(const float2 (&o)[xrow_P(N) 
 
 template <int N, bool C2R>
 __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ sims, Work w) {
+  chain_begin();
   constexpr int XR_NT = xrow_nt(N);
   constexpr int M = N / 2, P = xrow_P(N), Q = xrow_Q(N), T = xrow_T(N), RPW = 32 / T;
   constexpr int RB = Q * (P + 1);  // exchange buffer of a row (>= M + 1)
@@ -674,6 +680,7 @@ __global__ void __launch_bounds__(XTMA_NT, 1) k_x_tma(const Sim* __restrict__ si
     fence_mbar_init();
   }
   __syncthreads();
+  chain_begin();
   // warp 0 issues the copies of one unit: lane r copies rows r, r + 32, ...
   auto issue = [&](int unit, int st) {
     const int si = locate_sim(w, unit);
@@ -812,8 +819,8 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
   // leaves the CTAs that drew the dense tiles running alone at the end.
   // `order` (optional) lists the tiles dense-first; idx is the place in it.
   __shared__ int s_next;
-  auto take_next = [&](int idx) -> int {
-    return next_tile ? (int)gridDim.x * TPB + (int)atomicAdd(next_tile, (unsigned)TPB) : idx + (int)gridDim.x * TPB;
+  auto take_next = [&]() -> int {
+    return (int)gridDim.x * TPB + (int)atomicAdd(next_tile, (unsigned)TPB);
   };
   auto tile_at = [&](int idx) -> int { return order ? (int)__ldg(&order[idx]) : idx; };
   // the tile at place i of the order: its simulation and first row / plane (false: none)
@@ -840,16 +847,17 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
       if (tile_of(idx + (lane >> 3), si, y0, z0)) v = run_load(sims[si], row_start, y0, z0, lane & 7);
       return v;
     };
+    // The accumulators start zero, and each row is zeroed again by its transform lanes once
+    // they are done with it, so a tile needs no zeroing phase and barrier of its own
+    // (0.468 -> 0.460 ms early, 0.604 -> 0.587 ms at step 980, 256^3 on 512^3).
+    for (int i = threadIdx.x; i < TPB * NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
+    chain_begin();
     int idx = blockIdx.x * TPB;
     if (warp == 0 && idx < w.total) {
       const RunLoad v = load_tables(idx);
       const int tj = lane < TPB * 8 ? lane >> 3 : 0;
       run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
     }
-    // The accumulators start zero, and each row is zeroed again by its transform lanes once
-    // they are done with it, so a tile needs no zeroing phase and barrier of its own
-    // (0.468 -> 0.460 ms early, 0.604 -> 0.587 ms at step 980, 256^3 on 512^3).
-    for (int i = threadIdx.x; i < TPB * NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     while (idx < w.total) {
       {  // the particles of this group's tile (a group without a tile has an empty table)
@@ -884,7 +892,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
         // transform, so that the loads' latency hides behind it (the tables are free: the
         // particle loops are over, and the transform reads s_ts)
         int next = 0;
-        if (warp == 0) next = __shfl_sync(FULL, lane == 0 ? take_next(idx) : 0, 0);
+        if (warp == 0) next = __shfl_sync(FULL, lane == 0 ? take_next() : 0, 0);
         RunLoad nl{0u, 0u};
         if (warp == 0 && next < w.total) nl = load_tables(next);
         xrow_transform<N, false>(v2, o2, rb, t, S.tw);
@@ -912,6 +920,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
     }
     return;
   } else {
+    chain_begin();
     bool runs_ready = false;
     for (int idx = blockIdx.x; idx < w.total;) {
       int si, y0, z0;
@@ -946,7 +955,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
         const float2 o = cscale(mul_mi<false>(csub(zk, zc)), 0.5f);
         dst[row * P + k] = cadd(e, cmul(__ldg(&S.tw[k]), o));
       }
-      if (threadIdx.x == 0) s_next = take_next(idx);
+      if (threadIdx.x == 0) s_next = take_next();
       __syncthreads();
       idx = s_next;
     }
@@ -955,7 +964,7 @@ __global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
 
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
-                               int* err, unsigned* next_tile, const unsigned* order, int ctas, cudaStream_t st) {
+                               int* err, unsigned* next_tile, const unsigned* order, int ctas, Launch st) {
   if constexpr (!deposit_r2c_ok(N)) {
     return cudaErrorNotSupported;
   } else {
@@ -971,11 +980,7 @@ cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned*
   constexpr int NT = deposit_r2c_nt(N), TPB = dep_tiles(N);
   if (ctas > (w.total + TPB - 1) / TPB) ctas = (w.total + TPB - 1) / TPB;  // TPB tiles per CTA
   if (ctas <= 0) return cudaSuccess;
-  if (next_tile) {
-    const cudaError_t e = cudaMemsetAsync(next_tile, 0, sizeof(unsigned), st);
-    if (e) return e;
-  }
-  k_deposit_r2c<N><<<ctas, NT, sm, st>>>(sims, w, p, perm, row_start, err, next_tile, order);
+  launch_chained(k_deposit_r2c<N>, ctas, NT, sm, st, sims, w, p, perm, row_start, err, next_tile, order);
   return cudaGetLastError();
   }
 }
@@ -988,7 +993,7 @@ static cudaError_t max_shared(K kern, size_t bytes) {
 }
 
 template <int N>
-cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, cudaStream_t st,
+cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, Launch st,
                             const CUtensorMap* maps, int* err) {
   static DeviceOnce once;
   const size_t xs = x_smem_bytes(N), ls = line_smem_bytes(N);
@@ -1027,15 +1032,15 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, cu
       // ctas: the cap on the CTAs of the persistent row transform (the batch engine tunes it)
       const int per = xrow_nt(N) / 32, want = (w.total + per - 1) / per, cap = ctas > 0 ? ctas : device_sms() * 8;
       const int g = want < cap ? want : cap;
-      if (kind == SPEC_X_R2C) k_x_row<N, false><<<g, xrow_nt(N), 0, st>>>(sims, w);
-      else k_x_row<N, true><<<g, xrow_nt(N), 0, st>>>(sims, w);
+      if (kind == SPEC_X_R2C) launch_chained(k_x_row<N, false>, g, xrow_nt(N), 0, st, sims, w);
+      else launch_chained(k_x_row<N, true>, g, xrow_nt(N), 0, st, sims, w);
       return cudaGetLastError();
     }
   }
   if constexpr (tma_rows(N)) {
     if (kind == SPEC_X_R2C || kind == SPEC_X_C2R) {
-      if (kind == SPEC_X_R2C) k_x_tma<N, false><<<grid, XTMA_NT, xtma_smem_bytes(N), st>>>(sims, w, err);
-      else k_x_tma<N, true><<<grid, XTMA_NT, xtma_smem_bytes(N), st>>>(sims, w, err);
+      if (kind == SPEC_X_R2C) launch_chained(k_x_tma<N, false>, grid, XTMA_NT, xtma_smem_bytes(N), st, sims, w, err);
+      else launch_chained(k_x_tma<N, true>, grid, XTMA_NT, xtma_smem_bytes(N), st, sims, w, err);
       return cudaGetLastError();
     }
   }
@@ -1045,27 +1050,27 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, cu
       const int lcap = line_ctas_per_sm(N) * device_sms();
       const int grid = w.total < lcap ? w.total : lcap;
       switch (kind) {
-        case SPEC_Y_FWD: k_line_tma<N, 0><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Y_INV: k_line_tma<N, 1><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_GREEN: k_line_tma<N, 2><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_TABLE: k_line_tma<N, 3><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_FWD: k_line_tma<N, 4><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_INV: k_line_tma<N, 5><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_GRAD: k_line_tma<N, 6><<<grid, line_nt(N), sm, st>>>(maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Y_FWD: launch_chained(k_line_tma<N, 0>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Y_INV: launch_chained(k_line_tma<N, 1>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_GREEN: launch_chained(k_line_tma<N, 2>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_TABLE: launch_chained(k_line_tma<N, 3>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_FWD: launch_chained(k_line_tma<N, 4>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_INV: launch_chained(k_line_tma<N, 5>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_GRAD: launch_chained(k_line_tma<N, 6>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
         default: break;
       }
     }
   }
   switch (kind) {
-    case SPEC_X_R2C: k_x_r2c<N><<<ctas, SP_NT, xs, st>>>(sims, w); break;
-    case SPEC_X_C2R: k_x_c2r<N><<<ctas, SP_NT, xs, st>>>(sims, w); break;
-    case SPEC_Y_FWD: k_line_pass<N, false, false><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Y_INV: k_line_pass<N, false, true><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Z_FWD: k_line_pass<N, true, false><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Z_INV: k_line_pass<N, true, true><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Z_GREEN: k_z_green<N, false><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Z_TABLE: k_z_green<N, true><<<ctas, SP_NT, ls, st>>>(sims, w); break;
-    case SPEC_Z_GRAD: k_z_green<N, false, true><<<ctas, SP_NT, ls, st>>>(sims, w); break;
+    case SPEC_X_R2C: launch_chained(k_x_r2c<N>, ctas, SP_NT, xs, st, sims, w); break;
+    case SPEC_X_C2R: launch_chained(k_x_c2r<N>, ctas, SP_NT, xs, st, sims, w); break;
+    case SPEC_Y_FWD: launch_chained(k_line_pass<N, false, false>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Y_INV: launch_chained(k_line_pass<N, false, true>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Z_FWD: launch_chained(k_line_pass<N, true, false>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Z_INV: launch_chained(k_line_pass<N, true, true>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Z_GREEN: launch_chained(k_z_green<N, false>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Z_TABLE: launch_chained(k_z_green<N, true>, ctas, SP_NT, ls, st, sims, w); break;
+    case SPEC_Z_GRAD: launch_chained(k_z_green<N, false, true>, ctas, SP_NT, ls, st, sims, w); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

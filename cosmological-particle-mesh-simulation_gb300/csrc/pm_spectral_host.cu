@@ -6,18 +6,18 @@ namespace pm {
 
 #define PM_FOR_EACH_N(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024)
 
-#define PM_EXTERN(NN) extern template cudaError_t spectral_launch<NN>(SpecKind, const Sim*, Work, int, cudaStream_t, const CUtensorMap*, int*);
+#define PM_EXTERN(NN) extern template cudaError_t spectral_launch<NN>(SpecKind, const Sim*, Work, int, Launch, const CUtensorMap*, int*);
 PM_FOR_EACH_N(PM_EXTERN)
 #undef PM_EXTERN
 #define PM_EXTERN(NN)                                                                                         \
   extern template cudaError_t deposit_r2c_launch<NN>(const Sim*, Work, Parts, const unsigned*, const unsigned*, \
-                                                     int*, unsigned*, const unsigned*, int, cudaStream_t);
+                                                     int*, unsigned*, const unsigned*, int, Launch);
 PM_FOR_EACH_N(PM_EXTERN)
 #undef PM_EXTERN
 
 cudaError_t deposit_r2c_dispatch(int n, const Sim* sims, Work w, Parts p, const unsigned* perm,
                                  const unsigned* row_start, int* err, unsigned* next_tile,
-                                 const unsigned* order, int ctas, cudaStream_t st) {
+                                 const unsigned* order, int ctas, Launch st) {
   switch (n) {
 #define PM_CASE(NN) \
   case NN: return deposit_r2c_launch<NN>(sims, w, p, perm, row_start, err, next_tile, order, ctas, st);
@@ -63,7 +63,7 @@ int spectral_ctas_per_sm(SpecKind kind, int n) {
   return by_smem > 4 ? 4 : by_smem;
 }
 
-cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, cudaStream_t st,
+cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, Launch st,
                               const CUtensorMap* maps, int* err) {
   switch (n) {
 #define PM_CASE(NN) case NN: return spectral_launch<NN>(kind, sims, w, ctas, st, maps, err);
@@ -74,6 +74,7 @@ cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int
 }
 
 __global__ void k_fourier_grid(const Sim* __restrict__ sims) {
+  chain_begin();
   const Sim& S = sims[0];
   const long long n = S.n, total = n * n * n;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -84,8 +85,8 @@ __global__ void k_fourier_grid(const Sim* __restrict__ sims) {
   }
 }
 
-cudaError_t launch_fourier_grid(const Sim* sims, int ctas, cudaStream_t st) {
-  k_fourier_grid<<<ctas, 256, 0, st>>>(sims);
+cudaError_t launch_fourier_grid(const Sim* sims, int ctas, Launch st) {
+  launch_chained(k_fourier_grid, ctas, 256, 0, st, sims);
   return cudaGetLastError();
 }
 
