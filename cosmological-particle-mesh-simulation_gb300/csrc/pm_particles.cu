@@ -506,55 +506,91 @@ __global__ void k_row_keys_abs(const float* __restrict__ pos, long long np, int 
   }
 }
 
-// order (optional): slot off + i takes particle order[i] (the state is written in row order)
-__global__ void k_abs_to_disp(const float* __restrict__ pos, const float* __restrict__ vel, long long np,
+// Both conversions cross between particle order and row order, one float at a time and one array
+// after another (blockIdx.y: x y z vx vy vz, so that the blocks of one array run together): the
+// lines of one array that are being filled or read then stay in L2, where those of six at once do
+// not.  The slots are taken in chunks of one deposit tile's mean particle count, all z of one y
+// before the next y (row order has y before z): the particles in flight then cover whole lines
+// of the lattice (z is the fastest particle index).  For a clustered state the chunks only
+// roughly follow the tiles; every order gives the same result.  256^3 / 512^3 particles: to
+// displacements 1.12 / 14.1 ms (all arrays at once, slot order) -> 0.44 / 9.0, back 2.79 / 28.8 ->
+// 0.82 / 16.1; without the chunks 0.52 / 11.1 and 0.81 / 19.5.  Bound by the rate of 32-byte sectors
+// in L2, one per float (123 G/s at 256^3).
+struct ChunkOrder {
+  long long np;
+  int side;  // tiles per axis
+  unsigned size;
+  __host__ ChunkOrder(long long p, int n) : np(p), side(n / TY) {
+    size = (unsigned)((p + (long long)side * side - 1) / ((long long)side * side));
+  }
+  // f(s) for every slot s < np of this block's chunks
+  template <class F>
+  __device__ __forceinline__ void each(F f) const {
+    for (int c = blockIdx.x; c < side * side; c += gridDim.x) {
+      const long long s0 = (long long)(c % side * side + c / side) * size;
+      for (unsigned j = threadIdx.x; j < size && s0 + j < np; j += blockDim.x) f(s0 + j);
+    }
+  }
+};
+
+// slot off + s takes particle order[s]
+__global__ void k_abs_to_disp(const float* __restrict__ pos, const float* __restrict__ vel, ChunkOrder chunks,
                               int np1, int n, const int* __restrict__ q_int, const float* __restrict__ q_frac,
                               Parts out, long long off, const unsigned* __restrict__ order) {
   chain_begin();
+  const long long np = chunks.np;
   const float fn = (float)n, half = 0.5f * fn;
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < np;
-       s += (long long)gridDim.x * blockDim.x) {
-    const long long i = order ? (long long)__ldg(&order[s]) : s;  // the particle
-    const unsigned id = (unsigned)i, u1 = (unsigned)np1;
-    const unsigned ax[3] = {id / (u1 * u1), (id / u1) % u1, id % u1};
-    float* dst[3] = {out.x, out.y, out.z};
-    float* vdst[3] = {out.vx, out.vy, out.vz};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float q = (float)__ldg(&q_int[ax[k]]) + __ldg(&q_frac[ax[k]]);
-      float d = pos[k * np + i] - q;
-      if (d >= half) d -= fn;
-      if (d < -half) d += fn;
-      dst[k][off + s] = d;
-      vdst[k][off + s] = vel[k * np + i];
+  const unsigned u1 = (unsigned)np1;
+  const int k = blockIdx.y % 3;
+  const bool is_vel = blockIdx.y >= 3;
+  const float* __restrict__ src = (is_vel ? vel : pos) + k * np;
+  float* __restrict__ dst = (is_vel ? (k == 0 ? out.vx : (k == 1 ? out.vy : out.vz))
+                                    : (k == 0 ? out.x : (k == 1 ? out.y : out.z))) + off;
+  chunks.each([&](long long s) {
+    const unsigned i = __ldg(&order[s]);  // the particle
+    const float v = src[i];
+    if (is_vel) {
+      dst[s] = v;
+      return;
     }
-    out.id[off + s] = pack_lattice(ax[0], ax[1], ax[2]);
-  }
+    const unsigned iz = i % u1, t = i / u1, iy = t % u1, ix = t / u1;
+    const unsigned l = k == 0 ? ix : (k == 1 ? iy : iz);
+    const float q = (float)__ldg(&q_int[l]) + __ldg(&q_frac[l]);
+    float d = v - q;
+    if (d >= half) d -= fn;
+    if (d < -half) d += fn;
+    dst[s] = d;
+    if (k == 0) out.id[off + s] = pack_lattice(ix, iy, iz);
+  });
 }
 
-__global__ void k_disp_to_abs(Parts in, long long off, long long np, int np1, int n,
+__global__ void k_disp_to_abs(Parts in, long long off, ChunkOrder chunks, int np1, int n,
                               const int* __restrict__ q_int, const float* __restrict__ q_frac,
                               float* __restrict__ pos, float* __restrict__ vel) {
   chain_begin();
+  const long long np = chunks.np;
   const float fn = (float)n;
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < np;
-       j += (long long)gridDim.x * blockDim.x) {
-    const long long slot = off + j;
-    const unsigned pid = in.id[slot];
+  const int k = blockIdx.y % 3;
+  const bool is_vel = blockIdx.y >= 3;
+  const float* __restrict__ src = (is_vel ? (k == 0 ? in.vx : (k == 1 ? in.vy : in.vz))
+                                          : (k == 0 ? in.x : (k == 1 ? in.y : in.z))) + off;
+  const unsigned* __restrict__ ids = in.id + off;
+  float* __restrict__ dst = (is_vel ? vel : pos) + k * np;
+  chunks.each([&](long long j) {
+    const unsigned pid = __ldg(&ids[j]);
     const unsigned ax[3] = {pid >> 20, (pid >> 10) & 1023u, pid & 1023u};
     const long long id = ((long long)ax[0] * np1 + ax[1]) * np1 + ax[2];
-    const float dv[3] = {in.x[slot], in.y[slot], in.z[slot]};
-    const float vv[3] = {in.vx[slot], in.vy[slot], in.vz[slot]};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float s = __ldg(&q_frac[ax[k]]) + dv[k];
+    float v = __ldg(&src[j]);
+    if (!is_vel) {
+      const unsigned l = k == 0 ? ax[0] : (k == 1 ? ax[1] : ax[2]);
+      const float s = __ldg(&q_frac[l]) + v;
       const float fl = floorf(s);
-      float x = (float)wrap_int(__ldg(&q_int[ax[k]]) + (int)fl, n) + (s - fl);
+      float x = (float)wrap_int(__ldg(&q_int[l]) + (int)fl, n) + (s - fl);
       if (x >= fn) x -= fn;
-      pos[k * np + id] = x;
-      vel[k * np + id] = vv[k];
+      v = x;
     }
-  }
+    dst[id] = v;
+  });
 }
 
 // ---------------------------------------------------------------------------------
@@ -563,9 +599,9 @@ __global__ void k_disp_to_abs(Parts in, long long off, long long np, int np1, in
 cudaError_t launch_abs_to_disp(const float* pos, const float* vel, long long np, int np1, int n,
                                const int* q_int, const float* q_frac, Parts out, long long off,
                                Launch st, const unsigned* order) {
-  long long b = (np + 255) / 256;
-  if (b > 152 * 32) b = 152 * 32;
-  k_abs_to_disp<<<(int)b, 256, 0, st>>>(pos, vel, np, np1, n, q_int, q_frac, out, off, order);
+  const ChunkOrder c(np, n);
+  const int b = c.side * c.side < 152 * 16 ? c.side * c.side : 152 * 16;
+  k_abs_to_disp<<<dim3((unsigned)b, 6), 256, 0, st>>>(pos, vel, c, np1, n, q_int, q_frac, out, off, order);
   return cudaGetLastError();
 }
 
@@ -578,9 +614,9 @@ cudaError_t launch_row_keys_abs(const float* pos, long long np, int n, unsigned*
 
 cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, int n, const int* q_int,
                                const float* q_frac, float* pos, float* vel, Launch st) {
-  long long b = (np + 255) / 256;
-  if (b > 152 * 32) b = 152 * 32;
-  k_disp_to_abs<<<(int)b, 256, 0, st>>>(in, off, np, np1, n, q_int, q_frac, pos, vel);
+  const ChunkOrder c(np, n);
+  const int b = c.side * c.side < 152 * 16 ? c.side * c.side : 152 * 16;
+  k_disp_to_abs<<<dim3((unsigned)b, 6), 256, 0, st>>>(in, off, c, np1, n, q_int, q_frac, pos, vel);
   return cudaGetLastError();
 }
 
