@@ -15,12 +15,20 @@
 //     transform of a non-Hermitian rho_k is the inverse real transform of its Hermitian
 //     part (rho_k[k] + conj(rho_k[-k])) / 2, which is built directly in the half spectrum;
 //   * fftn of that field, the potential -rho_k / |l|^2 (k = 0 -> 0), -i l_d pot_k * res,
-//     and Re(ifftn(.)) * force_resolution per direction (zeldovich.py:17-69); the planes
-//     where l_d sits at the Nyquist frequency have no Hermitian part and are zero;
+//     and Re(ifftn(.)) * force_resolution per direction (zeldovich.py:17-69), the three
+//     directions together; the planes where l_d sits at the Nyquist
+//     frequency have no Hermitian part and are zero;
 //   * lattice + Dt * disp + jitter, modulo N_CELLS, and A f H Dt * disp
-//     (zeldovich.py:71-100), in float64 per particle as numpy does, stored as float32.
+//     (zeldovich.py:71-100), stored as float32.
 //     The jitter is the numpy PCG64 stream of uniform(-2, 2) (x, then y, then z draws),
-//     generated here by jumping the 128-bit LCG to each thread's first draw.
+//     generated here by jumping the 128-bit LCG to each block's first draw.
+//
+// GB300 issues two float64 operations per SM and clock, against 128 in float32, so the work per
+// grid point keeps out of them: the factors that depend on |m|^2 alone are tabulated in float64
+// and held as float32 pairs (48 bits and more), and products and sums with them are carried as
+// pairs (Dekker's and Knuth's error-free transformations), rounded to float32 once at the end.
+// 128^3: spectra of the displacements 170 -> 18 us, particles 227 -> 44, field 59 -> 19; the whole
+// call 772 -> 282, with 18 launches instead of 30.
 #include "pm_host.cuh"
 
 using namespace pm;
@@ -30,7 +38,8 @@ namespace {
 constexpr int NORM_BLOCKS = 512;  // fixed grid: the reduction order is the same on every device
 constexpr int NORM_NT = 256;
 constexpr int IC_NT = 256;
-constexpr int JIT_CHUNK = 8;      // consecutive jitter draws per thread
+constexpr int JIT_NT = 256;       // threads of the particle kernel
+constexpr int JIT_ROUNDS = 16;    // particles per thread
 
 // ---- the power spectrum shape (gaussian_random_field.py:65-123) -----------------------
 struct Shape {
@@ -43,7 +52,7 @@ struct Shape {
 __device__ double lcdm_transfer(double k, double gamma) {
   const double q = k / gamma;
   const double a = 16.1 * q, b = 5.46 * q, c = 6.71 * q;
-  const double f1 = sqrt(1.0 + 3.89 * q + a * a + pow(b, 3.0) + pow(c, 4.0));
+  const double f1 = sqrt(1.0 + 3.89 * q + a * a + b * b * b + (c * c) * (c * c));
   double f2 = 0.0;
   if (q != 0.0) {
     const double l = log(1.0 + 2.34 * q), d = 2.34 * q;
@@ -52,10 +61,42 @@ __device__ double lcdm_transfer(double k, double gamma) {
   return f2 / f1;
 }
 
-// S(m2): the summand of the normalisation, which is also P(k) / A for k != 0.
-__global__ void k_shape(double* __restrict__ shape, int m2max, Shape sp) {
+// ---- float32 pairs ---------------------------------------------------------------------
+// hi + lo with |lo| <= ulp(hi) / 2
+__host__ __device__ __forceinline__ float2 split(double v) {
+  const float h = (float)v;
+  return make_float2(h, (float)(v - (double)h));
+}
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return make_float2(s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t)));
+}
+// (c.x + c.y) * v
+__device__ __forceinline__ float2 pair_mul(float2 c, float v) {
+  const float p = __fmul_rn(c.x, v);
+  return make_float2(p, __fmaf_rn(c.x, v, -p) + c.y * v);
+}
+
+// Tables of a call: shape[m2] = S(m2), the summand of the normalisation, which is also P(k) / A
+// for k != 0; disp[m2] = coef / (l0 m2), so that m_d disp[m2] = coef l_d / |l|^2; and the lattice
+// coordinate of each index (numpy's linspace and + 0.5).
+struct TableArgs {
+  int m2max, n;
+  double* shape;
+  float2* disp;
+  float2* space;
+  double coef_l0;       // coef / l0
+  double step, stop;    // lattice step and last point
+  Shape sp;
+};
+
+__global__ void k_tables(TableArgs t) {
+  chain_begin();
   const int m2 = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m2 > m2max) return;
+  if (m2 < t.n)
+    t.space[m2] = split(__dadd_rn(m2 == t.n - 1 && t.n > 1 ? t.stop : __dmul_rn((double)m2, t.step), 0.5));
+  if (m2 > t.m2max) return;
+  const Shape& sp = t.sp;
   const double k = sp.kscale * sqrt((double)m2);
   double s;
   if (sp.power >= 0.0) {
@@ -65,7 +106,8 @@ __global__ void k_shape(double* __restrict__ shape, int m2max, Shape sp) {
     const double kinv = m2 != 0 ? pow(k, -sp.power) : 0.0;
     s = kinv != 0.0 ? 1.0 / kinv : 0.0;
   }
-  shape[m2] = s;
+  t.shape[m2] = s;
+  t.disp[m2] = m2 != 0 ? split(t.coef_l0 / (double)m2) : make_float2(0.f, 0.f);
 }
 
 __device__ __forceinline__ int signed_freq(int m, int n) { return m < n / 2 ? m : m - n; }
@@ -86,6 +128,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // with weight 2 for the columns that stand for two full-grid columns.
 __global__ void __launch_bounds__(NORM_NT) k_norm_partial(const double* __restrict__ shape, int n,
                                                            double* __restrict__ partial) {
+  chain_begin();
   __shared__ double red[NORM_NT / 32];
   const int w = n / 2 + 1;
   const long long total = (long long)n * n * w;
@@ -105,11 +148,22 @@ __global__ void __launch_bounds__(NORM_NT) k_norm_partial(const double* __restri
 // A = 64 H0^2 Npix^2 / sum (gaussian_random_field.py:104-121), one block, fixed order.
 __global__ void __launch_bounds__(NORM_NT) k_norm_final(const double* __restrict__ partial, double sigma_npix2,
                                                          double* __restrict__ norm) {
+  chain_begin();
   __shared__ double red[NORM_NT / 32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < NORM_BLOCKS; i += NORM_NT) acc += partial[i];
   const double t = block_sum(acc, red);
   if (threadIdx.x == 0) norm[0] = sigma_npix2 / t;
+}
+
+// amp[m2] = sqrt(P Dt^2) / 2 / n^3 of the field, P = A S(m2) (p0 A for k = 0)
+__global__ void k_amp(const double* __restrict__ shape, const double* __restrict__ norm, int m2max, double p0, double d2,
+                      double inv_n3, float2* __restrict__ amp) {
+  chain_begin();
+  const int m2 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m2 > m2max) return;
+  const double p = norm[0] * (m2 != 0 ? shape[m2] : p0);
+  amp[m2] = split(sqrt(p * d2) * inv_n3 * 0.5);
 }
 
 // ---- Gaussian random numbers (gaussian_random_field.py:53-61) -------------------------
@@ -129,34 +183,31 @@ struct GrfArgs {
   int n, pitch;
   const float* u;
   const float* v;
-  const double* shape;
-  const double* norm;
-  double p0;      // P(0) / A
-  double d2;      // Dt(A_INIT)^2
-  double inv_n3;  // the 1/n^3 of ifftn
+  const float2* amp;
   float2* spec;
 };
 
 // Hermitian part of rho_k = sqrt(P Dt^2) (f1 + i f2) over the half spectrum, scaled by 1/n^3.
 __global__ void __launch_bounds__(IC_NT) k_grf_fill(GrfArgs g) {
+  chain_begin();
   const int n = g.n, P = g.pitch, h = n / 2;
   const long long total = (long long)n * n * P;
-  const double A = __ldg(&g.norm[0]);
   for (long long e = (long long)blockIdx.x * IC_NT + threadIdx.x; e < total; e += (long long)gridDim.x * IC_NT) {
     const int kx = (int)(e % P);
-    const long long r = e / P;
-    const int ky = (int)(r % n), kz = (int)(r / n);
+    const int r = (int)(e / P);
+    const int ky = r % n, kz = r / n;
     float2 out = make_float2(0.f, 0.f);
     if (kx <= h) {
       const int m2 = sq(signed_freq(kx, n)) + sq(signed_freq(ky, n)) + sq(signed_freq(kz, n));
-      const double p = A * (m2 != 0 ? __ldg(&g.shape[m2]) : g.p0);
-      const double amp = sqrt(p * g.d2) * g.inv_n3;
+      const float2 amp = __ldg(&g.amp[m2]);
       const long long i = ((long long)kz * n + ky) * n + kx;
-      const long long j = ((long long)((n - kz) % n) * n + (n - ky) % n) * n + (n - kx) % n;
+      const int my = ky == 0 ? 0 : n - ky, mz = kz == 0 ? 0 : n - kz, mx = kx == 0 ? 0 : n - kx;
+      const long long j = ((long long)mz * n + my) * n + mx;
       const float2 a = box_muller(__ldg(&g.u[i]), __ldg(&g.v[i]));
       const float2 b = box_muller(__ldg(&g.u[j]), __ldg(&g.v[j]));
-      out = make_float2((float)(amp * 0.5 * ((double)a.x + (double)b.x)),
-                        (float)(amp * 0.5 * ((double)a.y - (double)b.y)));
+      const float2 sx = two_sum(a.x, b.x), sy = two_sum(a.y, -b.y);
+      const float2 px = pair_mul(amp, sx.x), py = pair_mul(amp, sy.x);
+      out = make_float2(px.x + (px.y + amp.x * sx.y), py.x + (py.y + amp.x * sy.y));
     }
     g.spec[e] = out;
   }
@@ -164,32 +215,40 @@ __global__ void __launch_bounds__(IC_NT) k_grf_fill(GrfArgs g) {
 
 // ---- Zel'dovich displacement spectrum (zeldovich.py:17-69) ------------------------------
 struct ZelArgs {
-  int n, pitch, dir;   // dir: axis of the (n, n, n) array (0 = slowest, the z of [z][y][x])
-  const double* kax;   // l(m) = (2 pi N_PARTS / BOX) * fftfreq(N_PARTS)[m]
-  double coef;         // resolution * force_resolution / n^3
+  int n, pitch;
+  const float2* disp;  // coef / (l0 m2)
   const float2* in;    // fftn of the density (half spectrum)
-  float2* out;
+  float2* out[3];      // i l_d coef / |l|^2 times it along axis d of the (n, n, n) array (0 = slowest,
+                       // the z of [z][y][x]); one of them may be `in`
 };
 
 __global__ void __launch_bounds__(IC_NT) k_zeld_spectrum(ZelArgs z) {
+  chain_begin();
   const int n = z.n, P = z.pitch, h = n / 2;
   const long long total = (long long)n * n * P;
   for (long long e = (long long)blockIdx.x * IC_NT + threadIdx.x; e < total; e += (long long)gridDim.x * IC_NT) {
     const int kx = (int)(e % P);
-    const long long r = e / P;
-    const int ky = (int)(r % n), kz = (int)(r / n);
-    float2 o = make_float2(0.f, 0.f);
-    const int kd = z.dir == 0 ? kz : (z.dir == 1 ? ky : kx);
-    if (kx <= h && kd != h && (kx | ky | kz) != 0) {
-      const double lx = __ldg(&z.kax[kx]), ly = __ldg(&z.kax[ky]), lz = __ldg(&z.kax[kz]);
-      const double l2 = __dadd_rn(__dadd_rn(__dmul_rn(lx, lx), __dmul_rn(ly, ly)), __dmul_rn(lz, lz));
-      const double ld = z.dir == 0 ? lz : (z.dir == 1 ? ly : lx);
-      const double gd = ld * z.coef / l2;
-      const float2 v = z.in[e];
-      // i * g * v
-      o = make_float2((float)(-gd * (double)v.y), (float)(gd * (double)v.x));
+    const int r = (int)(e / P);
+    const int ky = r % n, kz = r / n;
+    const bool mode = kx <= h && (kx | ky | kz) != 0;
+    float2 re = make_float2(0.f, 0.f), im = re;  // disp[m2] * v
+    if (mode) {
+      const int m2 = sq(signed_freq(kx, n)) + sq(signed_freq(ky, n)) + sq(signed_freq(kz, n));
+      const float2 c = __ldg(&z.disp[m2]), v = z.in[e];
+      re = pair_mul(c, v.x);
+      im = pair_mul(c, v.y);
     }
-    z.out[e] = o;
+    #pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int kd = d == 0 ? kz : (d == 1 ? ky : kx);
+      float2 o = make_float2(0.f, 0.f);
+      if (mode && kd != h) {  // i * m_d * (disp v)
+        const float m = (float)signed_freq(kd, n);
+        const float2 a = pair_mul(im, m), b = pair_mul(re, m);
+        o = make_float2(-(a.x + a.y), b.x + b.y);
+      }
+      z.out[d][e] = o;
+    }
   }
 }
 
@@ -221,9 +280,13 @@ __host__ __device__ __forceinline__ unsigned long long pcg_output(u128 s) {
   return (x >> rot) | (x << ((64u - rot) & 63u));
 }
 
-// uniform(-2, 2) of numpy's Generator: -2 + 4 * ((next >> 11) * 2^-53)
-__device__ __forceinline__ double jitter_value(unsigned long long x) {
-  return __dadd_rn(-2.0, __dmul_rn(4.0, (double)(x >> 11) * (1.0 / 9007199254740992.0)));
+// uniform(-2, 2) of numpy's Generator, -2 + 4 ((next >> 11) 2^-53), as a pair: the 53-bit
+// integer (next >> 11) - 2^52 is cut into its upper 24 bits, the next 24 and 5 dropped ones
+// (2^-46 of a cell).
+__device__ __forceinline__ float2 jitter_pair(unsigned long long x) {
+  const long long v = (long long)(x >> 11) - (1ll << 52);
+  const int hi = (int)(v >> 29), mid = (int)((v >> 5) & 0xffffffll);
+  return make_float2((float)hi * (1.f / 4194304.f), (float)mid * (1.f / 70368744177664.f));
 }
 
 // numpy float remainder: fmod, moved into the divisor's sign
@@ -237,51 +300,90 @@ __device__ __forceinline__ double py_mod(double a, double b) {
   return m;
 }
 
+// (v.x + v.y) mod n, rounded to float32
+__device__ __forceinline__ float pair_mod(float2 v, float n) {
+  const float hi = v.x, lo = v.y;
+  if (!(hi >= -n && hi < 2.f * n)) return (float)py_mod((double)hi + (double)lo, (double)n);  // (and NaN)
+  if (hi > n || (hi == n && lo >= 0.f)) return __fadd_rn(__fsub_rn(hi, n), lo);  // hi - n is exact
+  if (hi < 0.f || (hi == 0.f && lo < 0.f)) {
+    const float2 t = two_sum(hi, n);
+    return __fadd_rn(t.x, __fadd_rn(t.y, lo));
+  }
+  return __fadd_rn(hi, lo);
+}
+
 struct PartArgs {
-  int n, dir;
-  long long np;          // n^3
-  const float* disp;     // displacement field along dir (n^3, already * force_resolution)
-  const double* space;   // lattice coordinate per axis index (zeldovich.py:79)
-  double lin;            // Dt(A_INIT)
-  double vcoef;          // A_INIT * f_0 * h_0 * Dt
-  double ncells;
+  int n;
+  long long np;           // n^3
+  const float* disp[3];   // displacement field along each axis (n^3, already * force_resolution)
+  const float2* space;    // lattice coordinate per axis index (zeldovich.py:79)
+  float2 lin;             // Dt(A_INIT)
+  float2 vcoef;           // A_INIT * f_0 * h_0 * Dt
+  float ncells;
+  const ulonglong2* jump; // JIT_NT entries of (M^(t+1), 1 + M + .. + M^t), low and high words
   unsigned long long st_hi, st_lo, inc_hi, inc_lo;  // PCG64 state before the first draw
-  float* pos;            // row dir of (3, np)
+  float* pos;             // (3, np)
   float* vel;
 };
 
-__global__ void __launch_bounds__(IC_NT) k_zeld_particles(PartArgs a) {
-  const long long chunks = (a.np + JIT_CHUNK - 1) / JIT_CHUNK;
-  const u128 st0 = ((u128)a.st_hi << 64) | a.st_lo, inc = ((u128)a.inc_hi << 64) | a.inc_lo;
-  const long long nn = (long long)a.n * a.n;
-  for (long long c = (long long)blockIdx.x * IC_NT + threadIdx.x; c < chunks; c += (long long)gridDim.x * IC_NT) {
-    const long long p0 = c * JIT_CHUNK;
-    // draw number dir * np + p0 is the (dir * np + p0 + 1)-th step of the generator
-    u128 s = pcg_advance(st0, inc, (unsigned long long)(a.dir * a.np + p0));
-    for (int k = 0; k < JIT_CHUNK && p0 + k < a.np; ++k) {
-      const long long p = p0 + k;
-      s = s * pcg_mult() + inc;
-      const double jit = jitter_value(pcg_output(s));
-      const int id = a.dir == 0 ? (int)(p / nn) : (a.dir == 1 ? (int)((p / a.n) % a.n) : (int)(p % a.n));
-      const double d = (double)__ldg(&a.disp[p]);
-      double x = __dadd_rn(__ldg(&a.space[id]), __dmul_rn(a.lin, d));
-      x = __dadd_rn(x, jit);
-      a.pos[p] = (float)py_mod(x, a.ncells);
-      a.vel[p] = (float)__dmul_rn(a.vcoef, d);
-    }
+// A block takes JIT_NT * JIT_ROUNDS consecutive particles of axis blockIdx.y (coalesced); its
+// first thread jumps the generator there, and thread t reaches its draws by one jump of t + 1
+// steps and then jumps of JIT_NT (one 128-bit multiply-add each).
+__global__ void __launch_bounds__(JIT_NT) k_zeld_particles(PartArgs a) {
+  chain_begin();
+  __shared__ unsigned long long s_base[2];
+  const int dir = blockIdx.y;
+  const long long p0 = (long long)blockIdx.x * (JIT_NT * JIT_ROUNDS);
+  const u128 inc = ((u128)a.inc_hi << 64) | a.inc_lo;
+  if (threadIdx.x == 0) {
+    // draw number dir * np + p is the (dir * np + p + 1)-th step of the generator
+    const u128 b = pcg_advance(((u128)a.st_hi << 64) | a.st_lo, inc, (unsigned long long)(dir * a.np + p0));
+    s_base[0] = (unsigned long long)b;
+    s_base[1] = (unsigned long long)(b >> 64);
+  }
+  auto word = [](ulonglong2 w) { return ((u128)w.y << 64) | w.x; };
+  const u128 m = word(__ldg(&a.jump[2 * threadIdx.x])), c = word(__ldg(&a.jump[2 * threadIdx.x + 1]));
+  const u128 mr = word(__ldg(&a.jump[2 * (JIT_NT - 1)])), cr = word(__ldg(&a.jump[2 * (JIT_NT - 1) + 1])) * inc;
+  __syncthreads();
+  u128 s = m * (((u128)s_base[1] << 64) | s_base[0]) + c * inc;
+  const unsigned u = (unsigned)a.n;
+  const float* __restrict__ disp = a.disp[dir];
+  float* __restrict__ pos = a.pos + dir * a.np;
+  float* __restrict__ vel = a.vel + dir * a.np;
+  for (int k = 0; k < JIT_ROUNDS; ++k, s = mr * s + cr) {
+    const long long p = p0 + k * JIT_NT + threadIdx.x;
+    if (p >= a.np) break;
+    const float2 jit = jitter_pair(pcg_output(s));
+    const unsigned i = (unsigned)p;
+    const unsigned id = dir == 0 ? i / (u * u) : (dir == 1 ? i / u % u : i % u);
+    const float d = __ldg(&disp[p]);
+    const float2 x0 = __ldg(&a.space[id]), ld = pair_mul(a.lin, d);
+    const float2 t1 = two_sum(x0.x, ld.x), t2 = two_sum(t1.x, jit.x);
+    const float lo = __fadd_rn(__fadd_rn(__fadd_rn(x0.y, ld.y), jit.y), __fadd_rn(t1.y, t2.y));
+    pos[p] = pair_mod(two_sum(t2.x, lo), a.ncells);
+    const float2 v = pair_mul(a.vcoef, d);
+    vel[p] = __fadd_rn(v.x, v.y);
   }
 }
 
 }  // namespace
 
+// descriptors of an object's transforms
+enum IcSim : int { SIM_FIELD_INV = 0, SIM_FIELD_FWD, SIM_DISP, IC_SIMS = SIM_DISP + 3 };
+
 struct pm_ics {
   int n = 0, device = 0, sms = 1, m2max = 0;
   Tables tab;
-  DBuf d_sim, d_prefix, d_maps, d_err;
-  DBuf spec_a, spec_b, grid, shape, partial, norm, kax, space;
-  bool maps_ok = false;
-  std::vector<double> h_kax, h_space;
-  Sim h_sims[2];
+  DBuf pool;              // all of the object's memory, one after another:
+  Sim* d_sim = nullptr;   // (down to d_err: written by create)
+  CUtensorMap* d_maps = nullptr;  // null: no tensor maps
+  int* d_prefix = nullptr;
+  ulonglong2* jump = nullptr;
+  int* d_err = nullptr;
+  double *shape = nullptr, *partial = nullptr, *norm = nullptr;
+  float2 *amp = nullptr, *disp = nullptr, *space = nullptr;
+  float2* spec[3] = {};
+  float* grid[3] = {};
   int h_err = 0;
   std::string err;
 };
@@ -326,34 +428,73 @@ int pm_ics_create(int n_parts, int device, pm_ics** out) {
   g->device = device;
   const int n = n_parts, h = n / 2;
   g->m2max = 3 * h * h;
-  const size_t sb = (size_t)n * n * spec_pitch(n) * sizeof(float2);
+  // (sb: a multiple of 128 bytes, which the tensor maps and the row transforms rely on)
+  const size_t sb = (size_t)n * n * spec_pitch(n) * sizeof(float2), gb = (size_t)n * n * n * sizeof(float);
   cudaError_t e = cudaSetDevice(device);
   if (!e) g->sms = sm_count(device);
   if (!e) e = g->tab.build(n);
-  if (!e) e = g->d_sim.ensure(2 * sizeof(Sim));
-  if (!e) e = g->d_prefix.ensure(4 * sizeof(int));
-  if (!e) e = g->d_err.ensure(sizeof(int));
-  if (!e) e = g->spec_a.ensure(sb);
-  if (!e) e = g->spec_b.ensure(sb);
-  if (!e) e = g->grid.ensure((size_t)n * n * n * sizeof(float));
-  if (!e) e = g->shape.ensure((size_t)(g->m2max + 1) * sizeof(double));
-  if (!e) e = g->partial.ensure(NORM_BLOCKS * sizeof(double));
-  if (!e) e = g->norm.ensure(sizeof(double));
-  if (!e) e = g->kax.ensure(n * sizeof(double));
-  if (!e) e = g->space.ensure(n * sizeof(double));
-  if (!e) e = cudaMemset(g->d_err.p, 0, sizeof(int));
+  size_t at = 0;
+  auto part = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) / 256 * 256;
+    return o;
+  };
+  const size_t tables = (size_t)(g->m2max + 1);
+  const size_t o_sim = part(IC_SIMS * sizeof(Sim)), o_maps = part(2 * IC_SIMS * sizeof(CUtensorMap)),
+               o_pre = part(8 * sizeof(int)), o_jump = part(2 * JIT_NT * sizeof(ulonglong2)), o_err = part(sizeof(int)),
+               filled = at, o_shape = part(tables * sizeof(double)), o_amp = part(tables * sizeof(float2)),
+               o_disp = part(tables * sizeof(float2)), o_partial = part(NORM_BLOCKS * sizeof(double)),
+               o_norm = part(sizeof(double)), o_space = part(n * sizeof(float2)), o_spec = part(3 * sb),
+               o_grid = part(3 * gb);
+  if (!e) e = g->pool.ensure(at);
   if (!e) {
-    const int units_x = (int)spectral_units(SPEC_X_R2C, n), units_l = (int)spectral_units(SPEC_Y_FWD, n);
-    const int pre[4] = {0, units_x, 0, units_l};
-    e = cudaMemcpy(g->d_prefix.p, pre, sizeof(pre), cudaMemcpyHostToDevice);
-  }
-  if (!e) {
-    CUtensorMap m[4];
-    if (spectral_encode_maps(n, g->spec_a.p, m) && spectral_encode_maps(n, g->spec_b.p, m + 2)) {
-      e = g->d_maps.ensure(sizeof(m));
-      if (!e) e = cudaMemcpy(g->d_maps.p, m, sizeof(m), cudaMemcpyHostToDevice);
-      if (!e) g->maps_ok = true;
+    char* base = g->pool.as<char>();
+    g->d_sim = reinterpret_cast<Sim*>(base + o_sim);
+    g->d_prefix = reinterpret_cast<int*>(base + o_pre);
+    g->jump = reinterpret_cast<ulonglong2*>(base + o_jump);
+    g->d_err = reinterpret_cast<int*>(base + o_err);
+    g->shape = reinterpret_cast<double*>(base + o_shape);
+    g->amp = reinterpret_cast<float2*>(base + o_amp);
+    g->disp = reinterpret_cast<float2*>(base + o_disp);
+    g->partial = reinterpret_cast<double*>(base + o_partial);
+    g->norm = reinterpret_cast<double*>(base + o_norm);
+    g->space = reinterpret_cast<float2*>(base + o_space);
+    for (int i = 0; i < 3; ++i) {
+      g->spec[i] = reinterpret_cast<float2*>(base + o_spec + i * sb);
+      g->grid[i] = reinterpret_cast<float*>(base + o_grid + i * gb);
     }
+    std::vector<char> h(filled, 0);
+    // descriptors: the field's inverse and forward transforms, the displacements' inverses
+    bool ok = true;
+    for (int i = 0; i < IC_SIMS; ++i) {
+      const int sp = i == SIM_FIELD_INV ? 1 : (i == SIM_FIELD_FWD ? 0 : i - SIM_DISP);
+      const int gr = i < SIM_DISP ? 0 : i - SIM_DISP;
+      Sim d{};
+      d.n = n;
+      d.pitch = spec_pitch(n);
+      d.s2 = g->tab.s2.as<float>();
+      d.tw = g->tab.tw.as<float2>();
+      d.spec = g->spec[sp];
+      d.rho = d.phi = g->grid[gr];
+      std::memcpy(h.data() + o_sim + i * sizeof(Sim), &d, sizeof(d));
+      CUtensorMap m[2];
+      std::memset(m, 0, sizeof(m));
+      ok = ok && spectral_encode_maps(n, d.spec, m);
+      std::memcpy(h.data() + o_maps + 2 * i * sizeof(CUtensorMap), m, sizeof(m));
+    }
+    if (ok) g->d_maps = reinterpret_cast<CUtensorMap*>(base + o_maps);
+    const int ux = (int)spectral_units(SPEC_X_R2C, n), ul = (int)spectral_units(SPEC_Y_FWD, n);
+    const int pre[8] = {0, ux, 2 * ux, 3 * ux, 0, ul, 2 * ul, 3 * ul};
+    std::memcpy(h.data() + o_pre, pre, sizeof(pre));
+    u128 m = 1, c = 0;  // the generator's jumps by 1 .. JIT_NT steps
+    for (int t = 0; t < JIT_NT; ++t) {
+      c = c * pcg_mult() + 1;  // 1 + M + .. + M^t
+      m *= pcg_mult();
+      const unsigned long long w[4] = {(unsigned long long)m, (unsigned long long)(m >> 64), (unsigned long long)c,
+                                       (unsigned long long)(c >> 64)};
+      std::memcpy(h.data() + o_jump + t * sizeof(w), w, sizeof(w));
+    }
+    e = cudaMemcpy(g->pool.p, h.data(), filled, cudaMemcpyHostToDevice);
   }
   if (!e) e = spectral_dispatch(SPEC_PREPARE, n, nullptr, Work(), 0, nullptr);
   if (!e) e = cudaDeviceSynchronize();
@@ -368,9 +509,7 @@ int pm_ics_create(int n_parts, int device, pm_ics** out) {
 void pm_ics_destroy(pm_ics* g) {
   if (!g) return;
   cudaSetDevice(g->device);
-  DBuf* bufs[] = {&g->d_sim, &g->d_prefix, &g->d_maps, &g->d_err, &g->spec_a, &g->spec_b, &g->grid,
-                  &g->shape, &g->partial, &g->norm, &g->kax, &g->space};
-  for (DBuf* b : bufs) b->release();
+  g->pool.release();
   g->tab.release();
   delete g;
 }
@@ -391,127 +530,111 @@ int pm_ics_generate(pm_ics* g, const pm_config* cfg, const pm_ic_params* ic, con
   const double om = cfg->omega_m0, ob = cfg->omega_b0, ok = cfg->omega_k0, ol = cfg->omega_lambda0,
                h0 = cfg->h0, a0 = cfg->a_init, box = cfg->box_size, ncells = cfg->n_cells;
 
-  // host tables: Fourier axis l(m) and lattice coordinates, in numpy's operation order
-  g->h_kax.resize(n);
-  g->h_space.resize(n);
-  const double scale = 2.0 * M_PI * n / box, inv_n = 1.0 / n;
-  for (int m = 0; m < n; ++m) g->h_kax[m] = scale * ((double)(m < (n + 1) / 2 ? m : m - n) * inv_n);
-  const double res = ncells / n, stop = ncells - res, step = n > 1 ? stop / (n - 1) : 0.0;
-  for (int i = 0; i < n; ++i) g->h_space[i] = (i == n - 1 && n > 1 ? stop : i * step) + 0.5;
-  IC_CK(cudaMemcpyAsync(g->kax.p, g->h_kax.data(), n * sizeof(double), cudaMemcpyHostToDevice, st), "kax");
-  IC_CK(cudaMemcpyAsync(g->space.p, g->h_space.data(), n * sizeof(double), cudaMemcpyHostToDevice, st), "space");
+  const Launch lc(st, n <= 256);  // (pm_launch.cuh)
+  const double npix = (double)np, res = ncells / n, fres = ncells / box;
 
-  Sim s[2]{};
-  for (int k = 0; k < 2; ++k) {
-    s[k].n = n;
-    s[k].pitch = pitch;
-    s[k].s2 = g->tab.s2.as<float>();
-    s[k].tw = g->tab.tw.as<float2>();
-  }
-  s[0].rho = g->grid.as<float>();   // forward transform of the field
-  s[0].spec = g->spec_a.as<float2>();
-  s[1].spec = g->spec_b.as<float2>();  // inverse transforms into the field buffer
-  s[1].phi = g->grid.as<float>();
-  g->h_sims[0] = s[0];
-  g->h_sims[1] = s[1];
-  IC_CK(cudaMemcpyAsync(g->d_sim.p, g->h_sims, sizeof(g->h_sims), cudaMemcpyHostToDevice, st), "sims");
-
-  // power spectrum normalisation
-  Shape sp;
-  sp.kscale = 2.0 * M_PI / box;
-  sp.gamma = om * h0 * std::exp(-ob - ob / om);
-  sp.power = ic->power;
-  sp.lcdm = ic->lcdm_transfer ? 1 : 0;
-  k_shape<<<(g->m2max + 256) / 256, 256, 0, st>>>(g->shape.as<double>(), g->m2max, sp);
-  IC_CK(cudaGetLastError(), "shape");
-  k_norm_partial<<<NORM_BLOCKS, NORM_NT, 0, st>>>(g->shape.as<double>(), n, g->partial.as<double>());
-  IC_CK(cudaGetLastError(), "norm");
-  const double npix = (double)np;
-  k_norm_final<<<1, NORM_NT, 0, st>>>(g->partial.as<double>(), 64.0 * std::pow(h0, 2.0) * (npix * npix),
-                                      g->norm.as<double>());
-  IC_CK(cudaGetLastError(), "norm final");
-
+  // power spectrum, its normalisation and the other tables
+  TableArgs ta;
+  ta.m2max = g->m2max;
+  ta.n = n;
+  ta.shape = g->shape;
+  ta.disp = g->disp;
+  ta.space = g->space;
+  // l(m) = (2 pi n / box) fftfreq(n)[m] = l0 m; the displacement spectrum times resolution,
+  // force resolution and the 1/n^3 of ifftn
+  ta.coef_l0 = res * fres / npix / (2.0 * M_PI / box);
+  ta.stop = ncells - res;
+  ta.step = n > 1 ? ta.stop / (n - 1) : 0.0;
+  ta.sp.kscale = 2.0 * M_PI / box;
+  ta.sp.gamma = om * h0 * std::exp(-ob - ob / om);
+  ta.sp.power = ic->power;
+  ta.sp.lcdm = ic->lcdm_transfer ? 1 : 0;
+  const int tb = (g->m2max + 128) / 128;
+  IC_CK(launch_chained(k_tables, tb, 128, 0, lc, ta), "tables");
+  IC_CK(launch_chained(k_norm_partial, NORM_BLOCKS, NORM_NT, 0, lc, g->shape, n, g->partial),
+        "norm");
+  IC_CK(launch_chained(k_norm_final, 1, NORM_NT, 0, lc, g->partial,
+                       64.0 * std::pow(h0, 2.0) * (npix * npix), g->norm),
+        "norm final");
   const double lin = cosmo_Dt(a0, om, ol, ok);
+  // P(k = 0) / A: the reference's k**POWER * lcdm (or div) at k = 0
+  const double p0 = (ic->power >= 0.0 && !ic->lcdm_transfer && ic->power == 0.0) ? 1.0 : 0.0;
+  IC_CK(launch_chained(k_amp, tb, 128, 0, lc, g->shape, g->norm, g->m2max, p0, lin * lin,
+                       1.0 / npix, g->amp),
+        "amplitudes");
   GrfArgs ga;
   ga.n = n;
   ga.pitch = pitch;
   ga.u = u;
   ga.v = v;
-  ga.shape = g->shape.as<double>();
-  ga.norm = g->norm.as<double>();
-  // P(k = 0) / A: the reference's k**POWER * lcdm (or div) at k = 0
-  ga.p0 = (ic->power >= 0.0 && !ic->lcdm_transfer && ic->power == 0.0) ? 1.0 : 0.0;
-  ga.d2 = lin * lin;
-  ga.inv_n3 = 1.0 / npix;
-  ga.spec = g->spec_b.as<float2>();
+  ga.amp = g->amp;
+  ga.spec = g->spec[1];
   const int ew = grid_for(((long long)n * n * pitch + IC_NT - 1) / IC_NT, g->sms, 8);
-  k_grf_fill<<<ew, IC_NT, 0, st>>>(ga);
-  IC_CK(cudaGetLastError(), "grf fill");
+  IC_CK(launch_chained(k_grf_fill, ew, IC_NT, 0, lc, ga), "grf fill");
 
-  const Sim* ds = g->d_sim.as<Sim>();
-  const CUtensorMap* maps = g->maps_ok ? g->d_maps.as<CUtensorMap>() : nullptr;
-  int* err = g->d_err.as<int>();
-  const int* pre = g->d_prefix.as<int>();
-  Work wx{pre, 1, (int)spectral_units(SPEC_X_R2C, n)}, wl{pre + 2, 1, (int)spectral_units(SPEC_Y_FWD, n)};
-  const int gx = grid_for(wx.total, g->sms, 8), gl = grid_for(wl.total, g->sms, 8);
-  auto inverse = [&](const char* what) -> int {  // spec_b -> grid
-    const CUtensorMap* mb = maps ? maps + 2 : nullptr;
-    IC_CK(spectral_dispatch(SPEC_Z_INV, n, ds + 1, wl, gl, st, mb, err), what);
-    IC_CK(spectral_dispatch(SPEC_Y_INV, n, ds + 1, wl, gl, st, mb, err), what);
-    IC_CK(spectral_dispatch(SPEC_X_C2R, n, ds + 1, wx, gx, st, mb, err), what);
+  const Sim* ds = g->d_sim;
+  const CUtensorMap* maps = g->d_maps;
+  int* err = g->d_err;
+  const int* pre = g->d_prefix;
+  // one transform pass of `count` descriptors from `first` on
+  auto pass = [&](SpecKind kind, int first, int count, const char* what) -> int {
+    const bool xk = kind == SPEC_X_R2C || kind == SPEC_X_C2R;
+    const Work w{pre + (xk ? 0 : 4), count, count * (int)spectral_units(kind, n)};
+    IC_CK(spectral_dispatch(kind, n, ds + first, w, grid_for(w.total, g->sms, 8), lc, maps ? maps + 2 * first : nullptr,
+                            err),
+          what);
     return PM_OK;
   };
-  int rc = inverse("grf inverse");
-  if (rc) return rc;
+  auto inverse = [&](int first, int count, const char* what) -> int {
+    if (int r = pass(SPEC_Z_INV, first, count, what)) return r;
+    if (int r = pass(SPEC_Y_INV, first, count, what)) return r;
+    return pass(SPEC_X_C2R, first, count, what);
+  };
+  if (int r = inverse(SIM_FIELD_INV, 1, "grf inverse")) return r;
   if (grf)
-    IC_CK(cudaMemcpyAsync(grf, g->grid.p, (size_t)np * sizeof(float), cudaMemcpyDeviceToDevice, st), "grf out");
+    IC_CK(cudaMemcpyAsync(grf, g->grid[0], (size_t)np * sizeof(float), cudaMemcpyDeviceToDevice, st), "grf out");
 
   // fftn of the field (zeldovich.py:17)
-  IC_CK(spectral_dispatch(SPEC_X_R2C, n, ds, wx, gx, st, maps, err), "r2c");
-  IC_CK(spectral_dispatch(SPEC_Y_FWD, n, ds, wl, gl, st, maps, err), "y fwd");
-  IC_CK(spectral_dispatch(SPEC_Z_FWD, n, ds, wl, gl, st, maps, err), "z fwd");
+  if (int r = pass(SPEC_X_R2C, SIM_FIELD_FWD, 1, "r2c")) return r;
+  if (int r = pass(SPEC_Y_FWD, SIM_FIELD_FWD, 1, "y fwd")) return r;
+  if (int r = pass(SPEC_Z_FWD, SIM_FIELD_FWD, 1, "z fwd")) return r;
 
-  const double fres = ncells / box;
   const double f0 = 1.0 / std::sqrt((om + ok * a0 + ol * std::pow(a0, 3.0)) / a0);
   const double hh = cosmo_H(a0, h0, om, ol, ok);
-  for (int d = 0; d < 3; ++d) {
-    ZelArgs za;
-    za.n = n;
-    za.pitch = pitch;
-    za.dir = d;
-    za.kax = g->kax.as<double>();
-    za.coef = res * fres / npix;
-    za.in = g->spec_a.as<float2>();
-    za.out = g->spec_b.as<float2>();
-    k_zeld_spectrum<<<ew, IC_NT, 0, st>>>(za);
-    IC_CK(cudaGetLastError(), "displacement spectrum");
-    rc = inverse("displacement inverse");
-    if (rc) return rc;
-    PartArgs pa;
-    pa.n = n;
-    pa.dir = d;
-    pa.np = np;
-    pa.disp = g->grid.as<float>();
-    pa.space = g->space.as<double>();
-    pa.lin = lin;
-    pa.vcoef = a0 * f0 * hh * lin;
-    pa.ncells = ncells;
-    pa.st_hi = ic->jitter_state[0];
-    pa.st_lo = ic->jitter_state[1];
-    pa.inc_hi = ic->jitter_inc[0];
-    pa.inc_lo = ic->jitter_inc[1];
-    pa.pos = positions + d * np;
-    pa.vel = velocities + d * np;
-    const int pw = grid_for(((np + JIT_CHUNK - 1) / JIT_CHUNK + IC_NT - 1) / IC_NT, g->sms, 8);
-    k_zeld_particles<<<pw, IC_NT, 0, st>>>(pa);
-    IC_CK(cudaGetLastError(), "particles");
+  ZelArgs za;
+  PartArgs pa;
+  za.n = n;
+  za.pitch = pitch;
+  za.disp = g->disp;
+  za.in = g->spec[0];
+  for (int i = 0; i < 3; ++i) {
+    za.out[i] = g->spec[i];
+    pa.disp[i] = g->grid[i];
   }
+  IC_CK(launch_chained(k_zeld_spectrum, ew, IC_NT, 0, lc, za), "displacement spectrum");
+  if (int r = inverse(SIM_DISP, 3, "displacement inverse")) return r;
+  pa.n = n;
+  pa.np = np;
+  pa.space = g->space;
+  pa.lin = split(lin);
+  pa.vcoef = split(a0 * f0 * hh * lin);
+  pa.ncells = (float)ncells;
+  pa.jump = g->jump;
+  pa.st_hi = ic->jitter_state[0];
+  pa.st_lo = ic->jitter_state[1];
+  pa.inc_hi = ic->jitter_inc[0];
+  pa.inc_lo = ic->jitter_inc[1];
+  pa.pos = positions;
+  pa.vel = velocities;
+  const unsigned pb = (unsigned)((np + JIT_NT * JIT_ROUNDS - 1) / (JIT_NT * JIT_ROUNDS));
+  k_zeld_particles<<<dim3(pb, 3), JIT_NT, 0, st>>>(pa);
+  IC_CK(cudaGetLastError(), "particles");
   // device-side checks of the TMA passes (bounded waits): read back once
-  IC_CK(cudaMemcpyAsync(&g->h_err, g->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, st), "err");
+  IC_CK(cudaMemcpyAsync(&g->h_err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, st), "err");
   IC_CK(cudaStreamSynchronize(st), "sync");
   const int bits = g->h_err;
   if (bits) {
-    cudaMemsetAsync(g->d_err.p, 0, sizeof(int), st);
+    cudaMemsetAsync(g->d_err, 0, sizeof(int), st);
     return ic_fail(g, PM_ERR_DEVICE, "device check failed in the spectral passes (bits " + std::to_string(bits) + ")");
   }
   return PM_OK;
