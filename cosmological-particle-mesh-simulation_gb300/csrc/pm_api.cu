@@ -16,6 +16,8 @@ struct pm_ctx {
   DBuf hpos, hvel;                    // device copies for pm_step_host
   DBuf pk_partial, pk_out;            // power spectrum scratch
   DBuf row_count, scan_sums;  // row bin counts of a call (then 4 words: tile counter), block sums of their scan
+  DBuf group_max;             // largest count of each 16 row bins
+  DBuf dense;                 // the fused deposit's list of two-word tiles
   DBuf rec;                               // cell records in row order, then the forces
   // spectral gradient: spectra and force grids of the y and z axes (x uses spec and phi), the
   // three descriptors of the inverse passes and their work tables and tensor maps
@@ -159,11 +161,12 @@ int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy,
   PM_CK(c->row_start.ensure(((size_t)nrows + 1) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->row_count.ensure(((size_t)nrows + 4) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->scan_sums.ensure(row_sort_block_sums(nrows) * sizeof(unsigned)), "alloc rows");
+  PM_CK(c->group_max.ensure((size_t)nrows / 16 * sizeof(unsigned)), "alloc rows");
   unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
   unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
   if (int r = begin(c, k, st, count, ((size_t)nrows + 4) * sizeof(unsigned))) return r;
   PM_CK(launch_row_rank(positions, np, lattice_side(c, np), c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, lc), "row ranks");
-  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, lc), "row starts");
+  PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, lc, c->group_max.as<unsigned>()), "row starts");
   PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, lattice_side(c, np), c->n, start, ranks, place,
                          c->rec.as<uint4>(), lc),
         "row order");
@@ -173,7 +176,7 @@ int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy,
 int deposit(pm_ctx* c, Call& k, cudaStream_t st) {
   const Launch lc = chained(c, st);
   PM_CK(launch_deposit(c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
-                       c->row_start.as<unsigned>(), POS_DISP, c->d_err.as<int>(),
+                       c->row_start.as<unsigned>(), c->group_max.as<unsigned>(), POS_DISP, c->d_err.as<int>(),
                        grid_for(k.work.prefix[CALL_DEP][1], c->sms, 8), deposit_smem_bytes(c->n, TILE_Y, TILE_Z), lc),
         "deposit");
   return PM_OK;
@@ -353,6 +356,8 @@ void pm_ctx_destroy(pm_ctx* c) {
   if (c->ev_start) cudaEventDestroy(c->ev_start);
   if (c->ev_vel) cudaEventDestroy(c->ev_vel);
   c->scan_sums.release();
+  c->group_max.release();
+  c->dense.release();
   for (int i = 0; i < 2; ++i) { c->gspec[i].release(); c->ggrid[i].release(); }
   c->d_sim3.release();
   c->d_prefix3.release();
@@ -500,8 +505,10 @@ int step_core(pm_ctx* c, const StepIO& io, long long np, double mass, double a, 
   }
   if (!rho_out && deposit_r2c_supported(c->n)) {
     // the density is not requested: deposit straight into the x-transformed spectrum
+    PM_CK(c->dense.ensure(sizeof(unsigned) * k.work.prefix[CALL_DEP][1]), "alloc tiles");
     PM_CK(deposit_r2c_dispatch(c->n, c->d_sim.as<Sim>(), work(c, k, CALL_DEP), record_parts(c), nullptr,
-                               c->row_start.as<unsigned>(), c->d_err.as<int>(), c->row_count.as<unsigned>() + row_bins(c->n), nullptr,
+                               c->row_start.as<unsigned>(), c->group_max.as<unsigned>(), c->d_err.as<int>(),
+                               c->row_count.as<unsigned>() + row_bins(c->n), nullptr, c->dense.as<unsigned>(),
                                grid_for(k.work.prefix[CALL_DEP][1], c->sms, deposit_r2c_ctas_per_sm(c->n)), chained(c, st)),
           "fused deposit");
     if (int r = spectral(c, k, false, st, true, gradient)) return r;

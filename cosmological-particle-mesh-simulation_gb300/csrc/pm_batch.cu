@@ -113,10 +113,12 @@ struct pm_batch {
   int cur = 0;
   SortBufs sort;
   DBuf row_start, d_sims, d_prefix, d_err, d_maps;
-  DBuf tile_next;   // per distinct size: tile counter of the fused deposit, 2 words of ordering scratch
+  DBuf tile_next;   // per distinct size: tile counter and two-word count of the fused deposit, 2 words of ordering scratch
   DBuf tile_order;  // per distinct size (at its tile prefix): the fused deposit's tiles, dense first
+  DBuf tile_dense;  // the same for its list of two-word tiles
   DBuf d_one;       // descriptor + work table of a one-simulation deposit (pm_batch_density)
-  DBuf row_count, row_cursor, scan_sums;  // counting sort of the row keys
+  DBuf row_count, row_cursor, scan_sums;  // counting sort of the row bins
+  DBuf group_max;                         // largest count of each 16 row bins
   Plan plan;
   bool dirty = true, keys_valid = false;
   bool graphs = true;
@@ -420,6 +422,7 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     size_t tiles = 1;
     for (int t : P.fdep_total) tiles += (size_t)t;
     PB_CK(b->tile_order.ensure_geo(sizeof(unsigned) * tiles), "alloc tile order");
+    PB_CK(b->tile_dense.ensure_geo(sizeof(unsigned) * tiles), "alloc tile order");
     PB_CK(b->tile_next.ensure_geo(4 * sizeof(unsigned) * P.sizes.size()), "alloc tile counters");
     while (b->side.size() < P.sizes.size()) {
       cudaStream_t s = nullptr;
@@ -434,6 +437,7 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     }
   }
   PB_CK(b->row_cursor.ensure_geo(sizeof(unsigned) * (size_t)rows), "alloc rows");
+  PB_CK(b->group_max.ensure_geo(sizeof(unsigned) * (size_t)rows / 16), "alloc rows");
   PB_CK(b->scan_sums.ensure_geo(sizeof(unsigned) * row_sort_block_sums(rows)), "alloc rows");
   {  // tensor maps (for the TMA line passes), descriptors and work prefixes, through pinned staging
     const size_t mb = sizeof(CUtensorMap) * 2 * (size_t)S, sbytes = sizeof(Sim) * S, pbytes = sizeof(int) * pre.size();
@@ -476,7 +480,7 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     PB_CK(spectral_dispatch(SPEC_PREPARE, P.sizes[g], nullptr, Work(), 0, st), "prepare");
     if (P.fused[g])
       PB_CK(deposit_r2c_dispatch(P.sizes[g], nullptr, Work(), Parts(), nullptr, nullptr, nullptr, nullptr,
-                                 nullptr, 0, st),
+                                 nullptr, nullptr, nullptr, 0, st),
             "prepare fused deposit");
   }
   PB_CK(deposit_prepare(), "prepare deposit");
@@ -525,18 +529,19 @@ int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigne
   const Work wg = work_of(b, PH_FIXED + 3 * g + 2, tot);
   // this size's tile counter and ordering scratch, and its part of the tile order
   unsigned* next = b->tile_next.as<unsigned>() + 4 * g;
-  unsigned* order = b->tile_order.as<unsigned>();
-  for (int i = 0; i < g; ++i) order += P.fdep_total[i];
+  size_t at = 0;
+  for (int i = 0; i < g; ++i) at += P.fdep_total[i];
+  unsigned *order = b->tile_order.as<unsigned>() + at, *dense = b->tile_dense.as<unsigned>() + at;
   if (sh.dep == DEP_SEPARATE) {
-    PB_CK(launch_deposit(ds, wg, in, perm, b->row_start.as<unsigned>(), POS_DISP, err, grid_for(tot, b->sms, 3),
+    PB_CK(launch_deposit(ds, wg, in, perm, b->row_start.as<unsigned>(), b->group_max.as<unsigned>(), POS_DISP, err, grid_for(tot, b->sms, 3),
                          deposit_smem_bytes(n, TILE_Y, TILE_Z), st),
           "deposit");
     return PM_OK;
   }
   if (sh.dep == DEP_FUSED_DENSE_FIRST)
     PB_CK(launch_tile_order(ds, wg, b->row_start.as<unsigned>(), order, next + 2, b->sms, st), "tile order");
-  PB_CK(deposit_r2c_dispatch(n, ds, wg, in, perm, b->row_start.as<unsigned>(), err, next,
-                             sh.dep == DEP_FUSED_DENSE_FIRST ? order : nullptr,
+  PB_CK(deposit_r2c_dispatch(n, ds, wg, in, perm, b->row_start.as<unsigned>(), b->group_max.as<unsigned>(), err, next,
+                             sh.dep == DEP_FUSED_DENSE_FIRST ? order : nullptr, dense,
                              grid_for(tot, b->sms, sh.dep_cps ? sh.dep_cps : deposit_r2c_ctas_per_sm(n)), st),
         "fused deposit");
   return PM_OK;
@@ -557,13 +562,14 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   // clears it for this step's kick)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, Launch(st, P.max_n <= 256), true, true, b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size()),
+                          perm, err, b->sms, Launch(st, P.max_n <= 256), true, true, b->group_max.as<unsigned>(),
+                          b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size()),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
   if (P.fixed_total[PH_DEP] > 0)
     PB_CK(launch_deposit(ds, work_of(b, PH_DEP, P.fixed_total[PH_DEP]), in, perm, b->row_start.as<unsigned>(),
-                         POS_DISP, err, grid_for(P.fixed_total[PH_DEP], b->sms, 3), P.max_dep_smem, st),
+                         b->group_max.as<unsigned>(), POS_DISP, err, grid_for(P.fixed_total[PH_DEP], b->sms, 3), P.max_dep_smem, st),
           "deposit");
   const SpecKind order[5] = {SPEC_X_R2C, SPEC_Y_FWD, SPEC_Z_GREEN, SPEC_Y_INV, SPEC_X_C2R};
   auto spectral = [&](int o, int g, cudaStream_t s) -> int {
@@ -621,10 +627,10 @@ int launches_per_step(pm_batch* b) {
   const Plan& P = b->plan;
   // counting sort: 2 scan kernels and the scatter (the kick makes the histogram)
   int n = 3 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1 + 1;
-  // a fused size replaces its x R2C launch by the fused deposit (with a dense-first tile
+  // a fused size replaces its x R2C launch by the fused deposit's two (with a dense-first tile
   // order, one launch more); a separate one adds its deposit launch
   for (size_t g = 0; g < P.sizes.size(); ++g)
-    if (P.fused[g]) n += P.shape[g].dep == DEP_FUSED_INDEX ? 0 : 1;
+    if (P.fused[g]) n += P.shape[g].dep == DEP_FUSED_DENSE_FIRST ? 2 : 1;
   return n;
 }
 
@@ -670,7 +676,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
   // the row starts and permutation of the current keys (the step recomputes the same)
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, true),
+                          perm, err, b->sms, st, true, false, b->group_max.as<unsigned>()),
         "sort");
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   PB_CK(cudaEventCreate(&e0), "event");
@@ -948,11 +954,13 @@ void pm_batch_destroy(pm_batch* b) {
   b->row_count.release();
   b->row_cursor.release();
   b->scan_sums.release();
+  b->group_max.release();
   b->d_sims.release();
   b->d_prefix.release();
   b->d_err.release();
   b->tile_next.release();
   b->tile_order.release();
+  b->tile_dense.release();
   b->d_maps.release();
   b->d_one.release();
   if (b->own) cudaStreamDestroy(b->own);
@@ -1183,7 +1191,7 @@ int pm_batch_density(pm_batch* b, int sim_id, float* rho, void* stream) {
   PB_CK(cudaStreamWaitEvent(st, b->last_step, 0), "wait");
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
-                          perm, err, b->sms, st, true),
+                          perm, err, b->sms, st, true, false, b->group_max.as<unsigned>()),
         "sort");
   // this simulation's descriptor with the caller's grid as the deposit's output
   Sim s{};
@@ -1199,7 +1207,7 @@ int pm_batch_density(pm_batch* b, int sim_id, float* rho, void* stream) {
   auto* d = b->d_one.as<char>();
   const Work w{reinterpret_cast<const int*>(d + offsetof(decltype(one), prefix)), 1, one.prefix[1]};
   PB_CK(launch_deposit(reinterpret_cast<const Sim*>(d), w, state(b, b->cur), perm, b->row_start.as<unsigned>(),
-                       POS_DISP, err, grid_for(one.prefix[1], b->sms, 3), deposit_smem_bytes(s.n, TILE_Y, TILE_Z),
+                       b->group_max.as<unsigned>(), POS_DISP, err, grid_for(one.prefix[1], b->sms, 3), deposit_smem_bytes(s.n, TILE_Y, TILE_Z),
                        st),
         "deposit");
   PB_CK(cudaEventRecord(b->last_step, st), "event");

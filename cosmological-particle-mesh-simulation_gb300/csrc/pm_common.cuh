@@ -184,18 +184,19 @@ cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int
                               const CUtensorMap* maps = nullptr, int* err = nullptr);
 cudaError_t launch_fourier_grid(const Sim* sims, int ctas, Launch st);
 // fused deposit + x R2C (the density grid is not written); ctas <= 0 only prepares.
-// next_tile: one device word, the tile counter, 0 when the kernel starts.  order (optional, w.total entries): the tiles in the order to
+// next_tile: two device words, 0 at the start: the tile counter and the count of `dense`, a list (room
+// for w.total) of the tiles whose sums need two words.  order (optional, w.total entries): the tiles in the order to
 // take them (launch_tile_order).
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
-                               int* err, unsigned* next_tile, const unsigned* order, int ctas,
-                               Launch st);
+                               const unsigned* group_max, int* err, unsigned* next_tile, const unsigned* order,
+                               unsigned* dense, int ctas, Launch st);
 bool deposit_r2c_supported(int n);
 bool xrow_supported(int n);  // the x passes of size n transform rows in registers (their grid is tunable)
 int deposit_r2c_ctas_per_sm(int n);  // resident CTAs per SM of the fused deposit
 cudaError_t deposit_r2c_dispatch(int n, const Sim* sims, Work w, Parts p, const unsigned* perm,
-                                 const unsigned* row_start, int* err, unsigned* next_tile,
-                                 const unsigned* order, int ctas, Launch st);
+                                 const unsigned* row_start, const unsigned* group_max, int* err, unsigned* next_tile,
+                                 const unsigned* order, unsigned* dense, int ctas, Launch st);
 
 // sum of the first n_slices planes of an n^3 grid, float64 n^2 output (pm_diagnostics.cu)
 cudaError_t launch_project(const float* rho, int n, int n_slices, double* out, int ctas, cudaStream_t st);
@@ -214,8 +215,8 @@ cudaError_t launch_keys_disp(const Sim* sims, const Work& w, Parts p, unsigned* 
 cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsigned nrows,
                              unsigned* row_start, Launch st);
 cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsigned* perm,
-                           const unsigned* row_start, int mode, int* err, int ctas, size_t smem,
-                           Launch st);
+                           const unsigned* row_start, const unsigned* group_max, int mode, int* err, int ctas,
+                           size_t smem, Launch st);
 constexpr int KICK_UNIT = 512;  // particles per work unit of the kick
 // resident kick: the state in row order (through perm), the next keys and their row histogram
 cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, const unsigned* perm,
@@ -272,15 +273,18 @@ cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bi
 // specified).  Scratch: count and cursor (nrows each), block_sums (row_sort_block_sums).
 size_t row_sort_block_sums(unsigned nrows);
 // counted: count already holds the row histogram of keys (else it is zeroed and computed here);
-// zero: count is cleared once read; clear: nclear words set to 0.
+// zero: count is cleared once read; group_max: see row_scan; clear: nclear words set to 0.
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
                               int sms, Launch st, bool counted = false, bool zero = false,
-                              unsigned* clear = nullptr, int nclear = 0);
+                              unsigned* group_max = nullptr, unsigned* clear = nullptr, int nclear = 0);
 // row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows
-// entries; zero: count is cleared once read.  All arrays 16-byte aligned.
+// entries; zero: count is cleared once read; group_max (optional): the largest count of each 16
+// consecutive bins, for the deposit (pm_deposit.cuh).  All arrays 16-byte aligned.
 cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
-                     bool zero, Launch st);
+                     bool zero, Launch st, unsigned* group_max = nullptr);
+// group_max[g] = largest count of the row bins 16 g .. 16 g + 15 from their starts (row_scan: from the counts)
+cudaError_t launch_group_max(const unsigned* row_start, unsigned nrows, unsigned* group_max, Launch st);
 // count[r] = number of keys equal to r (count zeroed first)
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
                           Launch st);

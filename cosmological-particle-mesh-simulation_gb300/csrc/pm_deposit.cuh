@@ -4,8 +4,8 @@
 // rows (the tile plus one row and one plane below, periodic: 7 runs of the row-sorted
 // order) are found through the row starts; their CIC weights that land inside the tile are
 // added to integer accumulators in shared memory (TileSum: one 32-bit word per cell where the
-// tile's particle count allows, else a low word and a coarse word).  Integer sums do not
-// depend on the order of the atomics, so the deposit is bit-identical run to run.
+// particle counts of its row bins allow, else a low word and a coarse word).  Integer sums do
+// not depend on the order of the atomics, so the deposit is bit-identical run to run.
 #pragma once
 #include <type_traits>
 
@@ -14,7 +14,6 @@
 namespace pm {
 
 constexpr int DEP_NT = 512;
-constexpr int DEP_ROW_NT = 256;  // fused deposit with the register row transform
 
 constexpr int COARSE_SHIFT = 12;
 
@@ -29,23 +28,27 @@ __device__ __forceinline__ void acc_add(unsigned* lo, unsigned* co, int i, unsig
 // V = a 2^23 + b with a, b < 2^23; each is exact as a float (2^23 + a has a as its
 // mantissa), and fmaf(a, 2^23, b) rounds once: the value of a round-to-nearest 64-bit
 // conversion, computed on the FP32 pipe (GB300 issues 64-bit integer conversions to its
-// narrow FP64 pipe).
+// narrow FP64 pipe).  __fmul_rn: a contraction of the product with the transform's first sums would
+// make the fused deposit differ from the written density.
 __device__ __forceinline__ float fixed_to_float(unsigned l, unsigned c, float scale) {
   const unsigned est_lo = c << COARSE_SHIFT;
   const unsigned hi = (c >> (32 - COARSE_SHIFT)) + (l < est_lo ? 1u : 0u);
   const unsigned a = (hi << 9) | (l >> 23), b = l & 0x7fffffu;
   const float fa = __uint_as_float(0x4B000000u | a) - 8388608.f;
   const float fb = __uint_as_float(0x4B000000u | b) - 8388608.f;
-  return fmaf(fa, 8388608.f, fb) * scale;
+  return __fmul_rn(fmaf(fa, 8388608.f, fb), scale);
 }
 
 // How a tile's sums are held.  Every corner weight is quantised to an integer q <= 2^s and
 // added with integer atomics, so a cell's sum -- and the float made from it -- does not depend
-// on the order of the additions.  A cell receives at most one corner from each source entry
-// of its tile, so its sum is at most total * 2^s: a tile with total < 2^(32 - s) sums in one
-// 32-bit word per cell (one atomic per corner).  Tiles whose count allows s >= ONE_WORD_MIN
-// use one word at the largest such s (at most 26); denser tiles sum at 2^-26 in a low word
-// plus a coarse word (two atomics per corner).
+// on the order of the additions.  A cell receives at most one corner from each particle in four
+// rows (y, y - 1, z, z - 1) and two cells of each (x, x - 1), which lie in one row bin or two
+// adjacent ones: at most 4 or 8 times the largest count of a row bin of the tile and its three
+// lower neighbours, and at most the tile's source entries.  With that bound below 2^(32 - s) a
+// 32-bit word per cell holds the sum (one atomic per corner).  Tiles whose bound allows
+// s >= ONE_WORD_MIN use one word at the largest such s (at most 26; 23 to 24 for the 512 grid
+// of the README run, where the tile's source entries alone allowed 21); denser tiles sum at
+// 2^-26 in a low word plus a coarse word (two atomics per corner).
 constexpr int ONE_WORD_MIN = 20;
 
 struct TileSum {
@@ -53,8 +56,11 @@ struct TileSum {
   float ms;  // particle mass * 2^-(quantisation bits): the float of a sum times ms is its mass
 };
 
-__device__ __forceinline__ TileSum tile_sum(unsigned total, float mass_scale) {
-  const int bits = 32 - __clz(total);  // total < 2^bits
+// total: the tile's source entries; bin_max: the largest row bin count of the tile and its
+// lower neighbours (per_row bins to a row)
+__device__ __forceinline__ TileSum tile_sum(unsigned total, unsigned bin_max, int per_row, float mass_scale) {
+  const unsigned cap = bin_max < (1u << 28) ? bin_max * (per_row > 1 ? 8u : 4u) : 0xffffffffu;
+  const int bits = 32 - __clz(min(total, cap));  // entries of a cell < 2^bits
   const int s = min(PM_FIX_BITS, 32 - bits);
   TileSum t;
   t.s = s >= ONE_WORD_MIN ? s : 0;
@@ -67,7 +73,7 @@ __device__ __forceinline__ TileSum tile_sum(unsigned total, float mass_scale) {
 __device__ __forceinline__ float word_to_float(unsigned l, float scale) {
   const float fa = __uint_as_float(0x4B000000u | (l >> 23)) - 8388608.f;
   const float fb = __uint_as_float(0x4B000000u | (l & 0x7fffffu)) - 8388608.f;
-  return fmaf(fa, 8388608.f, fb) * scale;
+  return __fmul_rn(fmaf(fa, 8388608.f, fb), scale);
 }
 
 // The float of a cell's sum: low word l (and, for two-word tiles, coarse word c).
@@ -81,13 +87,16 @@ __device__ __forceinline__ float sum_to_float(const TileSum& t, unsigned l, unsi
 // order of cic_weights lie in rows (y, z), (y + 1, z), (y, z + 1), (y + 1, z + 1)); a row
 // outside the tile is skipped (a neighbouring tile adds it).  Four row predicates instead of a
 // test per corner measured 0.490 -> 0.468 ms per deposit (256^3 on 512^3).  ONE: one-word
-// sums (lo only).
+// sums of the whole tile (lo only); else two-word sums of the tile's planes z.x .. z.y - 1, the
+// first of which is at the start of lo and hi.
 template <bool ONE>
 __device__ __forceinline__ void deposit_particle(unsigned* lo, unsigned* hi, int n, int rs, int cx, int ly, int lz,
-                                                 const unsigned (&q)[8]) {
+                                                 int2 z, const unsigned (&q)[8]) {
   const int x1 = cx + 1 == n ? 0 : cx + 1;
-  const bool y0 = ly >= 0, y1 = ly + 1 < TY, z0 = lz >= 0, z1 = lz + 1 < TZ;
-  const int base = (lz * TY + ly) * rs;
+  const bool y0 = ly >= 0, y1 = ly + 1 < TY;
+  const bool z0 = ONE ? lz >= 0 : (lz >= z.x && lz < z.y);
+  const bool z1 = ONE ? lz + 1 < TZ : (lz + 1 >= z.x && lz + 1 < z.y);
+  const int base = ((ONE ? lz : lz - z.x) * TY + ly) * rs;
   auto add = [&](int i, unsigned v) {
     if (ONE) atomicAdd(&lo[i], v);  // result unused: a non-returning shared-memory reduction
     else acc_add(lo, hi, i, v);
@@ -119,11 +128,11 @@ __device__ __forceinline__ void quantised_weights(const Cell& c, float qscale, u
 // the deposit 6x slower on GB300.)
 template <bool ONE>
 __device__ __forceinline__ void deposit_entry(unsigned* lo, unsigned* hi, int n, int rs, float qscale, bool ok,
-                                              const Cell& c, int ly, int lz) {
+                                              const Cell& c, int ly, int lz, int2 z) {
   if (ok) {
     unsigned q[8];
     quantised_weights(c, qscale, q);
-    deposit_particle<ONE>(lo, hi, n, rs, c.x, ly, lz, q);
+    deposit_particle<ONE>(lo, hi, n, rs, c.x, ly, lz, z, q);
   }
 }
 
@@ -197,54 +206,73 @@ __device__ __forceinline__ bool source_cell(const Sim& S, const Parts& p, const 
   return ok;
 }
 
-// The 7 runs of the tile at (y0, z0): lane r < NRUN loads the first sorted index and the
-// particle count of run r.
+// The 7 runs of the tile at (y0, z0): lane r < NRUN of a group of eight loads the first sorted
+// index and the particle count of run r; and, with bin_max, the largest row bin count of the
+// tile and the three below it (all lanes of the group): group_max holds the maxima of 16
+// consecutive row bins, a tile's bins being x_bins such groups.
 struct RunLoad {
-  unsigned beg, cnt;
+  unsigned beg = 0, cnt = 0, bin_max = 0;
+  int per_row = 1;         // row bins to a row
+  float mass_scale = 0.f;  // of the simulation
 };
 
-__device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0,
-                                            int lane) {
-  RunLoad v{0u, 0u};
+__device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __restrict__ row_start,
+                                            const unsigned* __restrict__ group_max, int y0, int z0, int lane) {
+  RunLoad v;
+  const int n = S.n;
+  const int ym = y0 == 0 ? n - TY : y0 - TY, zm = z0 == 0 ? n - TZ : z0 - TZ;  // tiles below
+  const int ntile_y = n / TY;
+  const unsigned t_own = (unsigned)(z0 / TZ) * ntile_y + y0 / TY;
+  const unsigned t_zb = (unsigned)(zm / TZ) * ntile_y + y0 / TY;
+  const unsigned t_yb = (unsigned)(z0 / TZ) * ntile_y + ym / TY;
+  const unsigned t_c = (unsigned)(zm / TZ) * ntile_y + ym / TY;
+  const unsigned per_row = S.xbits ? 1u : (unsigned)x_bins(n);  // entries of row_start per x-row
+  v.per_row = (int)per_row;
+  v.mass_scale = S.mass_scale;
   if (lane < NRUN) {
-    const int n = S.n;
-    const int ym = y0 == 0 ? n - TY : y0 - TY, zm = z0 == 0 ? n - TZ : z0 - TZ;  // tiles below
-    const int ntile_y = n / TY;
-    const unsigned t_own = (unsigned)(z0 / TZ) * ntile_y + y0 / TY;
-    const unsigned t_zb = (unsigned)(zm / TZ) * ntile_y + y0 / TY;
-    const unsigned t_yb = (unsigned)(z0 / TZ) * ntile_y + ym / TY;
-    const unsigned t_c = (unsigned)(zm / TZ) * ntile_y + ym / TY;
     unsigned r0, nr;
     if (lane == 0) { r0 = t_own * (TZ * TY); nr = TZ * TY; }
     else if (lane == 1) { r0 = t_zb * (TZ * TY) + (TZ - 1) * TY; nr = TY; }
     else if (lane < 6) { r0 = t_yb * (TZ * TY) + (lane - 2) * TY + TY - 1; nr = 1; }
     else { r0 = t_c * (TZ * TY) + (TZ - 1) * TY + TY - 1; nr = 1; }
-    const unsigned per_row = S.xbits ? 1u : (unsigned)x_bins(n);  // entries of row_start per x-row
     const unsigned* s = row_start + (S.row_base + r0 * per_row);
     v.beg = __ldg(s);
     v.cnt = __ldg(s + nr * per_row) - v.beg;
+  }
+  if (group_max) {
+    const unsigned* g = group_max + S.row_base / (TZ * TY);
+    for (unsigned i = lane; i < 4 * per_row; i += 8) {
+      const unsigned t = i / per_row;
+      const unsigned tile = t == 0 ? t_own : (t == 1 ? t_zb : (t == 2 ? t_yb : t_c));
+      v.bin_max = max(v.bin_max, __ldg(&g[tile * per_row + i % per_row]));
+    }
   }
   return v;
 }
 
 // Warp-wide (all 32 lanes call it): the run table (first sorted index, and the inclusive scan
 // of the counts) of the tile whose runs the 8 lanes of this lane's group of eight loaded
-// (lane & 7 = the run).  The lanes with `write` store their group's table at s_begin / s_off.
-__device__ __forceinline__ void run_table(const RunLoad& v, int lane, unsigned* s_begin, unsigned* s_off,
-                                          bool write) {
+// (lane & 7 = the run).  The lanes with `write` store their group's table at s_begin / s_off
+// (NRUN and NRUN + 1 words).  Returns how the tile's sums are held.
+__device__ __forceinline__ TileSum run_table(const RunLoad& v, int lane, unsigned* s_begin, unsigned* s_off,
+                                             bool write) {
   const int r = lane & 7;
-  unsigned incl = v.cnt;
+  unsigned incl = v.cnt, m = v.bin_max;
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
     const unsigned t = __shfl_up_sync(FULL, incl, o, 8);
     if (r >= o) incl += t;
+    m = max(m, __shfl_xor_sync(FULL, m, o, 8));
   }
-  if (!write) return;
-  if (r < NRUN) {
-    s_begin[r] = v.beg;
-    s_off[r + 1] = incl;
+  const unsigned total = __shfl_sync(FULL, incl, NRUN - 1, 8);
+  if (write) {
+    if (r < NRUN) {
+      s_begin[r] = v.beg;
+      s_off[r + 1] = incl;
+    }
+    if (r == 0) s_off[0] = 0;
   }
-  if (r == 0) s_off[0] = 0;
+  return tile_sum(total, m, v.per_row, v.mass_scale);
 }
 
 // The particle loop of a tile: two source entries per lane and iteration, so that their
@@ -254,7 +282,7 @@ template <int MODE, int NT, bool ONE, int NN>
 __device__ __forceinline__ void deposit_sources(const Sim& S, const Parts& p, const unsigned* __restrict__ perm,
                                                 int* err, int y0, int z0, unsigned* lo, unsigned* hi, int rs,
                                                 const unsigned* s_begin, const unsigned* s_off, unsigned total,
-                                                float qscale, int tid) {
+                                                float qscale, int tid, int2 z) {
   const int lane = tid & 31, warp = tid >> 5;
   const int n = NN ? NN : S.n;
   using Runs = typename std::conditional<NN != 0, RunRegs, RunTable>::type;
@@ -270,53 +298,22 @@ __device__ __forceinline__ void deposit_sources(const Sim& S, const Parts& p, co
     int ly0 = 0, lz0 = 0, ly1 = 0, lz1 = 0;
     const bool ok0 = source_cell<MODE, NN>(S, p, q0, y0, z0, err, c0, ly0, lz0);
     const bool ok1 = source_cell<MODE, NN>(S, p, q1, y0, z0, err, c1, ly1, lz1);
-    deposit_entry<ONE>(lo, hi, n, rs, qscale, ok0, c0, ly0, lz0);
-    deposit_entry<ONE>(lo, hi, n, rs, qscale, ok1, c1, ly1, lz1);
+    deposit_entry<ONE>(lo, hi, n, rs, qscale, ok0, c0, ly0, lz0, z);
+    deposit_entry<ONE>(lo, hi, n, rs, qscale, ok1, c1, ly1, lz1, z);
   }
 }
 
-// Accumulate the tile at (y0, z0) of simulation S into lo/hi: TZ * TY rows of n cells, row r
-// of lo at word r * rs and of hi at the same offset from hi (hi is only written by two-word
-// tiles).  s_begin / s_off: NRUN + 1 words each, already holding the tile's run table when
-// runs_ready.  Done by NT threads, tid = 0 .. NT - 1 (a whole CTA, or a group of its warps
-// with one tile each: every group calls it together, it synchronises the whole CTA).  Returns
-// how the sums are held (tile_sum), also written to *ts_out when given.  NN: the grid size
-// when known at compile time (0: S.n).  zeroed: lo (and hi) are already zero, so the zeroing
-// phase and its barrier are skipped.
-template <int MODE, int NT, int NN = 0>
-__device__ __forceinline__ TileSum deposit_tile(const Sim& S, const Parts& p, const unsigned* __restrict__ perm,
-                                                const unsigned* __restrict__ row_start, int* err, int y0, int z0,
-                                                unsigned* lo, unsigned* hi, int rs, unsigned* s_begin,
-                                                unsigned* s_off, bool runs_ready = false, int tid = -1,
-                                                TileSum* ts_out = nullptr, bool zeroed = false) {
-  if (tid < 0) tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int n = NN ? NN : S.n;
-  if (!runs_ready) {
-    if (warp == 0) run_table(run_load(S, row_start, y0, z0, lane), lane, s_begin, s_off, lane < 8);
-    __syncthreads();
-  }
-  const unsigned total = s_off[NRUN];
-  const TileSum ts = tile_sum(total, S.mass_scale);
-  if (ts_out && tid == 0) *ts_out = ts;  // visible to the whole CTA after the barrier below
-  // zero the rows of lo (and of hi for two-word sums), 4 words per store
-  if (!zeroed) {
-    const int q4 = n / 4;
-    for (int i = tid; i < TZ * TY * q4; i += NT) {
-      const int off = (i / q4) * rs + (i % q4) * 4;
-      *reinterpret_cast<uint4*>(lo + off) = make_uint4(0u, 0u, 0u, 0u);
-      if (!ts.s) *reinterpret_cast<uint4*>(hi + off) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-  }
-  if (ts.s)
-    deposit_sources<MODE, NT, true, NN>(S, p, perm, err, y0, z0, lo, hi, rs, s_begin, s_off, total,
-                                    __uint_as_float((unsigned)(127 + ts.s) << 23), tid);
-  else
-    deposit_sources<MODE, NT, false, NN>(S, p, perm, err, y0, z0, lo, hi, rs, s_begin, s_off, total,
-                                     (float)(1u << PM_FIX_BITS), tid);
-  __syncthreads();
-  return ts;
+// Adds the tile at (y0, z0) of simulation S to zeroed accumulators, row r at word r * rs: one-word sums
+// (ONE, ts.s) of its TZ * TY rows of n cells in lo; two-word sums of its planes z.x .. z.y - 1 in lo
+// and hi.  s_begin / s_off: the tile's run table.  Done by NT threads, tid = 0 .. NT - 1 (a whole
+// CTA, or a group of its warps with one tile each); the caller synchronises.  NN: the grid size
+// when known at compile time (0: S.n).
+template <int MODE, int NT, bool ONE, int NN = 0>
+__device__ __forceinline__ void deposit_tile(const Sim& S, const Parts& p, const unsigned* __restrict__ perm, int* err,
+                                             int y0, int z0, unsigned* lo, unsigned* hi, int rs, const unsigned* s_begin,
+                                             const unsigned* s_off, const TileSum& ts, int2 z, int tid) {
+  const float qscale = ONE ? __uint_as_float((unsigned)(127 + ts.s) << 23) : (float)(1u << PM_FIX_BITS);
+  deposit_sources<MODE, NT, ONE, NN>(S, p, perm, err, y0, z0, lo, hi, rs, s_begin, s_off, s_off[NRUN], qscale, tid, z);
 }
 
 }  // namespace pm

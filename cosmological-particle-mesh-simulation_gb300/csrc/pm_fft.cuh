@@ -152,6 +152,14 @@ __device__ __forceinline__ void dft_composite(float2* v) {
   }
 }
 
+// exp(-2 pi i m / 6): multiples of 60 degrees
+struct W6 {
+  static __device__ __forceinline__ float2 w(int m) {
+    const float h = 0.5f, r = 0.866025403784438646763723f;
+    const float c[6] = {1.f, h, -h, -1.f, -h, h}, s[6] = {0.f, r, r, 0.f, -r, -r};
+    return make_float2(c[m], -s[m]);
+  }
+};
 // exp(-2 pi i m / 12) and exp(-2 pi i m / 24): multiples of 30 and 15 degrees
 struct W12 {
   static __device__ __forceinline__ float2 w(int m) {
@@ -171,6 +179,9 @@ struct W24 {
   }
 };
 
+template <bool INV> struct DFT<6, INV> {
+  static __device__ __forceinline__ void run(float2* v) { dft_composite<3, 2, W6, INV>(v); }
+};
 template <bool INV> struct DFT<12, INV> {
   static __device__ __forceinline__ void run(float2* v) { dft_composite<3, 4, W12, INV>(v); }
 };

@@ -64,18 +64,36 @@ __global__ void k_row_start(const unsigned* __restrict__ keys, long long n, int 
   }
 }
 
+// group_max[g] = largest particle count of the rows 16 g .. 16 g + 15 (the scan of the row counts
+// makes it where there is one, pm_sort.cu)
+__global__ void k_group_max(const unsigned* __restrict__ row_start, unsigned groups, unsigned* __restrict__ group_max) {
+  chain_begin();
+  const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= groups) return;
+  unsigned m = 0, prev = row_start[16 * g];
+  for (int i = 1; i <= 16; ++i) {
+    const unsigned next = row_start[16 * g + i];
+    m = max(m, next - prev);
+    prev = next;
+  }
+  group_max[g] = m;
+}
+
 // ---------------------------------------------------------------------------------
 // deposit: one CTA per tile (pm_deposit.cuh), then the tile's rows are written once
 // ---------------------------------------------------------------------------------
 template <int MODE>
 __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ sims, Work w, Parts p,
                                                        const unsigned* __restrict__ perm,
-                                                       const unsigned* __restrict__ row_start, int* err) {
+                                                       const unsigned* __restrict__ row_start,
+                                                       const unsigned* __restrict__ group_max, int* err) {
   chain_begin();
   extern __shared__ uint4 acc_raw[];
-  __shared__ unsigned s_begin[NSRC];
-  __shared__ unsigned s_off[NSRC + 1];
+  __shared__ unsigned s_begin[NRUN];
+  __shared__ unsigned s_off[NRUN + 1];
+  __shared__ TileSum s_ts;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   for (int unit = blockIdx.x; unit < w.total; unit += gridDim.x) {
     const int si = locate_sim(w, unit);
     const Sim& S = sims[si];
@@ -83,20 +101,37 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
     const int n = S.n;
     const int ntile_y = n / TY;
     const int y0 = (local % ntile_y) * TY, z0 = (local / ntile_y) * TZ;
-    unsigned* lo = reinterpret_cast<unsigned*>(acc_raw);
-    unsigned* hi = lo + TZ * TY * n;
-    const TileSum ts = deposit_tile<MODE, DEP_NT>(S, p, perm, row_start, err, y0, z0, lo, hi, S.n, s_begin, s_off);
-    for (int row = warp; row < TZ * TY; row += DEP_NT / 32) {
-      const uint4* l4 = reinterpret_cast<const uint4*>(lo + row * n);
-      const uint4* h4 = reinterpret_cast<const uint4*>(hi + row * n);
-      float4* dst = reinterpret_cast<float4*>(S.rho + ((long long)(z0 + row / TY) * n + (y0 + row % TY)) * n);
-      for (int x4 = lane; x4 < n / 4; x4 += 32) {
-        const uint4 l = l4[x4], h = ts.s ? make_uint4(0u, 0u, 0u, 0u) : h4[x4];
-        dst[x4] = make_float4(sum_to_float(ts, l.x, h.x), sum_to_float(ts, l.y, h.y), sum_to_float(ts, l.z, h.z),
-                              sum_to_float(ts, l.w, h.w));
-      }
+    if (warp == 0) {
+      const TileSum t =
+          run_table(run_load(S, row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off, lane < 8);
+      if (lane == 0) s_ts = t;
     }
+    for (int i = threadIdx.x; i < TZ * TY * n / 4; i += DEP_NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
+    const TileSum ts = s_ts;
+    const int rows = ts.s ? TZ * TY : TZ * TY / 2;
+    for (int half = 0; half < TZ * TY / rows; ++half) {
+      if (ts.s)
+        deposit_tile<MODE, DEP_NT, true>(S, p, perm, err, y0, z0, acc, nullptr, n, s_begin, s_off, ts, make_int2(0, TZ),
+                                         threadIdx.x);
+      else  // half the planes at a time: low words, then coarse words
+        deposit_tile<MODE, DEP_NT, false>(S, p, perm, err, y0, z0, acc, acc + TZ * TY / 2 * n, n, s_begin, s_off, ts,
+                                          make_int2(half * TZ / 2, (half + 1) * TZ / 2), threadIdx.x);
+      __syncthreads();
+      for (int r = warp; r < rows; r += DEP_NT / 32) {
+        const int row = half * rows + r;
+        uint4* l4 = reinterpret_cast<uint4*>(acc + r * n);
+        uint4* h4 = reinterpret_cast<uint4*>(acc + (r + TZ * TY / 2) * n);  // (two-word tiles)
+        float4* dst = reinterpret_cast<float4*>(S.rho + ((long long)(z0 + row / TY) * n + (y0 + row % TY)) * n);
+        for (int x4 = lane; x4 < n / 4; x4 += 32) {
+          const uint4 l = l4[x4], h = ts.s ? make_uint4(0u, 0u, 0u, 0u) : h4[x4];
+          dst[x4] = make_float4(sum_to_float(ts, l.x, h.x), sum_to_float(ts, l.y, h.y), sum_to_float(ts, l.z, h.z),
+                                sum_to_float(ts, l.w, h.w));
+          if (!ts.s) l4[x4] = h4[x4] = make_uint4(0u, 0u, 0u, 0u);  // for the other half
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -633,7 +668,7 @@ cudaError_t deposit_prepare() {
   });
 }
 
-size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * sizeof(unsigned long long); }
+size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * sizeof(unsigned); }
 
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
                             int* err, int ctas, Launch st) {
@@ -655,6 +690,11 @@ cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsig
   return cudaGetLastError();
 }
 
+cudaError_t launch_group_max(const unsigned* row_start, unsigned nrows, unsigned* group_max, Launch st) {
+  launch_chained(k_group_max, (int)((nrows / 16 + 127) / 128), 128, 0, st, row_start, nrows / 16, group_max);
+  return cudaGetLastError();
+}
+
 // Order in which the fused deposit takes its tiles: the dense tiles first.  A tile's work is
 // its source-entry count, which clustering makes very uneven; a dense tile taken late runs on
 // alone after the others have finished.  Tiles with more than twice the mean count go to the
@@ -670,7 +710,7 @@ __global__ void k_tile_order(const Sim* __restrict__ sims, Work w, const unsigne
     const int y0 = (local % (n / TY)) * TY, z0 = (local / (n / TY)) * TZ;
     unsigned cnt = 0;
 #pragma unroll
-    for (int r = 0; r < NRUN; ++r) cnt += run_load(S, row_start, y0, z0, r).cnt;
+    for (int r = 0; r < NRUN; ++r) cnt += run_load(S, row_start, nullptr, y0, z0, r).cnt;
     // mean source entries per tile: each particle once, plus its tile's last plane / row / corner
     const double ntiles = (double)(n / TY) * (n / TZ);
     const double mean = (double)S.np * (1.0 + 1.0 / TZ + 1.0 / TY + 1.0 / (TY * TZ)) / ntiles;
@@ -688,11 +728,11 @@ cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* ro
 }
 
 cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsigned* perm,
-                           const unsigned* row_start, int mode, int* err, int ctas, size_t smem,
-                           Launch st) {
+                           const unsigned* row_start, const unsigned* group_max, int mode, int* err, int ctas,
+                           size_t smem, Launch st) {
   if (cudaError_t e = deposit_prepare()) return e;
-  if (mode == POS_ABS) launch_chained(k_deposit<POS_ABS>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, err);
-  else launch_chained(k_deposit<POS_DISP>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, err);
+  if (mode == POS_ABS) launch_chained(k_deposit<POS_ABS>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, group_max, err);
+  else launch_chained(k_deposit<POS_DISP>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, group_max, err);
   return cudaGetLastError();
 }
 

@@ -54,44 +54,41 @@ __host__ __device__ constexpr bool tma_lines(int n) { return n >= 32 && line_box
 // transformed line by line, runs 1024.
 __host__ __device__ constexpr int line_nt(int n) { return line_small(n) ? 256 : (n == 768 ? 1024 : 512); }
 __host__ __device__ constexpr int line_ctas_per_sm(int n) { return line_small(n) ? 2 : 1; }
-constexpr int XTMA_NT = 1024;  // x passes
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
   return (size_t)n * cline_width(n) * cline_bpc(n) * sizeof(float2);
 }
 __host__ __device__ constexpr size_t tma_smem_bytes(int n) { return TMA_STAGES * tma_stage_bytes(n) + 64; }
 
-// x passes with the row transform in registers (power-of-two n, 64 <= n <= 512): a row of
-// M = n/2 complex points is factored M = P x Q and held by T lanes of a warp
-// (n: P x Q, T) -- 64: 8x4, 4; 128: 8x8, 8; 256: 16x8, 8; 512: 16x16, 16;
-// 96: 4x12, 4; 192: 8x12, 4; 384: 8x24, 8
-__host__ __device__ constexpr bool xrow_ok(int n) {
-  return n == 64 || n == 128 || n == 256 || n == 512 || n == 96 || n == 192 || n == 384;
-}
+// x passes with the row transform in registers (n >= 32): a row of M = n/2 complex points is held
+// by T lanes of a warp and transformed in passes of radix A, (B,) C, M = A C or A B C, through an
+// exchange buffer of the row that only its warp synchronises on
+// (n: radices, T) -- 32: 4x4, 4; 48: 4x6, 2; 64: 8x4, 4; 96: 4x12, 4; 128: 8x8, 8; 192: 8x12, 4;
+// 256: 16x8, 8; 384: 8x24, 8; 512: 16x16, 16; 768: 8x8x6, 16; 1024: 8x8x8, 32
 // (the radix-3 rows with the smaller factor first: x C2R per 134M cells 96: 0.119 -> 0.115,
-// 192: 0.315 -> 0.257, 384: 0.269 -> 0.256 ms)
-__host__ __device__ constexpr int xrow_P(int n) {
-  return n % 3 == 0 ? (n == 96 ? 4 : 8) : (n >= 256 ? 16 : 8);
+// 192: 0.315 -> 0.257, 384: 0.269 -> 0.256 ms.  Two passes for 768 and 1024 would hold 24 x 16 or
+// 32 x 16 points in 64 registers a lane and more; three passes hold 24 and 16 points.)
+__host__ __device__ constexpr bool xrow_ok(int n) { return n >= 32; }
+__host__ __device__ constexpr int xrow_A(int n) {
+  return n >= 768 ? 8 : (n % 3 == 0 ? (n <= 96 ? 4 : 8) : (n >= 256 ? 16 : (n == 32 ? 4 : 8)));
 }
-__host__ __device__ constexpr int xrow_Q(int n) { return n / 2 / xrow_P(n); }
+__host__ __device__ constexpr int xrow_B(int n) { return n >= 768 ? 8 : 1; }
+__host__ __device__ constexpr int xrow_C(int n) { return n / 2 / (xrow_A(n) * xrow_B(n)); }
 __host__ __device__ constexpr int xrow_T(int n) {
-  return n == 192 ? 4 : (xrow_Q(n) < xrow_P(n) ? xrow_Q(n) : xrow_P(n));
+  return n == 1024 ? 32 : (n == 768 || n == 512 ? 16 : (n == 48 ? 2 : (n % 3 == 0 && n != 384 ? 4 : (n <= 64 ? 4 : 8))));
 }
 __host__ __device__ constexpr int xrow_rows_per_warp(int n) { return 32 / xrow_T(n); }
+// complex elements of a row's exchange buffer: C rows of A (padded) in two passes; in three,
+// the row with one element of padding after every A
+__host__ __device__ constexpr int xrow_exchange(int n) {
+  return xrow_B(n) == 1 ? xrow_C(n) * (xrow_A(n) + 1) : n / 2 + n / 2 / xrow_A(n);
+}
 // threads of a row-transform CTA: up to 8 warps, their exchange buffers within 40 KB of
 // static shared memory
-__host__ __device__ constexpr int xrow_warp_bytes(int n) {
-  return xrow_rows_per_warp(n) * xrow_Q(n) * (xrow_P(n) + 1) * 8;
-}
+__host__ __device__ constexpr int xrow_warp_bytes(int n) { return xrow_rows_per_warp(n) * xrow_exchange(n) * 8; }
 __host__ __device__ constexpr int xrow_nt(int n) {
   return 32 * (40960 / xrow_warp_bytes(n) < 8 ? (40960 / xrow_warp_bytes(n) < 1 ? 1 : 40960 / xrow_warp_bytes(n)) : 8);
 }
-
-// x passes fed by bulk copies into a double-buffered staging area (one simulation per launch)
-__host__ __device__ constexpr bool tma_rows(int n);
-__host__ __device__ constexpr int xrow_stage_floats(int n) { return n + 4; }  // (n/2 + 2) complex: bulk size % 16 == 0
-__host__ __device__ constexpr size_t xtma_fft_bytes(int n);
-__host__ __device__ constexpr size_t xtma_smem_bytes(int n);
 
 __host__ __device__ constexpr size_t x_smem_bytes(int n) {
   return (size_t)(n / 2 + 1) * (cx_rows(n) + 1) * sizeof(float2);
@@ -99,13 +96,6 @@ __host__ __device__ constexpr size_t x_smem_bytes(int n) {
 __host__ __device__ constexpr size_t line_smem_bytes(int n) {
   return (size_t)n * cline_width(n) * cline_bpc(n) * sizeof(float2);
 }
-__host__ __device__ constexpr size_t xtma_fft_bytes(int n) { return x_smem_bytes(n); }
-// two staging buffers of cx_rows(n) rows x (n + 4) floats, the FFT buffer, two mbarriers
-__host__ __device__ constexpr size_t xtma_smem_bytes(int n) {
-  return 2 * (size_t)cx_rows(n) * xrow_stage_floats(n) * sizeof(float) + xtma_fft_bytes(n) + 64;
-}
-__host__ __device__ constexpr bool tma_rows(int n) { return n >= 32 && xtma_smem_bytes(n) <= 227 * 1024; }
-
 // ---------------------------------------------------------------------------------
 // x_r2c
 // ---------------------------------------------------------------------------------
@@ -500,59 +490,105 @@ __global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(co
 }
 
 // ---------------------------------------------------------------------------------
-// x passes, row transform in registers (xrow_ok sizes).  T lanes of a warp own one row of
-// M = P Q complex points, j = Q a + b, k = c + P d:
-//   pass 1  lane t, b = t + T i: P-point DFT over a of z[Q a + b], times w_M^(b c)
+// x passes, row transform in registers (xrow_ok sizes).  T lanes of a warp own one row of M
+// complex points.  Two passes, M = A C, j = C a + b, k = c + A d:
+//   pass 1  lane t, b = t + T i: A-point DFT over a of z[C a + b], times w_M^(b c)
 //   (shared-memory exchange inside the row, synchronised by the warp alone)
-//   pass 2  lane t, c = t + T i: Q-point DFT over b -> Z[c + P d]
+//   pass 2  lane t, c = t + T i: C-point DFT over b -> Z[c + A d]
+// Three passes, M = A B C: Stockham passes of radix A, B, C on the row's exchange buffer, element
+// e at e + e / A (pass 1 stores A e + r: without the padding all lanes would hit one bank).
 // R2C: z[j] = x[2j] + i x[2j+1] read straight from the density rows, Z untangled into the
 // half spectrum.  C2R: the spectrum row is staged, tangled into pass 1, and z written as
 // pairs of reals.  Loads and stores of T lanes are consecutive (coalesced).  A work unit
 // is the 32 / T rows of one warp.
 // ---------------------------------------------------------------------------------
-// Pass 1, the in-row exchange and pass 2 of a row transform; v holds z[Q a + t + T i] on
-// entry, o holds Z[t + T i + P d] on exit.  rb: the row's exchange buffer (Q (P + 1)).
+// A row's passes; v holds z[(M / A) a + t + T i] on entry, o holds Z[t + T i + (M / C) d] on exit.
+// rb: the row's exchange buffer.
+template <int N> constexpr int xrow_NB1 = N / 2 / xrow_A(N) / xrow_T(N);  // A-point DFTs of a lane
+template <int N> constexpr int xrow_NB2 = N / 2 / xrow_C(N) / xrow_T(N);  // C-point DFTs of a lane
+
 template <int N, bool INV>
-__device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_Q(N) / xrow_T(N)][xrow_P(N)],
-                                               float2 (&o)[xrow_P(N) / xrow_T(N)][xrow_Q(N)], float2* rb, int t,
-                                               const float2* __restrict__ tw) {
-  constexpr int M = N / 2, P = xrow_P(N), Q = xrow_Q(N), T = xrow_T(N);
-  constexpr int NB1 = Q / T, NB2 = P / T;
+__device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N>][xrow_A(N)], float2 (&o)[xrow_NB2<N>][xrow_C(N)],
+                                               float2* rb, int t, const float2* __restrict__ tw) {
+  constexpr int M = N / 2, A = xrow_A(N), B = xrow_B(N), C = xrow_C(N), T = xrow_T(N);
+  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
+  auto twiddle = [&](int m) {
+    float2 w = __ldg(&tw[m * 2]);
+    if (INV) w.y = -w.y;
+    return w;
+  };
+  if constexpr (B == 1) {
 #pragma unroll
-  for (int i = 0; i < NB1; ++i) {
-    const int b = t + T * i;
-    DFT<P, INV>::run(v[i]);
+    for (int i = 0; i < NB1; ++i) {
+      const int b = t + T * i;
+      DFT<A, INV>::run(v[i]);
 #pragma unroll
-    for (int c = 1; c < P; ++c) {
-      float2 wv = __ldg(&tw[((b * c) % M) * 2]);
-      if (INV) wv.y = -wv.y;
-      v[i][c] = cmul(v[i][c], wv);
+      for (int c = 1; c < A; ++c) v[i][c] = cmul(v[i][c], twiddle((b * c) % M));
     }
-  }
-  __syncwarp();
+    __syncwarp();
 #pragma unroll
-  for (int i = 0; i < NB1; ++i)
+    for (int i = 0; i < NB1; ++i)
 #pragma unroll
-    for (int c = 0; c < P; ++c) rb[(t + T * i) * (P + 1) + c] = v[i][c];
-  __syncwarp();
+      for (int c = 0; c < A; ++c) rb[(t + T * i) * (A + 1) + c] = v[i][c];
+    __syncwarp();
 #pragma unroll
-  for (int i = 0; i < NB2; ++i) {
+    for (int i = 0; i < NB2; ++i) {
 #pragma unroll
-    for (int b = 0; b < Q; ++b) o[i][b] = rb[b * (P + 1) + t + T * i];
-    DFT<Q, INV>::run(o[i]);
+      for (int b = 0; b < C; ++b) o[i][b] = rb[b * (A + 1) + t + T * i];
+      DFT<C, INV>::run(o[i]);
+    }
+  } else {
+    constexpr int NB = M / B / T;  // B-point DFTs of a lane
+    static_assert(M / B % T == 0, "row plan");
+    auto at = [](int e) { return e + e / A; };
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NB1; ++i) {
+      DFT<A, INV>::run(v[i]);
+#pragma unroll
+      for (int r = 0; r < A; ++r) rb[at((t + T * i) * A + r)] = v[i][r];
+    }
+    __syncwarp();
+    float2 u[NB][B];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int j = t + T * i, k = j % A;
+#pragma unroll
+      for (int r = 0; r < B; ++r) u[i][r] = rb[at(j + r * (M / B))];
+#pragma unroll
+      for (int r = 1; r < B; ++r) u[i][r] = cmul(u[i][r], twiddle(r * k * (M / (A * B))));
+      DFT<B, INV>::run(u[i]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int j = t + T * i, k = j % A, base = (j - k) * B + k;
+#pragma unroll
+      for (int r = 0; r < B; ++r) rb[at(base + r * A)] = u[i][r];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NB2; ++i) {
+      const int j = t + T * i;
+#pragma unroll
+      for (int r = 0; r < C; ++r) o[i][r] = rb[at(j + r * (M / C))];
+#pragma unroll
+      for (int r = 1; r < C; ++r) o[i][r] = cmul(o[i][r], twiddle(r * j));
+      DFT<C, INV>::run(o[i]);
+    }
   }
 }
 
 // R2C end of a row: Z (in o) is untangled into the half-spectrum row dst[0..M].
 template <int N>
-__device__ __forceinline__ void xrow_untangle_store(const float2 (&o)[xrow_P(N) / xrow_T(N)][xrow_Q(N)], float2* rb,
+__device__ __forceinline__ void xrow_untangle_store(const float2 (&o)[xrow_NB2<N>][xrow_C(N)], float2* rb,
                                                     int t, const float2* __restrict__ tw, float2* __restrict__ dst) {
-  constexpr int M = N / 2, P = xrow_P(N), Q = xrow_Q(N), T = xrow_T(N), NB2 = P / T;
+  constexpr int M = N / 2, C = xrow_C(N), T = xrow_T(N);
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < NB2; ++i)
+  for (int i = 0; i < xrow_NB2<N>; ++i)
 #pragma unroll
-    for (int d = 0; d < Q; ++d) rb[t + T * i + P * d] = o[i][d];
+    for (int d = 0; d < C; ++d) rb[t + T * i + M / C * d] = o[i][d];
   __syncwarp();
   // X[k] = E[k] + W^k O[k], k = 0..M
   for (int k = t; k <= M; k += T) {
@@ -568,10 +604,10 @@ template <int N, bool C2R>
 __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ sims, Work w) {
   chain_begin();
   constexpr int XR_NT = xrow_nt(N);
-  constexpr int M = N / 2, P = xrow_P(N), Q = xrow_Q(N), T = xrow_T(N), RPW = 32 / T;
-  constexpr int RB = Q * (P + 1);  // exchange buffer of a row (>= M + 1)
-  constexpr int NB1 = Q / T, NB2 = P / T;
-  static_assert(P * Q == M && Q % T == 0 && P % T == 0 && RB >= M + 1, "row plan");
+  constexpr int M = N / 2, A = xrow_A(N), B = xrow_B(N), C = xrow_C(N), T = xrow_T(N), RPW = 32 / T;
+  constexpr int RB = xrow_exchange(N);  // exchange buffer of a row (>= M + 1)
+  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
+  static_assert(A * B * C == M && NB1 * A * T == M && NB2 * C * T == M && RB >= M + 1, "row plan");
   __shared__ float2 sbuf[XR_NT / 32][RPW][RB];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane / T, t = lane % T;
@@ -582,14 +618,14 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
     const Sim& S = sims[si];
     const long long row = ((long long)unit - __ldg(&w.prefix[si])) * RPW + sub;
     const float2* __restrict__ tw = S.tw;
-    float2 v[NB1][P];
-    float2 o[NB2][Q];
+    float2 v[NB1][A];
+    float2 o[NB2][C];
     if (!C2R) {
       const float2* __restrict__ src = reinterpret_cast<const float2*>(S.rho) + row * M;
 #pragma unroll
       for (int i = 0; i < NB1; ++i)
 #pragma unroll
-        for (int a = 0; a < P; ++a) v[i][a] = __ldg(&src[Q * a + t + T * i]);
+        for (int a = 0; a < A; ++a) v[i][a] = __ldg(&src[M / A * a + t + T * i]);
       xrow_transform<N, false>(v, o, rb, t, tw);
       xrow_untangle_store<N>(o, rb, t, tw, S.spec + row * S.pitch);
     } else {
@@ -611,8 +647,8 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
 #pragma unroll
       for (int i = 0; i < NB1; ++i)
 #pragma unroll
-        for (int a = 0; a < P; ++a) {
-          const int j = Q * a + t + T * i;
+        for (int a = 0; a < A; ++a) {
+          const int j = M / A * a + t + T * i;
           const float2 xk = rb[j], xm = rb[M - j];
           const float2 ap = cadd(xk, conjf2(xm)), bm = csub(xk, conjf2(xm));
           const float2 tt = cmul(conjf2(__ldg(&tw[j])), bm);
@@ -623,7 +659,7 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
 #pragma unroll
       for (int i = 0; i < NB2; ++i)
 #pragma unroll
-        for (int d = 0; d < Q; ++d) dst[t + T * i + P * d] = o[i][d];
+        for (int d = 0; d < C; ++d) dst[t + T * i + M / C * d] = o[i][d];
     }
   }
 }
@@ -653,335 +689,248 @@ inline bool encode_spectrum_map(CUtensorMap* tm, const void* spec, int n, bool z
 }
 
 // ---------------------------------------------------------------------------------
-// x passes fed by bulk copies, one simulation per launch.
-//
-// Persistent CTA with two staging buffers.  The NR rows of a unit stream into a staging
-// buffer (one 1-D bulk copy per row, completing on an mbarrier); unit i is transposed out
-// of its buffer into the padded line-interleaved FFT buffer, the buffer is refilled at
-// once with unit i+2, and the transform and its coalesced global stores follow.
+// fused deposit + x R2C (the sizes with a register row transform): a CTA deposits tiles of
+// TZ x TY rows into shared memory (pm_deposit.cuh), transforms each row along x in place and
+// writes the half-spectrum rows, so the density grid never goes to HBM.
 // ---------------------------------------------------------------------------------
-template <int N, bool C2R>
-__global__ void __launch_bounds__(XTMA_NT, 1) k_x_tma(const Sim* __restrict__ sims, Work w, int* err) {
-  constexpr int M = N / 2, NR = cx_rows(N), LS = NR + 1, RS = xrow_stage_floats(N);
-  constexpr int NT = XTMA_NT;
-  // bytes copied per row: R2C reads n floats; C2R reads M + 2 complex (= RS floats)
-  constexpr unsigned ROWB = C2R ? RS * 4u : N * 4u;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  float* stage[2] = {reinterpret_cast<float*>(smem_raw),
-                     reinterpret_cast<float*>(smem_raw + (size_t)NR * RS * sizeof(float))};
-  float2* F = reinterpret_cast<float2*>(smem_raw + 2 * (size_t)NR * RS * sizeof(float));
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * (size_t)NR * RS * sizeof(float) + xtma_fft_bytes(N));
-  const long long nrows = (long long)N * N;
-  const int nunits = w.total;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  chain_begin();
-  // warp 0 issues the copies of one unit: lane r copies rows r, r + 32, ...
-  auto issue = [&](int unit, int st) {
-    const int si = locate_sim(w, unit);
-    const Sim& S = sims[si];
-    const long long row0 = (long long)(unit - __ldg(&w.prefix[si])) * NR;
-    const int rows = (int)(nrows - row0 < NR ? nrows - row0 : NR);
-    if (lane == 0) mbar_expect_tx(&bar[st], (unsigned)rows * ROWB);
-    __syncwarp();
-    for (int r = lane; r < rows; r += 32) {
-      const void* src = C2R ? (const void*)(S.spec + (row0 + r) * S.pitch) : (const void*)(S.rho + (row0 + r) * N);
-      bulk_load(stage[st] + r * RS, src, ROWB, &bar[st]);
-    }
-  };
-  int unit = blockIdx.x;
-  if (warp == 0) {
-    if (unit < nunits) issue(unit, 0);
-    if (unit + (int)gridDim.x < nunits) issue(unit + gridDim.x, 1);
-  }
-  unsigned parity = 0;
-  for (int it = 0; unit < nunits; unit += gridDim.x, ++it) {
-    const int st = it & 1;
-    const int si = locate_sim(w, unit);
-    const Sim& S = sims[si];
-    const long long row0 = (long long)(unit - __ldg(&w.prefix[si])) * NR;
-    const bool ok = mbar_wait(&bar[st], (parity >> st) & 1u);
-    parity ^= 1u << st;
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) set_error(err, ERR_TIMEOUT);
-      break;
-    }
-    const float2* sg = reinterpret_cast<const float2*>(stage[st]);
-    if (!C2R) {
-      // z[j] = x[2j] + i x[2j+1]: staged row r, complex j -> F[j][r]
-      for (int u = threadIdx.x; u < NR * M; u += NT) {
-        const int r = u / M, j = u % M;
-        F[j * LS + r] = sg[r * (RS / 2) + j];
-      }
-    } else {
-      // tangle: Z[k] = (X[k] + X*[M-k]) + i W^-k (X[k] - X*[M-k]), pairs (k, M-k)
-      for (int u = threadIdx.x; u < NR * (M / 2 + 1); u += NT) {
-        const int r = u / (M / 2 + 1), k = u % (M / 2 + 1);
-        const float2 xk = sg[r * (RS / 2) + k];
-        const float2 xm = sg[r * (RS / 2) + (M - k)];
-        const float2 a = cadd(xk, conjf2(xm));
-        const float2 b = csub(xk, conjf2(xm));
-        const float2 w = __ldg(&S.tw[k]);
-        const float2 t = cmul(conjf2(w), b);
-        F[k * LS + r] = make_float2(a.x - t.y, a.y + t.x);
-        if (k != 0 && 2 * k != M) {
-          const float2 t2 = cmul(w, conjf2(b));
-          F[(M - k) * LS + r] = make_float2(a.x - t2.y, -a.y + t2.x);
-        }
-      }
-    }
-    __syncthreads();  // staging buffer st is free again: refill it with the unit after next
-    const int after = unit + 2 * (int)gridDim.x;
-    if (warp == 0 && after < nunits) issue(after, st);
-    fft_lines<M, NR, LS, NT, C2R>(F, S.tw, 2);
-    if (!C2R) {
-      float2* __restrict__ dst = S.spec;
-      const int P = S.pitch;
-      for (int u = threadIdx.x; u < NR * (M + 1); u += NT) {
-        const int r = u / (M + 1), k = u % (M + 1);
-        if (row0 + r >= nrows) continue;
-        const float2 zk = F[(k == M ? 0 : k) * LS + r];
-        const float2 zc = conjf2(F[(k == 0 ? 0 : M - k) * LS + r]);
-        const float2 e = cscale(cadd(zk, zc), 0.5f);
-        const float2 o = cscale(mul_mi<false>(csub(zk, zc)), 0.5f);
-        dst[(row0 + r) * P + k] = cadd(e, cmul(__ldg(&S.tw[k]), o));
-      }
-    } else {
-      float2* __restrict__ dst = reinterpret_cast<float2*>(S.phi);
-      for (int u = threadIdx.x; u < NR * M; u += NT) {
-        const int r = u / M, j = u % M;
-        if (row0 + r < nrows) dst[(row0 + r) * M + j] = F[j * LS + r];
-      }
-    }
-    __syncthreads();  // F is rewritten by the next unit
-  }
+__host__ __device__ constexpr bool deposit_r2c_ok(int n) { return xrow_ok(n); }
+// words of a tile row: its cells, or the exchange buffer of its transform, which overlays them
+__host__ __device__ constexpr int dep_row_words(int n) {
+  return 2 * xrow_exchange(n) > n ? 2 * xrow_exchange(n) : n;
+}
+__host__ __device__ constexpr size_t dep_tile_bytes(int n) { return (size_t)TZ * TY * dep_row_words(n) * sizeof(unsigned); }
+constexpr int DEP_ROW_NT = 256;  // threads (the 16 rows of a 1024 tile take them twice: 3.95 ms, 512 threads 4.34)
+// Tiles per CTA: the row transform of a tile's 16 rows keeps 16 / T warps busy (T lanes per row),
+// so on the sizes with T < 16 a CTA takes several tiles at once -- its warps split into one
+// group per tile for the particle loop and share all the rows in the transform.
+__host__ __device__ constexpr int dep_tiles(int n) {
+  return n == 1024 ? 1 : (16 / xrow_T(n) > 4 ? 4 : 16 / xrow_T(n));
+}
+// CTAs per SM, which bounds the registers of a thread: four (64) where the row plan leaves few
+// spills (512: 423 us, three 466; 256 in an ensemble 234, three 262; 64 and 96 lose 10%), else three
+// (192: 134, two 144; 768: 1589, two 1717); five spill (512: 495).  With one-word sums alone in the
+// kernel the 512 grid then takes 402 us early and clustered, the 1024 grid 3.61 ms (start of this
+// layout: 442, 445 and 6.12, with a low and a coarse word for every cell at three CTAs).
+__host__ __device__ constexpr int dep_ctas_bound(int n) { return n == 128 || n == 256 || n == 512 ? 4 : 3; }
+
+// The tile at place i of the order (`order`, optional, lists the tiles dense-first): its
+// simulation and first row / plane (false: none).
+template <int N>
+__device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restrict__ order, int i, int& si, int& y0,
+                                         int& z0) {
+  si = 0; y0 = z0 = 0;
+  if (i >= w.total) return false;
+  const int unit = order ? (int)__ldg(&order[i]) : i;
+  si = locate_sim(w, unit);
+  const int local = unit - __ldg(&w.prefix[si]);
+  y0 = (local % (N / TY)) * TY;
+  z0 = (local / (N / TY)) * TZ;
+  return true;
 }
 
-// ---------------------------------------------------------------------------------
-// fused deposit + x R2C: one CTA per deposit tile.  The tile's TZ x TY rows are deposited
-// into shared memory (pm_deposit.cuh), converted to float and transformed along x -- by
-// the register row transform (T lanes per row) where the size has one, else transposed
-// into a padded line-interleaved buffer (reusing the accumulator space) -- and the
-// half-spectrum rows are written directly, so the density grid never goes to HBM.
-// ---------------------------------------------------------------------------------
-// accumulators: 2 words per cell, >= (n/2) * (TZ*TY + 1) * sizeof(float2) for the
-// shared-memory transform; with the register row transform each row's low and high words
-// are adjacent (row r at word 2 r n) and the row's exchange buffer overlays them
-__host__ __device__ constexpr size_t deposit_r2c_smem_bytes(int n) { return (size_t)2 * TZ * TY * n * sizeof(unsigned); }
-__host__ __device__ constexpr int deposit_r2c_nt(int n) { return xrow_ok(n) ? DEP_ROW_NT : DEP_NT; }
-// sizes whose tile (TZ * TY rows of n cells) divides evenly over the block
-__host__ __device__ constexpr bool deposit_r2c_ok(int n) { return (TZ * TY * n) % deposit_r2c_nt(n) == 0; }
-
-// Tiles per CTA of the fused deposit: the register row transform of a tile's 16 rows keeps
-// 16 / T warps busy (T lanes per row), so on the sizes with T < 16 a CTA takes several tiles
-// at once -- its warps split into one group per tile for the particle loop and share all the
-// rows in the transform -- as long as their accumulators stay within 72 KB (three CTAs per
-// SM).  The 192 grid (T = 4, 48 complex values per lane) takes its four tiles at two CTAs per
-// SM with 128 registers instead (measured 0.90 -> 0.87 ms per 134M-cell deposit).
-__host__ __device__ constexpr int dep_ctas_bound(int n) { return n == 192 ? 2 : (xrow_ok(n) ? 3 : 2); }
-__host__ __device__ constexpr int dep_tiles(int n) {
-  int t = xrow_ok(n) ? 16 / xrow_T(n) : 1;
-  while (t > 1 && (size_t)t * deposit_r2c_smem_bytes(n) > (n == 192 ? 100 : 72) * 1024) t /= 2;
-  return t;
+// The x R2C of tile rows: row r's sums at acc + r * stride (TWO: its coarse words HO words further
+// on); T lanes to a row, whose exchange buffer overlays its low words once they are read.  A
+// batch is the rows that the CTA's warps hold at once.  f(tg): whether to store tile tg's rows and
+// where they belong; `between` runs in warp 0 before the first transform, `after` behind the
+// last; every row is left zero.
+template <int N, int NT, int TPB, bool TWO, class H, class F, class G>
+__device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsigned* acc, int stride, const TileSum* s_ts,
+                                              H tile, F between, G after) {
+  constexpr int NL = TZ * TY, M = N / 2, A = xrow_A(N), C = xrow_C(N), T = xrow_T(N), RPW = 32 / T;
+  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
+  constexpr int BROWS = NT / 32 * RPW, NBATCH = (TPB * NL + BROWS - 1) / BROWS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sub = lane / T, t = lane % T;
+#pragma unroll 1
+  for (int batch = 0; batch < NBATCH; ++batch) {
+    if (batch * BROWS + warp * RPW >= TPB * NL) break;  // warp-uniform (a warp's rows are all in or all out)
+    const int R = batch * BROWS + warp * RPW + sub, tg = R / NL, r = R % NL;
+    unsigned* row = acc + R * stride;
+    float2* rb = reinterpret_cast<float2*>(row);
+    int si, y0, z0;
+    const bool has = tile(tg, si, y0, z0);
+    const Sim& S = sims[si];
+    const TileSum ts = s_ts[tg];
+    float2 v2[NB1][A];
+    float2 o2[NB2][C];
+    const uint2* l2 = reinterpret_cast<const uint2*>(row);
+    const uint2* h2 = reinterpret_cast<const uint2*>(row + dep_row_words(N));
+#pragma unroll
+    for (int i = 0; i < NB1; ++i)
+#pragma unroll
+      for (int a = 0; a < A; ++a) {
+        const int j = M / A * a + t + T * i;  // z[j] = x[2j] + i x[2j+1]
+        const uint2 l = l2[j];
+        if (!TWO) {
+          v2[i][a] = make_float2(word_to_float(l.x, ts.ms), word_to_float(l.y, ts.ms));
+        } else {
+          const uint2 h = h2[j];
+          v2[i][a] = make_float2(fixed_to_float(l.x, h.x, ts.ms), fixed_to_float(l.y, h.y, ts.ms));
+        }
+      }
+    if (warp == 0 && batch == 0) between();
+    xrow_transform<N, false>(v2, o2, rb, t, S.tw);
+    if (has)
+      xrow_untangle_store<N>(o2, rb, t, S.tw, S.spec + ((long long)(z0 + r / TY) * N + (y0 + r % TY)) * S.pitch);
+    __syncwarp();  // the row's lanes are done with its words
+    uint4* z4 = reinterpret_cast<uint4*>(row);
+    for (int i = t; i < stride / 4; i += T) z4[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (warp == 0 && batch == NBATCH - 1) after();
+  }
 }
 
 template <int N>
-__global__ void __launch_bounds__(deposit_r2c_nt(N), dep_ctas_bound(N))
+__global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
     k_deposit_r2c(const Sim* __restrict__ sims, Work w, Parts p, const unsigned* __restrict__ perm,
-                  const unsigned* __restrict__ row_start, int* err, unsigned* __restrict__ next_tile,
-                  const unsigned* __restrict__ order) {
-  constexpr int NT = deposit_r2c_nt(N);
-  constexpr int M = N / 2, NL = TZ * TY, LS = NL + 1;
-  constexpr int PER = NL * N / NT;
-  constexpr int TPB = dep_tiles(N);  // tiles per CTA
-  static_assert(NL * N % NT == 0, "tile cells must divide by the block size");
-  static_assert((size_t)M * LS * sizeof(float2) <= deposit_r2c_smem_bytes(N), "FFT buffer must fit");
+                  const unsigned* __restrict__ row_start, const unsigned* __restrict__ group_max, int* err,
+                  unsigned* __restrict__ next_tile, const unsigned* __restrict__ order, unsigned* __restrict__ dense) {
+  constexpr int NT = DEP_ROW_NT, NL = TZ * TY, TPB = dep_tiles(N);
+  constexpr int RS = dep_row_words(N);  // words from a tile row to the next
+  constexpr int NTT = NT / TPB;         // threads per tile group
   static_assert(TPB * 8 <= 32 && NT % (TPB * 32) == 0, "one warp loads the run tables of a CTA's tiles");
+  static_assert(RS % 4 == 0, "rows zeroed 4 words at a time");
   extern __shared__ uint4 acc_raw[];
   // run tables of the CTA's tiles (7 runs each: first sorted index, and inclusive offsets)
   __shared__ unsigned s_begin[TPB][8];
   __shared__ unsigned s_off[TPB][8];
-  __shared__ TileSum s_ts[TPB];
-  unsigned* lo = reinterpret_cast<unsigned*>(acc_raw);
-  // row r: lo at r * RS, hi at r * RS + HO (tiles one after another, NL rows each)
-  constexpr int RS = xrow_ok(N) ? 2 * N : N, HO = xrow_ok(N) ? N : NL * N;
-  unsigned* hi = lo + HO;
-  float2* F = reinterpret_cast<float2*>(acc_raw);
-  float* Ff = reinterpret_cast<float*>(acc_raw);
+  __shared__ TileSum s_ts[2][TPB];  // of the tiles at hand and the next ones, in turn
+  __shared__ int s_next;
+  unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // warp 0: the run tables of the tiles at places idx .. idx + TPB - 1 (8 lanes per tile)
+  auto load_tables = [&](int idx) -> RunLoad {
+    RunLoad v;
+    int si, y0, z0;
+    if (dep_tile<N>(w, order, idx + (lane >> 3), si, y0, z0))
+      v = run_load(sims[si], row_start, group_max, y0, z0, lane & 7);
+    return v;
+  };
+  // warp 0: stores the tables and how the tiles' sums are held; a tile with two-word sums goes to
+  // the list of k_deposit_r2c_dense and is left out here
+  auto store_tables = [&](const RunLoad& v, int idx, TileSum* ts) {
+    const int tj = lane < TPB * 8 ? lane >> 3 : 0;
+    const TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
+    if (lane < TPB * 8 && (lane & 7) == 0) {
+      ts[tj] = t;
+      if (t.s == 0) dense[atomicAdd(next_tile + 1, 1u)] = (unsigned)(idx + tj);
+    }
+  };
   // Tiles are taken from a counter (zero at launch) after the first, TPB per CTA: a tile's
   // work is its particle count, which clustering makes very uneven, so a fixed stride
-  // leaves the CTAs that drew the dense tiles running alone at the end.
-  // `order` (optional) lists the tiles dense-first; idx is the place in it.
-  __shared__ int s_next;
-  auto take_next = [&]() -> int {
-    return (int)gridDim.x * TPB + (int)atomicAdd(next_tile, (unsigned)TPB);
+  // leaves the CTAs that drew the dense tiles running alone at the end.  Warp 0 takes the next
+  // tiles and loads their run tables before the transform and stores them after it, so that
+  // the loads' latency hides behind it (the particle loops are over).
+  int next = 0, turn = 0;
+  RunLoad nl;
+  auto take = [&]() {
+    next = __shfl_sync(FULL, lane == 0 ? (int)gridDim.x * TPB + (int)atomicAdd(next_tile, (unsigned)TPB) : 0, 0);
+    if (next < w.total) nl = load_tables(next);
   };
-  auto tile_at = [&](int idx) -> int { return order ? (int)__ldg(&order[idx]) : idx; };
-  // the tile at place i of the order: its simulation and first row / plane (false: none)
-  auto tile_of = [&](int i, int& si, int& y0, int& z0) -> bool {
-    si = 0; y0 = z0 = 0;
-    if (i >= w.total) return false;
-    const int unit = tile_at(i);
-    si = locate_sim(w, unit);
-    const int local = unit - __ldg(&w.prefix[si]);
-    y0 = (local % (N / TY)) * TY;
-    z0 = (local / (N / TY)) * TZ;
-    return true;
+  auto store = [&]() {
+    if (next < w.total) store_tables(nl, next, s_ts[turn ^ 1]);
+    if (lane == 0) s_next = next;
   };
-  if constexpr (xrow_ok(N)) {
-    constexpr int NTT = NT / TPB;  // threads per tile group
-    constexpr int P = xrow_P(N), Q = xrow_Q(N), T = xrow_T(N), RPW = 32 / T;
-    constexpr int NB1 = Q / T, NB2 = P / T;
-    static_assert(Q * (P + 1) * sizeof(float2) <= 2 * N * sizeof(unsigned), "exchange buffer in the row");
-    const int g = threadIdx.x / NTT, gtid = threadIdx.x % NTT;
-    // warp 0: the run tables of the tiles at places idx .. idx + TPB - 1 (8 lanes per tile)
-    auto load_tables = [&](int idx) -> RunLoad {
-      RunLoad v{0u, 0u};
+  // The accumulators start zero, and each row is zeroed again by its transform lanes once
+  // they are done with it, so a tile needs no zeroing phase and barrier of its own
+  // (0.468 -> 0.460 ms early, 0.604 -> 0.587 ms at step 980, 256^3 on 512^3).
+  for (int i = threadIdx.x; i < TPB * NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
+  chain_begin();
+  int idx = blockIdx.x * TPB;
+  if (warp == 0 && idx < w.total) store_tables(load_tables(idx), idx, s_ts[0]);
+  __syncthreads();
+  for (; idx < w.total; turn ^= 1) {
+    {  // the particles of this group's tile (a group without a tile has an empty table)
+      const int g = threadIdx.x / NTT, gtid = threadIdx.x % NTT;
       int si, y0, z0;
-      if (tile_of(idx + (lane >> 3), si, y0, z0)) v = run_load(sims[si], row_start, y0, z0, lane & 7);
-      return v;
-    };
-    // The accumulators start zero, and each row is zeroed again by its transform lanes once
-    // they are done with it, so a tile needs no zeroing phase and barrier of its own
-    // (0.468 -> 0.460 ms early, 0.604 -> 0.587 ms at step 980, 256^3 on 512^3).
-    for (int i = threadIdx.x; i < TPB * NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
-    chain_begin();
-    int idx = blockIdx.x * TPB;
-    if (warp == 0 && idx < w.total) {
-      const RunLoad v = load_tables(idx);
-      const int tj = lane < TPB * 8 ? lane >> 3 : 0;
-      run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
+      dep_tile<N>(w, order, idx + g, si, y0, z0);
+      const TileSum ts = s_ts[turn][g];
+      if (ts.s)
+        deposit_tile<POS_DISP, NTT, true, N>(sims[si], p, perm, err, y0, z0, acc + g * NL * RS, nullptr, RS, s_begin[g],
+                                             s_off[g], ts, make_int2(0, TZ), gtid);
     }
     __syncthreads();
-    while (idx < w.total) {
-      {  // the particles of this group's tile (a group without a tile has an empty table)
-        int si, y0, z0;
-        tile_of(idx + g, si, y0, z0);
-        deposit_tile<POS_DISP, NTT, N>(sims[si], p, perm, row_start, err, y0, z0, lo + g * NL * RS, hi + g * NL * RS, RS,
-                                s_begin[g], s_off[g], true, gtid, &s_ts[g], true);
-      }
-      // the CTA's TPB * NL rows: T lanes per row, rows R = warp * RPW + sub; a row's exchange
-      // buffer overlays its own accumulator words once they are read
-      const int sub = lane / T, t = lane % T;
-      const int R = warp * RPW + sub, tg = R / NL, r = R % NL;
-      float2* rb = reinterpret_cast<float2*>(lo + R * RS);
-      if (warp * RPW < TPB * NL) {  // warp-uniform
-        int tsi, ty0, tz0;
-        const bool thas = tile_of(idx + tg, tsi, ty0, tz0);
-        const Sim& S = sims[tsi];
-        const TileSum ts = s_ts[tg];
-        float2 v2[NB1][P];
-        float2 o2[NB2][Q];
-        const uint2* l2 = reinterpret_cast<const uint2*>(lo + R * RS);
-        const uint2* h2 = reinterpret_cast<const uint2*>(lo + R * RS + HO);
-#pragma unroll
-        for (int i = 0; i < NB1; ++i)
-#pragma unroll
-          for (int a = 0; a < P; ++a) {
-            const int j = Q * a + t + T * i;  // z[j] = x[2j] + i x[2j+1]
-            const uint2 ll = l2[j], hh = ts.s ? make_uint2(0u, 0u) : h2[j];
-            v2[i][a] = make_float2(sum_to_float(ts, ll.x, hh.x), sum_to_float(ts, ll.y, hh.y));
-          }
-        // warp 0 takes the next tiles and loads their run tables now, and stores them after the
-        // transform, so that the loads' latency hides behind it (the tables are free: the
-        // particle loops are over, and the transform reads s_ts)
-        int next = 0;
-        if (warp == 0) next = __shfl_sync(FULL, lane == 0 ? take_next() : 0, 0);
-        RunLoad nl{0u, 0u};
-        if (warp == 0 && next < w.total) nl = load_tables(next);
-        xrow_transform<N, false>(v2, o2, rb, t, S.tw);
-        if (thas) {
-          const long long row = (long long)(tz0 + r / TY) * N + (ty0 + r % TY);
-          xrow_untangle_store<N>(o2, rb, t, S.tw, S.spec + row * S.pitch);
-        }
-        __syncwarp();  // the row's lanes are done with its words
-        {  // zero what this tile dirtied: the low words and the exchange buffer (which reaches
-           // into the high words), and the high words after a two-word tile
-          constexpr int XW = 2 * Q * (P + 1);  // words of the exchange buffer
-          static_assert(XW % 4 == 0 && RS % 4 == 0, "rows zeroed 4 words at a time");
-          const int zw = ts.s ? (XW > N ? XW : N) : RS;
-          uint4* z4 = reinterpret_cast<uint4*>(lo + R * RS);
-          for (int i = t; i < zw / 4; i += T) z4[i] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        if (warp == 0 && next < w.total) {
-          const int tj = lane < TPB * 8 ? lane >> 3 : 0;
-          run_table(nl, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
-        }
-        if (threadIdx.x == 0) s_next = next;
-      }
-      __syncthreads();
-      idx = s_next;
+    dep_transform<N, NT, TPB, false>(
+        sims, acc, RS, s_ts[turn],
+        [&](int tg, int& si, int& y0, int& z0) { return dep_tile<N>(w, order, idx + tg, si, y0, z0) && s_ts[turn][tg].s; },
+        take, store);
+    __syncthreads();
+    idx = s_next;
+  }
+}
+
+// The tiles that k_deposit_r2c left: those with two-word sums, one to a CTA of 1024 threads (such
+// tiles hold thousands of particles).  A kernel of its own: next to the one-word path its
+// registers and code cost that path 10% (442 -> 498 us on the 512 grid).
+constexpr int DEP_DENSE_NT = 1024;
+__host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, coarse words
+
+template <int N>
+__global__ void __launch_bounds__(DEP_DENSE_NT, 1)
+    k_deposit_r2c_dense(const Sim* __restrict__ sims, Work w, Parts p, const unsigned* __restrict__ perm,
+                        const unsigned* __restrict__ row_start, const unsigned* __restrict__ group_max, int* err,
+                        const unsigned* __restrict__ next_tile, const unsigned* __restrict__ order,
+                        const unsigned* __restrict__ dense) {
+  constexpr int NT = DEP_DENSE_NT, NL = TZ * TY, RS = dep_dense_stride(N);
+  static_assert(RS % 4 == 0, "rows zeroed 4 words at a time");
+  extern __shared__ uint4 acc_raw[];
+  __shared__ unsigned s_begin[8];
+  __shared__ unsigned s_off[8];
+  __shared__ TileSum s_ts;
+  unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  chain_begin();
+  const unsigned count = next_tile[1];
+  if (blockIdx.x >= count) return;
+  for (int i = threadIdx.x; i < NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
+    int si, y0, z0;
+    dep_tile<N>(w, order, (int)dense[i], si, y0, z0);
+    if (warp == 0) {
+      const TileSum t = run_table(run_load(sims[si], row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off,
+                                  lane < 8);
+      if (lane == 0) s_ts = t;
     }
-    return;
-  } else {
-    chain_begin();
-    bool runs_ready = false;
-    for (int idx = blockIdx.x; idx < w.total;) {
-      int si, y0, z0;
-      tile_of(idx, si, y0, z0);
-      const Sim& S = sims[si];
-      const TileSum ts = deposit_tile<POS_DISP, NT, N>(S, p, perm, row_start, err, y0, z0, lo, hi, RS, s_begin[0], s_off[0],
-                                                runs_ready);
-      runs_ready = false;
-      float v[PER];
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const int i = threadIdx.x + k * NT;
-        v[k] = sum_to_float(ts, lo[i], ts.s ? 0u : hi[i]);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const int i = threadIdx.x + k * NT;
-        const int r = i / N, x = i % N;
-        Ff[((x >> 1) * LS + r) * 2 + (x & 1)] = v[k];  // z[j] = x[2j] + i x[2j+1] of row r
-      }
-      __syncthreads();
-      fft_lines<M, NL, LS, NT, false>(F, S.tw, 2);
-      float2* __restrict__ dst = S.spec;
-      const int P = S.pitch;
-      for (int u = threadIdx.x; u < NL * (M + 1); u += NT) {
-        const int r = u / (M + 1), k = u % (M + 1);
-        const long long row = (long long)(z0 + r / TY) * N + (y0 + r % TY);
-        const float2 zk = F[(k == M ? 0 : k) * LS + r];
-        const float2 zc = conjf2(F[(k == 0 ? 0 : M - k) * LS + r]);
-        const float2 e = cscale(cadd(zk, zc), 0.5f);
-        const float2 o = cscale(mul_mi<false>(csub(zk, zc)), 0.5f);
-        dst[row * P + k] = cadd(e, cmul(__ldg(&S.tw[k]), o));
-      }
-      if (threadIdx.x == 0) s_next = take_next();
-      __syncthreads();
-      idx = s_next;
-    }
+    __syncthreads();
+    deposit_tile<POS_DISP, NT, false, N>(sims[si], p, perm, err, y0, z0, acc, acc + dep_row_words(N), RS, s_begin, s_off,
+                                         s_ts, make_int2(0, TZ), threadIdx.x);
+    __syncthreads();
+    dep_transform<N, NT, 1, true>(
+        sims, acc, RS, &s_ts, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0; return true; }, []() {},
+        []() {});
+    __syncthreads();
   }
 }
 
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,
-                               int* err, unsigned* next_tile, const unsigned* order, int ctas, Launch st) {
+                               const unsigned* group_max, int* err, unsigned* next_tile, const unsigned* order,
+                               unsigned* dense, int ctas, Launch st) {
   if constexpr (!deposit_r2c_ok(N)) {
     return cudaErrorNotSupported;
   } else {
-  static DeviceOnce once;
-  const size_t sm = dep_tiles(N) * deposit_r2c_smem_bytes(N);
-  const cudaError_t ie = once.run([&]() {
-    cudaError_t e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    return e;
-  });
-  if (ie) return ie;
-  if (ctas <= 0) return cudaSuccess;  // attribute setup only
-  constexpr int NT = deposit_r2c_nt(N), TPB = dep_tiles(N);
-  if (ctas > (w.total + TPB - 1) / TPB) ctas = (w.total + TPB - 1) / TPB;  // TPB tiles per CTA
-  if (ctas <= 0) return cudaSuccess;
-  launch_chained(k_deposit_r2c<N>, ctas, NT, sm, st, sims, w, p, perm, row_start, err, next_tile, order);
-  return cudaGetLastError();
+    static DeviceOnce once;
+    const size_t sm = dep_tiles(N) * dep_tile_bytes(N);
+    const size_t smd = (size_t)TZ * TY * dep_dense_stride(N) * sizeof(unsigned);
+    const cudaError_t ie = once.run([&]() {
+      cudaError_t e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      if (!e)
+        e = cudaFuncSetAttribute(k_deposit_r2c_dense<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smd);
+      if (!e) e = cudaFuncSetAttribute(k_deposit_r2c_dense<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      return e;
+    });
+    if (ie) return ie;
+    if (ctas <= 0) return cudaSuccess;  // attribute setup only
+    constexpr int NT = DEP_ROW_NT, TPB = dep_tiles(N);
+    if (ctas > (w.total + TPB - 1) / TPB) ctas = (w.total + TPB - 1) / TPB;  // TPB tiles per CTA
+    if (ctas <= 0) return cudaSuccess;
+    launch_chained(k_deposit_r2c<N>, ctas, NT, sm, st, sims, w, p, perm, row_start, group_max, err, next_tile, order,
+                   dense);
+    if (cudaError_t e = cudaGetLastError()) return e;
+    const int few = w.total < device_sms() ? w.total : device_sms();
+    launch_chained(k_deposit_r2c_dense<N>, few, DEP_DENSE_NT, smd, st, sims, w, p, perm, row_start, group_max, err, next_tile,
+                   order, dense);
+    return cudaGetLastError();
   }
 }
 
@@ -998,11 +947,6 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
   static DeviceOnce once;
   const size_t xs = x_smem_bytes(N), ls = line_smem_bytes(N);
   const cudaError_t ie = once.run([&]() -> cudaError_t {
-    if constexpr (tma_rows(N)) {
-      cudaError_t e = max_shared(k_x_tma<N, false>, xtma_smem_bytes(N));
-      if (!e) e = max_shared(k_x_tma<N, true>, xtma_smem_bytes(N));
-      if (e) return e;
-    }
     if constexpr (tma_lines(N)) {
       cudaError_t e = max_shared(k_line_tma<N, 0>, tma_smem_bytes(N));
       if (!e) e = max_shared(k_line_tma<N, 1>, tma_smem_bytes(N));
@@ -1013,8 +957,11 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
       if (!e) e = max_shared(k_line_tma<N, 6>, tma_smem_bytes(N));
       if (e) return e;
     }
-    cudaError_t e = max_shared(k_x_r2c<N>, xs);
-    if (!e) e = max_shared(k_x_c2r<N>, xs);
+    cudaError_t e = cudaSuccess;
+    if constexpr (!xrow_ok(N)) {
+      e = max_shared(k_x_r2c<N>, xs);
+      if (!e) e = max_shared(k_x_c2r<N>, xs);
+    }
     if (!e) e = max_shared(k_line_pass<N, false, false>, ls);
     if (!e) e = max_shared(k_line_pass<N, false, true>, ls);
     if (!e) e = max_shared(k_line_pass<N, true, false>, ls);
@@ -1026,7 +973,6 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
   });
   if (ie) return ie;
   if (kind == SPEC_PREPARE) return cudaSuccess;
-  const int grid = w.total < device_sms() ? w.total : device_sms();
   if constexpr (xrow_ok(N)) {
     if (kind == SPEC_X_R2C || kind == SPEC_X_C2R) {
       // ctas: the cap on the CTAs of the persistent row transform (the batch engine tunes it)
@@ -1037,10 +983,10 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
       return cudaGetLastError();
     }
   }
-  if constexpr (tma_rows(N)) {
+  if constexpr (!xrow_ok(N)) {
     if (kind == SPEC_X_R2C || kind == SPEC_X_C2R) {
-      if (kind == SPEC_X_R2C) launch_chained(k_x_tma<N, false>, grid, XTMA_NT, xtma_smem_bytes(N), st, sims, w, err);
-      else launch_chained(k_x_tma<N, true>, grid, XTMA_NT, xtma_smem_bytes(N), st, sims, w, err);
+      if (kind == SPEC_X_R2C) launch_chained(k_x_r2c<N>, ctas, SP_NT, xs, st, sims, w);
+      else launch_chained(k_x_c2r<N>, ctas, SP_NT, xs, st, sims, w);
       return cudaGetLastError();
     }
   }
@@ -1062,8 +1008,6 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
     }
   }
   switch (kind) {
-    case SPEC_X_R2C: launch_chained(k_x_r2c<N>, ctas, SP_NT, xs, st, sims, w); break;
-    case SPEC_X_C2R: launch_chained(k_x_c2r<N>, ctas, SP_NT, xs, st, sims, w); break;
     case SPEC_Y_FWD: launch_chained(k_line_pass<N, false, false>, ctas, SP_NT, ls, st, sims, w); break;
     case SPEC_Y_INV: launch_chained(k_line_pass<N, false, true>, ctas, SP_NT, ls, st, sims, w); break;
     case SPEC_Z_FWD: launch_chained(k_line_pass<N, true, false>, ctas, SP_NT, ls, st, sims, w); break;

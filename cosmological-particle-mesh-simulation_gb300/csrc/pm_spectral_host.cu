@@ -11,16 +11,17 @@ PM_FOR_EACH_N(PM_EXTERN)
 #undef PM_EXTERN
 #define PM_EXTERN(NN)                                                                                         \
   extern template cudaError_t deposit_r2c_launch<NN>(const Sim*, Work, Parts, const unsigned*, const unsigned*, \
-                                                     int*, unsigned*, const unsigned*, int, Launch);
+                                                     const unsigned*, int*, unsigned*, const unsigned*, unsigned*, int, \
+                                                     Launch);
 PM_FOR_EACH_N(PM_EXTERN)
 #undef PM_EXTERN
 
 cudaError_t deposit_r2c_dispatch(int n, const Sim* sims, Work w, Parts p, const unsigned* perm,
-                                 const unsigned* row_start, int* err, unsigned* next_tile,
-                                 const unsigned* order, int ctas, Launch st) {
+                                 const unsigned* row_start, const unsigned* group_max, int* err, unsigned* next_tile,
+                                 const unsigned* order, unsigned* dense, int ctas, Launch st) {
   switch (n) {
 #define PM_CASE(NN) \
-  case NN: return deposit_r2c_launch<NN>(sims, w, p, perm, row_start, err, next_tile, order, ctas, st);
+  case NN: return deposit_r2c_launch<NN>(sims, w, p, perm, row_start, group_max, err, next_tile, order, dense, ctas, st);
     PM_FOR_EACH_N(PM_CASE)
 #undef PM_CASE
     default: return cudaErrorInvalidValue;
@@ -35,7 +36,7 @@ bool spectral_encode_maps(int n, const void* spec, CUtensorMap out[2]) {
 bool deposit_r2c_supported(int n) { return spectral_supported(n) && deposit_r2c_ok(n); }
 bool xrow_supported(int n) { return spectral_supported(n) && xrow_ok(n); }
 
-int deposit_r2c_ctas_per_sm(int n) { return xrow_ok(n) ? 3 : 2; }
+int deposit_r2c_ctas_per_sm(int n) { return dep_ctas_bound(n); }
 
 bool spectral_supported(int n) {
   switch (n) {

@@ -7,6 +7,6 @@
 
 namespace pm {
 template cudaError_t spectral_launch<PM_N>(SpecKind, const Sim*, Work, int, Launch, const CUtensorMap*, int*);
-template cudaError_t deposit_r2c_launch<PM_N>(const Sim*, Work, Parts, const unsigned*, const unsigned*, int*, unsigned*,
-                                              const unsigned*, int, Launch);
+template cudaError_t deposit_r2c_launch<PM_N>(const Sim*, Work, Parts, const unsigned*, const unsigned*, const unsigned*, int*,
+                                              unsigned*, const unsigned*, unsigned*, int, Launch);
 }
