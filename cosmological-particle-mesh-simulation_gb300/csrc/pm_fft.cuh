@@ -189,6 +189,21 @@ template <bool INV> struct DFT<24, INV> {
   static __device__ __forceinline__ void run(float2* v) { dft_composite<3, 8, W24, INV>(v); }
 };
 
+// exp(-2 pi i m / 32): multiples of 11.25 degrees
+struct W32 {
+  static __device__ __forceinline__ float2 w(int m) {
+    const float a = 0.980785280403230449126182f, b = 0.923879532511286756128183f, d = 0.831469612302545237078788f;
+    const float e = 0.707106781186547524400844f, f = 0.555570233019602224742831f, g = 0.382683432365089771728460f;
+    const float h = 0.195090322016128267848285f;
+    const float c[32] = {1.f, a, b, d, e, f, g, h, 0.f, -h, -g, -f, -e, -d, -b, -a,
+                         -1.f, -a, -b, -d, -e, -f, -g, -h, 0.f, h, g, f, e, d, b, a};
+    return make_float2(c[m], -c[(m + 24) % 32]);  // sin(t) = cos(t - 90 degrees)
+  }
+};
+template <bool INV> struct DFT<32, INV> {
+  static __device__ __forceinline__ void run(float2* v) { dft_composite<4, 8, W32, INV>(v); }
+};
+
 // ---------------------------------------------------------------------------------
 // Radix plans (product of radices == L).  Fewer passes mean fewer shared-memory round trips:
 // the two-pass plans of 128, 192, 256 and 384 and the three-pass plan of 1024 measured, per
@@ -197,11 +212,17 @@ template <bool INV> struct DFT<24, INV> {
 // 1.07G cells): 1.88 -> 1.51.  512 keeps three radix-8 passes on pairs of lines (16 x 32 line
 // by line: z 0.291 -> 0.303 ms, half the threads idle in the radix-32 pass).
 // ---------------------------------------------------------------------------------
+// Lengths whose blocked transforms run on pairs of lines: the plans of radix 8 or less, and
+// 128 (8 x 16).  The radix-12/16/24 plans hold too many values per pair of lines and run
+// line by line (on pairs they spill).
+__host__ __device__ constexpr bool blocked_pairs(int L) { return L % 3 != 0 && L != 256 && L != 1024; }
+
 template <int L> struct Plan;
 #define PM_PLAN(L_, ...)                                   \
   template <> struct Plan<L_> {                            \
     static constexpr int r[] = {__VA_ARGS__};              \
     static constexpr int np = sizeof(r) / sizeof(int);     \
+    static constexpr bool pairs = blocked_pairs(L_);       \
   };
 PM_PLAN(8, 8)
 PM_PLAN(12, 3, 4)
@@ -219,6 +240,19 @@ PM_PLAN(512, 8, 8, 8)
 PM_PLAN(768, 3, 4, 8, 8)
 PM_PLAN(1024, 16, 8, 8)
 #undef PM_PLAN
+
+// Plan of the forward / map / inverse turn (the larger radices halve its shared-memory round trips;
+// 1024 as 32 x 32 takes the same 3.48 ms as 16 x 8 x 8).
+template <int L> struct TurnPlan : Plan<L> {};
+#define PM_TURN_PLAN(L_, ...)                              \
+  template <> struct TurnPlan<L_> {                        \
+    static constexpr int r[] = {__VA_ARGS__};              \
+    static constexpr int np = sizeof(r) / sizeof(int);     \
+    static constexpr bool pairs = false;                   \
+  };
+PM_TURN_PLAN(512, 16, 32)
+PM_TURN_PLAN(768, 24, 32)
+#undef PM_TURN_PLAN
 
 template <int LS>
 struct Interleaved {
@@ -292,11 +326,6 @@ __device__ __forceinline__ void fft_passes(float2* s, const float2* __restrict__
     }
   }
 }
-
-// Lengths whose blocked transforms run on pairs of lines: the plans of radix 8 or less, and
-// 128 (8 x 16).  The radix-12/16/24 plans hold too many values per pair of lines and run
-// line by line (on pairs they spill).
-__host__ __device__ constexpr bool blocked_pairs(int L) { return L % 3 != 0 && L != 256 && L != 1024; }
 
 // Whether task j of a stride-1 pass over NP pairs of lines stores its R outputs in the order
 // r ^ 1: with 4 pairs, the 8 lanes of a quarter-warp (one phase of a 128-bit shared-memory
@@ -394,30 +423,29 @@ __device__ __forceinline__ void fft_passes_pairs(float2* s, const float2* __rest
 // registers -- the map is applied between them -- instead of through shared memory: one
 // shared-memory round trip and two barriers fewer per transform pair.
 // ---------------------------------------------------------------------------------
-template <int L, int P, bool REV>
+template <class PL, int P, bool REV>
 __host__ __device__ constexpr int plan_radix() {
-  return REV ? Plan<L>::r[Plan<L>::np - 1 - P] : Plan<L>::r[P];
+  return REV ? PL::r[PL::np - 1 - P] : PL::r[P];
 }
 
 // Passes P .. PEND-1 of the plan (reversed with REV), entered with stride NS.
-template <int L, int P, int PEND, int NS, int NL, int BW, int NT, bool INV, bool REV>
+template <int L, class PL, int P, int PEND, int NS, int NL, int BW, int NT, bool INV, bool REV>
 __device__ __forceinline__ void passes_span(float2* s, const float2* __restrict__ tw, int tws) {
   if constexpr (P < PEND) {
-    constexpr int R = plan_radix<L, P, REV>();
-    if constexpr (blocked_pairs(L))
+    constexpr int R = plan_radix<PL, P, REV>();
+    if constexpr (PL::pairs)
       stockham_pass_pairs<L, R, NS, NL, BW, NT, INV, NoEpi, true>(s, tw, tws);
     else
       stockham_pass<L, R, NS, NL, Blocked<L, BW>, NT, INV>(s, tw, tws);
-    passes_span<L, P + 1, PEND, NS * R, NL, BW, NT, INV, REV>(s, tw, tws);
+    passes_span<L, PL, P + 1, PEND, NS * R, NL, BW, NT, INV, REV>(s, tw, tws);
   }
 }
 
 // The turn: last forward pass, `epi` on each output (element e of line), first inverse pass.
-template <int L, int R, int NL, int BW, int NT, class EPI>
+template <int L, int R, bool PAIRS, int NL, int BW, int NT, class EPI>
 __device__ __forceinline__ void stockham_turn(float2* s, const float2* __restrict__ tw, int tws, const EPI& epi) {
   using LAY = Blocked<L, BW>;
   constexpr int NS = L / R;  // forward stride of the last pass == the inverse's block count
-  constexpr bool PAIRS = blocked_pairs(L);
   constexpr int NG = PAIRS ? NL / 2 : NL;  // line groups: pairs of lines, or lines
   constexpr int NTASK = NG * NS;
   constexpr int TPT = (NTASK + NT - 1) / NT;
@@ -487,10 +515,11 @@ __device__ __forceinline__ void stockham_turn(float2* s, const float2* __restric
 template <int L, int NL, int BW, int NT, class EPI>
 __device__ __forceinline__ void fft_lines_blocked_turn(float2* s, const float2* __restrict__ tw, int tws,
                                                        const EPI& epi) {
-  constexpr int NPL = Plan<L>::np, RL = Plan<L>::r[NPL - 1];
-  passes_span<L, 0, NPL - 1, 1, NL, BW, NT, false, false>(s, tw, tws);
-  stockham_turn<L, RL, NL, BW, NT>(s, tw, tws, epi);
-  passes_span<L, 1, NPL, RL, NL, BW, NT, true, true>(s, tw, tws);
+  using PL = TurnPlan<L>;
+  constexpr int NPL = PL::np, RL = PL::r[NPL - 1];
+  passes_span<L, PL, 0, NPL - 1, 1, NL, BW, NT, false, false>(s, tw, tws);
+  stockham_turn<L, RL, PL::pairs, NL, BW, NT>(s, tw, tws, epi);
+  passes_span<L, PL, 1, NPL, RL, NL, BW, NT, true, true>(s, tw, tws);
 }
 
 // Unnormalised DFT of NL interleaved lines of length L held in shared memory.

@@ -54,11 +54,23 @@ __host__ __device__ constexpr bool tma_lines(int n) { return n >= 32 && line_box
 // transformed line by line, runs 1024.
 __host__ __device__ constexpr int line_nt(int n) { return line_small(n) ? 256 : (n == 768 ? 1024 : 512); }
 __host__ __device__ constexpr int line_ctas_per_sm(int n) { return line_small(n) ? 2 : 1; }
+// The z pass with the Green function (the turn) has plans of its own (pm_fft.cuh: TurnPlan), and on
+// these grids its own threads, CTAs per SM and ring stages: 512 in two passes of 16 and 32, one
+// radix-32 transform per thread of 128, three CTAs of two stages (256 us; three radix-8 passes on
+// pairs of lines 288, two CTAs of three stages 284, 256 threads of which half idle 299); 768 of 24
+// and 32 with 256 threads (1.31 ms; radix 3, 4, 8, 8 with 1024 threads 2.9).  The same passes on
+// bundles of 4 columns (32-byte rows for the copies) take twice the time.
+__host__ __device__ constexpr int turn_stages(int n) { return n == 512 ? 2 : 3; }
+__host__ __device__ constexpr int turn_nt(int n) { return n == 512 ? 128 : (n == 768 ? 256 : line_nt(n)); }
+__host__ __device__ constexpr int turn_ctas_per_sm(int n) { return n == 512 ? 3 : line_ctas_per_sm(n); }
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
   return (size_t)n * cline_width(n) * cline_bpc(n) * sizeof(float2);
 }
-__host__ __device__ constexpr size_t tma_smem_bytes(int n) { return TMA_STAGES * tma_stage_bytes(n) + 64; }
+__host__ __device__ constexpr size_t tma_smem_bytes(int n, bool turn) {
+  return (turn ? turn_stages(n) : TMA_STAGES) * tma_stage_bytes(n) + 64;
+}
+__host__ __device__ constexpr bool line_turn(int mode) { return mode == 2 || mode == 3 || mode == 6; }
 
 // x passes with the row transform in registers (n >= 32): a row of M = n/2 complex points is held
 // by T lanes of a warp and transformed in passes of radix A, (B,) C, M = A C or A B C, through an
@@ -399,8 +411,10 @@ struct GreenEpi {
 // MODE 0: y forward, 1: y inverse, 2: z Green, 3: z Green (caller table), 4: z forward, 5: z inverse,
 // 6: z Green times -i sin(k_d) (spectral gradient of axis S.grad_axis - 1)
 template <int N, int MODE>
-__global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(const CUtensorMap* __restrict__ maps,
-                                                        const Sim* __restrict__ sims, Work w, int* err) {
+__global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
+                                  line_turn(MODE) ? turn_ctas_per_sm(N) : line_ctas_per_sm(N))
+    k_line_tma(const CUtensorMap* __restrict__ maps, const Sim* __restrict__ sims, Work w, int* err) {
+  constexpr int STAGES = line_turn(MODE) ? turn_stages(N) : TMA_STAGES;
   constexpr int BW = cline_width(N), BPC = cline_bpc(N), NL = BW * BPC;
   constexpr int BOX = line_box_rows(N), NBOX = N / BOX;
   constexpr int NBP = cbundles_per_plane(N), W = chalf(N), NB = N * NBP;
@@ -409,10 +423,10 @@ __global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(co
   constexpr bool ZAX = MODE >= 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float2* stg0 = reinterpret_cast<float2*>(smem_raw);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + TMA_STAGES * STAGE);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + STAGES * STAGE);
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < TMA_STAGES; ++i) mbar_init(&bar[i], 1);
+    for (int i = 0; i < STAGES; ++i) mbar_init(&bar[i], 1);
     fence_mbar_init();
   }
   __syncthreads();
@@ -447,11 +461,11 @@ __global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(co
   if (threadIdx.x == 0 && unit < w.total) issue_load(unit, 0);
   unsigned parity = 0;  // bit st: parity of the next phase of stage st
   for (int it = 0; unit < w.total; unit += gridDim.x, ++it) {
-    const int st = it % TMA_STAGES;
+    const int st = it % STAGES;
     const int next = unit + gridDim.x;
     if (threadIdx.x == 0 && next < w.total) {
-      bulk_wait_read<TMA_STAGES - 2>();  // the store that last read stage (it+1)%3 is done
-      issue_load(next, (it + 1) % TMA_STAGES);
+      bulk_wait_read<STAGES - 2>();  // the store that last read the stage is done
+      issue_load(next, (it + 1) % STAGES);
     }
     const bool ok = mbar_wait(&bar[st], (parity >> st) & 1u);
     parity ^= 1u << st;
@@ -470,7 +484,7 @@ __global__ void __launch_bounds__(line_nt(N), line_ctas_per_sm(N)) k_line_tma(co
     } else {
       // forward z transform, the Green function, inverse z transform (meeting in registers)
       const GreenEpi<N, MODE == 3, MODE == 6> epi{S.green, S.s2, S.fgrid, b0, cnt, S.sn, S.grad_axis};
-      fft_lines_blocked_turn<N, NL, BW, line_nt(N)>(s, S.tw, 1, epi);
+      fft_lines_blocked_turn<N, NL, BW, turn_nt(N)>(s, S.tw, 1, epi);
     }
     fence_proxy_async_smem();
     __syncthreads();
@@ -948,13 +962,13 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
   const size_t xs = x_smem_bytes(N), ls = line_smem_bytes(N);
   const cudaError_t ie = once.run([&]() -> cudaError_t {
     if constexpr (tma_lines(N)) {
-      cudaError_t e = max_shared(k_line_tma<N, 0>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 1>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 2>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 3>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 4>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 5>, tma_smem_bytes(N));
-      if (!e) e = max_shared(k_line_tma<N, 6>, tma_smem_bytes(N));
+      cudaError_t e = max_shared(k_line_tma<N, 0>, tma_smem_bytes(N, false));
+      if (!e) e = max_shared(k_line_tma<N, 1>, tma_smem_bytes(N, false));
+      if (!e) e = max_shared(k_line_tma<N, 2>, tma_smem_bytes(N, true));
+      if (!e) e = max_shared(k_line_tma<N, 3>, tma_smem_bytes(N, true));
+      if (!e) e = max_shared(k_line_tma<N, 4>, tma_smem_bytes(N, false));
+      if (!e) e = max_shared(k_line_tma<N, 5>, tma_smem_bytes(N, false));
+      if (!e) e = max_shared(k_line_tma<N, 6>, tma_smem_bytes(N, true));
       if (e) return e;
     }
     cudaError_t e = cudaSuccess;
@@ -992,17 +1006,19 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
   }
   if constexpr (tma_lines(N)) {
     if (maps) {
-      const size_t sm = tma_smem_bytes(N);
-      const int lcap = line_ctas_per_sm(N) * device_sms();
+      const bool turn = kind == SPEC_Z_GREEN || kind == SPEC_Z_TABLE || kind == SPEC_Z_GRAD;
+      const size_t sm = tma_smem_bytes(N, turn);
+      const int nt = turn ? turn_nt(N) : line_nt(N);
+      const int lcap = (turn ? turn_ctas_per_sm(N) : line_ctas_per_sm(N)) * device_sms();
       const int grid = w.total < lcap ? w.total : lcap;
       switch (kind) {
-        case SPEC_Y_FWD: launch_chained(k_line_tma<N, 0>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Y_INV: launch_chained(k_line_tma<N, 1>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_GREEN: launch_chained(k_line_tma<N, 2>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_TABLE: launch_chained(k_line_tma<N, 3>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_FWD: launch_chained(k_line_tma<N, 4>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_INV: launch_chained(k_line_tma<N, 5>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
-        case SPEC_Z_GRAD: launch_chained(k_line_tma<N, 6>, grid, line_nt(N), sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Y_FWD: launch_chained(k_line_tma<N, 0>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Y_INV: launch_chained(k_line_tma<N, 1>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_GREEN: launch_chained(k_line_tma<N, 2>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_TABLE: launch_chained(k_line_tma<N, 3>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_FWD: launch_chained(k_line_tma<N, 4>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_INV: launch_chained(k_line_tma<N, 5>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
+        case SPEC_Z_GRAD: launch_chained(k_line_tma<N, 6>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
         default: break;
       }
     }
