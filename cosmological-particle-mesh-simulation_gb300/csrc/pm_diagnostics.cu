@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(PK_NT) k_pk_bins(const float2* __restrict__ sp
   const long long rows = (long long)n * n;
   const long long gw = (long long)blockIdx.x * PK_WARPS + warp, nw = (long long)gridDim.x * PK_WARPS;
   for (long long r = gw; r < rows; r += nw) {
-    const int ky = (int)(r % n), kz = (int)(r / n);
+    const int ky = spec_row_y(n, r), kz = spec_row_z(n, r);
     const int fy = pk_freq(ky, n), fz = pk_freq(kz, n);
     const int base = fy * fy + fz * fz;
     if (base >= nbins * nbins) continue;  // the whole row lies outside the last shell

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(IC_NT) k_grf_fill(GrfArgs g) {
   for (long long e = (long long)blockIdx.x * IC_NT + threadIdx.x; e < total; e += (long long)gridDim.x * IC_NT) {
     const int kx = (int)(e % P);
     const int r = (int)(e / P);
-    const int ky = r % n, kz = r / n;
+    const int ky = spec_row_y(n, r), kz = spec_row_z(n, r);
     float2 out = make_float2(0.f, 0.f);
     if (kx <= h) {
       const int m2 = sq(signed_freq(kx, n)) + sq(signed_freq(ky, n)) + sq(signed_freq(kz, n));
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(IC_NT) k_zeld_spectrum(ZelArgs z) {
   for (long long e = (long long)blockIdx.x * IC_NT + threadIdx.x; e < total; e += (long long)gridDim.x * IC_NT) {
     const int kx = (int)(e % P);
     const int r = (int)(e / P);
-    const int ky = r % n, kz = r / n;
+    const int ky = spec_row_y(n, r), kz = spec_row_z(n, r);
     const bool mode = kx <= h && (kx | ky | kz) != 0;
     float2 re = make_float2(0.f, 0.f), im = re;  // disp[m2] * v
     if (mode) {

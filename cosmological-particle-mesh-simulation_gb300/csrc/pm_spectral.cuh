@@ -58,10 +58,11 @@ __host__ __device__ constexpr int line_ctas_per_sm(int n) { return line_small(n)
 // these grids its own threads, CTAs per SM and ring stages: 512 in two passes of 16 and 32, one
 // radix-32 transform per thread of 128, three CTAs of two stages (256 us; three radix-8 passes on
 // pairs of lines 288, two CTAs of three stages 284, 256 threads of which half idle 299); 768 of 24
-// and 32 with 256 threads (1.31 ms; radix 3, 4, 8, 8 with 1024 threads 2.9).  The same passes on
-// bundles of 4 columns (32-byte rows for the copies) take twice the time.
+// and 32 with 256 threads (1.22 ms; radix 3, 4, 8, 8 with 1024 threads 2.9); 1024 of 32 and 32 with
+// 256 threads (2.36 ms; 16, 8, 8 with 512 threads 2.67).  The same passes on bundles of 4 columns
+// (32-byte rows for the copies) take twice the time.
 __host__ __device__ constexpr int turn_stages(int n) { return n == 512 ? 2 : 3; }
-__host__ __device__ constexpr int turn_nt(int n) { return n == 512 ? 128 : (n == 768 ? 256 : line_nt(n)); }
+__host__ __device__ constexpr int turn_nt(int n) { return n == 512 ? 128 : (n >= 768 ? 256 : line_nt(n)); }
 __host__ __device__ constexpr int turn_ctas_per_sm(int n) { return n == 512 ? 3 : line_ctas_per_sm(n); }
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
@@ -240,8 +241,6 @@ __device__ __forceinline__ void load_bundles(const Sim& S, int unit, float2* s) 
   constexpr int NT = SP_NT;
   constexpr int KU = (NU + NT - 1) / NT;
   const long long P = S.pitch;
-  const long long es = ZAXIS ? (long long)N * P : P;
-  const long long ps = ZAXIS ? P : (long long)N * P;
   const int nb = N * NBP;
   const float2* __restrict__ src = S.spec;
   float4 buf[KU];
@@ -255,7 +254,7 @@ __device__ __forceinline__ void load_bundles(const Sim& S, int unit, float2* s) 
     if ((NU % NT == 0 || u < NU) && b < nb) {
       const int plane = b / NBP, kx0 = (b % NBP) * BW;
       if (kx0 + c < W) {
-        buf[k] = __ldg(reinterpret_cast<const float4*>(src + plane * ps + j * es + kx0 + c));
+        buf[k] = __ldg(reinterpret_cast<const float4*>(src + (ZAXIS ? spec_row(N, plane, j) : spec_row(N, j, plane)) * P + kx0 + c));
         if (kx0 + c + 1 >= W) { buf[k].z = 0.f; buf[k].w = 0.f; }
       }
     }
@@ -279,8 +278,6 @@ __device__ __forceinline__ void store_bundles(const Sim& S, int unit, const floa
   constexpr int NU = BPC * N * U;
   constexpr int NT = SP_NT;
   const long long P = S.pitch;
-  const long long es = ZAXIS ? (long long)N * P : P;
-  const long long ps = ZAXIS ? P : (long long)N * P;
   const int nb = N * NBP;
   float2* __restrict__ dst = S.spec;
   for (int u = threadIdx.x; u < NU; u += NT) {
@@ -290,7 +287,7 @@ __device__ __forceinline__ void store_bundles(const Sim& S, int unit, const floa
     if (b >= nb) continue;
     const int plane = b / NBP, kx0 = (b % NBP) * BW;
     if (kx0 + c < W)
-      *reinterpret_cast<float4*>(dst + plane * ps + j * es + kx0 + c) =
+      *reinterpret_cast<float4*>(dst + (ZAXIS ? spec_row(N, plane, j) : spec_row(N, j, plane)) * P + kx0 + c) =
           *reinterpret_cast<const float4*>(&s[j * LS + i * BW + c]);
   }
 }
@@ -438,11 +435,14 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
     b0 = (unit - __ldg(&w.prefix[si])) * BPC;
     cnt = NB - b0 < BPC ? NB - b0 : BPC;
   };
-  auto coords = [&](int b, int box, int& c0, int& c1, int& c2) {
-    const int plane = b / NBP, kx0 = (b % NBP) * BW;
+  // (the map's axes: 2 kx, y in its block, z, block of y)
+  auto coords = [&](int b, int box, int& c0, int& c1, int& c2, int& c3) {
+    constexpr int YB = spec_block(N);
+    const int plane = b / NBP, kx0 = (b % NBP) * BW, y = ZAX ? plane : box * BOX;
     c0 = 2 * kx0;
-    c1 = ZAX ? plane : box * BOX;
+    c1 = y % YB;
     c2 = ZAX ? box * BOX : plane;
+    c3 = y / YB;
   };
   auto issue_load = [&](int unit, int st) {
     int si, b0, cnt;
@@ -452,9 +452,9 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
     for (int i = 0; i < cnt; ++i)
 #pragma unroll
       for (int box = 0; box < NBOX; ++box) {
-        int c0, c1, c2;
-        coords(b0 + i, box, c0, c1, c2);
-        tma_load_3d(stage_ptr(st) + (i * N + box * BOX) * BW, tm, c0, c1, c2, &bar[st]);
+        int c0, c1, c2, c3;
+        coords(b0 + i, box, c0, c1, c2, c3);
+        tma_load_4d(stage_ptr(st) + (i * N + box * BOX) * BW, tm, c0, c1, c2, c3, &bar[st]);
       }
   };
   int unit = blockIdx.x;
@@ -493,9 +493,9 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
       for (int i = 0; i < cnt; ++i)
 #pragma unroll
         for (int box = 0; box < NBOX; ++box) {
-          int c0, c1, c2;
-          coords(b0 + i, box, c0, c1, c2);
-          tma_store_3d(tm, c0, c1, c2, s + (i * N + box * BOX) * BW);
+          int c0, c1, c2, c3;
+          coords(b0 + i, box, c0, c1, c2, c3);
+          tma_store_4d(tm, c0, c1, c2, c3, s + (i * N + box * BOX) * BW);
         }
       bulk_commit();
     }
@@ -641,9 +641,9 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
 #pragma unroll
         for (int a = 0; a < A; ++a) v[i][a] = __ldg(&src[M / A * a + t + T * i]);
       xrow_transform<N, false>(v, o, rb, t, tw);
-      xrow_untangle_store<N>(o, rb, t, tw, S.spec + row * S.pitch);
+      xrow_untangle_store<N>(o, rb, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch);
     } else {
-      const float2* __restrict__ src = S.spec + row * S.pitch;
+      const float2* __restrict__ src = S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch;
       // all loads of the row issued before any store (the row is M + 1 values)
       constexpr int NLD = (M + 1 + T - 1) / T;
       float2 ld[NLD];
@@ -678,8 +678,8 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
   }
 }
 
-// Tensor map of a half spectrum seen as float32 [z][y][2*pitch], box {2 BW, BOX, 1} for the
-// y pass and {2 BW, 1, BOX} for the z pass.
+// Tensor map of a half spectrum seen as float32 [y / YB][z][y % YB][2*pitch] (spec_row): boxes of BOX
+// rows, {2 BW, min(YB, BOX), 1, rest} for the y pass and {2 BW, 1, BOX, 1} for the z pass.
 inline bool encode_spectrum_map(CUtensorMap* tm, const void* spec, int n, bool zaxis) {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   if (!fn) {
@@ -693,11 +693,13 @@ inline bool encode_spectrum_map(CUtensorMap* tm, const void* spec, int n, bool z
   }
   const cuuint64_t row = (cuuint64_t)2 * cpitch(n);
   const cuuint32_t box_rows = (cuuint32_t)line_box_rows(n);
-  cuuint64_t dims[3] = {row, (cuuint64_t)n, (cuuint64_t)n};
-  cuuint64_t strides[2] = {row * 4, row * 4 * (cuuint64_t)n};
-  cuuint32_t box[3] = {(cuuint32_t)(2 * cline_width(n)), zaxis ? 1u : box_rows, zaxis ? box_rows : 1u};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(spec), dims, strides, box, estr,
+  const cuuint32_t yb = (cuuint32_t)spec_block(n), yrows = yb < box_rows ? yb : box_rows;
+  cuuint64_t dims[4] = {row, yb, (cuuint64_t)n, (cuuint64_t)n / yb};
+  cuuint64_t strides[3] = {row * 4, row * 4 * yb, row * 4 * yb * (cuuint64_t)n};
+  cuuint32_t box[4] = {(cuuint32_t)(2 * cline_width(n)), zaxis ? 1u : yrows, zaxis ? box_rows : 1u,
+                       zaxis ? 1u : box_rows / yrows};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(spec), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -785,7 +787,7 @@ __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsi
     if (warp == 0 && batch == 0) between();
     xrow_transform<N, false>(v2, o2, rb, t, S.tw);
     if (has)
-      xrow_untangle_store<N>(o2, rb, t, S.tw, S.spec + ((long long)(z0 + r / TY) * N + (y0 + r % TY)) * S.pitch);
+      xrow_untangle_store<N>(o2, rb, t, S.tw, S.spec + spec_row(N, y0 + r % TY, z0 + r / TY) * S.pitch);
     __syncwarp();  // the row's lanes are done with its words
     uint4* z4 = reinterpret_cast<uint4*>(row);
     for (int i = t; i < stride / 4; i += T) z4[i] = make_uint4(0u, 0u, 0u, 0u);
