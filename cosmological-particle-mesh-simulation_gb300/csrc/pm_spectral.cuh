@@ -55,21 +55,33 @@ __host__ __device__ constexpr bool tma_lines(int n) { return n >= 32 && line_box
 __host__ __device__ constexpr int line_nt(int n) { return line_small(n) ? 256 : (n == 768 ? 1024 : 512); }
 __host__ __device__ constexpr int line_ctas_per_sm(int n) { return line_small(n) ? 2 : 1; }
 // The z pass with the Green function (the turn) has plans of its own (pm_fft.cuh: TurnPlan), and on
-// these grids its own threads, CTAs per SM and ring stages: 512 in two passes of 16 and 32, one
-// radix-32 transform per thread of 128, three CTAs of two stages (256 us; three radix-8 passes on
-// pairs of lines 288, two CTAs of three stages 284, 256 threads of which half idle 299); 768 of 24
-// and 32 with 256 threads (1.22 ms; radix 3, 4, 8, 8 with 1024 threads 2.9); 1024 of 32 and 32 with
-// 256 threads (2.36 ms; 16, 8, 8 with 512 threads 2.67).  The same passes on bundles of 4 columns
-// (32-byte rows for the copies) take twice the time.
-__host__ __device__ constexpr int turn_stages(int n) { return n == 512 ? 2 : 3; }
-__host__ __device__ constexpr int turn_nt(int n) { return n == 512 ? 128 : (n >= 768 ? 256 : line_nt(n)); }
-__host__ __device__ constexpr int turn_ctas_per_sm(int n) { return n == 512 ? 3 : line_ctas_per_sm(n); }
+// these grids its own threads, CTAs per SM and ring stages, a unit's bundles taken in turn_parts
+// parts: several thin CTAs cover one another's barriers and copies better than one wide one, as
+// long as every thread has a transform of the larger radix to do.  Measured in us a launch:
+//   512  16 x 32, 128 threads, 3 CTAs of 2 stages 256 (8 x 8 x 8 on pairs of lines, 2 x 256 threads,
+//        288; 2 CTAs of 3 stages 284; 256 threads, half idle in the radix-32 pass, 299)
+//   384  24 x 16, 128 threads, 4 CTAs of 2 stages 113 (256 threads 190, 3 CTAs of 3 stages 117)
+//   256  one bundle of the two, 256 threads, 2 CTAs 146 in an ensemble (1 x 512 threads 156, 3 CTAs
+//        of 2 stages 236: spills)
+//   128  one bundle of the four, 128 threads, 4 CTAs 45 for eight grids (1 x 512 threads 52)
+//   768  24 x 32, 256 threads 1.22 ms (3, 4, 8, 8 with 1024 threads 2.9); 1024 32 x 32, 256 threads
+//        2.36 ms (16, 8, 8 with 512 threads 2.67)
+// 192 and below gain nothing.  Bundles of 4 columns on the large grids (32-byte rows for the
+// copies) take twice the time.
+__host__ __device__ constexpr int turn_parts(int n) { return n == 256 ? 2 : (n == 128 ? 4 : 1); }
+__host__ __device__ constexpr int turn_stages(int n) { return n == 512 || n == 384 ? 2 : 3; }
+__host__ __device__ constexpr int turn_nt(int n) {
+  return n == 512 || n == 384 || n == 128 ? 128 : (n == 256 || n >= 768 ? 256 : line_nt(n));
+}
+__host__ __device__ constexpr int turn_ctas_per_sm(int n) {
+  return n == 384 || n == 128 ? 4 : (n == 512 ? 3 : (n == 256 ? 2 : line_ctas_per_sm(n)));
+}
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
   return (size_t)n * cline_width(n) * cline_bpc(n) * sizeof(float2);
 }
 __host__ __device__ constexpr size_t tma_smem_bytes(int n, bool turn) {
-  return (turn ? turn_stages(n) : TMA_STAGES) * tma_stage_bytes(n) + 64;
+  return (turn ? turn_stages(n) * tma_stage_bytes(n) / turn_parts(n) : TMA_STAGES * tma_stage_bytes(n)) + 64;
 }
 __host__ __device__ constexpr bool line_turn(int mode) { return mode == 2 || mode == 3 || mode == 6; }
 
@@ -412,10 +424,13 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
                                   line_turn(MODE) ? turn_ctas_per_sm(N) : line_ctas_per_sm(N))
     k_line_tma(const CUtensorMap* __restrict__ maps, const Sim* __restrict__ sims, Work w, int* err) {
   constexpr int STAGES = line_turn(MODE) ? turn_stages(N) : TMA_STAGES;
-  constexpr int BW = cline_width(N), BPC = cline_bpc(N), NL = BW * BPC;
+  // the turn takes the bundles of a unit in PARTS parts of BPC bundles
+  constexpr int PARTS = line_turn(MODE) ? turn_parts(N) : 1;
+  constexpr int BW = cline_width(N), BPC = cline_bpc(N) / PARTS, NL = BW * BPC;
+  static_assert(BPC * PARTS == cline_bpc(N), "whole bundles");
   constexpr int BOX = line_box_rows(N), NBOX = N / BOX;
   constexpr int NBP = cbundles_per_plane(N), W = chalf(N), NB = N * NBP;
-  constexpr unsigned STAGE = (unsigned)tma_stage_bytes(N);
+  constexpr unsigned STAGE = (unsigned)tma_stage_bytes(N) / PARTS;
   constexpr unsigned BUNDLE = (unsigned)N * BW * sizeof(float2);
   constexpr bool ZAX = MODE >= 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -429,11 +444,11 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
   __syncthreads();
   chain_begin();
   auto stage_ptr = [&](int st) { return stg0 + (size_t)st * (STAGE / sizeof(float2)); };
-  // unit -> (simulation, first bundle, bundles in the unit)
-  auto unit_info = [&](int unit, int& si, int& b0, int& cnt) {
-    si = locate_sim(w, unit);
-    b0 = (unit - __ldg(&w.prefix[si])) * BPC;
-    cnt = NB - b0 < BPC ? NB - b0 : BPC;
+  // part u of the launch -> (simulation, first bundle, bundles in the part: none past the last)
+  auto unit_info = [&](int u, int& si, int& b0, int& cnt) {
+    si = locate_sim(w, u / PARTS);
+    b0 = (u - __ldg(&w.prefix[si]) * PARTS) * BPC;
+    cnt = NB - b0 < BPC ? (NB > b0 ? NB - b0 : 0) : BPC;
   };
   // (the map's axes: 2 kx, y in its block, z, block of y)
   auto coords = [&](int b, int box, int& c0, int& c1, int& c2, int& c3) {
@@ -457,13 +472,14 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
         tma_load_4d(stage_ptr(st) + (i * N + box * BOX) * BW, tm, c0, c1, c2, c3, &bar[st]);
       }
   };
+  const int total = w.total * PARTS;
   int unit = blockIdx.x;
-  if (threadIdx.x == 0 && unit < w.total) issue_load(unit, 0);
+  if (threadIdx.x == 0 && unit < total) issue_load(unit, 0);
   unsigned parity = 0;  // bit st: parity of the next phase of stage st
-  for (int it = 0; unit < w.total; unit += gridDim.x, ++it) {
+  for (int it = 0; unit < total; unit += gridDim.x, ++it) {
     const int st = it % STAGES;
     const int next = unit + gridDim.x;
-    if (threadIdx.x == 0 && next < w.total) {
+    if (threadIdx.x == 0 && next < total) {
       bulk_wait_read<STAGES - 2>();  // the store that last read the stage is done
       issue_load(next, (it + 1) % STAGES);
     }
@@ -1012,7 +1028,7 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
       const size_t sm = tma_smem_bytes(N, turn);
       const int nt = turn ? turn_nt(N) : line_nt(N);
       const int lcap = (turn ? turn_ctas_per_sm(N) : line_ctas_per_sm(N)) * device_sms();
-      const int grid = w.total < lcap ? w.total : lcap;
+      const int units = turn ? w.total * turn_parts(N) : w.total, grid = units < lcap ? units : lcap;
       switch (kind) {
         case SPEC_Y_FWD: launch_chained(k_line_tma<N, 0>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
         case SPEC_Y_INV: launch_chained(k_line_tma<N, 1>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
