@@ -473,7 +473,6 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     PB_CK(cudaEventRecord(b->plan_ev[t], st), "event");
     b->plan_turn = 1 - t;
   }
-  PB_CK(launch_coef(b->d_sims.as<Sim>(), S, 0, st), "coef");
   // (the uploads are ordered on `st` after the steps already enqueued: pageable host memory is
   // staged before cudaMemcpyAsync returns, so no synchronisation is needed here)
   for (size_t g = 0; g < P.sizes.size(); ++g) {
@@ -563,7 +562,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
                           perm, err, b->sms, Launch(st, P.max_n <= 256), true, true, b->group_max.as<unsigned>(),
-                          b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size()),
+                          b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size(), b->d_sims.as<Sim>(), P.nsims),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
@@ -611,13 +610,13 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
       PB_CK(mark(1 + PP_X_R2C + o), "event");
     }
   }
-  // the kick writes the next keys and counts them per row bin for the next step's sort
+  // the kick writes the next keys and counts them per row bin for the next step's sort; the next
+  // step's scatter moves the scale factor on
   PB_CK(launch_kick(ds, work_of(b, PH_KICK, P.fixed_total[PH_KICK]), in, out, perm, b->sort.keys.as<unsigned>(),
                     err, grid_for(P.fixed_total[PH_KICK], b->sms, P.kick_cps), st,
                     b->row_count.as<unsigned>()),
         "kick");
   PB_CK(mark(1 + PP_KICK), "event");
-  PB_CK(launch_coef(b->d_sims.as<Sim>(), P.nsims, 1, Launch(st, P.max_n <= 256)), "coef");
   PB_CK(mark(1 + PP_COEF), "event");
   return PM_OK;
 }
@@ -626,7 +625,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
 int launches_per_step(pm_batch* b) {
   const Plan& P = b->plan;
   // counting sort: 2 scan kernels and the scatter (the kick makes the histogram)
-  int n = 3 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1 + 1;
+  int n = 3 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1;
   // a fused size replaces its x R2C launch by the fused deposit's two (with a dense-first tile
   // order, one launch more); a separate one adds its deposit launch
   for (size_t g = 0; g < P.sizes.size(); ++g)

@@ -111,7 +111,7 @@ struct Sim {
   long long slot_off;  // first particle slot of this simulation in the state being read by the
                        // keys kernel (differs from part_off right after a retirement)
   unsigned row_base;   // first global row (xbits != 0) or row-bin (xbits == 0) of this simulation
-  unsigned pad1;
+  int started;         // 0 until the first step of the plan (step_coefficients)
   float* rho;          // density n^3 (output of the deposit)
   float2* spec;        // half spectrum (rows in the order of spec_row)
   float* phi;          // potential n^3
@@ -135,6 +135,25 @@ struct Sim {
   double a, da, om, ol, ok, h0;
   int step, nsteps, active, fix_f;
 };
+
+// The coefficients of the step at hand, in fp64 (integrate.py:11-13, potential.py:15,
+// cosmology.py:20-27); every step but a plan's first moves the scale factor on.  (A resident step
+// has one thread per simulation do it in the sort's scatter: a kernel of its own took 4 us.)
+__device__ __forceinline__ void step_coefficients(Sim& S) {
+  if (S.started) {
+    S.a += S.da;
+    S.step += 1;
+  }
+  S.started = 1;
+  const double a = S.a, da = S.da, a1 = a + da;
+  const double n3 = (double)S.n * S.n * S.n;
+  S.green = (float)(-3.0 * S.om / 8.0 / a / n3);
+  // integrate.py:12 passes [H0, OL, OK]: H0 in the Omega_m slot unless fix_f is set
+  const double om_slot = S.fix_f ? S.om : S.h0;
+  const double fa1 = 1.0 / sqrt((om_slot + S.ok * a1 + S.ol * a1 * a1 * a1) / a1);
+  S.kick = (float)(da * fa1);
+  S.drift = (float)(da / (a1 * a1) * fa1);
+}
 
 // CTA -> simulation map of one phase: prefix[s] = first work unit of simulation s.
 struct Work {
@@ -253,7 +272,6 @@ cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, con
 cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, Launch st);
 cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
                            const float* pos, const float* vel, float* pos_out, float* vel_out, int* err, Launch st);
-cudaError_t launch_coef(Sim* sims, int nsims, int advance, Launch st);
 cudaError_t deposit_prepare();  // sets kernel attributes of the current device (call before graph capture)
 // order of the fused deposit's tiles (dense tiles first); counts: 2 device words, 0 when the kernel starts
 cudaError_t launch_tile_order(const Sim* sims, const Work& w, const unsigned* row_start, unsigned* order,
@@ -290,11 +308,13 @@ cudaError_t radix_sort(unsigned* keys, unsigned* vals, long long n, int begin_bi
 // specified).  Scratch: count and cursor (nrows each), block_sums (row_sort_block_sums).
 size_t row_sort_block_sums(unsigned nrows);
 // counted: count already holds the row histogram of keys (else it is zeroed and computed here);
-// zero: count is cleared once read; group_max: see row_scan; clear: nclear words set to 0.
+// zero: count is cleared once read; group_max: see row_scan; clear: nclear words set to 0; sims:
+// nsims simulations brought to the step at hand (step_coefficients).
 cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows, unsigned* count,
                               unsigned* row_start, unsigned* cursor, unsigned* block_sums, unsigned* perm, int* err,
                               int sms, Launch st, bool counted = false, bool zero = false,
-                              unsigned* group_max = nullptr, unsigned* clear = nullptr, int nclear = 0);
+                              unsigned* group_max = nullptr, unsigned* clear = nullptr, int nclear = 0, Sim* sims = nullptr,
+                              int nsims = 0);
 // row_start[0..nrows]: exclusive prefix of count; cursor (optional): a copy of its first nrows
 // entries; zero: count is cleared once read; group_max (optional): the largest count of each 16
 // consecutive bins, for the deposit (pm_deposit.cuh).  All arrays 16-byte aligned.

@@ -5,8 +5,6 @@
 //   deposit  deterministic CIC deposit             (density.py:7-48)
 //   kick     CIC gather of the central-difference force, kick and drift
 //                                                  (integrate.py:15-97)
-//   coef     per-step coefficients from the scale factor, in fp64 (integrate.py:11-13,
-//            potential.py:15, cosmology.py:20-27)
 //
 // Cells, weights and keys are defined in pm_cells.cuh, the deposit's accumulation in
 // pm_deposit.cuh (shared with the fused deposit + x-transform kernel).
@@ -506,28 +504,6 @@ __global__ void k_call_begin(Sim* __restrict__ dsim, CallWork* __restrict__ dwor
 }
 
 // ---------------------------------------------------------------------------------
-// coefficients (one thread per simulation, fp64)
-// ---------------------------------------------------------------------------------
-__global__ void k_coef(Sim* sims, int nsims, int advance) {
-  chain_begin();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsims) return;
-  Sim& S = sims[s];
-  if (advance) {
-    S.a += S.da;
-    S.step += 1;
-  }
-  const double a = S.a, da = S.da, a1 = a + da;
-  const double n3 = (double)S.n * S.n * S.n;
-  S.green = (float)(-3.0 * S.om / 8.0 / a / n3);
-  // integrate.py:12 passes [H0, OL, OK]: H0 in the Omega_m slot unless fix_f is set
-  const double om_slot = S.fix_f ? S.om : S.h0;
-  const double fa1 = 1.0 / sqrt((om_slot + S.ok * a1 + S.ol * a1 * a1 * a1) / a1);
-  S.kick = (float)(da * fa1);
-  S.drift = (float)(da / (a1 * a1) * fa1);
-}
-
-// ---------------------------------------------------------------------------------
 // resident-state conversion: absolute (3, np) arrays in particle order <-> displacement
 // state at slots [off, off + np)
 // ---------------------------------------------------------------------------------
@@ -778,9 +754,5 @@ cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* 
   return cudaGetLastError();
 }
 
-cudaError_t launch_coef(Sim* sims, int nsims, int advance, Launch st) {
-  launch_chained(k_coef, (nsims + 127) / 128, 128, 0, st, sims, nsims, advance);
-  return cudaGetLastError();
-}
 
 }  // namespace pm
