@@ -30,14 +30,20 @@ __host__ __device__ constexpr int cx_rows(int n) {
   // rows of the x passes per CTA: ~SP_ELEMS complex, a multiple of 8, at most n*n
   return (SP_ELEMS / (n / 2)) / 8 * 8 > n * n ? n * n : (SP_ELEMS / (n / 2)) / 8 * 8;
 }
-// Line passes of the 512 and 384 grids run two CTAs per SM, each with 32 / 24 KB TMA
-// stages of bundles 8 columns wide; the others one CTA with 64 KB stages (measured: 8-wide
-// bundles slow the 256 grid's z pass 0.34 -> 0.41 ms and the 192 grid's 0.50 -> 0.52 ms).
+// Line passes: units of bundles of 16 columns (8 on 384 and above, where a bundle is 24 KB and more),
+// one unit to a TMA stage of a persistent CTA.  Thin CTAs, two to four to an SM with one or two
+// bundles to a unit, cover one another's barriers and copies, and give a small grid enough units
+// for 152 SMs: with 64 KB stages a 64^3 grid had 24 (y 5.2 us -> 3.3, z 7.3 -> 4.2); 128: y 8.2 ->
+// 5.8; 192 (512 threads on two bundles -> 256 on one, three CTAs): a Poisson solve 91 -> 82 us;
+// 256 the same with two CTAs: 40 resident steps 10.74 -> 10.56 ms.  768 and 1024 keep one CTA with
+// 48 / 64 KB stages.  (8-wide bundles on 256 and 192: z 20% and 4% slower.)
 __host__ __device__ constexpr bool line_small(int n) { return n == 512 || n == 384; }
+__host__ __device__ constexpr bool line_thin(int n) { return n >= 32 && n <= 256; }
 // columns of a line-pass bundle
 __host__ __device__ constexpr int cline_width(int n) { return n >= 512 || line_small(n) ? 8 : 16; }
 // bundles per unit (per TMA stage)
 __host__ __device__ constexpr int cline_bpc(int n) {
+  if (line_thin(n)) return n >= 128 ? 1 : 2;
   return line_small(n) ? SP_ELEMS / 2 / (n * 8)
                        : (SP_ELEMS / (n * cline_width(n)) < 1 ? 1 : SP_ELEMS / (n * cline_width(n)));
 }
@@ -50,38 +56,36 @@ __host__ __device__ constexpr int cpitch(int n) { return (chalf(n) + 15) / 16 * 
 // Line passes that stream through a TMA ring: boxes of at most 256 rows tiling n.
 __host__ __device__ constexpr int line_box_rows(int n) { return n <= 256 ? n : (n % 256 == 0 ? 256 : n / 2); }
 __host__ __device__ constexpr bool tma_lines(int n) { return n >= 32 && line_box_rows(n) <= 256; }
-// Threads of a line-pass CTA: 512 (up to 128 registers), 256 for the two-CTA sizes; 768,
-// transformed line by line, runs 1024.
-__host__ __device__ constexpr int line_nt(int n) { return line_small(n) ? 256 : (n == 768 ? 1024 : 512); }
-__host__ __device__ constexpr int line_ctas_per_sm(int n) { return line_small(n) ? 2 : 1; }
+// Threads of a line-pass CTA and CTAs per SM.  (768, transformed line by
+// line, runs 1024 threads.)
+__host__ __device__ constexpr int line_nt(int n) {
+  return line_small(n) || n == 96 || n == 192 || n == 256 ? 256 : (line_thin(n) ? 128 : (n == 768 ? 1024 : 512));
+}
+__host__ __device__ constexpr int line_ctas_per_sm(int n) {
+  return line_small(n) || n == 256 ? 2 : (n == 96 || n == 192 ? 3 : (line_thin(n) ? 4 : 1));
+}
 // The z pass with the Green function (the turn) has plans of its own (pm_fft.cuh: TurnPlan), and on
-// these grids its own threads, CTAs per SM and ring stages, a unit's bundles taken in turn_parts
-// parts: several thin CTAs cover one another's barriers and copies better than one wide one, as
-// long as every thread has a transform of the larger radix to do.  Measured in us a launch:
+// the larger grids its own threads, CTAs per SM and ring stages, as thin as every thread still
+// has a transform of the larger radix to do.  Measured in us a launch:
 //   512  16 x 32, 128 threads, 3 CTAs of 2 stages 256 (8 x 8 x 8 on pairs of lines, 2 x 256 threads,
 //        288; 2 CTAs of 3 stages 284; 256 threads, half idle in the radix-32 pass, 299)
 //   384  24 x 16, 128 threads, 4 CTAs of 2 stages 113 (256 threads 190, 3 CTAs of 3 stages 117)
-//   256  one bundle of the two, 256 threads, 2 CTAs 146 in an ensemble (1 x 512 threads 156, 3 CTAs
-//        of 2 stages 236: spills)
-//   128  one bundle of the four, 128 threads, 4 CTAs 45 for eight grids (1 x 512 threads 52)
 //   768  24 x 32, 256 threads 1.22 ms (3, 4, 8, 8 with 1024 threads 2.9); 1024 32 x 32, 256 threads
 //        2.36 ms (16, 8, 8 with 512 threads 2.67)
-// 192 and below gain nothing.  Bundles of 4 columns on the large grids (32-byte rows for the
-// copies) take twice the time.
-__host__ __device__ constexpr int turn_parts(int n) { return n == 256 ? 2 : (n == 128 ? 4 : 1); }
+// Bundles of 4 columns on 768 and 1024 (32-byte rows for the copies) take twice the time.
 __host__ __device__ constexpr int turn_stages(int n) { return n == 512 || n == 384 ? 2 : 3; }
 __host__ __device__ constexpr int turn_nt(int n) {
-  return n == 512 || n == 384 || n == 128 ? 128 : (n == 256 || n >= 768 ? 256 : line_nt(n));
+  return n == 512 || n == 384 ? 128 : (n >= 768 ? 256 : line_nt(n));
 }
 __host__ __device__ constexpr int turn_ctas_per_sm(int n) {
-  return n == 384 || n == 128 ? 4 : (n == 512 ? 3 : (n == 256 ? 2 : line_ctas_per_sm(n)));
+  return n == 384 ? 4 : (n == 512 ? 3 : line_ctas_per_sm(n));
 }
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
   return (size_t)n * cline_width(n) * cline_bpc(n) * sizeof(float2);
 }
 __host__ __device__ constexpr size_t tma_smem_bytes(int n, bool turn) {
-  return (turn ? turn_stages(n) * tma_stage_bytes(n) / turn_parts(n) : TMA_STAGES * tma_stage_bytes(n)) + 64;
+  return (turn ? turn_stages(n) * tma_stage_bytes(n) : TMA_STAGES * tma_stage_bytes(n)) + 64;
 }
 __host__ __device__ constexpr bool line_turn(int mode) { return mode == 2 || mode == 3 || mode == 6; }
 
@@ -424,13 +428,10 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
                                   line_turn(MODE) ? turn_ctas_per_sm(N) : line_ctas_per_sm(N))
     k_line_tma(const CUtensorMap* __restrict__ maps, const Sim* __restrict__ sims, Work w, int* err) {
   constexpr int STAGES = line_turn(MODE) ? turn_stages(N) : TMA_STAGES;
-  // the turn takes the bundles of a unit in PARTS parts of BPC bundles
-  constexpr int PARTS = line_turn(MODE) ? turn_parts(N) : 1;
-  constexpr int BW = cline_width(N), BPC = cline_bpc(N) / PARTS, NL = BW * BPC;
-  static_assert(BPC * PARTS == cline_bpc(N), "whole bundles");
+  constexpr int BW = cline_width(N), BPC = cline_bpc(N), NL = BW * BPC;
   constexpr int BOX = line_box_rows(N), NBOX = N / BOX;
   constexpr int NBP = cbundles_per_plane(N), W = chalf(N), NB = N * NBP;
-  constexpr unsigned STAGE = (unsigned)tma_stage_bytes(N) / PARTS;
+  constexpr unsigned STAGE = (unsigned)tma_stage_bytes(N);
   constexpr unsigned BUNDLE = (unsigned)N * BW * sizeof(float2);
   constexpr bool ZAX = MODE >= 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -444,11 +445,11 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
   __syncthreads();
   chain_begin();
   auto stage_ptr = [&](int st) { return stg0 + (size_t)st * (STAGE / sizeof(float2)); };
-  // part u of the launch -> (simulation, first bundle, bundles in the part: none past the last)
-  auto unit_info = [&](int u, int& si, int& b0, int& cnt) {
-    si = locate_sim(w, u / PARTS);
-    b0 = (u - __ldg(&w.prefix[si]) * PARTS) * BPC;
-    cnt = NB - b0 < BPC ? (NB > b0 ? NB - b0 : 0) : BPC;
+  // unit -> (simulation, first bundle, bundles in the unit)
+  auto unit_info = [&](int unit, int& si, int& b0, int& cnt) {
+    si = locate_sim(w, unit);
+    b0 = (unit - __ldg(&w.prefix[si])) * BPC;
+    cnt = NB - b0 < BPC ? NB - b0 : BPC;
   };
   // (the map's axes: 2 kx, y in its block, z, block of y)
   auto coords = [&](int b, int box, int& c0, int& c1, int& c2, int& c3) {
@@ -472,14 +473,13 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
         tma_load_4d(stage_ptr(st) + (i * N + box * BOX) * BW, tm, c0, c1, c2, c3, &bar[st]);
       }
   };
-  const int total = w.total * PARTS;
   int unit = blockIdx.x;
-  if (threadIdx.x == 0 && unit < total) issue_load(unit, 0);
+  if (threadIdx.x == 0 && unit < w.total) issue_load(unit, 0);
   unsigned parity = 0;  // bit st: parity of the next phase of stage st
-  for (int it = 0; unit < total; unit += gridDim.x, ++it) {
+  for (int it = 0; unit < w.total; unit += gridDim.x, ++it) {
     const int st = it % STAGES;
     const int next = unit + gridDim.x;
-    if (threadIdx.x == 0 && next < total) {
+    if (threadIdx.x == 0 && next < w.total) {
       bulk_wait_read<STAGES - 2>();  // the store that last read the stage is done
       issue_load(next, (it + 1) % STAGES);
     }
@@ -1028,7 +1028,7 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
       const size_t sm = tma_smem_bytes(N, turn);
       const int nt = turn ? turn_nt(N) : line_nt(N);
       const int lcap = (turn ? turn_ctas_per_sm(N) : line_ctas_per_sm(N)) * device_sms();
-      const int units = turn ? w.total * turn_parts(N) : w.total, grid = units < lcap ? units : lcap;
+      const int grid = w.total < lcap ? w.total : lcap;
       switch (kind) {
         case SPEC_Y_FWD: launch_chained(k_line_tma<N, 0>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
         case SPEC_Y_INV: launch_chained(k_line_tma<N, 1>, grid, nt, sm, st, maps, sims, w, err); return cudaGetLastError();
