@@ -93,30 +93,39 @@ __host__ __device__ constexpr bool line_turn(int mode) { return mode == 2 || mod
 // by T lanes of a warp and transformed in passes of radix A, (B,) C, M = A C or A B C, through an
 // exchange buffer of the row that only its warp synchronises on
 // (n: radices, T) -- 32: 4x4, 4; 48: 4x6, 2; 64: 8x4, 4; 96: 4x12, 4; 128: 8x8, 8; 192: 8x12, 4;
-// 256: 16x8, 8; 384: 8x24, 8; 512: 16x16, 16; 768: 8x8x6, 16; 1024: 8x8x8, 32
+// 256: 16x8, 8; 384: 8x24, 8; 512: 16x16, 16; 768: 8x8x6, 16; 1024: 8x8x8, 32, inverse 16x32, 16
 // (the radix-3 rows with the smaller factor first: x C2R per 134M cells 96: 0.119 -> 0.115,
-// 192: 0.315 -> 0.257, 384: 0.269 -> 0.256 ms.  Two passes for 768 and 1024 would hold 24 x 16 or
-// 32 x 16 points in 64 registers a lane and more; three passes hold 24 and 16 points.)
+// 192: 0.315 -> 0.257, 384: 0.269 -> 0.256 ms.  1024 in two passes holds 32 points, 64 registers, a
+// lane: the C2R pass, which is alone in its kernel, 1.90 -> 1.39 ms, but the fused deposit, left with
+// two CTAs per SM, 3.35 -> 3.67; the plain R2C keeps the fused one's plan, and so its bits.  768 in
+// two passes would hold 48 points.)
 __host__ __device__ constexpr bool xrow_ok(int n) { return n >= 32; }
-__host__ __device__ constexpr int xrow_A(int n) {
+__host__ __device__ constexpr int xrow_A(int n, bool inv) {
+  if (n == 1024) return inv ? 16 : 8;
   return n >= 768 ? 8 : (n % 3 == 0 ? (n <= 96 ? 4 : 8) : (n >= 256 ? 16 : (n == 32 ? 4 : 8)));
 }
-__host__ __device__ constexpr int xrow_B(int n) { return n >= 768 ? 8 : 1; }
-__host__ __device__ constexpr int xrow_C(int n) { return n / 2 / (xrow_A(n) * xrow_B(n)); }
-__host__ __device__ constexpr int xrow_T(int n) {
-  return n == 1024 ? 32 : (n == 768 || n == 512 ? 16 : (n == 48 ? 2 : (n % 3 == 0 && n != 384 ? 4 : (n <= 64 ? 4 : 8))));
+__host__ __device__ constexpr int xrow_B(int n, bool inv) { return n == 768 || (n == 1024 && !inv) ? 8 : 1; }
+__host__ __device__ constexpr int xrow_C(int n, bool inv) { return n / 2 / (xrow_A(n, inv) * xrow_B(n, inv)); }
+__host__ __device__ constexpr int xrow_T(int n, bool inv) {
+  return n == 1024 && !inv ? 32 : (n >= 768 || n == 512 ? 16 : (n == 48 ? 2 : (n % 3 == 0 && n != 384 ? 4 : (n <= 64 ? 4 : 8))));
 }
-__host__ __device__ constexpr int xrow_rows_per_warp(int n) { return 32 / xrow_T(n); }
+__host__ __device__ constexpr int xrow_rows_per_warp(int n, bool inv) { return 32 / xrow_T(n, inv); }
+// rows of a work unit, which a warp takes: one unit for both directions
+__host__ __device__ constexpr int xrow_unit_rows(int n) {
+  return xrow_rows_per_warp(n, true) > xrow_rows_per_warp(n, false) ? xrow_rows_per_warp(n, true)
+                                                                    : xrow_rows_per_warp(n, false);
+}
 // complex elements of a row's exchange buffer: C rows of A (padded) in two passes; in three,
 // the row with one element of padding after every A
-__host__ __device__ constexpr int xrow_exchange(int n) {
-  return xrow_B(n) == 1 ? xrow_C(n) * (xrow_A(n) + 1) : n / 2 + n / 2 / xrow_A(n);
+__host__ __device__ constexpr int xrow_exchange(int n, bool inv) {
+  return xrow_B(n, inv) == 1 ? xrow_C(n, inv) * (xrow_A(n, inv) + 1) : n / 2 + n / 2 / xrow_A(n, inv);
 }
 // threads of a row-transform CTA: up to 8 warps, their exchange buffers within 40 KB of
 // static shared memory
-__host__ __device__ constexpr int xrow_warp_bytes(int n) { return xrow_rows_per_warp(n) * xrow_exchange(n) * 8; }
-__host__ __device__ constexpr int xrow_nt(int n) {
-  return 32 * (40960 / xrow_warp_bytes(n) < 8 ? (40960 / xrow_warp_bytes(n) < 1 ? 1 : 40960 / xrow_warp_bytes(n)) : 8);
+__host__ __device__ constexpr int xrow_warp_bytes(int n, bool inv) { return xrow_rows_per_warp(n, inv) * xrow_exchange(n, inv) * 8; }
+__host__ __device__ constexpr int xrow_nt(int n, bool inv) {
+  const int warps = 40960 / xrow_warp_bytes(n, inv);
+  return 32 * (warps < 8 ? (warps < 1 ? 1 : warps) : 8);
 }
 
 __host__ __device__ constexpr size_t x_smem_bytes(int n) {
@@ -528,20 +537,20 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
 // Three passes, M = A B C: Stockham passes of radix A, B, C on the row's exchange buffer, element
 // e at e + e / A (pass 1 stores A e + r: without the padding all lanes would hit one bank).
 // R2C: z[j] = x[2j] + i x[2j+1] read straight from the density rows, Z untangled into the
-// half spectrum.  C2R: the spectrum row is staged, tangled into pass 1, and z written as
-// pairs of reals.  Loads and stores of T lanes are consecutive (coalesced).  A work unit
-// is the 32 / T rows of one warp.
+// half spectrum.  C2R: the spectrum row is tangled into pass 1, and z written as pairs of reals.  Loads and stores of T lanes are consecutive (coalesced).  A work unit
+// is the 32 / T rows of one warp (of the direction that takes more).
 // ---------------------------------------------------------------------------------
 // A row's passes; v holds z[(M / A) a + t + T i] on entry, o holds Z[t + T i + (M / C) d] on exit.
 // rb: the row's exchange buffer.
-template <int N> constexpr int xrow_NB1 = N / 2 / xrow_A(N) / xrow_T(N);  // A-point DFTs of a lane
-template <int N> constexpr int xrow_NB2 = N / 2 / xrow_C(N) / xrow_T(N);  // C-point DFTs of a lane
+// A-point and C-point DFTs of a lane
+template <int N, bool INV> constexpr int xrow_NB1 = N / 2 / xrow_A(N, INV) / xrow_T(N, INV);
+template <int N, bool INV> constexpr int xrow_NB2 = N / 2 / xrow_C(N, INV) / xrow_T(N, INV);
 
 template <int N, bool INV>
-__device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N>][xrow_A(N)], float2 (&o)[xrow_NB2<N>][xrow_C(N)],
-                                               float2* rb, int t, const float2* __restrict__ tw) {
-  constexpr int M = N / 2, A = xrow_A(N), B = xrow_B(N), C = xrow_C(N), T = xrow_T(N);
-  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
+__device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xrow_A(N, INV)],
+                                               float2 (&o)[xrow_NB2<N, INV>][xrow_C(N, INV)], float2* rb, int t, const float2* __restrict__ tw) {
+  constexpr int M = N / 2, A = xrow_A(N, INV), B = xrow_B(N, INV), C = xrow_C(N, INV), T = xrow_T(N, INV);
+  constexpr int NB1 = xrow_NB1<N, INV>, NB2 = xrow_NB2<N, INV>;
   auto twiddle = [&](int m) {
     float2 w = __ldg(&tw[m * 2]);
     if (INV) w.y = -w.y;
@@ -609,35 +618,83 @@ __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N>][xrow_A(N
   }
 }
 
-// R2C end of a row: Z (in o) is untangled into the half-spectrum row dst[0..M].
+// The ends of a row work on the pairs (k, M - k).  Lane t holds the K = M / T elements t + T m: the
+// partner of element m is element K - 1 - m of lane T - t -- lane 0's is its own K - m, and k = 0
+// goes with k = M -- so each lane takes the pairs of its lower half, with the partners brought by
+// shuffles.  (Through the exchange buffer, every element written once and read twice, the ends
+// took more of the shared-memory pipe than the transform itself: x C2R of 192^3 20.6 -> 17.7 us, 512^3
+// 195 -> 174, R2C of 192^3 21.5 -> 15.7, the fused deposit of 1024^3 3.64 -> 3.35 ms.)  Lane 0 is one pair ahead in the
+// upper half (its k = M / 2, alone, starts it), so that the T elements of a step are consecutive
+// and aligned there too.
+template <int T>
+__device__ __forceinline__ float2 xrow_partner(float2 v, int t) {
+  const int src = (T - t) & (T - 1);
+  return make_float2(__shfl_sync(FULL, v.x, src, T), __shfl_sync(FULL, v.y, src, T));
+}
+__device__ __forceinline__ float2 cselect(bool c, float2 a, float2 b) { return make_float2(c ? a.x : b.x, c ? a.y : b.y); }
+
+// R2C end of a row: Z (in o) is untangled into the half-spectrum row dst[0..M] (if `store`).
+// Every lane of the warp calls it.
 template <int N>
-__device__ __forceinline__ void xrow_untangle_store(const float2 (&o)[xrow_NB2<N>][xrow_C(N)], float2* rb,
-                                                    int t, const float2* __restrict__ tw, float2* __restrict__ dst) {
-  constexpr int M = N / 2, C = xrow_C(N), T = xrow_T(N);
-  __syncwarp();
+__device__ __forceinline__ void xrow_untangle_store(const float2 (&o)[xrow_NB2<N, false>][xrow_C(N, false)], int t,
+                                                    const float2* __restrict__ tw, float2* __restrict__ dst, bool store) {
+  constexpr int M = N / 2, T = xrow_T(N, false), NB = xrow_NB2<N, false>, K = M / T;
+  static_assert(K % 2 == 0 && (T & (T - 1)) == 0, "pairs of a lane");
+  // X[k] = E + W^k O, X[M - k] = conj(E - W^k O)
+  float2 up = conjf2(o[K / 2 % NB][K / 2 / NB]);  // lane 0: X[M / 2]
 #pragma unroll
-  for (int i = 0; i < xrow_NB2<N>; ++i)
-#pragma unroll
-    for (int d = 0; d < C; ++d) rb[t + T * i + M / C * d] = o[i][d];
-  __syncwarp();
-  // X[k] = E[k] + W^k O[k], k = 0..M
-  for (int k = t; k <= M; k += T) {
-    const float2 zk = rb[k == M ? 0 : k];
-    const float2 zc = conjf2(rb[k == 0 ? 0 : M - k]);
+  for (int m = K / 2 - 1; m >= 0; --m) {
+    const int j = K - 1 - m, j0 = (K - m) % K, k = t + T * m;
+    const float2 zk = o[m % NB][m / NB];
+    const float2 zc = conjf2(xrow_partner<T>(cselect(t == 0, o[j0 % NB][j0 / NB], o[j % NB][j / NB]), t));
     const float2 e = cscale(cadd(zk, zc), 0.5f);
     const float2 od = cscale(mul_mi<false>(csub(zk, zc)), 0.5f);
-    dst[k] = cadd(e, cmul(__ldg(&tw[k]), od));
+    const float2 wo = cmul(__ldg(&tw[k]), od);
+    const float2 xm = conjf2(csub(e, wo));
+    if (store) {
+      dst[k] = cadd(e, wo);
+      dst[(t == 0 ? M - T : M - t) - T * m] = cselect(t == 0, up, xm);
+    }
+    up = xm;
+  }
+  if (store && t == 0) dst[M] = up;
+}
+
+// C2R start of a row: the half-spectrum row src[0..M] is loaded and tangled into pass 1's input,
+// Z[k] = (X[k] + X*[M-k]) + i W^-k (X[k] - X*[M-k]).  Every lane of the warp calls it.
+template <int N>
+__device__ __forceinline__ void xrow_load_tangle(float2 (&v)[xrow_NB1<N, true>][xrow_A(N, true)], int t,
+                                                 const float2* __restrict__ tw, const float2* __restrict__ src) {
+  constexpr int M = N / 2, T = xrow_T(N, true), NB = xrow_NB1<N, true>, K = M / T;
+  static_assert(K % 2 == 0 && (T & (T - 1)) == 0, "pairs of a lane");
+#pragma unroll
+  for (int m = 0; m < K; ++m) v[m % NB][m / NB] = __ldg(&src[t + T * m]);
+  const float2 top = t == 0 ? __ldg(&src[M]) : make_float2(0.f, 0.f);
+  float2 up = v[K / 2 % NB][K / 2 / NB];  // lane 0: Z[M / 2] = 2 conj(X[M / 2])
+  up = make_float2(2.f * up.x, -2.f * up.y);
+#pragma unroll
+  for (int m = K / 2 - 1; m >= 0; --m) {
+    const int j = K - 1 - m, j0 = K - m;
+    const float2 xk = v[m % NB][m / NB];
+    const float2 x0 = m == 0 ? top : v[j0 % K % NB][j0 % K / NB];
+    const float2 xm = xrow_partner<T>(cselect(t == 0, x0, v[j % NB][j / NB]), t);
+    const float2 ap = cadd(xk, conjf2(xm)), bm = csub(xk, conjf2(xm));
+    const float2 tt = cmul(conjf2(__ldg(&tw[t + T * m])), bm);
+    v[m % NB][m / NB] = make_float2(ap.x - tt.y, ap.y + tt.x);
+    const float2 back = xrow_partner<T>(make_float2(ap.x + tt.y, tt.x - ap.y), t);
+    v[j % NB][j / NB] = cselect(t == 0, up, back);
+    up = back;
   }
 }
 
 template <int N, bool C2R>
-__global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ sims, Work w) {
+__global__ void __launch_bounds__(xrow_nt(N, C2R)) k_x_row(const Sim* __restrict__ sims, Work w) {
   chain_begin();
-  constexpr int XR_NT = xrow_nt(N);
-  constexpr int M = N / 2, A = xrow_A(N), B = xrow_B(N), C = xrow_C(N), T = xrow_T(N), RPW = 32 / T;
-  constexpr int RB = xrow_exchange(N);  // exchange buffer of a row (>= M + 1)
-  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
-  static_assert(A * B * C == M && NB1 * A * T == M && NB2 * C * T == M && RB >= M + 1, "row plan");
+  constexpr int XR_NT = xrow_nt(N, C2R);
+  constexpr int M = N / 2, A = xrow_A(N, C2R), B = xrow_B(N, C2R), C = xrow_C(N, C2R), T = xrow_T(N, C2R), RPW = 32 / T;
+  constexpr int UR = xrow_unit_rows(N), RB = xrow_exchange(N, C2R);  // exchange buffer of a row
+  constexpr int NB1 = xrow_NB1<N, C2R>, NB2 = xrow_NB2<N, C2R>;
+  static_assert(A * B * C == M && NB1 * A * T == M && NB2 * C * T == M, "row plan");
   __shared__ float2 sbuf[XR_NT / 32][RPW][RB];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane / T, t = lane % T;
@@ -646,50 +703,29 @@ __global__ void __launch_bounds__(xrow_nt(N)) k_x_row(const Sim* __restrict__ si
   for (long long unit = (long long)blockIdx.x * (XR_NT / 32) + wid; unit < w.total; unit += nw) {
     const int si = locate_sim(w, (int)unit);
     const Sim& S = sims[si];
-    const long long row = ((long long)unit - __ldg(&w.prefix[si])) * RPW + sub;
     const float2* __restrict__ tw = S.tw;
-    float2 v[NB1][A];
-    float2 o[NB2][C];
-    if (!C2R) {
-      const float2* __restrict__ src = reinterpret_cast<const float2*>(S.rho) + row * M;
+    long long row = ((long long)unit - __ldg(&w.prefix[si])) * UR + sub;
+#pragma unroll 1
+    for (int r = 0; r < UR; r += RPW, row += RPW) {
+      float2 v[NB1][A];
+      float2 o[NB2][C];
+      if constexpr (!C2R) {
+        const float2* __restrict__ src = reinterpret_cast<const float2*>(S.rho) + row * M;
 #pragma unroll
-      for (int i = 0; i < NB1; ++i)
+        for (int i = 0; i < NB1; ++i)
 #pragma unroll
-        for (int a = 0; a < A; ++a) v[i][a] = __ldg(&src[M / A * a + t + T * i]);
-      xrow_transform<N, false>(v, o, rb, t, tw);
-      xrow_untangle_store<N>(o, rb, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch);
-    } else {
-      const float2* __restrict__ src = S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch;
-      // all loads of the row issued before any store (the row is M + 1 values)
-      constexpr int NLD = (M + 1 + T - 1) / T;
-      float2 ld[NLD];
+          for (int a = 0; a < A; ++a) v[i][a] = __ldg(&src[M / A * a + t + T * i]);
+        xrow_transform<N, false>(v, o, rb, t, tw);
+        xrow_untangle_store<N>(o, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch, true);
+      } else {
+        xrow_load_tangle<N>(v, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch);
+        xrow_transform<N, true>(v, o, rb, t, tw);
+        float2* __restrict__ dst = reinterpret_cast<float2*>(S.phi) + row * M;
 #pragma unroll
-      for (int i = 0; i < NLD; ++i) {
-        const int k = t + T * i;
-        ld[i] = k <= M ? __ldg(&src[k]) : make_float2(0.f, 0.f);
+        for (int i = 0; i < NB2; ++i)
+#pragma unroll
+          for (int d = 0; d < C; ++d) dst[t + T * i + M / C * d] = o[i][d];
       }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < NLD; ++i)
-        if (t + T * i <= M) rb[t + T * i] = ld[i];
-      __syncwarp();
-      // tangle: Z[j] = (X[j] + X*[M-j]) + i W^-j (X[j] - X*[M-j])
-#pragma unroll
-      for (int i = 0; i < NB1; ++i)
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-          const int j = M / A * a + t + T * i;
-          const float2 xk = rb[j], xm = rb[M - j];
-          const float2 ap = cadd(xk, conjf2(xm)), bm = csub(xk, conjf2(xm));
-          const float2 tt = cmul(conjf2(__ldg(&tw[j])), bm);
-          v[i][a] = make_float2(ap.x - tt.y, ap.y + tt.x);
-        }
-      xrow_transform<N, true>(v, o, rb, t, tw);
-      float2* __restrict__ dst = reinterpret_cast<float2*>(S.phi) + row * M;
-#pragma unroll
-      for (int i = 0; i < NB2; ++i)
-#pragma unroll
-        for (int d = 0; d < C; ++d) dst[t + T * i + M / C * d] = o[i][d];
     }
   }
 }
@@ -728,7 +764,7 @@ inline bool encode_spectrum_map(CUtensorMap* tm, const void* spec, int n, bool z
 __host__ __device__ constexpr bool deposit_r2c_ok(int n) { return xrow_ok(n); }
 // words of a tile row: its cells, or the exchange buffer of its transform, which overlays them
 __host__ __device__ constexpr int dep_row_words(int n) {
-  return 2 * xrow_exchange(n) > n ? 2 * xrow_exchange(n) : n;
+  return 2 * xrow_exchange(n, false) > n ? 2 * xrow_exchange(n, false) : n;
 }
 __host__ __device__ constexpr size_t dep_tile_bytes(int n) { return (size_t)TZ * TY * dep_row_words(n) * sizeof(unsigned); }
 constexpr int DEP_ROW_NT = 256;  // threads (the 16 rows of a 1024 tile take them twice: 3.95 ms, 512 threads 4.34)
@@ -736,7 +772,7 @@ constexpr int DEP_ROW_NT = 256;  // threads (the 16 rows of a 1024 tile take the
 // so on the sizes with T < 16 a CTA takes several tiles at once -- its warps split into one
 // group per tile for the particle loop and share all the rows in the transform.
 __host__ __device__ constexpr int dep_tiles(int n) {
-  return n == 1024 ? 1 : (16 / xrow_T(n) > 4 ? 4 : 16 / xrow_T(n));
+  return n == 1024 ? 1 : (16 / xrow_T(n, false) > 4 ? 4 : 16 / xrow_T(n, false));
 }
 // CTAs per SM, which bounds the registers of a thread: four (64) where the row plan leaves few
 // spills (512: 423 us, three 466; 256 in an ensemble 234, three 262; 64 and 96 lose 10%), else three
@@ -768,8 +804,8 @@ __device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restri
 template <int N, int NT, int TPB, bool TWO, class H, class F, class G>
 __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsigned* acc, int stride, const TileSum* s_ts,
                                               H tile, F between, G after) {
-  constexpr int NL = TZ * TY, M = N / 2, A = xrow_A(N), C = xrow_C(N), T = xrow_T(N), RPW = 32 / T;
-  constexpr int NB1 = xrow_NB1<N>, NB2 = xrow_NB2<N>;
+  constexpr int NL = TZ * TY, M = N / 2, A = xrow_A(N, false), C = xrow_C(N, false), T = xrow_T(N, false), RPW = 32 / T;
+  constexpr int NB1 = xrow_NB1<N, false>, NB2 = xrow_NB2<N, false>;
   constexpr int BROWS = NT / 32 * RPW, NBATCH = (TPB * NL + BROWS - 1) / BROWS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / T, t = lane % T;
@@ -802,8 +838,7 @@ __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsi
       }
     if (warp == 0 && batch == 0) between();
     xrow_transform<N, false>(v2, o2, rb, t, S.tw);
-    if (has)
-      xrow_untangle_store<N>(o2, rb, t, S.tw, S.spec + spec_row(N, y0 + r % TY, z0 + r / TY) * S.pitch);
+    xrow_untangle_store<N>(o2, t, S.tw, S.spec + spec_row(N, y0 + r % TY, z0 + r / TY) * S.pitch, has);
     __syncwarp();  // the row's lanes are done with its words
     uint4* z4 = reinterpret_cast<uint4*>(row);
     for (int i = t; i < stride / 4; i += T) z4[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -1008,10 +1043,11 @@ cudaError_t spectral_launch(SpecKind kind, const Sim* sims, Work w, int ctas, La
   if constexpr (xrow_ok(N)) {
     if (kind == SPEC_X_R2C || kind == SPEC_X_C2R) {
       // ctas: the cap on the CTAs of the persistent row transform (the batch engine tunes it)
-      const int per = xrow_nt(N) / 32, want = (w.total + per - 1) / per, cap = ctas > 0 ? ctas : device_sms() * 8;
+      const int nt = xrow_nt(N, kind == SPEC_X_C2R);
+      const int per = nt / 32, want = (w.total + per - 1) / per, cap = ctas > 0 ? ctas : device_sms() * 8;
       const int g = want < cap ? want : cap;
-      if (kind == SPEC_X_R2C) launch_chained(k_x_row<N, false>, g, xrow_nt(N), 0, st, sims, w);
-      else launch_chained(k_x_row<N, true>, g, xrow_nt(N), 0, st, sims, w);
+      if (kind == SPEC_X_R2C) launch_chained(k_x_row<N, false>, g, nt, 0, st, sims, w);
+      else launch_chained(k_x_row<N, true>, g, nt, 0, st, sims, w);
       return cudaGetLastError();
     }
   }
