@@ -70,15 +70,16 @@ __host__ __device__ constexpr int line_ctas_per_sm(int n) {
 //   512  16 x 32, 128 threads, 3 CTAs of 2 stages 256 (8 x 8 x 8 on pairs of lines, 2 x 256 threads,
 //        288; 2 CTAs of 3 stages 284; 256 threads, half idle in the radix-32 pass, 299)
 //   384  24 x 16, 128 threads, 4 CTAs of 2 stages 113 (256 threads 190, 3 CTAs of 3 stages 117)
-//   768  24 x 32, 256 threads 1.22 ms (3, 4, 8, 8 with 1024 threads 2.9); 1024 32 x 32, 256 threads
-//        2.36 ms (16, 8, 8 with 512 threads 2.67)
+//   768  24 x 32, 256 threads, 2 CTAs of 2 stages 1.05 ms (one CTA of 3 stages 1.22, 2 of one stage
+//        1.20; 3, 4, 8, 8 with 1024 threads 2.9)
+//   1024 32 x 32, 256 threads 2.36 ms (16, 8, 8 with 512 threads 2.67; 2 CTAs of one stage the same)
 // Bundles of 4 columns on 768 and 1024 (32-byte rows for the copies) take twice the time.
-__host__ __device__ constexpr int turn_stages(int n) { return n == 512 || n == 384 ? 2 : 3; }
+__host__ __device__ constexpr int turn_stages(int n) { return n == 512 || n == 384 || n == 768 ? 2 : 3; }
 __host__ __device__ constexpr int turn_nt(int n) {
   return n == 512 || n == 384 ? 128 : (n >= 768 ? 256 : line_nt(n));
 }
 __host__ __device__ constexpr int turn_ctas_per_sm(int n) {
-  return n == 384 ? 4 : (n == 512 ? 3 : line_ctas_per_sm(n));
+  return n == 384 ? 4 : (n == 512 ? 3 : (n == 768 ? 2 : line_ctas_per_sm(n)));
 }
 constexpr int TMA_STAGES = 3;
 __host__ __device__ constexpr size_t tma_stage_bytes(int n) {
