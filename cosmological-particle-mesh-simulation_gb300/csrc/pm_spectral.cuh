@@ -538,8 +538,9 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
 // Three passes, M = A B C: Stockham passes of radix A, B, C on the row's exchange buffer, element
 // e at e + e / A (pass 1 stores A e + r: without the padding all lanes would hit one bank).
 // R2C: z[j] = x[2j] + i x[2j+1] read straight from the density rows, Z untangled into the
-// half spectrum.  C2R: the spectrum row is tangled into pass 1, and z written as pairs of reals.  Loads and stores of T lanes are consecutive (coalesced).  A work unit
-// is the 32 / T rows of one warp (of the direction that takes more).
+// half spectrum.  C2R: the spectrum row is tangled into pass 1, and z written as pairs of reals.
+// Loads and stores of T lanes are consecutive (coalesced).  A work unit is the 32 / T rows of one
+// warp (of the direction that takes more).
 // ---------------------------------------------------------------------------------
 // A row's passes; v holds z[(M / A) a + t + T i] on entry, o holds Z[t + T i + (M / C) d] on exit.
 // rb: the row's exchange buffer.
@@ -547,12 +548,49 @@ __global__ void __launch_bounds__(line_turn(MODE) ? turn_nt(N) : line_nt(N),
 template <int N, bool INV> constexpr int xrow_NB1 = N / 2 / xrow_A(N, INV) / xrow_T(N, INV);
 template <int N, bool INV> constexpr int xrow_NB2 = N / 2 / xrow_C(N, INV) / xrow_T(N, INV);
 
-template <int N, bool INV>
+// The twiddles between a row's passes, in shared memory in the order in which the lanes use them.  Read
+// from the table by their exponent, the lanes' words lie up to 15 apart -- 8 to 16 cache lines a
+// load, a quarter to a half of the L1 wavefronts of the x passes.  From 256 cells a side (x C2R of
+// 384^3 88 -> 77 us, 512^3 171 -> 167, 768^3 721 -> 643, 1024^3 1.38 -> 1.31 ms), in the fused deposit
+// from 192 (256^3 59 -> 55 us, 512^3 400 -> 356, 768^3 1.60 -> 1.42 ms, 1024^3 3.33 -> 3.16; eight
+// 192^3 204 -> 193 us); shorter rows have few lines to a load (192 x passes 15.4 -> 16.2).
+__host__ __device__ constexpr bool xrow_table(int n, bool fused) { return n >= (fused ? 192 : 256); }
+// j's of the third pass that are in the table (three CTAs of the fused deposit on 1024 leave 2.7 KB each)
+__host__ __device__ constexpr int xrow_table_j(int n, bool inv) {
+  return n == 1024 ? xrow_T(n, inv) : n / 2 / xrow_C(n, inv);
+}
+template <int N, bool INV, bool FUSED>
+__host__ __device__ constexpr int xrow_table_size() {
+  constexpr int M = N / 2, A = xrow_A(N, INV), B = xrow_B(N, INV), C = xrow_C(N, INV);
+  return !xrow_table(N, FUSED) ? 1 : (B == 1 ? (A - 1) * (M / A) : (B - 1) * A + (C - 1) * xrow_table_j(N, INV));
+}
+// Filled by the CTA, which synchronises.  Two passes: w_M^(b c) at (c - 1) M / A + b; three:
+// w_M^(r k M / (A B)) at (r - 1) A + k, then w_M^(r j) at (r - 1) J + j, j < J = xrow_table_j.
+template <int N, bool INV, bool FUSED, int NT>
+__device__ __forceinline__ void xrow_table_fill(float2* wt, const float2* __restrict__ tw) {
+  constexpr int M = N / 2, A = xrow_A(N, INV), B = xrow_B(N, INV), C = xrow_C(N, INV);
+  constexpr int J = xrow_table_j(N, INV);
+  if (!xrow_table(N, FUSED)) return;
+  for (int e = threadIdx.x; e < xrow_table_size<N, INV, FUSED>(); e += NT) {
+    int m;
+    if (B == 1) m = (e / (M / A) + 1) * (e % (M / A));
+    else if (e < (B - 1) * A) m = (e / A + 1) * (e % A) * (M / (A * B));
+    else m = ((e - (B - 1) * A) / J + 1) * ((e - (B - 1) * A) % J);
+    float2 w = __ldg(&tw[m % M * 2]);
+    if (INV) w.y = -w.y;
+    wt[e] = w;
+  }
+}
+
+template <int N, bool INV, bool FUSED>
 __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xrow_A(N, INV)],
-                                               float2 (&o)[xrow_NB2<N, INV>][xrow_C(N, INV)], float2* rb, int t, const float2* __restrict__ tw) {
+                                               float2 (&o)[xrow_NB2<N, INV>][xrow_C(N, INV)], float2* rb, int t,
+                                               const float2* __restrict__ tw, const float2* wt) {
   constexpr int M = N / 2, A = xrow_A(N, INV), B = xrow_B(N, INV), C = xrow_C(N, INV), T = xrow_T(N, INV);
   constexpr int NB1 = xrow_NB1<N, INV>, NB2 = xrow_NB2<N, INV>;
-  auto twiddle = [&](int m) {
+  // w_M^m, at place e of the table (if it is there)
+  auto twiddle = [&](int m, int e, bool in = true) {
+    if (xrow_table(N, FUSED) && in) return wt[e];
     float2 w = __ldg(&tw[m * 2]);
     if (INV) w.y = -w.y;
     return w;
@@ -563,7 +601,7 @@ __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xro
       const int b = t + T * i;
       DFT<A, INV>::run(v[i]);
 #pragma unroll
-      for (int c = 1; c < A; ++c) v[i][c] = cmul(v[i][c], twiddle((b * c) % M));
+      for (int c = 1; c < A; ++c) v[i][c] = cmul(v[i][c], twiddle((b * c) % M, (c - 1) * (M / A) + b));
     }
     __syncwarp();
 #pragma unroll
@@ -578,7 +616,7 @@ __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xro
       DFT<C, INV>::run(o[i]);
     }
   } else {
-    constexpr int NB = M / B / T;  // B-point DFTs of a lane
+    constexpr int NB = M / B / T, J = xrow_table_j(N, INV);  // NB: B-point DFTs of a lane
     static_assert(M / B % T == 0, "row plan");
     auto at = [](int e) { return e + e / A; };
     __syncwarp();
@@ -596,7 +634,7 @@ __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xro
 #pragma unroll
       for (int r = 0; r < B; ++r) u[i][r] = rb[at(j + r * (M / B))];
 #pragma unroll
-      for (int r = 1; r < B; ++r) u[i][r] = cmul(u[i][r], twiddle(r * k * (M / (A * B))));
+      for (int r = 1; r < B; ++r) u[i][r] = cmul(u[i][r], twiddle(r * k * (M / (A * B)), (r - 1) * A + k));
       DFT<B, INV>::run(u[i]);
     }
     __syncwarp();
@@ -613,7 +651,7 @@ __device__ __forceinline__ void xrow_transform(float2 (&v)[xrow_NB1<N, INV>][xro
 #pragma unroll
       for (int r = 0; r < C; ++r) o[i][r] = rb[at(j + r * (M / C))];
 #pragma unroll
-      for (int r = 1; r < C; ++r) o[i][r] = cmul(o[i][r], twiddle(r * j));
+      for (int r = 1; r < C; ++r) o[i][r] = cmul(o[i][r], twiddle(r * j, (B - 1) * A + (r - 1) * J + j, T * i < J));
       DFT<C, INV>::run(o[i]);
     }
   }
@@ -697,6 +735,11 @@ __global__ void __launch_bounds__(xrow_nt(N, C2R)) k_x_row(const Sim* __restrict
   constexpr int NB1 = xrow_NB1<N, C2R>, NB2 = xrow_NB2<N, C2R>;
   static_assert(A * B * C == M && NB1 * A * T == M && NB2 * C * T == M, "row plan");
   __shared__ float2 sbuf[XR_NT / 32][RPW][RB];
+  __shared__ float2 wt[xrow_table_size<N, C2R, false>()];
+  if (xrow_table(N, false)) {
+    xrow_table_fill<N, C2R, false, XR_NT>(wt, sims[locate_sim(w, 0)].tw);
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane / T, t = lane % T;
   float2* rb = sbuf[wid][sub];
@@ -716,11 +759,11 @@ __global__ void __launch_bounds__(xrow_nt(N, C2R)) k_x_row(const Sim* __restrict
         for (int i = 0; i < NB1; ++i)
 #pragma unroll
           for (int a = 0; a < A; ++a) v[i][a] = __ldg(&src[M / A * a + t + T * i]);
-        xrow_transform<N, false>(v, o, rb, t, tw);
+        xrow_transform<N, false, false>(v, o, rb, t, tw, wt);
         xrow_untangle_store<N>(o, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch, true);
       } else {
         xrow_load_tangle<N>(v, t, tw, S.spec + spec_row(N, (int)(row % N), (int)(row / N)) * S.pitch);
-        xrow_transform<N, true>(v, o, rb, t, tw);
+        xrow_transform<N, true, false>(v, o, rb, t, tw, wt);
         float2* __restrict__ dst = reinterpret_cast<float2*>(S.phi) + row * M;
 #pragma unroll
         for (int i = 0; i < NB2; ++i)
@@ -777,9 +820,9 @@ __host__ __device__ constexpr int dep_tiles(int n) {
 }
 // CTAs per SM, which bounds the registers of a thread: four (64) where the row plan leaves few
 // spills (512: 423 us, three 466; 256 in an ensemble 234, three 262; 64 and 96 lose 10%), else three
-// (192: 134, two 144; 768: 1589, two 1717); five spill (512: 495).  With one-word sums alone in the
-// kernel the 512 grid then takes 402 us early and clustered, the 1024 grid 3.61 ms (start of this
-// layout: 442, 445 and 6.12, with a low and a coarse word for every cell at three CTAs).
+// (192: 134, two 144; 768: 1589, two 1717); five spill (512: 495; all before the row ends and
+// twiddles below).  The 512 grid now takes 356 us, the 1024 grid 3.16 ms (442 us and 6.12 ms with a low
+// and a coarse word for every cell at three CTAs).
 __host__ __device__ constexpr int dep_ctas_bound(int n) { return n == 128 || n == 256 || n == 512 ? 4 : 3; }
 
 // The tile at place i of the order (`order`, optional, lists the tiles dense-first): its
@@ -804,7 +847,7 @@ __device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restri
 // last; every row is left zero.
 template <int N, int NT, int TPB, bool TWO, class H, class F, class G>
 __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsigned* acc, int stride, const TileSum* s_ts,
-                                              H tile, F between, G after) {
+                                              const float2* wt, H tile, F between, G after) {
   constexpr int NL = TZ * TY, M = N / 2, A = xrow_A(N, false), C = xrow_C(N, false), T = xrow_T(N, false), RPW = 32 / T;
   constexpr int NB1 = xrow_NB1<N, false>, NB2 = xrow_NB2<N, false>;
   constexpr int BROWS = NT / 32 * RPW, NBATCH = (TPB * NL + BROWS - 1) / BROWS;
@@ -838,7 +881,7 @@ __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsi
         }
       }
     if (warp == 0 && batch == 0) between();
-    xrow_transform<N, false>(v2, o2, rb, t, S.tw);
+    xrow_transform<N, false, true>(v2, o2, rb, t, S.tw, wt);
     xrow_untangle_store<N>(o2, t, S.tw, S.spec + spec_row(N, y0 + r % TY, z0 + r / TY) * S.pitch, has);
     __syncwarp();  // the row's lanes are done with its words
     uint4* z4 = reinterpret_cast<uint4*>(row);
@@ -863,6 +906,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
   __shared__ unsigned s_off[TPB][8];
   __shared__ TileSum s_ts[2][TPB];  // of the tiles at hand and the next ones, in turn
   __shared__ int s_next;
+  __shared__ float2 wt[xrow_table_size<N, false, true>()];
   unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // warp 0: the run tables of the tiles at places idx .. idx + TPB - 1 (8 lanes per tile)
@@ -903,6 +947,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
   // (0.468 -> 0.460 ms early, 0.604 -> 0.587 ms at step 980, 256^3 on 512^3).
   for (int i = threadIdx.x; i < TPB * NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
   chain_begin();
+  xrow_table_fill<N, false, true, NT>(wt, sims[locate_sim(w, 0)].tw);
   int idx = blockIdx.x * TPB;
   if (warp == 0 && idx < w.total) store_tables(load_tables(idx), idx, s_ts[0]);
   __syncthreads();
@@ -918,7 +963,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
     }
     __syncthreads();
     dep_transform<N, NT, TPB, false>(
-        sims, acc, RS, s_ts[turn],
+        sims, acc, RS, s_ts[turn], wt,
         [&](int tg, int& si, int& y0, int& z0) { return dep_tile<N>(w, order, idx + tg, si, y0, z0) && s_ts[turn][tg].s; },
         take, store);
     __syncthreads();
@@ -944,11 +989,13 @@ __global__ void __launch_bounds__(DEP_DENSE_NT, 1)
   __shared__ unsigned s_begin[8];
   __shared__ unsigned s_off[8];
   __shared__ TileSum s_ts;
+  __shared__ float2 wt[xrow_table_size<N, false, true>()];
   unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   chain_begin();
   const unsigned count = next_tile[1];
   if (blockIdx.x >= count) return;
+  xrow_table_fill<N, false, true, NT>(wt, sims[locate_sim(w, 0)].tw);
   for (int i = threadIdx.x; i < NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
   for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
     int si, y0, z0;
@@ -963,7 +1010,7 @@ __global__ void __launch_bounds__(DEP_DENSE_NT, 1)
                                          s_ts, make_int2(0, TZ), threadIdx.x);
     __syncthreads();
     dep_transform<N, NT, 1, true>(
-        sims, acc, RS, &s_ts, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0; return true; }, []() {},
+        sims, acc, RS, &s_ts, wt, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0; return true; }, []() {},
         []() {});
     __syncthreads();
   }
