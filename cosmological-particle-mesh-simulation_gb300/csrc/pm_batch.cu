@@ -46,6 +46,7 @@ struct SimRec {
   unsigned row_base = 0;
 };
 
+constexpr int TILE_WORDS = 6, TILE_ORDER = 4;  // words of a size in pm_batch::tile_next, place of the scratch
 enum Phase { PH_KEYS = 0, PH_DEP, PH_KICK, PH_FIXED };
 
 // Schedule of the phases of one grid size, chosen by the autotuner (autotune below).  Every
@@ -118,7 +119,7 @@ struct pm_batch {
   int cur = 0;
   SortBufs sort;
   DBuf row_start, d_sims, d_prefix, d_err, d_maps;
-  DBuf tile_next;   // per distinct size: tile counter and two-word count of the fused deposit, 2 words of ordering scratch
+  DBuf tile_next;   // per distinct size, TILE_WORDS: the fused deposit's (pm_common.cuh), 2 words of ordering scratch
   DBuf tile_order;  // per distinct size (at its tile prefix): the fused deposit's tiles, dense first
   DBuf tile_dense;  // the same for its list of two-word tiles
   DBuf d_one;       // descriptor + work table of a one-simulation deposit (pm_batch_density)
@@ -428,7 +429,7 @@ int build_plan(pm_batch* b, cudaStream_t st) {
     for (int t : P.fdep_total) tiles += (size_t)t;
     PB_CK(b->tile_order.ensure_geo(sizeof(unsigned) * tiles), "alloc tile order");
     PB_CK(b->tile_dense.ensure_geo(sizeof(unsigned) * tiles), "alloc tile order");
-    PB_CK(b->tile_next.ensure_geo(4 * sizeof(unsigned) * P.sizes.size()), "alloc tile counters");
+    PB_CK(b->tile_next.ensure_geo(TILE_WORDS * sizeof(unsigned) * P.sizes.size()), "alloc tile counters");
     while (b->side.size() < P.sizes.size()) {
       cudaStream_t s = nullptr;
       cudaEvent_t e = nullptr;
@@ -532,7 +533,7 @@ int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigne
   const int n = P.sizes[g], tot = P.fdep_total[g];
   const Work wg = work_of(b, PH_FIXED + 3 * g + 2, tot);
   // this size's tile counter and ordering scratch, and its part of the tile order
-  unsigned* next = b->tile_next.as<unsigned>() + 4 * g;
+  unsigned* next = b->tile_next.as<unsigned>() + TILE_WORDS * g;
   size_t at = 0;
   for (int i = 0; i < g; ++i) at += P.fdep_total[i];
   unsigned *order = b->tile_order.as<unsigned>() + at, *dense = b->tile_dense.as<unsigned>() + at;
@@ -543,7 +544,7 @@ int enqueue_deposit(pm_batch* b, int g, const Shape& sh, Parts in, const unsigne
     return PM_OK;
   }
   if (sh.dep == DEP_FUSED_DENSE_FIRST)
-    PB_CK(launch_tile_order(ds, wg, b->row_start.as<unsigned>(), order, next + 2, b->sms, st), "tile order");
+    PB_CK(launch_tile_order(ds, wg, b->row_start.as<unsigned>(), order, next + TILE_ORDER, b->sms, st), "tile order");
   PB_CK(deposit_r2c_dispatch(n, ds, wg, in, perm, b->row_start.as<unsigned>(), b->group_max.as<unsigned>(), err, next,
                              sh.dep == DEP_FUSED_DENSE_FIRST ? order : nullptr, dense,
                              grid_for(tot, b->sms, sh.dep_cps ? sh.dep_cps : deposit_r2c_ctas_per_sm(n)), st),
@@ -567,7 +568,7 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
   PB_CK(row_counting_sort(b->sort.keys.as<unsigned>(), P.sort_n, P.rows, b->row_count.as<unsigned>(),
                           b->row_start.as<unsigned>(), b->row_cursor.as<unsigned>(), b->scan_sums.as<unsigned>(),
                           perm, err, b->sms, Launch(st, chained(P)), true, true, b->group_max.as<unsigned>(),
-                          b->tile_next.as<unsigned>(), 4 * (int)P.sizes.size(), b->d_sims.as<Sim>(), P.nsims),
+                          b->tile_next.as<unsigned>(), TILE_WORDS * (int)P.sizes.size(), b->d_sims.as<Sim>(), P.nsims),
         "sort");
   PB_CK(mark(1 + PP_SORT), "event");
   PB_CK(mark(1 + PP_ROWS), "event");  // the row starts come out of the counting sort
@@ -717,7 +718,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
       for (const Shape& c : cands) {
         float ms = 0.f;
         rc = time3([&]() -> int {
-          PB_CK(cudaMemsetAsync(b->tile_next.p, 0, 4 * sizeof(unsigned) * P.sizes.size(), st), "clear");
+          PB_CK(cudaMemsetAsync(b->tile_next.p, 0, TILE_WORDS * sizeof(unsigned) * P.sizes.size(), st), "clear");
           if (int r = enqueue_deposit(b, (int)g, c, in, perm, st)) return r;
           if (c.dep == DEP_SEPARATE)
             PB_CK(spectral_dispatch(SPEC_X_R2C, n, ds, wx, grid_for(wx.total, b->sms, c.x_cps), st,
@@ -914,7 +915,7 @@ int pm_batch_create(int device, size_t mem_cap_bytes, pm_batch** out) {
   cudaError_t e = cudaSetDevice(device);
   if (!e) b->sms = sm_count(device);
   if (!e) e = b->d_err.ensure(sizeof(int));
-  if (!e) e = b->tile_next.ensure(4 * sizeof(unsigned));
+  if (!e) e = b->tile_next.ensure(TILE_WORDS * sizeof(unsigned));
   if (!e) e = cudaMemset(b->d_err.p, 0, sizeof(int));
   if (!e) e = cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking);
   if (!e) e = cudaStreamCreateWithFlags(&b->admit, cudaStreamNonBlocking);

@@ -46,9 +46,10 @@ __device__ __forceinline__ float fixed_to_float(unsigned l, unsigned c, float sc
 // adjacent ones: at most 4 or 8 times the largest count of a row bin of the tile and its three
 // lower neighbours, and at most the tile's source entries.  With that bound below 2^(32 - s) a
 // 32-bit word per cell holds the sum (one atomic per corner).  Tiles whose bound allows
-// s >= ONE_WORD_MIN use one word at the largest such s (at most 26; 23 to 24 for the 512 grid
-// of the README run, where the tile's source entries alone allowed 21); denser tiles sum at
-// 2^-26 in a low word plus a coarse word (two atomics per corner).
+// s >= ONE_WORD_MIN use one word at the largest such s (at most 26; 23 to 24 for 256^3 particles
+// on 512^3 early, where the tile's source entries alone allowed 21).  Where it does not, the counts
+// themselves are read (tight_sum): the largest sum of a row's four source rows over two
+// adjacent bins.  The tiles left sum at 2^-26 in a low word plus a coarse word (two atomics per corner).
 constexpr int ONE_WORD_MIN = 20;
 
 struct TileSum {
@@ -56,11 +57,9 @@ struct TileSum {
   float ms;  // particle mass * 2^-(quantisation bits): the float of a sum times ms is its mass
 };
 
-// total: the tile's source entries; bin_max: the largest row bin count of the tile and its
-// lower neighbours (per_row bins to a row)
-__device__ __forceinline__ TileSum tile_sum(unsigned total, unsigned bin_max, int per_row, float mass_scale) {
-  const unsigned cap = bin_max < (1u << 28) ? bin_max * (per_row > 1 ? 8u : 4u) : 0xffffffffu;
-  const int bits = 32 - __clz(min(total, cap));  // entries of a cell < 2^bits
+// cap: a cell receives at most that many corners
+__device__ __forceinline__ TileSum tile_sum(unsigned cap, float mass_scale) {
+  const int bits = 32 - __clz(cap);  // entries of a cell < 2^bits
   const int s = min(PM_FIX_BITS, 32 - bits);
   TileSum t;
   t.s = s >= ONE_WORD_MIN ? s : 0;
@@ -250,6 +249,21 @@ __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __rest
   return v;
 }
 
+// The runs of plane z0 + p of the tile alone: the rows of the plane and of the one below it, and
+// the row before each.
+__device__ __forceinline__ RunLoad plane_load(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0, int p,
+                                              int lane) {
+  RunLoad v;
+  if (lane >= 4) return v;
+  const int n = S.n, ym = y0 == 0 ? n - 1 : y0 - 1, zp = z0 + p, zm = zp == 0 ? n - 1 : zp - 1;
+  const unsigned per_row = S.xbits ? 1u : (unsigned)x_bins(n);
+  const unsigned r0 = row_number(lane < 2 ? y0 : ym, lane & 1 ? zm : zp, n), nr = lane < 2 ? TY : 1u;
+  const unsigned* s = row_start + (S.row_base + r0 * per_row);
+  v.beg = __ldg(s);
+  v.cnt = __ldg(s + nr * per_row) - v.beg;
+  return v;
+}
+
 // Warp-wide (all 32 lanes call it): the run table (first sorted index, and the inclusive scan
 // of the counts) of the tile whose runs the 8 lanes of this lane's group of eight loaded
 // (lane & 7 = the run).  The lanes with `write` store their group's table at s_begin / s_off
@@ -272,7 +286,32 @@ __device__ __forceinline__ TileSum run_table(const RunLoad& v, int lane, unsigne
     }
     if (r == 0) s_off[0] = 0;
   }
-  return tile_sum(total, m, v.per_row, v.mass_scale);
+  const unsigned cap = m < (1u << 28) ? m * (v.per_row > 1 ? 8u : 4u) : 0xffffffffu;
+  return tile_sum(min(total, cap), v.mass_scale);
+}
+
+// Warp-wide, for a tile whose maxima do not allow one word: from the counts of its row bins.  A cell
+// of row (y, z) and bin b receives corners from rows (y, z), (y - 1, z), (y, z - 1), (y - 1, z - 1)
+// and bins b and b - 1.  total: the tile's source entries.  (Few tiles come here: of 256^3
+// particles on 512^3 the halos' at late times.)
+__device__ __forceinline__ TileSum tight_sum(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0,
+                                             unsigned total, int lane) {
+  const int n = S.n, bins = S.xbits ? 1 : x_bins(n);
+  const int y = y0 + lane % TY, z = z0 + lane / TY % TZ;  // two lanes to a row, each with every other bin
+  unsigned cap = 0;
+  for (int b = lane / (TY * TZ); b < bins; b += 32 / (TY * TZ)) {
+    unsigned sum = 0;
+    for (int k = 0; k < 4; ++k) {
+      const int ys = k & 1 ? (y == 0 ? n - 1 : y - 1) : y, zs = k & 2 ? (z == 0 ? n - 1 : z - 1) : z;
+      const unsigned* c = row_start + (S.row_base + row_number(ys, zs, n) * (unsigned)bins);
+      const int prev = b == 0 ? bins - 1 : b - 1;
+      sum += __ldg(c + b + 1) - __ldg(c + b);
+      if (bins > 1) sum += __ldg(c + prev + 1) - __ldg(c + prev);
+    }
+    cap = max(cap, sum);
+  }
+  cap = __reduce_max_sync(FULL, cap);
+  return tile_sum(min(total, cap), S.mass_scale);
 }
 
 // The particle loop of a tile: two source entries per lane and iteration, so that their

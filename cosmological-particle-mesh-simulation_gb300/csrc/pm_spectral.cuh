@@ -840,27 +840,29 @@ __device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restri
   return true;
 }
 
-// The x R2C of tile rows: row r's sums at acc + r * stride (TWO: its coarse words HO words further
+// The x R2C of the NL rows of each tile (or plane of one): row r's sums at acc + r * stride (TWO: its coarse words HO words further
 // on); T lanes to a row, whose exchange buffer overlays its low words once they are read.  A
 // batch is the rows that the CTA's warps hold at once.  f(tg): whether to store tile tg's rows and
 // where they belong; `between` runs in warp 0 before the first transform, `after` behind the
 // last; every row is left zero.
-template <int N, int NT, int TPB, bool TWO, class H, class F, class G>
+template <int N, int NT, int TPB, int NL, bool TWO, class H, class F, class G>
 __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsigned* acc, int stride, const TileSum* s_ts,
                                               const float2* wt, H tile, F between, G after) {
-  constexpr int NL = TZ * TY, M = N / 2, A = xrow_A(N, false), C = xrow_C(N, false), T = xrow_T(N, false), RPW = 32 / T;
+  constexpr int M = N / 2, A = xrow_A(N, false), C = xrow_C(N, false), T = xrow_T(N, false), RPW = 32 / T;
   constexpr int NB1 = xrow_NB1<N, false>, NB2 = xrow_NB2<N, false>;
   constexpr int BROWS = NT / 32 * RPW, NBATCH = (TPB * NL + BROWS - 1) / BROWS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / T, t = lane % T;
 #pragma unroll 1
   for (int batch = 0; batch < NBATCH; ++batch) {
-    if (batch * BROWS + warp * RPW >= TPB * NL) break;  // warp-uniform (a warp's rows are all in or all out)
-    const int R = batch * BROWS + warp * RPW + sub, tg = R / NL, r = R % NL;
+    if (batch * BROWS + warp * RPW >= TPB * NL) break;  // warp-uniform
+    // (where a warp holds more rows than there are, its other lanes repeat the last one)
+    const int R0 = batch * BROWS + warp * RPW + sub, R = TPB * NL % RPW == 0 || R0 < TPB * NL ? R0 : TPB * NL - 1;
+    const int tg = R / NL, r = R % NL;
     unsigned* row = acc + R * stride;
     float2* rb = reinterpret_cast<float2*>(row);
     int si, y0, z0;
-    const bool has = tile(tg, si, y0, z0);
+    const bool has = tile(tg, si, y0, z0) && R == R0;
     const Sim& S = sims[si];
     const TileSum ts = s_ts[tg];
     float2 v2[NB1][A];
@@ -921,7 +923,15 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
   // the list of k_deposit_r2c_dense and is left out here
   auto store_tables = [&](const RunLoad& v, int idx, TileSum* ts) {
     const int tj = lane < TPB * 8 ? lane >> 3 : 0;
-    const TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
+    TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
+    for (unsigned m = __ballot_sync(FULL, lane < TPB * 8 && (lane & 7) == 0 && !t.s); m; m &= m - 1) {
+      const int j = (__ffs(m) - 1) >> 3;
+      int si, y0, z0;
+      dep_tile<N>(w, order, idx + j, si, y0, z0);
+      __syncwarp();
+      const TileSum u = tight_sum(sims[si], row_start, y0, z0, s_off[j][NRUN], lane);
+      if (lane >> 3 == j) t = u;
+    }
     if (lane < TPB * 8 && (lane & 7) == 0) {
       ts[tj] = t;
       if (t.s == 0) dense[atomicAdd(next_tile + 1, 1u)] = (unsigned)(idx + tj);
@@ -962,7 +972,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
                                              s_off[g], ts, make_int2(0, TZ), gtid);
     }
     __syncthreads();
-    dep_transform<N, NT, TPB, false>(
+    dep_transform<N, NT, TPB, NL, false>(
         sims, acc, RS, s_ts[turn], wt,
         [&](int tg, int& si, int& y0, int& z0) { return dep_tile<N>(w, order, idx + tg, si, y0, z0) && s_ts[turn][tg].s; },
         take, store);
@@ -971,48 +981,71 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
   }
 }
 
-// The tiles that k_deposit_r2c left: those with two-word sums, one to a CTA of 1024 threads (such
-// tiles hold thousands of particles).  A kernel of its own: next to the one-word path its
-// registers and code cost that path 10% (442 -> 498 us on the 512 grid).
-constexpr int DEP_DENSE_NT = 1024;
+// The tiles that k_deposit_r2c left: those with two-word sums, one plane at a time, taken from a
+// counter.  A kernel of its own: next to the one-word path its registers and code cost that path 10%
+// (442 -> 498 us on the 512 grid).  By planes: the heart of a large halo is one tile, whose atomics
+// on a few cells alone would otherwise outlast the rest of the kernel.  256^3 particles on 512^3 at
+// steps 400 / 600 / 980 of 1000, in us: whole tiles on 1024 threads in a fixed stride 292 / 414 / 560,
+// taken from a counter, 2 CTAs of 512 threads, 233 / 296 / 416, without those that tight_sum finds
+// 181 / 228 / 361, planes 107 / 164 / 249 (256 threads, 4 CTAs: 117 / 181 / 280; rows 146 / 209 / 312).
+constexpr int DEP_DENSE_NT = 512;
 __host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, coarse words
+__host__ __device__ constexpr size_t dep_dense_bytes(int n) { return (size_t)TY * dep_dense_stride(n) * sizeof(unsigned); }
+constexpr int DEP_DENSE_CTAS = 2;
 
 template <int N>
-__global__ void __launch_bounds__(DEP_DENSE_NT, 1)
+__global__ void __launch_bounds__(DEP_DENSE_NT, DEP_DENSE_CTAS)
     k_deposit_r2c_dense(const Sim* __restrict__ sims, Work w, Parts p, const unsigned* __restrict__ perm,
-                        const unsigned* __restrict__ row_start, const unsigned* __restrict__ group_max, int* err,
-                        const unsigned* __restrict__ next_tile, const unsigned* __restrict__ order,
-                        const unsigned* __restrict__ dense) {
-  constexpr int NT = DEP_DENSE_NT, NL = TZ * TY, RS = dep_dense_stride(N);
+                        const unsigned* __restrict__ row_start, int* err, unsigned* __restrict__ next_tile,
+                        const unsigned* __restrict__ order, const unsigned* __restrict__ dense) {
+  constexpr int NT = DEP_DENSE_NT, RS = dep_dense_stride(N);
   static_assert(RS % 4 == 0, "rows zeroed 4 words at a time");
   extern __shared__ uint4 acc_raw[];
   __shared__ unsigned s_begin[8];
   __shared__ unsigned s_off[8];
-  __shared__ TileSum s_ts;
+  __shared__ unsigned s_next;
   __shared__ float2 wt[xrow_table_size<N, false, true>()];
   unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   chain_begin();
-  const unsigned count = next_tile[1];
+  const unsigned count = next_tile[1] * TZ;
   if (blockIdx.x >= count) return;
+  for (int i = threadIdx.x; i < TY * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
   xrow_table_fill<N, false, true, NT>(wt, sims[locate_sim(w, 0)].tw);
-  for (int i = threadIdx.x; i < NL * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (unsigned i = blockIdx.x; i < count; i += gridDim.x) {
+  // warp 0 takes the next plane and loads its run table before the transform and stores it after
+  unsigned i = blockIdx.x, next = 0;
+  RunLoad nl;
+  auto load = [&](unsigned unit) {
     int si, y0, z0;
-    dep_tile<N>(w, order, (int)dense[i], si, y0, z0);
-    if (warp == 0) {
-      const TileSum t = run_table(run_load(sims[si], row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off,
-                                  lane < 8);
-      if (lane == 0) s_ts = t;
-    }
+    dep_tile<N>(w, order, (int)dense[unit / TZ], si, y0, z0);
+    nl = plane_load(sims[si], row_start, y0, z0, (int)(unit % TZ), lane & 7);
+  };
+  auto take = [&]() {
+    next = __shfl_sync(FULL, lane == 0 ? gridDim.x + atomicAdd(next_tile + 2, 1u) : 0u, 0);
+    if (next < count) load(next);
+  };
+  auto store = [&]() {
+    if (next < count) run_table(nl, lane, s_begin, s_off, lane < 8);
+    if (lane == 0) s_next = next;
+  };
+  if (warp == 0) {
+    load(i);
+    run_table(nl, lane, s_begin, s_off, lane < 8);
+  }
+  __syncthreads();
+  while (i < count) {
+    int si, y0, z0;
+    dep_tile<N>(w, order, (int)dense[i / TZ], si, y0, z0);
+    const int zp = (int)(i % TZ);
+    const TileSum ts{0, sims[si].mass_scale};
+    deposit_tile<POS_DISP, NT, false, N>(sims[si], p, perm, err, y0, z0, acc, acc + dep_row_words(N), RS, s_begin, s_off, ts,
+                                         make_int2(zp, zp + 1), threadIdx.x);
     __syncthreads();
-    deposit_tile<POS_DISP, NT, false, N>(sims[si], p, perm, err, y0, z0, acc, acc + dep_row_words(N), RS, s_begin, s_off,
-                                         s_ts, make_int2(0, TZ), threadIdx.x);
+    dep_transform<N, NT, 1, TY, true>(
+        sims, acc, RS, &ts, wt, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0 + zp; return true; }, take,
+        store);
     __syncthreads();
-    dep_transform<N, NT, 1, true>(
-        sims, acc, RS, &s_ts, wt, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0; return true; }, []() {},
-        []() {});
-    __syncthreads();
+    i = s_next;
   }
 }
 
@@ -1025,7 +1058,7 @@ cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned*
   } else {
     static DeviceOnce once;
     const size_t sm = dep_tiles(N) * dep_tile_bytes(N);
-    const size_t smd = (size_t)TZ * TY * dep_dense_stride(N) * sizeof(unsigned);
+    const size_t smd = dep_dense_bytes(N);
     const cudaError_t ie = once.run([&]() {
       cudaError_t e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (!e) e = cudaFuncSetAttribute(k_deposit_r2c<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -1042,8 +1075,8 @@ cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned*
     launch_chained(k_deposit_r2c<N>, ctas, NT, sm, st, sims, w, p, perm, row_start, group_max, err, next_tile, order,
                    dense);
     if (cudaError_t e = cudaGetLastError()) return e;
-    const int few = w.total < device_sms() ? w.total : device_sms();
-    launch_chained(k_deposit_r2c_dense<N>, few, DEP_DENSE_NT, smd, st, sims, w, p, perm, row_start, group_max, err, next_tile,
+    const int cap = device_sms() * DEP_DENSE_CTAS, few = w.total < cap / TZ ? w.total * TZ : cap;
+    launch_chained(k_deposit_r2c_dense<N>, few, DEP_DENSE_NT, smd, st, sims, w, p, perm, row_start, err, next_tile,
                    order, dense);
     return cudaGetLastError();
   }
