@@ -215,7 +215,6 @@ bool spectral_supported(int n);
 // work units (CTAs' worth of work) of one spectral pass for a grid of size n
 long long spectral_units(SpecKind kind, int n);
 // resident CTAs per SM of a spectral pass for size n (for persistent grid sizing)
-int spectral_ctas_per_sm(SpecKind kind, int n);
 cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, Launch st,
                               const CUtensorMap* maps = nullptr, int* err = nullptr);
 cudaError_t launch_fourier_grid(const Sim* sims, int ctas, Launch st);

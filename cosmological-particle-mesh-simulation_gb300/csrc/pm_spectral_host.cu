@@ -57,13 +57,6 @@ long long spectral_units(SpecKind kind, int n) {
   return (nb + bpc - 1) / bpc;
 }
 
-int spectral_ctas_per_sm(SpecKind kind, int n) {
-  const size_t sm = (kind == SPEC_X_R2C || kind == SPEC_X_C2R) ? x_smem_bytes(n) : line_smem_bytes(n);
-  int by_smem = (int)((228u * 1024u) / (sm + 1024));
-  if (by_smem < 1) by_smem = 1;
-  return by_smem > 4 ? 4 : by_smem;
-}
-
 cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int ctas, Launch st,
                               const CUtensorMap* maps, int* err) {
   switch (n) {

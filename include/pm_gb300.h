@@ -75,7 +75,7 @@ int pm_supported_n(int n);
 
 /* ---- drop-in hot path ----------------------------------------------------------- */
 /* src/density.py:7-48  density(positions, mass) -> grid.
-   Deterministic: cell-key radix sort + tiled integer-accumulated CIC deposit. */
+   Deterministic: particles grouped by grid row + tiled integer-accumulated CIC deposit. */
 int pm_density(pm_ctx* ctx, const float* positions, long long np, double mass, float* rho,
                void* stream);
 
@@ -209,7 +209,8 @@ int pm_batch_set_graphs(pm_batch* b, int enable);
 int pm_batch_check(pm_batch* b, void* stream, int* bits);
 /* Runs up to nsteps steps with direct launches and CUDA events between phases, and
    writes the mean milliseconds of each phase to phase_ms[0..9]: sort, row starts,
-   deposit, x R2C, y forward, z Green, y inverse, x C2R, kick/drift, coefficients. */
+   deposit, x R2C, y forward, z Green, y inverse, x C2R, kick/drift, coefficients (made
+   inside the sort: the last is 0 up to the events). */
 int pm_batch_profile(pm_batch* b, int nsteps, float* phase_ms, int nphase, void* stream);
 /* Kernel launches per step for the resident simulations (-1 on error). */
 int pm_batch_launches_per_step(pm_batch* b);
