@@ -529,8 +529,10 @@ __global__ void k_row_keys_abs(const float* __restrict__ pos, long long np, int 
 // of the lattice (z is the fastest particle index).  For a clustered state the chunks only
 // roughly follow the tiles; every order gives the same result.  256^3 / 512^3 particles: to
 // displacements 1.12 / 14.1 ms (all arrays at once, slot order) -> 0.44 / 9.0, back 2.79 / 28.8 ->
-// 0.82 / 16.1; without the chunks 0.52 / 11.1 and 0.81 / 19.5.  Bound by the rate of 32-byte sectors
-// in L2, one per float (123 G/s at 256^3).
+// 0.82 / 16.1; without the chunks 0.52 / 11.1 and 0.81 / 19.5.  The way back reads its slots
+// evict-first, which leaves L2 to the lines being filled: 0.78 / 14.3 (its stores evict-first as well 24;
+// several slots' loads issued together 0.79 / 17; a quarter of the CTAs 0.95 / 20).  Bound by
+// the rate of 32-byte sectors in L2, one per float (123 G/s at 256^3).
 struct ChunkOrder {
   long long np;
   int side;  // tiles per axis
@@ -592,10 +594,10 @@ __global__ void k_disp_to_abs(Parts in, long long off, ChunkOrder chunks, int np
   const unsigned* __restrict__ ids = in.id + off;
   float* __restrict__ dst = (is_vel ? vel : pos) + k * np;
   chunks.each([&](long long j) {
-    const unsigned pid = __ldg(&ids[j]);
+    const unsigned pid = __ldcs(&ids[j]);
     const unsigned ax[3] = {pid >> 20, (pid >> 10) & 1023u, pid & 1023u};
     const long long id = ((long long)ax[0] * np1 + ax[1]) * np1 + ax[2];
-    float v = __ldg(&src[j]);
+    float v = __ldcs(&src[j]);
     if (!is_vel) {
       const unsigned l = k == 0 ? ax[0] : (k == 1 ? ax[1] : ax[2]);
       const float s = __ldg(&q_frac[l]) + v;
