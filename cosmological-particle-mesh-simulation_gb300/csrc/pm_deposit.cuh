@@ -41,28 +41,28 @@ __device__ __forceinline__ float fixed_to_float(unsigned l, unsigned c, float sc
 
 // How a tile's sums are held.  Every corner weight is quantised to an integer q <= 2^s and
 // added with integer atomics, so a cell's sum -- and the float made from it -- does not depend
-// on the order of the additions.  A cell receives at most one corner from each particle in four
-// rows (y, y - 1, z, z - 1) and two cells of each (x, x - 1), which lie in one row bin or two
-// adjacent ones: at most 4 or 8 times the largest count of a row bin of the tile and its three
-// lower neighbours, and at most the tile's source entries.  With that bound below 2^(32 - s) a
-// 32-bit word per cell holds the sum (one atomic per corner).  Tiles whose bound allows
-// s >= ONE_WORD_MIN use one word at the largest such s (at most 26; 23 to 24 for 256^3 particles
-// on 512^3 early, where the tile's source entries alone allowed 21).  Where it does not, the counts
-// themselves are read (tight_sum): the largest sum of a row's four source rows over two
-// adjacent bins.  The tiles left sum at 2^-26 in a low word plus a coarse word (two atomics per corner).
-constexpr int ONE_WORD_MIN = 20;
+// on the order of the additions.  A tile of up to ONE_WORD_TOTAL - 1 source entries sums in one 32-bit
+// word per cell (one atomic per corner), at the largest s <= 26 that cannot overflow.  A cell
+// receives at most one corner from each particle in four rows (y, y - 1, z, z - 1) and two cells of
+// each (x, x - 1), which lie in one row bin or two adjacent ones: at most 4 or 8 times the largest count of a
+// row bin of the tile and its three lower neighbours, and at most the tile's source entries, which
+// alone would allow s = 20 to 26 (256^3 on 512^3 early: 21; with the bins 23 to 24).
+// Denser tiles sum at 2^-26 in a low word plus a coarse word (two atomics per corner): bounds from the
+// bins would put most of them in one word too, but at s = 20 to 22, and the quantisation would
+// then be the largest error of their density -- one particle per cell of 256^3, uniform:
+// 3.4e-7 in relative L2 instead of 3.2e-8.
+constexpr unsigned ONE_WORD_TOTAL = 4096;
 
 struct TileSum {
   int s;     // one-word quantisation 2^s; 0: two-word sums at 2^-26
   float ms;  // particle mass * 2^-(quantisation bits): the float of a sum times ms is its mass
 };
 
-// cap: a cell receives at most that many corners
-__device__ __forceinline__ TileSum tile_sum(unsigned cap, float mass_scale) {
-  const int bits = 32 - __clz(cap);  // entries of a cell < 2^bits
-  const int s = min(PM_FIX_BITS, 32 - bits);
+// total: source entries of the tile; cap: a cell receives at most that many corners
+__device__ __forceinline__ TileSum tile_sum(unsigned total, unsigned cap, float mass_scale) {
+  const int bits = 32 - __clz(min(total, cap));  // entries of a cell < 2^bits
   TileSum t;
-  t.s = s >= ONE_WORD_MIN ? s : 0;
+  t.s = total < ONE_WORD_TOTAL ? min(PM_FIX_BITS, 32 - bits) : 0;
   // mass_scale = mass * 2^-26; one-word sums at 2^-s: times 2^(26 - s), exactly
   t.ms = t.s ? mass_scale * __uint_as_float((unsigned)(127 + PM_FIX_BITS - t.s) << 23) : mass_scale;
   return t;
@@ -287,31 +287,7 @@ __device__ __forceinline__ TileSum run_table(const RunLoad& v, int lane, unsigne
     if (r == 0) s_off[0] = 0;
   }
   const unsigned cap = m < (1u << 28) ? m * (v.per_row > 1 ? 8u : 4u) : 0xffffffffu;
-  return tile_sum(min(total, cap), v.mass_scale);
-}
-
-// Warp-wide, for a tile whose maxima do not allow one word: from the counts of its row bins.  A cell
-// of row (y, z) and bin b receives corners from rows (y, z), (y - 1, z), (y, z - 1), (y - 1, z - 1)
-// and bins b and b - 1.  total: the tile's source entries.  (Few tiles come here: of 256^3
-// particles on 512^3 the halos' at late times.)
-__device__ __forceinline__ TileSum tight_sum(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0,
-                                             unsigned total, int lane) {
-  const int n = S.n, bins = S.xbits ? 1 : x_bins(n);
-  const int y = y0 + lane % TY, z = z0 + lane / TY % TZ;  // two lanes to a row, each with every other bin
-  unsigned cap = 0;
-  for (int b = lane / (TY * TZ); b < bins; b += 32 / (TY * TZ)) {
-    unsigned sum = 0;
-    for (int k = 0; k < 4; ++k) {
-      const int ys = k & 1 ? (y == 0 ? n - 1 : y - 1) : y, zs = k & 2 ? (z == 0 ? n - 1 : z - 1) : z;
-      const unsigned* c = row_start + (S.row_base + row_number(ys, zs, n) * (unsigned)bins);
-      const int prev = b == 0 ? bins - 1 : b - 1;
-      sum += __ldg(c + b + 1) - __ldg(c + b);
-      if (bins > 1) sum += __ldg(c + prev + 1) - __ldg(c + prev);
-    }
-    cap = max(cap, sum);
-  }
-  cap = __reduce_max_sync(FULL, cap);
-  return tile_sum(min(total, cap), S.mass_scale);
+  return tile_sum(total, cap, v.mass_scale);
 }
 
 // The particle loop of a tile: two source entries per lane and iteration, so that their

@@ -923,15 +923,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
   // the list of k_deposit_r2c_dense and is left out here
   auto store_tables = [&](const RunLoad& v, int idx, TileSum* ts) {
     const int tj = lane < TPB * 8 ? lane >> 3 : 0;
-    TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
-    for (unsigned m = __ballot_sync(FULL, lane < TPB * 8 && (lane & 7) == 0 && !t.s); m; m &= m - 1) {
-      const int j = (__ffs(m) - 1) >> 3;
-      int si, y0, z0;
-      dep_tile<N>(w, order, idx + j, si, y0, z0);
-      __syncwarp();
-      const TileSum u = tight_sum(sims[si], row_start, y0, z0, s_off[j][NRUN], lane);
-      if (lane >> 3 == j) t = u;
-    }
+    const TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
     if (lane < TPB * 8 && (lane & 7) == 0) {
       ts[tj] = t;
       if (t.s == 0) dense[atomicAdd(next_tile + 1, 1u)] = (unsigned)(idx + tj);
@@ -984,10 +976,9 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
 // The tiles that k_deposit_r2c left: those with two-word sums, one plane at a time, taken from a
 // counter.  A kernel of its own: next to the one-word path its registers and code cost that path 10%
 // (442 -> 498 us on the 512 grid).  By planes: the heart of a large halo is one tile, whose atomics
-// on a few cells alone would otherwise outlast the rest of the kernel.  256^3 particles on 512^3 at
-// steps 400 / 600 / 980 of 1000, in us: whole tiles on 1024 threads in a fixed stride 292 / 414 / 560,
-// taken from a counter, 2 CTAs of 512 threads, 233 / 296 / 416, without those that tight_sum finds
-// 181 / 228 / 361, planes 107 / 164 / 249 (256 threads, 4 CTAs: 117 / 181 / 280; rows 146 / 209 / 312).
+// on a few cells alone would otherwise outlast the rest of the kernel (256^3 particles on 512^3 at step
+// 980 of 1000, half of these tiles: planes 249 us, whole tiles 361, single rows 312, planes on 4 CTAs of
+// 256 threads 280).  All tiles of 4096 and more entries at steps 400 / 600 / 980: 222 / 266 / 338 us.
 constexpr int DEP_DENSE_NT = 512;
 __host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, coarse words
 __host__ __device__ constexpr size_t dep_dense_bytes(int n) { return (size_t)TY * dep_dense_stride(n) * sizeof(unsigned); }
