@@ -30,6 +30,7 @@
 // 128^3: spectra of the displacements 170 -> 18 us, particles 227 -> 44, field 59 -> 19; the whole
 // call 772 -> 282, with 18 launches instead of 30.
 #include "pm_host.cuh"
+#include "pm_pair.cuh"
 
 using namespace pm;
 
@@ -59,22 +60,6 @@ __device__ double lcdm_transfer(double k, double gamma) {
     f2 = (l * l) / (d * d);
   }
   return f2 / f1;
-}
-
-// ---- float32 pairs ---------------------------------------------------------------------
-// hi + lo with |lo| <= ulp(hi) / 2
-__host__ __device__ __forceinline__ float2 split(double v) {
-  const float h = (float)v;
-  return make_float2(h, (float)(v - (double)h));
-}
-__device__ __forceinline__ float2 two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-  return make_float2(s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t)));
-}
-// (c.x + c.y) * v
-__device__ __forceinline__ float2 pair_mul(float2 c, float v) {
-  const float p = __fmul_rn(c.x, v);
-  return make_float2(p, __fmaf_rn(c.x, v, -p) + c.y * v);
 }
 
 // Tables of a call: shape[m2] = S(m2), the summand of the normalisation, which is also P(k) / A
@@ -287,29 +272,6 @@ __device__ __forceinline__ float2 jitter_pair(unsigned long long x) {
   const long long v = (long long)(x >> 11) - (1ll << 52);
   const int hi = (int)(v >> 29), mid = (int)((v >> 5) & 0xffffffll);
   return make_float2((float)hi * (1.f / 4194304.f), (float)mid * (1.f / 70368744177664.f));
-}
-
-// numpy float remainder: fmod, moved into the divisor's sign
-__device__ __forceinline__ double py_mod(double a, double b) {
-  double m = fmod(a, b);
-  if (m != 0.0) {
-    if ((b < 0.0) != (m < 0.0)) m += b;
-  } else {
-    m = copysign(0.0, b);
-  }
-  return m;
-}
-
-// (v.x + v.y) mod n, rounded to float32
-__device__ __forceinline__ float pair_mod(float2 v, float n) {
-  const float hi = v.x, lo = v.y;
-  if (!(hi >= -n && hi < 2.f * n)) return (float)py_mod((double)hi + (double)lo, (double)n);  // (and NaN)
-  if (hi > n || (hi == n && lo >= 0.f)) return __fadd_rn(__fsub_rn(hi, n), lo);  // hi - n is exact
-  if (hi < 0.f || (hi == 0.f && lo < 0.f)) {
-    const float2 t = two_sum(hi, n);
-    return __fadd_rn(t.x, __fadd_rn(t.y, lo));
-  }
-  return __fadd_rn(hi, lo);
 }
 
 struct PartArgs {
