@@ -209,9 +209,12 @@ size_t footprint(const pm_config& c) {
   size_t f = n * n * n * sizeof(float);                          // potential / density
   if (c.flags & PM_FLAG_KEEP_DENSITY) f += n * n * n * sizeof(float);
   f += n * n * (size_t)spec_pitch((int)n) * sizeof(float2);      // spectrum
-  f += np * (2 * kStateBytes + 4 * 4);                           // state x2, keys/vals x2
+  f += np * (2 * kStateBytes + 2 * 4);                           // state x2, keys and order of the sort
   f += np * 6 * sizeof(float);                                   // final state
-  f += 3 * n * n * sizeof(unsigned) + 4096;                      // row starts, counts, cursors, tables
+  const size_t bins = row_bins((int)n);
+  f += (3 * bins + bins / 16) * sizeof(unsigned);                // bin starts, counts, cursors; largest of 16
+  f += 2 * (n / TILE_Y) * (n / TILE_Z) * sizeof(unsigned);       // tile order, two-word tiles
+  f += 4096;                                                     // descriptor, tables
   return f;
 }
 
