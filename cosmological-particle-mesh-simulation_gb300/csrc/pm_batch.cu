@@ -633,8 +633,8 @@ int enqueue_step(pm_batch* b, int cur, cudaStream_t st, cudaEvent_t* ev = nullpt
 // Kernel launches of one step for the current plan.
 int launches_per_step(pm_batch* b) {
   const Plan& P = b->plan;
-  // counting sort: 2 scan kernels and the scatter (the kick makes the histogram)
-  int n = 3 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1;
+  // counting sort: the scan and the scatter (the kick makes the histogram)
+  int n = row_scan_launches(P.rows) + 1 + (P.fixed_total[PH_DEP] > 0 ? 1 : 0) + 5 * (int)P.sizes.size() + 1;
   // a fused size replaces its x R2C launch by the fused deposit's two (with a dense-first tile
   // order, one launch more); a separate one adds its deposit launch
   for (size_t g = 0; g < P.sizes.size(); ++g)

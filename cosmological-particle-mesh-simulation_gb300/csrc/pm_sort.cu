@@ -471,13 +471,20 @@ cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, uns
   return cudaGetLastError();
 }
 
+// More blocks than this (33 M bins): adding up the earlier blocks' sums in every block costs more than
+// a scan of the sums.
+constexpr int SCANNED_BLOCKS = 8192;
+
+int row_scan_launches(unsigned nrows) {
+  const size_t nb = row_sort_block_sums(nrows);
+  return 1 + (nb > 1 ? 1 : 0) + (nb > SCANNED_BLOCKS ? 1 : 0);
+}
+
 cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
                      bool zero, Launch st, unsigned* group_max) {
   if (nrows == 0) return cudaErrorInvalidValue;
   const int nb = (int)row_sort_block_sums(nrows);
-  // from 8192 blocks on (33 M bins) adding up the earlier blocks' sums in every block costs more
-  // than a scan of the sums
-  const bool scanned = nb > 8192;
+  const bool scanned = nb > SCANNED_BLOCKS;
   if (nb > 1) launch_chained(k_scan_reduce, nb, CS_NT, 0, st, count, nrows, block_sums);
   if (scanned) launch_chained(k_scan_top, 1, CS_NT, 0, st, block_sums, nb);
   launch_chained(k_scan_apply, nb, CS_NT, 0, st, count, nrows, block_sums, scanned, zero, row_start, cursor, group_max);
