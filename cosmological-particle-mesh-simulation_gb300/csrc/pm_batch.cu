@@ -671,8 +671,8 @@ constexpr int TUNE_AFTER_STEPS = 2;
 // win on the even particle distribution of early steps, where it is timed, and then loses
 // badly once particles cluster -- 1.01 against 0.72 ms at step 980 of the 256^3 / 512^3 run.)  Runs between steps: the trials write
 // only buffers that the next step rewrites from scratch (spectra, grids, the next state, tile
-// counters) or scratch (the kick's keys and histogram go to unused sort buffers), never the
-// state the step reads or the histogram its sort consumes.
+// counters, the sort's cursors) and the keys, which are then made again from the state; never the
+// state the step reads.  Nothing is allocated.
 int autotune(pm_batch* b, cudaStream_t st) {
   Plan& P = b->plan;
   if (b->tuned || !b->autotune) return PM_OK;
@@ -758,16 +758,16 @@ int autotune(pm_batch* b, cudaStream_t st) {
     std::lock_guard<std::mutex> lk(g_tune_lock);
     kick_known = g_kick_cps.count(kkey) != 0;
   }
-  if (!rc && !kick_known) {  // the kick's grid; its keys and histogram go to scratch buffers
+  if (!rc && !kick_known) {
+    // the kick's grid; its keys go over the current ones, which are made again behind the trials
+    // (its histogram goes to scratch)
     const Work wk = work_of(b, PH_KICK, P.fixed_total[PH_KICK]);
     float best_ms = 1e30f;
-    DBuf keys;
-    if (cudaError_t e = keys.ensure(sizeof(unsigned) * (size_t)P.ptot)) rc = bcuda(b, e, "alloc keys");
+    b->keys_valid = false;
     for (int cps : {4, 8, 16, 32}) {
-      if (rc) break;
       float ms = 0.f;
       rc = time3([&]() -> int {
-        PB_CK(launch_kick(ds, wk, in, out, perm, keys.as<unsigned>(), err,
+        PB_CK(launch_kick(ds, wk, in, out, perm, b->sort.keys.as<unsigned>(), err,
                           grid_for(wk.total, b->sms, cps), st, b->row_cursor.as<unsigned>()),
               "kick");
         return PM_OK;
@@ -775,7 +775,7 @@ int autotune(pm_batch* b, cudaStream_t st) {
       if (rc) break;
       if (ms < best_ms) { best_ms = ms; P.kick_cps = cps; }
     }
-    keys.release();
+    if (int r = ensure_keys(b, st); r && !rc) rc = r;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
