@@ -15,8 +15,8 @@
 //     transform of a non-Hermitian rho_k is the inverse real transform of its Hermitian
 //     part (rho_k[k] + conj(rho_k[-k])) / 2, which is built directly in the half spectrum;
 //   * fftn of that field, the potential -rho_k / |l|^2 (k = 0 -> 0), -i l_d pot_k * res,
-//     and Re(ifftn(.)) * force_resolution per direction (zeldovich.py:17-69), the three
-//     directions together; the planes where l_d sits at the Nyquist
+//     and Re(ifftn(.)) * force_resolution per direction (zeldovich.py:17-69), up to 256^3 the
+//     three directions together; the planes where l_d sits at the Nyquist
 //     frequency have no Hermitian part and are zero;
 //   * lattice + Dt * disp + jitter, modulo N_CELLS, and A f H Dt * disp
 //     (zeldovich.py:71-100), stored as float32.
@@ -204,7 +204,7 @@ struct ZelArgs {
   const float2* disp;  // coef / (l0 m2)
   const float2* in;    // fftn of the density (half spectrum)
   float2* out[3];      // i l_d coef / |l|^2 times it along axis d of the (n, n, n) array (0 = slowest,
-                       // the z of [z][y][x]); one of them may be `in`
+                       // the z of [z][y][x]); null: not wanted; one of them may be `in`
 };
 
 __global__ void __launch_bounds__(IC_NT) k_zeld_spectrum(ZelArgs z) {
@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(IC_NT) k_zeld_spectrum(ZelArgs z) {
     }
     #pragma unroll
     for (int d = 0; d < 3; ++d) {
+      if (!z.out[d]) continue;
       const int kd = d == 0 ? kz : (d == 1 ? ky : kx);
       float2 o = make_float2(0.f, 0.f);
       if (mode && kd != h) {  // i * m_d * (disp v)
@@ -275,7 +276,7 @@ __device__ __forceinline__ float2 jitter_pair(unsigned long long x) {
 }
 
 struct PartArgs {
-  int n;
+  int n, first;           // particles per side, axis of blockIdx.y = 0
   long long np;           // n^3
   const float* disp[3];   // displacement field along each axis (n^3, already * force_resolution)
   const float2* space;    // lattice coordinate per axis index (zeldovich.py:79)
@@ -288,13 +289,13 @@ struct PartArgs {
   float* vel;
 };
 
-// A block takes JIT_NT * JIT_ROUNDS consecutive particles of axis blockIdx.y (coalesced); its
+// A block takes JIT_NT * JIT_ROUNDS consecutive particles of axis first + blockIdx.y (coalesced); its
 // first thread jumps the generator there, and thread t reaches its draws by one jump of t + 1
 // steps and then jumps of JIT_NT (one 128-bit multiply-add each).
 __global__ void __launch_bounds__(JIT_NT) k_zeld_particles(PartArgs a) {
   chain_begin();
   __shared__ unsigned long long s_base[2];
-  const int dir = blockIdx.y;
+  const int dir = a.first + blockIdx.y;
   const long long p0 = (long long)blockIdx.x * (JIT_NT * JIT_ROUNDS);
   const u128 inc = ((u128)a.inc_hi << 64) | a.inc_lo;
   if (threadIdx.x == 0) {
@@ -332,6 +333,12 @@ __global__ void __launch_bounds__(JIT_NT) k_zeld_particles(PartArgs a) {
 
 // descriptors of an object's transforms
 enum IcSim : int { SIM_FIELD_INV = 0, SIM_FIELD_FWD, SIM_DISP, IC_SIMS = SIM_DISP + 3 };
+
+// Directions of the displacement whose transforms run together.  Three keep the launches of a small
+// lattice few and its passes full (128^3: 18 launches instead of 28) and make their spectra in one pass, but
+// take three spectra and grids where one after another takes two and one: 3.3 GB instead of 1.7 at
+// 512^3 and 26 instead of 13 at 1024^3, for 7.1 ms instead of 8.1 at 512^3.
+constexpr int ic_together(int n) { return n <= 256 ? 3 : 1; }
 
 struct pm_ics {
   int n = 0, device = 0, sms = 1, m2max = 0;
@@ -402,12 +409,13 @@ int pm_ics_create(int n_parts, int device, pm_ics** out) {
     return o;
   };
   const size_t tables = (size_t)(g->m2max + 1);
+  const int ngrids = ic_together(n), nspecs = ngrids < 2 ? 2 : ngrids;
   const size_t o_sim = part(IC_SIMS * sizeof(Sim)), o_maps = part(2 * IC_SIMS * sizeof(CUtensorMap)),
                o_pre = part(8 * sizeof(int)), o_jump = part(2 * JIT_NT * sizeof(ulonglong2)), o_err = part(sizeof(int)),
                filled = at, o_shape = part(tables * sizeof(double)), o_amp = part(tables * sizeof(float2)),
                o_disp = part(tables * sizeof(float2)), o_partial = part(NORM_BLOCKS * sizeof(double)),
-               o_norm = part(sizeof(double)), o_space = part(n * sizeof(float2)), o_spec = part(3 * sb),
-               o_grid = part(3 * gb);
+               o_norm = part(sizeof(double)), o_space = part(n * sizeof(float2)), o_spec = part(nspecs * sb),
+               o_grid = part(ngrids * gb);
   if (!e) e = g->pool.ensure(at);
   if (!e) {
     char* base = g->pool.as<char>();
@@ -421,16 +429,14 @@ int pm_ics_create(int n_parts, int device, pm_ics** out) {
     g->partial = reinterpret_cast<double*>(base + o_partial);
     g->norm = reinterpret_cast<double*>(base + o_norm);
     g->space = reinterpret_cast<float2*>(base + o_space);
-    for (int i = 0; i < 3; ++i) {
-      g->spec[i] = reinterpret_cast<float2*>(base + o_spec + i * sb);
-      g->grid[i] = reinterpret_cast<float*>(base + o_grid + i * gb);
-    }
+    for (int i = 0; i < nspecs; ++i) g->spec[i] = reinterpret_cast<float2*>(base + o_spec + i * sb);
+    for (int i = 0; i < ngrids; ++i) g->grid[i] = reinterpret_cast<float*>(base + o_grid + i * gb);
     std::vector<char> h(filled, 0);
     // descriptors: the field's inverse and forward transforms, the displacements' inverses
     bool ok = true;
     for (int i = 0; i < IC_SIMS; ++i) {
-      const int sp = i == SIM_FIELD_INV ? 1 : (i == SIM_FIELD_FWD ? 0 : i - SIM_DISP);
-      const int gr = i < SIM_DISP ? 0 : i - SIM_DISP;
+      const int sp = i == SIM_FIELD_INV ? 1 : (i == SIM_FIELD_FWD ? 0 : (ngrids == 3 ? i - SIM_DISP : 1));
+      const int gr = i < SIM_DISP || ngrids == 1 ? 0 : i - SIM_DISP;
       Sim d{};
       d.n = n;
       d.pitch = spec_pitch(n);
@@ -569,12 +575,6 @@ int pm_ics_generate(pm_ics* g, const pm_config* cfg, const pm_ic_params* ic, con
   za.pitch = pitch;
   za.disp = g->disp;
   za.in = g->spec[0];
-  for (int i = 0; i < 3; ++i) {
-    za.out[i] = g->spec[i];
-    pa.disp[i] = g->grid[i];
-  }
-  IC_CK(launch_chained(k_zeld_spectrum, ew, IC_NT, 0, lc, za), "displacement spectrum");
-  if (int r = inverse(SIM_DISP, 3, "displacement inverse")) return r;
   pa.n = n;
   pa.np = np;
   pa.space = g->space;
@@ -589,8 +589,19 @@ int pm_ics_generate(pm_ics* g, const pm_config* cfg, const pm_ic_params* ic, con
   pa.pos = positions;
   pa.vel = velocities;
   const unsigned pb = (unsigned)((np + JIT_NT * JIT_ROUNDS - 1) / (JIT_NT * JIT_ROUNDS));
-  k_zeld_particles<<<dim3(pb, 3), JIT_NT, 0, st>>>(pa);
-  IC_CK(cudaGetLastError(), "particles");
+  const int together = ic_together(n);
+  for (int first = 0; first < 3; first += together) {
+    pa.first = first;
+    for (int d = 0; d < 3; ++d) {
+      const bool now = d >= first && d < first + together;
+      za.out[d] = now ? g->spec[together == 3 ? d : 1] : nullptr;
+      pa.disp[d] = now ? g->grid[together == 3 ? d : 0] : nullptr;
+    }
+    IC_CK(launch_chained(k_zeld_spectrum, ew, IC_NT, 0, lc, za), "displacement spectrum");
+    if (int r = inverse(SIM_DISP + first, together, "displacement inverse")) return r;
+    k_zeld_particles<<<dim3(pb, together), JIT_NT, 0, st>>>(pa);
+    IC_CK(cudaGetLastError(), "particles");
+  }
   // device-side checks of the TMA passes (bounded waits): read back once
   IC_CK(cudaMemcpyAsync(&g->h_err, g->d_err, sizeof(int), cudaMemcpyDeviceToHost, st), "err");
   IC_CK(cudaStreamSynchronize(st), "sync");
