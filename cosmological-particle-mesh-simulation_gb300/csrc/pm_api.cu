@@ -15,7 +15,8 @@ struct pm_ctx {
   DBuf row_start, spec, phi, rho;     // scratch grids
   DBuf hpos, hvel;                    // device copies for pm_step_host
   DBuf pk_partial, pk_out;            // power spectrum scratch
-  DBuf row_count, scan_sums;  // row bin counts of a call (then 4 words: tile counter), block sums of their scan
+  DBuf row_count, scan_sums;  // row bin counts of a call (then 3 words of the fused deposit, the vote on the
+                              // particles' order), block sums of their scan
   DBuf group_max;             // largest count of each 16 row bins
   DBuf dense;                 // the fused deposit's list of two-word tiles
   DBuf rec;                               // cell records in row order, then the forces
@@ -141,7 +142,7 @@ int sort_particles(pm_ctx* c, Call& k, const float* positions, cudaStream_t st, 
 }
 
 // Particles per side if np is the configuration's whole lattice (the caller's arrays are then
-// taken to be in lattice order; any other order gives the same results, slower), else 0.
+// probably in lattice order), else 0.
 int lattice_side(pm_ctx* c, long long np) {
   const long long l = c->cfg.n_parts;
   return l * l * l == np ? (int)l : 0;
@@ -165,10 +166,12 @@ int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy,
   unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
   unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
   if (int r = begin(c, k, st, count, ((size_t)nrows + 4) * sizeof(unsigned))) return r;
-  PM_CK(launch_row_rank(positions, np, lattice_side(c, np), c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, lc), "row ranks");
+  const int side = lattice_side(c, np);
+  int* vote = reinterpret_cast<int*>(count + nrows + 3);
+  PM_CK(launch_row_rank(positions, np, side, c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, vote, lc), "row ranks");
   PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, lc, c->group_max.as<unsigned>()), "row starts");
-  PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, lattice_side(c, np), c->n, start, ranks, place,
-                         c->rec.as<uint4>(), lc),
+  PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, side, c->n, start, ranks, place, c->rec.as<uint4>(), vote,
+                         lc),
         "row order");
   return PM_OK;
 }
@@ -295,7 +298,7 @@ int force(pm_ctx* c, const Call& k, Launch l) {
 
 int advance(pm_ctx* c, const Call& k, const float* pos, const float* vel, float* pos_out, float* vel_out,
             cudaStream_t st) {
-  PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, lattice_side(c, k.sim.np), c->rec.as<uint4>(),
+  PM_CK(launch_advance(c->d_sim.as<Sim>(), k.sim.np, c->rec.as<uint4>(),
                        c->sort.keys.as<unsigned>(), pos, vel, pos_out, vel_out, c->d_err.as<int>(), chained(c, st)),
         "kick");
   return PM_OK;

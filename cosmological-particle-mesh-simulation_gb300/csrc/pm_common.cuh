@@ -260,16 +260,18 @@ cudaError_t launch_kick(const Sim* sims, const Work& w, Parts in, Parts out, con
 // descriptor and work table of one call (from kernel arguments); zero_bytes: a multiple of 16
 cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const CallWork& work, void* zero,
                               size_t zero_bytes, Launch st);
-// np1: particles per side when the particles are in lattice order (np = np1^3), else 0
-// row key and rank inside its row of every particle; count (zero before) ends as the row counts
+// np1: particles per side when np = np1^3 (they may be in lattice order), else 0
+// row key and rank inside its row of every particle; count (zero before) ends as the row counts;
+// vote (np1; 0 before): positive if the particles are in lattice order
 cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
-                            unsigned* ranks, int* err, float* copy, Launch st);
-// cell records in row order; place: in the keys, out each particle's place in row order
+                            unsigned* ranks, int* err, float* copy, int* vote, Launch st);
+// cell records in row order, taken in boxes of the lattice if the vote is for it; place: in the keys,
+// out each particle's place in row order
 cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
-                             const unsigned* ranks, unsigned* place, uint4* rec, Launch st);
+                             const unsigned* ranks, unsigned* place, uint4* rec, const int* vote, Launch st);
 // rec: in the cell records, out the forces (3 floats in the first words of each entry)
 cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, Launch st);
-cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
+cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place,
                            const float* pos, const float* vel, float* pos_out, float* vel_out, int* err, Launch st);
 cudaError_t deposit_prepare();  // sets kernel attributes of the current device (call before graph capture)
 // order of the fused deposit's tiles (dense tiles first); counts: 2 device words, 0 when the kernel starts

@@ -333,12 +333,16 @@ constexpr int ORD_PPT = 4;  // particles per thread: their loads and atomics ove
 // 16 ix, boxes along ix first: a box's particles lie in a few neighbouring rows, and the boxes in
 // flight fill whole rows, so the words they write stay in L2 until their lines are full.  Plain
 // order sweeps all rows once per ix plane.  np1 = 0: plain order.
+// np1^3 particles in another order are better off in plain order (k_row_place, 256^3 particles with
+// the lattice's axes reversed 139 us, in boxes 334; shuffled 420 and 531), so the boxes are taken
+// only if the positions vote for them (lattice_vote).
 struct ParticleOrder {
   long long np;
   int np1, bx, by;  // boxes per axis ix, iy
   __host__ __device__ ParticleOrder(long long n, int l) : np(n), np1(l), bx((l + 15) / 16), by((l + 3) / 4) {}
-  __host__ long long blocks() const {
-    return np1 ? (long long)bx * by * bx : (np + ORD_NT * ORD_PPT - 1) / (ORD_NT * ORD_PPT);
+  __host__ long long blocks() const {  // enough for both orders
+    const long long plain = (np + ORD_NT * ORD_PPT - 1) / (ORD_NT * ORD_PPT), boxes = (long long)bx * by * bx;
+    return np1 && boxes > plain ? boxes : plain;
   }
   __device__ __forceinline__ long long at(int q) const {
     if (!np1) {
@@ -352,12 +356,30 @@ struct ParticleOrder {
   }
 };
 
+// A warp's vote on the order of the np1^3 particles, of which its lanes hold (x, y, z) of 32
+// consecutive ones from i0 on: along a lattice line (iz) the z of a particle and of one m further on
+// are m n / np1 cells apart, and their x and y about the same; m n / np1 is kept to n / 4, far beyond the
+// displacements of neighbours relative to one another in most of the box.  Votes are summed.
+__device__ __forceinline__ void lattice_vote(int np1, int n, long long i0, float x, float y, float z, int* vote) {
+  const int left = np1 - 1 - (int)(i0 % np1), m = min(min(31, np1 / 4), left);  // (warp-uniform)
+  if (m < 1) return;
+  const float fn = (float)n;
+  auto apart = [&](float v) {  // to the nearest image
+    const float d = __shfl_sync(FULL, v, m) - __shfl_sync(FULL, v, 0);
+    return fabsf(d - fn * rintf(d / fn));
+  };
+  const float dx = apart(x), dy = apart(y), dz = apart(z);
+  if ((threadIdx.x & 31) == 0) atomicAdd(vote, dz > 2.f * fmaxf(dx, dy) ? 1 : -1);
+}
+
+// np1 (optional): whether np = np1^3 particles are in lattice order is voted on by every 16th block
+// (vote: 0 before; positive: yes).
 // copy (optional): the positions are also written there (they are read once, e.g. from host
 // memory, and leave a device copy)
 __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ pos, ParticleOrder ord, int n,
                                                      unsigned* __restrict__ count, unsigned* __restrict__ keys,
                                                      unsigned* __restrict__ ranks, int* err,
-                                                     float* __restrict__ copy) {
+                                                     float* __restrict__ copy, int np1, int* __restrict__ vote) {
   chain_begin();
   const int lane = threadIdx.x & 31;
   const long long np = ord.np;
@@ -367,6 +389,10 @@ __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ p
     const long long i = ord.at(q);
     x[q] = y[q] = z[q] = 0.f;
     if (i >= 0) { x[q] = pos[i]; y[q] = pos[np + i]; z[q] = pos[2 * np + i]; }
+  }
+  if (np1 && blockIdx.x % 16 == 0) {
+    const long long i0 = (long long)blockIdx.x * (ORD_NT * ORD_PPT) + threadIdx.x - lane;
+    if (i0 + 31 < np) lattice_vote(np1, n, i0, x[0], y[0], z[0], vote);
   }
   unsigned key[ORD_PPT], grp[ORD_PPT], base[ORD_PPT];
 #pragma unroll
@@ -395,13 +421,14 @@ __global__ void __launch_bounds__(ORD_NT) k_row_rank(const float* __restrict__ p
   }
 }
 
-// place: in the row key of each particle, out its place in row order
+// place: in the row key of each particle, out its place in row order; vote: k_row_rank's
 __global__ void __launch_bounds__(ORD_NT) k_row_place(const float* __restrict__ pos, ParticleOrder ord, int n,
                                                       const unsigned* __restrict__ row_start,
                                                       const unsigned* __restrict__ ranks, unsigned* __restrict__ place,
-                                                      uint4* __restrict__ rec) {
+                                                      uint4* __restrict__ rec, const int* __restrict__ vote) {
   chain_begin();
   const long long np = ord.np;
+  if (ord.np1 && *vote <= 0) ord.np1 = 0;
   Parts out{};
   out.rec = rec;
 #pragma unroll
@@ -729,16 +756,16 @@ cudaError_t launch_call_begin(Sim* dsim, CallWork* dwork, const Sim& sim, const 
 }
 
 cudaError_t launch_row_rank(const float* pos, long long np, int np1, int n, unsigned* count, unsigned* keys,
-                            unsigned* ranks, int* err, float* copy, Launch st) {
+                            unsigned* ranks, int* err, float* copy, int* vote, Launch st) {
   const ParticleOrder o(np, 0);
-  launch_chained(k_row_rank, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, count, keys, ranks, err, copy);
+  launch_chained(k_row_rank, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, count, keys, ranks, err, copy, np1, vote);
   return cudaGetLastError();
 }
 
 cudaError_t launch_row_place(const float* pos, long long np, int np1, int n, const unsigned* row_start,
-                             const unsigned* ranks, unsigned* place, uint4* rec, Launch st) {
+                             const unsigned* ranks, unsigned* place, uint4* rec, const int* vote, Launch st) {
   const ParticleOrder o(np, np1);
-  launch_chained(k_row_place, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, row_start, ranks, place, rec);
+  launch_chained(k_row_place, (int)o.blocks(), ORD_NT, 0, st, pos, o, n, row_start, ranks, place, rec, vote);
   return cudaGetLastError();
 }
 
@@ -748,13 +775,12 @@ cudaError_t launch_force(const Sim* sims, long long np, uint4* rec, int sms, Lau
   return cudaGetLastError();
 }
 
-cudaError_t launch_advance(const Sim* sims, long long np, int np1, const uint4* force, const unsigned* place,
+cudaError_t launch_advance(const Sim* sims, long long np, const uint4* force, const unsigned* place,
                            const float* pos, const float* vel, float* pos_out, float* vel_out, int* err,
                            Launch st) {
   const ParticleOrder o(np, 0);
   launch_chained(k_advance, (int)o.blocks(), ORD_NT, 0, st, sims, o, force, place, pos, vel, pos_out, vel_out, err);
   return cudaGetLastError();
 }
-
 
 }  // namespace pm
