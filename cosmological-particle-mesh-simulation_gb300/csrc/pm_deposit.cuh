@@ -4,7 +4,7 @@
 // rows (the tile plus one row and one plane below, periodic: 7 runs of the row-sorted
 // order) are found through the row starts; their CIC weights that land inside the tile are
 // added to integer accumulators in shared memory (TileSum: one 32-bit word per cell where the
-// particle counts of its row bins allow, else a low word and a coarse word).  Integer sums do
+// number of its source entries allows, else a low word and a high word).  Integer sums do
 // not depend on the order of the atomics, so the deposit is bit-identical run to run.
 #pragma once
 #include <type_traits>
@@ -15,25 +15,22 @@ namespace pm {
 
 constexpr int DEP_NT = 512;
 
-constexpr int COARSE_SHIFT = 12;
-
-__device__ __forceinline__ void acc_add(unsigned* lo, unsigned* co, int i, unsigned q) {
-  atomicAdd(&lo[i], q);  // results unused: non-returning shared-memory reductions
-  atomicAdd(&co[i], q >> COARSE_SHIFT);
+// A two-word sum: the carry out of the low word, seen from the value that was there, is added to the
+// high word.  It is rare, so a corner takes one atomic, as in a one-word sum; a second one for every
+// corner (a word of q >> 12, from which the carries follow) cost the halos' tiles more (256^3
+// particles on 512^3 at steps 400 / 600 / 980 of 1000: 222 / 266 / 338 us -> 175 / 216 / 254).
+__device__ __forceinline__ void acc_add(unsigned* lo, unsigned* hi, int i, unsigned q) {
+  if (atomicAdd(&lo[i], q) > ~q) atomicAdd(&hi[i], 1u);
 }
 
-// The exact sum V from its low word l and its coarse sum c, rounded to float32, times scale.
-// V - (c << 12) lies in [0, 2^32), so V = (c << 12) + (l - (c << 12) mod 2^32): its low word
-// is l and its high word is c >> 20 plus the carry of that addition.  V < 2^44, so
-// V = a 2^23 + b with a, b < 2^23; each is exact as a float (2^23 + a has a as its
-// mantissa), and fmaf(a, 2^23, b) rounds once: the value of a round-to-nearest 64-bit
-// conversion, computed on the FP32 pipe (GB300 issues 64-bit integer conversions to its
-// narrow FP64 pipe).  __fmul_rn: a contraction of the product with the transform's first sums would
+// The exact sum V of low word l and high word h, rounded to float32, times scale.  V < 2^46 (a
+// million particles in a cell), so V = a 2^23 + b with a, b < 2^23; each is exact as a float
+// (2^23 + a has a as its mantissa), and fmaf(a, 2^23, b) rounds once: the value of a
+// round-to-nearest 64-bit conversion, computed on the FP32 pipe (GB300 issues 64-bit integer
+// conversions to its narrow FP64 pipe).  __fmul_rn: a contraction of the product with the transform's first sums would
 // make the fused deposit differ from the written density.
-__device__ __forceinline__ float fixed_to_float(unsigned l, unsigned c, float scale) {
-  const unsigned est_lo = c << COARSE_SHIFT;
-  const unsigned hi = (c >> (32 - COARSE_SHIFT)) + (l < est_lo ? 1u : 0u);
-  const unsigned a = (hi << 9) | (l >> 23), b = l & 0x7fffffu;
+__device__ __forceinline__ float fixed_to_float(unsigned l, unsigned h, float scale) {
+  const unsigned a = (h << 9) | (l >> 23), b = l & 0x7fffffu;
   const float fa = __uint_as_float(0x4B000000u | a) - 8388608.f;
   const float fb = __uint_as_float(0x4B000000u | b) - 8388608.f;
   return __fmul_rn(fmaf(fa, 8388608.f, fb), scale);
@@ -47,7 +44,7 @@ __device__ __forceinline__ float fixed_to_float(unsigned l, unsigned c, float sc
 // each (x, x - 1), which lie in one row bin or two adjacent ones: at most 4 or 8 times the largest count of a
 // row bin of the tile and its three lower neighbours, and at most the tile's source entries, which
 // alone would allow s = 20 to 26 (256^3 on 512^3 early: 21; with the bins 23 to 24).
-// Denser tiles sum at 2^-26 in a low word plus a coarse word (two atomics per corner): bounds from the
+// Denser tiles sum at 2^-26 in a low word and a high word: bounds from the
 // bins would put most of them in one word too, but at s = 20 to 22, and the quantisation would
 // then be the largest error of their density -- one particle per cell of 256^3, uniform:
 // 3.4e-7 in relative L2 instead of 3.2e-8.
@@ -75,9 +72,9 @@ __device__ __forceinline__ float word_to_float(unsigned l, float scale) {
   return __fmul_rn(fmaf(fa, 8388608.f, fb), scale);
 }
 
-// The float of a cell's sum: low word l (and, for two-word tiles, coarse word c).
-__device__ __forceinline__ float sum_to_float(const TileSum& t, unsigned l, unsigned c) {
-  return t.s ? word_to_float(l, t.ms) : fixed_to_float(l, c, t.ms);
+// The float of a cell's sum: low word l (and, for two-word tiles, high word h).
+__device__ __forceinline__ float sum_to_float(const TileSum& t, unsigned l, unsigned h) {
+  return t.s ? word_to_float(l, t.ms) : fixed_to_float(l, h, t.ms);
 }
 
 // Adds the 8 quantised weights q of a particle with base cell (cx, ly, lz) (ly, lz relative

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
       if (ts.s)
         deposit_tile<MODE, DEP_NT, true>(S, p, perm, err, y0, z0, acc, nullptr, n, s_begin, s_off, ts, make_int2(0, TZ),
                                          threadIdx.x);
-      else  // half the planes at a time: low words, then coarse words
+      else  // half the planes at a time: low words, then high words
         deposit_tile<MODE, DEP_NT, false>(S, p, perm, err, y0, z0, acc, acc + TZ * TY / 2 * n, n, s_begin, s_off, ts,
                                           make_int2(half * TZ / 2, (half + 1) * TZ / 2), threadIdx.x);
       __syncthreads();

@@ -840,7 +840,7 @@ __device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restri
   return true;
 }
 
-// The x R2C of the NL rows of each tile (or plane of one): row r's sums at acc + r * stride (TWO: its coarse words HO words further
+// The x R2C of the NL rows of each tile (or plane of one): row r's sums at acc + r * stride (TWO: its high words dep_row_words further
 // on); T lanes to a row, whose exchange buffer overlays its low words once they are read.  A
 // batch is the rows that the CTA's warps hold at once.  f(tg): whether to store tile tg's rows and
 // where they belong; `between` runs in warp 0 before the first transform, `after` behind the
@@ -978,9 +978,9 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
 // (442 -> 498 us on the 512 grid).  By planes: the heart of a large halo is one tile, whose atomics
 // on a few cells alone would otherwise outlast the rest of the kernel (256^3 particles on 512^3 at step
 // 980 of 1000, half of these tiles: planes 249 us, whole tiles 361, single rows 312, planes on 4 CTAs of
-// 256 threads 280).  All tiles of 4096 and more entries at steps 400 / 600 / 980: 222 / 266 / 338 us.
+// 256 threads 280).  All tiles of 4096 and more entries at steps 400 / 600 / 980: 175 / 216 / 254 us.
 constexpr int DEP_DENSE_NT = 512;
-__host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, coarse words
+__host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, high words
 __host__ __device__ constexpr size_t dep_dense_bytes(int n) { return (size_t)TY * dep_dense_stride(n) * sizeof(unsigned); }
 constexpr int DEP_DENSE_CTAS = 2;
 

@@ -114,3 +114,24 @@ def test_dense_ensemble(cuda):
         alone = run((i,), False)[0]
         for got in (mixed[i], tuned[i]):
             assert torch.equal(got[0], alone[0]) and torch.equal(got[1], alone[1])
+
+
+@pytest.mark.parametrize("n", [16, 64, 256])
+@pytest.mark.parametrize("count", [300_000, 2 ** 20 - 1])
+def test_a_million_particles_in_a_cell(cuda, n, count):
+    """Two words hold a cell's sum up to 2^20 particles (2^46), exactly."""
+    torch = cuda
+    from pmgpu.config import Config
+    from pmgpu.context import PMContext
+    pos = torch.tensor([n - 1.0, 5.0, 6.0], device="cuda")[:, None].expand(3, count).contiguous()
+    ctx = PMContext(Config(n_parts=n // 2, n_cells=n, box_size=100.0))
+    want = torch.zeros((n, n, n), device="cuda")
+    want[6, 5, n - 1] = count
+    assert torch.equal(ctx.density(pos, 1.0), want)
+    p1, p2, out = pos.clone(), pos.clone(), ctx.grid()
+    v1, v2 = torch.zeros_like(pos), torch.zeros_like(pos)
+    ctx.step(p1, v1, 1.0, 0.02, 0.00098)
+    ctx.step(p2, v2, 1.0, 0.02, 0.00098, rho_out=out)
+    ctx.check_device()
+    assert torch.equal(out, want) and torch.equal(p1, p2) and torch.equal(v1, v2)
+    ctx.close()
