@@ -142,10 +142,12 @@ int sort_particles(pm_ctx* c, Call& k, const float* positions, cudaStream_t st, 
 }
 
 // Particles per side if np is the configuration's whole lattice (the caller's arrays are then
-// probably in lattice order), else 0.
+// probably in lattice order), else 0.  Also 0 below 128 a side, where all words being written stay in L2 in any
+// order (density() of a lattice in boxes and in plain order, in us: 64^3 particles 64 and 58, 96^3 60
+// and 60, 128^3 113 and 116, 192^3 350 and 380) and the vote would add 0.4 us.
 int lattice_side(pm_ctx* c, long long np) {
   const long long l = c->cfg.n_parts;
-  return l * l * l == np ? (int)l : 0;
+  return l >= 128 && l * l * l == np ? (int)l : 0;
 }
 
 // Writes the call's descriptor and groups the particles by row bin: bin starts in c->row_start,

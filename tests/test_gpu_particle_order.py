@@ -6,7 +6,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("side,n", [(5, 32), (15, 32), (16, 48), (17, 64), (33, 64), (48, 32), (130, 192)])
+@pytest.mark.parametrize("side,n", [(5, 32), (127, 128), (128, 192), (130, 192), (131, 64), (143, 256), (145, 192)])
 @pytest.mark.parametrize("order", ["lattice", "reversed", "shuffled"])
 def test_orders(cuda, side, n, order):
     torch = cuda
