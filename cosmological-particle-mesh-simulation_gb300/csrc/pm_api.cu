@@ -15,7 +15,7 @@ struct pm_ctx {
   DBuf row_start, spec, phi, rho;     // scratch grids
   DBuf hpos, hvel;                    // device copies for pm_step_host
   DBuf pk_partial, pk_out;            // power spectrum scratch
-  DBuf row_count, scan_sums;  // row bin counts of a call (then 3 words of the fused deposit, the vote on the
+  DBuf row_count, scan_sums;  // row bin counts of a call (then 4 words of the fused deposit, the vote on the
                               // particles' order), block sums of their scan
   DBuf group_max;             // largest count of each 16 row bins
   DBuf dense;                 // the fused deposit's list of two-word tiles
@@ -162,14 +162,14 @@ int place_particles(pm_ctx* c, Call& k, const float* positions, float* pos_copy,
   PM_CK(c->sort.ensure(np), "alloc sort");
   PM_CK(c->rec.ensure((size_t)np * sizeof(uint4)), "alloc records");
   PM_CK(c->row_start.ensure(((size_t)nrows + 1) * sizeof(unsigned)), "alloc rows");
-  PM_CK(c->row_count.ensure(((size_t)nrows + 4) * sizeof(unsigned)), "alloc rows");
+  PM_CK(c->row_count.ensure(((size_t)nrows + 8) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->scan_sums.ensure(row_sort_block_sums(nrows) * sizeof(unsigned)), "alloc rows");
   PM_CK(c->group_max.ensure((size_t)nrows / 16 * sizeof(unsigned)), "alloc rows");
   unsigned *count = c->row_count.as<unsigned>(), *start = c->row_start.as<unsigned>();
   unsigned *place = c->sort.keys.as<unsigned>(), *ranks = c->sort.vals.as<unsigned>();
-  if (int r = begin(c, k, st, count, ((size_t)nrows + 4) * sizeof(unsigned))) return r;
+  if (int r = begin(c, k, st, count, ((size_t)nrows + 8) * sizeof(unsigned))) return r;
   const int side = lattice_side(c, np);
-  int* vote = reinterpret_cast<int*>(count + nrows + 3);
+  int* vote = reinterpret_cast<int*>(count + nrows + 4);
   PM_CK(launch_row_rank(positions, np, side, c->n, count, place, ranks, c->d_err.as<int>(), pos_copy, vote, lc), "row ranks");
   PM_CK(row_scan(count, nrows, start, nullptr, c->scan_sums.as<unsigned>(), false, lc, c->group_max.as<unsigned>()), "row starts");
   PM_CK(launch_row_place(pos_copy ? pos_copy : positions, np, side, c->n, start, ranks, place, c->rec.as<uint4>(), vote,

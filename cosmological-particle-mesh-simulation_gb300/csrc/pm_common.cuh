@@ -219,8 +219,9 @@ cudaError_t spectral_dispatch(SpecKind kind, int n, const Sim* sims, Work w, int
                               const CUtensorMap* maps = nullptr, int* err = nullptr);
 cudaError_t launch_fourier_grid(const Sim* sims, int ctas, Launch st);
 // fused deposit + x R2C (the density grid is not written); ctas <= 0 only prepares.
-// next_tile: three device words, 0 at the start: the tile counter, the count of `dense`, a list (room
-// for w.total) of the tiles whose sums need two words, and the counter of that list.  order (optional, w.total entries): the tiles in the order to
+// next_tile: four device words, 0 at the start: the tile counter, and of `dense`, a list (room for
+// w.total) of the tiles whose sums need two words, the count from its front, the counter of its work and
+// the count from its back.  order (optional, w.total entries): the tiles in the order to
 // take them (launch_tile_order).
 template <int N>
 cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned* perm, const unsigned* row_start,

@@ -246,27 +246,29 @@ __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __rest
   return v;
 }
 
-// The runs of plane z0 + p of the tile alone: the rows of the plane and of the one below it, and
-// the row before each.
-__device__ __forceinline__ RunLoad plane_load(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0, int p,
-                                              int lane) {
+// The runs of planes z0 + p0 .. z0 + p1 - 1 of the tile alone: their rows and those of the plane below
+// them, and the row before each of these planes.
+__device__ __forceinline__ RunLoad plane_load(const Sim& S, const unsigned* __restrict__ row_start, int y0, int z0, int p0,
+                                              int p1, int lane) {
   RunLoad v;
-  if (lane >= 4) return v;
-  const int n = S.n, ym = y0 == 0 ? n - 1 : y0 - 1, zp = z0 + p, zm = zp == 0 ? n - 1 : zp - 1;
+  const int n = S.n, ym = y0 == 0 ? n - 1 : y0 - 1, own = p0 > 0 ? p0 - 1 : 0, p = p0 - 3 + lane;
+  int y = y0, z = z0 + own, rows = (p1 - own) * TY;  // lane 0: the tile's own
+  if (lane == 1) { z = z0 - 1; rows = p0 == 0 ? TY : 0; }
+  if (lane >= 2) { y = ym; z = z0 + p; rows = lane < NRUN && p < p1 ? 1 : 0; }
+  if (rows == 0) return v;
   const unsigned per_row = S.xbits ? 1u : (unsigned)x_bins(n);
-  const unsigned r0 = row_number(lane < 2 ? y0 : ym, lane & 1 ? zm : zp, n), nr = lane < 2 ? TY : 1u;
-  const unsigned* s = row_start + (S.row_base + r0 * per_row);
+  const unsigned* s = row_start + (S.row_base + row_number(y, z < 0 ? n - 1 : z, n) * per_row);
   v.beg = __ldg(s);
-  v.cnt = __ldg(s + nr * per_row) - v.beg;
+  v.cnt = __ldg(s + rows * per_row) - v.beg;
   return v;
 }
 
 // Warp-wide (all 32 lanes call it): the run table (first sorted index, and the inclusive scan
 // of the counts) of the tile whose runs the 8 lanes of this lane's group of eight loaded
 // (lane & 7 = the run).  The lanes with `write` store their group's table at s_begin / s_off
-// (NRUN and NRUN + 1 words).  Returns how the tile's sums are held.
+// (NRUN and NRUN + 1 words).  total: the tile's source entries.  Returns how its sums are held.
 __device__ __forceinline__ TileSum run_table(const RunLoad& v, int lane, unsigned* s_begin, unsigned* s_off,
-                                             bool write) {
+                                             bool write, unsigned& total) {
   const int r = lane & 7;
   unsigned incl = v.cnt, m = v.bin_max;
 #pragma unroll
@@ -275,7 +277,7 @@ __device__ __forceinline__ TileSum run_table(const RunLoad& v, int lane, unsigne
     if (r >= o) incl += t;
     m = max(m, __shfl_xor_sync(FULL, m, o, 8));
   }
-  const unsigned total = __shfl_sync(FULL, incl, NRUN - 1, 8);
+  total = __shfl_sync(FULL, incl, NRUN - 1, 8);
   if (write) {
     if (r < NRUN) {
       s_begin[r] = v.beg;

@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
     const int ntile_y = n / TY;
     const int y0 = (local % ntile_y) * TY, z0 = (local / ntile_y) * TZ;
     if (warp == 0) {
-      const TileSum t = run_table(run_load(S, row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off, lane < 8);
+      unsigned total;
+      const TileSum t = run_table(run_load(S, row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off, lane < 8, total);
       if (lane == 0) s_ts = t;
     }
     for (int i = threadIdx.x; i < TZ * TY * n / 4; i += DEP_NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);

@@ -844,10 +844,10 @@ __device__ __forceinline__ bool dep_tile(const Work& w, const unsigned* __restri
 // on); T lanes to a row, whose exchange buffer overlays its low words once they are read.  A
 // batch is the rows that the CTA's warps hold at once.  f(tg): whether to store tile tg's rows and
 // where they belong; `between` runs in warp 0 before the first transform, `after` behind the
-// last; every row is left zero.
+// last; every row is left zero.  rows: all of the TPB * NL, or the first ones.
 template <int N, int NT, int TPB, int NL, bool TWO, class H, class F, class G>
 __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsigned* acc, int stride, const TileSum* s_ts,
-                                              const float2* wt, H tile, F between, G after) {
+                                              const float2* wt, H tile, F between, G after, int rows = TPB * NL) {
   constexpr int M = N / 2, A = xrow_A(N, false), C = xrow_C(N, false), T = xrow_T(N, false), RPW = 32 / T;
   constexpr int NB1 = xrow_NB1<N, false>, NB2 = xrow_NB2<N, false>;
   constexpr int BROWS = NT / 32 * RPW, NBATCH = (TPB * NL + BROWS - 1) / BROWS;
@@ -855,9 +855,9 @@ __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsi
   const int sub = lane / T, t = lane % T;
 #pragma unroll 1
   for (int batch = 0; batch < NBATCH; ++batch) {
-    if (batch * BROWS + warp * RPW >= TPB * NL) break;  // warp-uniform
+    if (batch * BROWS + warp * RPW >= rows) break;  // warp-uniform
     // (where a warp holds more rows than there are, its other lanes repeat the last one)
-    const int R0 = batch * BROWS + warp * RPW + sub, R = TPB * NL % RPW == 0 || R0 < TPB * NL ? R0 : TPB * NL - 1;
+    const int R0 = batch * BROWS + warp * RPW + sub, R = (!TWO && TPB * NL % RPW == 0) || R0 < rows ? R0 : rows - 1;
     const int tg = R / NL, r = R % NL;
     unsigned* row = acc + R * stride;
     float2* rb = reinterpret_cast<float2*>(row);
@@ -888,9 +888,12 @@ __device__ __forceinline__ void dep_transform(const Sim* __restrict__ sims, unsi
     __syncwarp();  // the row's lanes are done with its words
     uint4* z4 = reinterpret_cast<uint4*>(row);
     for (int i = t; i < stride / 4; i += T) z4[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == 0 && batch == NBATCH - 1) after();
+    if (warp == 0 && (batch == NBATCH - 1 || (batch + 1) * BROWS >= rows)) after();
   }
 }
+
+// Source entries from which on a tile of two-word sums is taken apart by planes (k_deposit_r2c_dense).
+constexpr unsigned DEP_HEAVY = 16384;
 
 template <int N>
 __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
@@ -920,13 +923,18 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
     return v;
   };
   // warp 0: stores the tables and how the tiles' sums are held; a tile with two-word sums goes to
-  // the list of k_deposit_r2c_dense and is left out here
+  // the list of k_deposit_r2c_dense (at its back if heavy) and is left out here
   auto store_tables = [&](const RunLoad& v, int idx, TileSum* ts) {
     const int tj = lane < TPB * 8 ? lane >> 3 : 0;
-    const TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8);
+    unsigned total;
+    const TileSum t = run_table(v, lane, s_begin[tj], s_off[tj], lane < TPB * 8, total);
     if (lane < TPB * 8 && (lane & 7) == 0) {
       ts[tj] = t;
-      if (t.s == 0) dense[atomicAdd(next_tile + 1, 1u)] = (unsigned)(idx + tj);
+      if (t.s == 0) {
+        const bool heavy = total >= DEP_HEAVY;
+        const unsigned at = atomicAdd(next_tile + (heavy ? 3 : 1), 1u);
+        dense[heavy ? w.total - 1 - at : at] = (unsigned)(idx + tj);
+      }
     }
   };
   // Tiles are taken from a counter (zero at launch) after the first, TPB per CTA: a tile's
@@ -964,32 +972,53 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
                                              s_off[g], ts, make_int2(0, TZ), gtid);
     }
     __syncthreads();
-    dep_transform<N, NT, TPB, NL, false>(
-        sims, acc, RS, s_ts[turn], wt,
-        [&](int tg, int& si, int& y0, int& z0) { return dep_tile<N>(w, order, idx + tg, si, y0, z0) && s_ts[turn][tg].s; },
-        take, store);
+    bool any = false;  // (without a one-word tile there is nothing to transform)
+#pragma unroll
+    for (int j = 0; j < TPB; ++j) any = any || s_ts[turn][j].s;
+    if (any) {
+      dep_transform<N, NT, TPB, NL, false>(
+          sims, acc, RS, s_ts[turn], wt,
+          [&](int tg, int& si, int& y0, int& z0) { return dep_tile<N>(w, order, idx + tg, si, y0, z0) && s_ts[turn][tg].s; },
+          take, store);
+    } else if (warp == 0) {
+      take();
+      store();
+    }
     __syncthreads();
     idx = s_next;
   }
 }
 
-// The tiles that k_deposit_r2c left: those with two-word sums, one plane at a time, taken from a
-// counter.  A kernel of its own: next to the one-word path its registers and code cost that path 10%
-// (442 -> 498 us on the 512 grid).  By planes: the heart of a large halo is one tile, whose atomics
-// on a few cells alone would otherwise outlast the rest of the kernel (256^3 particles on 512^3 at step
-// 980 of 1000, half of these tiles: planes 249 us, whole tiles 361, single rows 312, planes on 4 CTAs of
-// 256 threads 280).  All tiles of 4096 and more entries at steps 400 / 600 / 980: 175 / 216 / 254 us.
+// The tiles that k_deposit_r2c left: those with two-word sums.  A kernel of its own: next to the
+// one-word path its registers and code cost that path 10% (442 -> 498 us on the 512 grid).  A unit of
+// work, taken from a counter, is a whole tile (half of one on 1024, where four planes would leave room for one
+// CTA).  Planes are units of their own, and read every particle up to twice, in two cases:
+// * heavy tiles, which come first: the heart of a large halo is one tile, whose atomics on a few
+//   cells alone would otherwise outlast the rest of the kernel (256^3 particles on 512^3 at step 980
+//   of 1000: all tiles whole 385 us, heavy from 8192 entries on 236, from 16384 on 213 -- these with
+//   256 threads; with 512 178; all by planes 254);
+// * fewer tiles than CTAs (128^3 particles on 128^3 at step 20: 47 us whole, 34 by planes).
+// By planes alone a state with most of its tiles dense takes twice the time (256^3 on 256^3 early 466 us
+// against 242; 357^3 on 512^3 1423 against 745).  512 threads, 2 CTAs per SM, against 256
+// threads and up to 4: 1024^3 late 1736 against 2104 us, 96^3 on 128^3 late 64 against 90, the dense early
+// states 745 against 723 and 242 against 212; 384 threads lie between.
 constexpr int DEP_DENSE_NT = 512;
+__host__ __device__ constexpr int dep_dense_planes(int n) { return n == 1024 ? 2 : TZ; }  // planes of a large unit
 __host__ __device__ constexpr int dep_dense_stride(int n) { return dep_row_words(n) + n; }  // low words, high words
-__host__ __device__ constexpr size_t dep_dense_bytes(int n) { return (size_t)TY * dep_dense_stride(n) * sizeof(unsigned); }
-constexpr int DEP_DENSE_CTAS = 2;
+__host__ __device__ constexpr size_t dep_dense_bytes(int n) {
+  return (size_t)dep_dense_planes(n) * TY * dep_dense_stride(n) * sizeof(unsigned);
+}
+__host__ __device__ constexpr int dep_dense_ctas(int n) {
+  const int by_smem = (int)((220 * 1024) / (dep_dense_bytes(n) + 6 * 1024));
+  return by_smem > 2 ? 2 : by_smem;
+}
 
 template <int N>
-__global__ void __launch_bounds__(DEP_DENSE_NT, DEP_DENSE_CTAS)
+__global__ void __launch_bounds__(DEP_DENSE_NT, dep_dense_ctas(N))
     k_deposit_r2c_dense(const Sim* __restrict__ sims, Work w, Parts p, const unsigned* __restrict__ perm,
                         const unsigned* __restrict__ row_start, int* err, unsigned* __restrict__ next_tile,
                         const unsigned* __restrict__ order, const unsigned* __restrict__ dense) {
-  constexpr int NT = DEP_DENSE_NT, RS = dep_dense_stride(N);
+  constexpr int NT = DEP_DENSE_NT, RS = dep_dense_stride(N), PU = dep_dense_planes(N);
   static_assert(RS % 4 == 0, "rows zeroed 4 words at a time");
   extern __shared__ uint4 acc_raw[];
   __shared__ unsigned s_begin[8];
@@ -999,42 +1028,51 @@ __global__ void __launch_bounds__(DEP_DENSE_NT, DEP_DENSE_CTAS)
   unsigned* acc = reinterpret_cast<unsigned*>(acc_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   chain_begin();
-  const unsigned count = next_tile[1] * TZ;
+  const unsigned light = next_tile[1], heavy = next_tile[3] * TZ;
+  const int pu = light < gridDim.x ? 1 : PU;  // planes of a unit of a light tile
+  const unsigned count = heavy + light * (unsigned)(TZ / pu);
   if (blockIdx.x >= count) return;
-  for (int i = threadIdx.x; i < TY * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = threadIdx.x; i < PU * TY * RS / 4; i += NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
   xrow_table_fill<N, false, true, NT>(wt, sims[locate_sim(w, 0)].tw);
-  // warp 0 takes the next plane and loads its run table before the transform and stores it after
-  unsigned i = blockIdx.x, next = 0;
+  // unit u: planes p0 .. p1 - 1 of a tile (a heavy one from the back of the list, a light one from its front)
+  auto unit = [&](unsigned u, int& si, int& y0, int& z0, int& p0, int& p1) {
+    const bool hv = u < heavy;
+    const unsigned v = hv ? u : u - heavy, k = hv ? 1u : (unsigned)pu, parts = TZ / k;
+    p0 = (int)(v % parts * k);
+    p1 = p0 + (int)k;
+    dep_tile<N>(w, order, (int)dense[hv ? (unsigned)w.total - 1 - v / parts : v / parts], si, y0, z0);
+  };
+  // warp 0 takes the next unit and loads its run table before the transform and stores it after
+  unsigned i = blockIdx.x, next = 0, total;
   RunLoad nl;
-  auto load = [&](unsigned unit) {
-    int si, y0, z0;
-    dep_tile<N>(w, order, (int)dense[unit / TZ], si, y0, z0);
-    nl = plane_load(sims[si], row_start, y0, z0, (int)(unit % TZ), lane & 7);
+  auto load = [&](unsigned u) {
+    int si, y0, z0, p0, p1;
+    unit(u, si, y0, z0, p0, p1);
+    nl = plane_load(sims[si], row_start, y0, z0, p0, p1, lane & 7);
   };
   auto take = [&]() {
     next = __shfl_sync(FULL, lane == 0 ? gridDim.x + atomicAdd(next_tile + 2, 1u) : 0u, 0);
     if (next < count) load(next);
   };
   auto store = [&]() {
-    if (next < count) run_table(nl, lane, s_begin, s_off, lane < 8);
+    if (next < count) run_table(nl, lane, s_begin, s_off, lane < 8, total);
     if (lane == 0) s_next = next;
   };
   if (warp == 0) {
     load(i);
-    run_table(nl, lane, s_begin, s_off, lane < 8);
+    run_table(nl, lane, s_begin, s_off, lane < 8, total);
   }
   __syncthreads();
   while (i < count) {
-    int si, y0, z0;
-    dep_tile<N>(w, order, (int)dense[i / TZ], si, y0, z0);
-    const int zp = (int)(i % TZ);
+    int si, y0, z0, p0, p1;
+    unit(i, si, y0, z0, p0, p1);
     const TileSum ts{0, sims[si].mass_scale};
     deposit_tile<POS_DISP, NT, false, N>(sims[si], p, perm, err, y0, z0, acc, acc + dep_row_words(N), RS, s_begin, s_off, ts,
-                                         make_int2(zp, zp + 1), threadIdx.x);
+                                         make_int2(p0, p1), threadIdx.x);
     __syncthreads();
-    dep_transform<N, NT, 1, TY, true>(
-        sims, acc, RS, &ts, wt, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0 + zp; return true; }, take,
-        store);
+    dep_transform<N, NT, 1, PU * TY, true>(
+        sims, acc, RS, &ts, wt, [&](int, int& a, int& b, int& c) { a = si; b = y0; c = z0 + p0; return true; }, take,
+        store, (p1 - p0) * TY);
     __syncthreads();
     i = s_next;
   }
@@ -1066,7 +1104,7 @@ cudaError_t deposit_r2c_launch(const Sim* sims, Work w, Parts p, const unsigned*
     launch_chained(k_deposit_r2c<N>, ctas, NT, sm, st, sims, w, p, perm, row_start, group_max, err, next_tile, order,
                    dense);
     if (cudaError_t e = cudaGetLastError()) return e;
-    const int cap = device_sms() * DEP_DENSE_CTAS, few = w.total < cap / TZ ? w.total * TZ : cap;
+    const int cap = device_sms() * dep_dense_ctas(N), few = w.total < cap / TZ ? w.total * TZ : cap;
     launch_chained(k_deposit_r2c_dense<N>, few, DEP_DENSE_NT, smd, st, sims, w, p, perm, row_start, err, next_tile,
                    order, dense);
     return cudaGetLastError();

@@ -99,6 +99,8 @@ def test_dense_ensemble(cuda):
         vel = torch.randn(pos.shape, generator=g, device="cuda") * 0.01
         sims.append((Config(n_parts=p, n_cells=n, box_size=100.0, random_seed=seed, steps=1000), pos, vel))
 
+    torch.cuda.synchronize()  # (admission reads complete arrays)
+
     def run(sel, tune):
         b = Batch(autotune=tune)
         ids = [b.add(*sims[i]) for i in sel]
