@@ -323,8 +323,6 @@ cudaError_t row_counting_sort(const unsigned* keys, long long n, unsigned nrows,
 cudaError_t row_scan(unsigned* count, unsigned nrows, unsigned* row_start, unsigned* cursor, unsigned* block_sums,
                      bool zero, Launch st, unsigned* group_max = nullptr);
 int row_scan_launches(unsigned nrows);  // its kernels
-// group_max[g] = largest count of the row bins 16 g .. 16 g + 15 from their starts (row_scan: from the counts)
-cudaError_t launch_group_max(const unsigned* row_start, unsigned nrows, unsigned* group_max, Launch st);
 // count[r] = number of keys equal to r (count zeroed first)
 cudaError_t row_histogram(const unsigned* keys, long long n, unsigned nrows, unsigned* count, int* err, int sms,
                           Launch st);

@@ -203,15 +203,19 @@ __device__ __forceinline__ bool source_cell(const Sim& S, const Parts& p, const 
 }
 
 // The 7 runs of the tile at (y0, z0): lane r < NRUN of a group of eight loads the first sorted
-// index and the particle count of run r; and, with bin_max, the largest row bin count of the
-// tile and the three below it (all lanes of the group): group_max holds the maxima of 16
-// consecutive row bins, a tile's bins being x_bins such groups.
+// index and the particle count of run r; and, unless MAX is BINS_NOT, the largest row bin count of the
+// tile and the three below it (all lanes of the group) -- BINS_MAXIMA: group_max holds the maxima of 16
+// consecutive row bins, a tile's bins being x_bins such groups; BINS_STARTS: from row_start, eight times
+// the loads, where a kernel to make the maxima would cost more (4 us of a 60 us call).
+enum BinsMode : int { BINS_NOT = 0, BINS_MAXIMA, BINS_STARTS };
+
 struct RunLoad {
   unsigned beg = 0, cnt = 0, bin_max = 0;
   int per_row = 1;         // row bins to a row
   float mass_scale = 0.f;  // of the simulation
 };
 
+template <int MAX>
 __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __restrict__ row_start,
                                             const unsigned* __restrict__ group_max, int y0, int z0, int lane) {
   RunLoad v;
@@ -235,12 +239,13 @@ __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __rest
     v.beg = __ldg(s);
     v.cnt = __ldg(s + nr * per_row) - v.beg;
   }
-  if (group_max) {
-    const unsigned* g = group_max + S.row_base / (TZ * TY);
-    for (unsigned i = lane; i < 4 * per_row; i += 8) {
-      const unsigned t = i / per_row;
-      const unsigned tile = t == 0 ? t_own : (t == 1 ? t_zb : (t == 2 ? t_yb : t_c));
-      v.bin_max = max(v.bin_max, __ldg(&g[tile * per_row + i % per_row]));
+  if (MAX != BINS_NOT) {
+    const unsigned each = MAX == BINS_MAXIMA ? per_row : per_row * (TZ * TY);  // words of a tile
+    for (unsigned i = lane; i < 4 * each; i += 8) {
+      const unsigned t = i / each;
+      const unsigned tile = t == 0 ? t_own : (t == 1 ? t_zb : (t == 2 ? t_yb : t_c)), at = tile * each + i % each;
+      const unsigned* b = MAX == BINS_MAXIMA ? group_max + S.row_base / (TZ * TY) + at : row_start + (S.row_base + at);
+      v.bin_max = max(v.bin_max, MAX == BINS_MAXIMA ? __ldg(b) : __ldg(b + 1) - __ldg(b));
     }
   }
   return v;

@@ -49,7 +49,6 @@ struct NoAllocScratch {
   unsigned hist[SORT_DIGIT_TOTALS * NOALLOC_MAX_BLOCKS];
   unsigned digit_tot[SORT_DIGIT_TOTALS];
   unsigned row_start[NOALLOC_MAX_ROWS + 1];
-  unsigned group_max[NOALLOC_MAX_ROWS / 16];
 };
 
 // The scratch: about 4.3 MB.
@@ -142,8 +141,7 @@ extern "C" int pm_density_noalloc(const float* positions, long long np, int n_ce
   unsigned* perm = alt ? s->vals_alt : s->vals;
   unsigned* skeys = alt ? s->keys_alt : s->keys;
   if (launch_row_start(skeys, np, d.xbits, (unsigned)nrows, s->row_start, st)) return PM_ERR_CUDA;
-  if (launch_group_max(s->row_start, (unsigned)nrows, s->group_max, st)) return PM_ERR_CUDA;
-  if (launch_deposit(&s->sim, wd, p, perm, s->row_start, s->group_max, POS_ABS, &s->err, grid_for(dep_units, sms, 3),
+  if (launch_deposit(&s->sim, wd, p, perm, s->row_start, nullptr, POS_ABS, &s->err, grid_for(dep_units, sms, 3),
                      deposit_smem_bytes(n_cells, TILE_Y, TILE_Z), st))
     return PM_ERR_CUDA;
   return PM_OK;

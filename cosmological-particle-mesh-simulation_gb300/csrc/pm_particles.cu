@@ -62,25 +62,10 @@ __global__ void k_row_start(const unsigned* __restrict__ keys, long long n, int 
   }
 }
 
-// group_max[g] = largest particle count of the rows 16 g .. 16 g + 15 (the scan of the row counts
-// makes it where there is one, pm_sort.cu)
-__global__ void k_group_max(const unsigned* __restrict__ row_start, unsigned groups, unsigned* __restrict__ group_max) {
-  chain_begin();
-  const unsigned g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= groups) return;
-  unsigned m = 0, prev = row_start[16 * g];
-  for (int i = 1; i <= 16; ++i) {
-    const unsigned next = row_start[16 * g + i];
-    m = max(m, next - prev);
-    prev = next;
-  }
-  group_max[g] = m;
-}
-
 // ---------------------------------------------------------------------------------
 // deposit: one CTA per tile (pm_deposit.cuh), then the tile's rows are written once
 // ---------------------------------------------------------------------------------
-template <int MODE>
+template <int MODE, int BINS>
 __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ sims, Work w, Parts p,
                                                        const unsigned* __restrict__ perm,
                                                        const unsigned* __restrict__ row_start,
@@ -101,7 +86,8 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
     const int y0 = (local % ntile_y) * TY, z0 = (local / ntile_y) * TZ;
     if (warp == 0) {
       unsigned total;
-      const TileSum t = run_table(run_load(S, row_start, group_max, y0, z0, lane & 7), lane, s_begin, s_off, lane < 8, total);
+      const RunLoad v = run_load<BINS>(S, row_start, group_max, y0, z0, lane & 7);
+      const TileSum t = run_table(v, lane, s_begin, s_off, lane < 8, total);
       if (lane == 0) s_ts = t;
     }
     for (int i = threadIdx.x; i < TZ * TY * n / 4; i += DEP_NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -664,13 +650,13 @@ cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, i
 cudaError_t deposit_prepare() {
   static DeviceOnce once;
   return once.run([]() {
-  cudaError_t e = cudaFuncSetAttribute(k_deposit<POS_ABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)deposit_smem_bytes(PM_MAX_N, 4, 4));
-  if (!e) e = cudaFuncSetAttribute(k_deposit<POS_DISP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)deposit_smem_bytes(PM_MAX_N, 4, 4));
-  if (!e) e = cudaFuncSetAttribute(k_deposit<POS_ABS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (!e) e = cudaFuncSetAttribute(k_deposit<POS_DISP>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  return e;
+    const int sm = (int)deposit_smem_bytes(PM_MAX_N, 4, 4);
+    cudaError_t e = cudaSuccess;
+    for (auto k : {k_deposit<POS_ABS, BINS_STARTS>, k_deposit<POS_DISP, BINS_MAXIMA>}) {
+      if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    }
+    return e;
   });
 }
 
@@ -696,11 +682,6 @@ cudaError_t launch_row_start(const unsigned* keys, long long n, int xbits, unsig
   return cudaGetLastError();
 }
 
-cudaError_t launch_group_max(const unsigned* row_start, unsigned nrows, unsigned* group_max, Launch st) {
-  launch_chained(k_group_max, (int)((nrows / 16 + 127) / 128), 128, 0, st, row_start, nrows / 16, group_max);
-  return cudaGetLastError();
-}
-
 // Order in which the fused deposit takes its tiles: the dense tiles first.  A tile's work is
 // its source-entry count, which clustering makes very uneven; a dense tile taken late runs on
 // alone after the others have finished.  Tiles with more than twice the mean count go to the
@@ -716,7 +697,7 @@ __global__ void k_tile_order(const Sim* __restrict__ sims, Work w, const unsigne
     const int y0 = (local % (n / TY)) * TY, z0 = (local / (n / TY)) * TZ;
     unsigned cnt = 0;
 #pragma unroll
-    for (int r = 0; r < NRUN; ++r) cnt += run_load(S, row_start, nullptr, y0, z0, r).cnt;
+    for (int r = 0; r < NRUN; ++r) cnt += run_load<BINS_NOT>(S, row_start, nullptr, y0, z0, r).cnt;
     // mean source entries per tile: each particle once, plus its tile's last plane / row / corner
     const double ntiles = (double)(n / TY) * (n / TZ);
     const double mean = (double)S.np * (1.0 + 1.0 / TZ + 1.0 / TY + 1.0 / (TY * TZ)) / ntiles;
@@ -737,8 +718,9 @@ cudaError_t launch_deposit(const Sim* sims, const Work& w, Parts p, const unsign
                            const unsigned* row_start, const unsigned* group_max, int mode, int* err, int ctas,
                            size_t smem, Launch st) {
   if (cudaError_t e = deposit_prepare()) return e;
-  if (mode == POS_ABS) launch_chained(k_deposit<POS_ABS>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, group_max, err);
-  else launch_chained(k_deposit<POS_DISP>, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, group_max, err);
+  // (absolute positions come without bin maxima)
+  auto kernel = mode == POS_ABS ? k_deposit<POS_ABS, BINS_STARTS> : k_deposit<POS_DISP, BINS_MAXIMA>;
+  launch_chained(kernel, ctas, DEP_NT, smem, st, sims, w, p, perm, row_start, group_max, err);
   return cudaGetLastError();
 }
 

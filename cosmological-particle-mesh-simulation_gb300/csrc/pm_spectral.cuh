@@ -919,7 +919,7 @@ __global__ void __launch_bounds__(DEP_ROW_NT, dep_ctas_bound(N))
     RunLoad v;
     int si, y0, z0;
     if (dep_tile<N>(w, order, idx + (lane >> 3), si, y0, z0))
-      v = run_load(sims[si], row_start, group_max, y0, z0, lane & 7);
+      v = run_load<BINS_MAXIMA>(sims[si], row_start, group_max, y0, z0, lane & 7);
     return v;
   };
   // warp 0: stores the tables and how the tiles' sums are held; a tile with two-word sums goes to

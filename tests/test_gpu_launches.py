@@ -51,3 +51,23 @@ def test_scan_of_many_bins(cuda):
         alone.close()
         assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
     b.close()
+
+
+def test_launches_of_the_noalloc_deposit(cuda):
+    """Descriptor, keys, three kernels for each of the two digits of an 18-bit key, row starts, deposit:
+    the bin maxima of the deposit's bound take no launch of their own."""
+    import ctypes
+
+    torch = cuda
+    from pmgpu import _lib
+    from torch.profiler import ProfilerActivity, profile
+    lib, n = _lib.load(), 64
+    pos = torch.rand((3, 10000), device="cuda") * n
+    rho = torch.empty((n, n, n), device="cuda")
+    for _ in range(3):
+        with profile(activities=[ProfilerActivity.CUDA, ProfilerActivity.CPU]) as p:
+            assert lib.pm_density_noalloc(ctypes.c_void_p(pos.data_ptr()), 10000, n, 1.0, ctypes.c_void_p(rho.data_ptr()),
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+            torch.cuda.synchronize()
+    names = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert len([k for k in names if not k.startswith(("Memset", "Memcpy"))]) == 10, names
