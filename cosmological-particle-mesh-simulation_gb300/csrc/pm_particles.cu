@@ -65,6 +65,10 @@ __global__ void k_row_start(const unsigned* __restrict__ keys, long long n, int 
 // ---------------------------------------------------------------------------------
 // deposit: one CTA per tile (pm_deposit.cuh), then the tile's rows are written once
 // ---------------------------------------------------------------------------------
+// Words of a cell's sum that there is room for: two up to 512 cells, at three CTAs per SM; above, tiles
+// in two words are done half their planes at a time.
+__host__ __device__ constexpr int deposit_words(int n) { return n <= 512 ? 2 : 1; }
+
 template <int MODE, int BINS>
 __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ sims, Work w, Parts p,
                                                        const unsigned* __restrict__ perm,
@@ -90,22 +94,23 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
       const TileSum t = run_table(v, lane, s_begin, s_off, lane < 8, total);
       if (lane == 0) s_ts = t;
     }
-    for (int i = threadIdx.x; i < TZ * TY * n / 4; i += DEP_NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
+    const int words = deposit_words(n);  // of a cell
+    for (int i = threadIdx.x; i < words * TZ * TY * n / 4; i += DEP_NT) acc_raw[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const TileSum ts = s_ts;
-    const int rows = ts.s ? TZ * TY : TZ * TY / 2;
+    const int rows = ts.s || words == 2 ? TZ * TY : TZ * TY / 2;
     for (int half = 0; half < TZ * TY / rows; ++half) {
       if (ts.s)
         deposit_tile<MODE, DEP_NT, true>(S, p, perm, err, y0, z0, acc, nullptr, n, s_begin, s_off, ts, make_int2(0, TZ),
                                          threadIdx.x);
-      else  // half the planes at a time: low words, then high words
-        deposit_tile<MODE, DEP_NT, false>(S, p, perm, err, y0, z0, acc, acc + TZ * TY / 2 * n, n, s_begin, s_off, ts,
-                                          make_int2(half * TZ / 2, (half + 1) * TZ / 2), threadIdx.x);
+      else  // low words, then high words (of half the planes at a time)
+        deposit_tile<MODE, DEP_NT, false>(S, p, perm, err, y0, z0, acc, acc + rows * n, n, s_begin, s_off, ts,
+                                          make_int2(half * rows / TY, (half + 1) * rows / TY), threadIdx.x);
       __syncthreads();
       for (int r = warp; r < rows; r += DEP_NT / 32) {
         const int row = half * rows + r;
         uint4* l4 = reinterpret_cast<uint4*>(acc + r * n);
-        uint4* h4 = reinterpret_cast<uint4*>(acc + (r + TZ * TY / 2) * n);  // (two-word tiles)
+        uint4* h4 = reinterpret_cast<uint4*>(acc + (r + rows) * n);  // (two-word tiles)
         float4* dst = reinterpret_cast<float4*>(S.rho + ((long long)(z0 + row / TY) * n + (y0 + row % TY)) * n);
         for (int x4 = lane; x4 < n / 4; x4 += 32) {
           const uint4 l = l4[x4], h = ts.s ? make_uint4(0u, 0u, 0u, 0u) : h4[x4];
@@ -650,7 +655,8 @@ cudaError_t launch_disp_to_abs(Parts in, long long off, long long np, int np1, i
 cudaError_t deposit_prepare() {
   static DeviceOnce once;
   return once.run([]() {
-    const int sm = (int)deposit_smem_bytes(PM_MAX_N, 4, 4);
+    int sm = 0;
+    for (int n = 16; n <= PM_MAX_N; n *= 2) sm = std::max(sm, (int)deposit_smem_bytes(n, TY, TZ));
     cudaError_t e = cudaSuccess;
     for (auto k : {k_deposit<POS_ABS, BINS_STARTS>, k_deposit<POS_DISP, BINS_MAXIMA>}) {
       if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -660,7 +666,7 @@ cudaError_t deposit_prepare() {
   });
 }
 
-size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * sizeof(unsigned); }
+size_t deposit_smem_bytes(int n, int ty, int tz) { return (size_t)n * ty * tz * deposit_words(n) * sizeof(unsigned); }
 
 cudaError_t launch_keys_abs(const Sim* sims, const Work& w, Parts p, unsigned* keys, unsigned* vals,
                             int* err, int ctas, Launch st) {
