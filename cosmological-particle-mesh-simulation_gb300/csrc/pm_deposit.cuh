@@ -205,8 +205,9 @@ __device__ __forceinline__ bool source_cell(const Sim& S, const Parts& p, const 
 // The 7 runs of the tile at (y0, z0): lane r < NRUN of a group of eight loads the first sorted
 // index and the particle count of run r; and, unless MAX is BINS_NOT, the largest row bin count of the
 // tile and the three below it (all lanes of the group) -- BINS_MAXIMA: group_max holds the maxima of 16
-// consecutive row bins, a tile's bins being x_bins such groups; BINS_STARTS: from row_start, eight times
-// the loads, where a kernel to make the maxima would cost more (4 us of a 60 us call).
+// consecutive row bins, a tile's bins being x_bins such groups; BINS_STARTS: from row_start, where a
+// kernel to make the maxima would cost more (4 us of a 60 us call), all 32 lanes of a warp for one
+// tile (lane32), each with the maximum of its part.
 enum BinsMode : int { BINS_NOT = 0, BINS_MAXIMA, BINS_STARTS };
 
 struct RunLoad {
@@ -217,7 +218,8 @@ struct RunLoad {
 
 template <int MAX>
 __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __restrict__ row_start,
-                                            const unsigned* __restrict__ group_max, int y0, int z0, int lane) {
+                                            const unsigned* __restrict__ group_max, int y0, int z0, int lane,
+                                            int lane32 = 0) {
   RunLoad v;
   const int n = S.n;
   const int ym = y0 == 0 ? n - TY : y0 - TY, zm = z0 == 0 ? n - TZ : z0 - TZ;  // tiles below
@@ -241,7 +243,7 @@ __device__ __forceinline__ RunLoad run_load(const Sim& S, const unsigned* __rest
   }
   if (MAX != BINS_NOT) {
     const unsigned each = MAX == BINS_MAXIMA ? per_row : per_row * (TZ * TY);  // words of a tile
-    for (unsigned i = lane; i < 4 * each; i += 8) {
+    for (unsigned i = MAX == BINS_MAXIMA ? lane : lane32; i < 4 * each; i += MAX == BINS_MAXIMA ? 8 : 32) {
       const unsigned t = i / each;
       const unsigned tile = t == 0 ? t_own : (t == 1 ? t_zb : (t == 2 ? t_yb : t_c)), at = tile * each + i % each;
       const unsigned* b = MAX == BINS_MAXIMA ? group_max + S.row_base / (TZ * TY) + at : row_start + (S.row_base + at);

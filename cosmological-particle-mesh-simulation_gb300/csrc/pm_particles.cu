@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(DEP_NT, 3) k_deposit(const Sim* __restrict__ s
     const int y0 = (local % ntile_y) * TY, z0 = (local / ntile_y) * TZ;
     if (warp == 0) {
       unsigned total;
-      const RunLoad v = run_load<BINS>(S, row_start, group_max, y0, z0, lane & 7);
+      RunLoad v = run_load<BINS>(S, row_start, group_max, y0, z0, lane & 7, lane);
+      if (BINS == BINS_STARTS) v.bin_max = __reduce_max_sync(FULL, v.bin_max);
       const TileSum t = run_table(v, lane, s_begin, s_off, lane < 8, total);
       if (lane == 0) s_ts = t;
     }
