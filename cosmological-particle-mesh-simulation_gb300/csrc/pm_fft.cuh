@@ -211,8 +211,9 @@ template <bool INV> struct DFT<32, INV> {
 // the two-pass plans of 128, 192, 256 and 384 and the three-pass plan of 1024 measured, per
 // 134M cells (y, z in ms), 128: 0.191, 0.311 -> 0.174, 0.265; 192: 0.243, 0.497 -> 0.228,
 // 0.335; 256: 0.208, 0.340 -> 0.190, 0.281; 384: 0.304, 0.843 -> 0.243, 0.631; 1024 (y, per
-// 1.07G cells): 1.88 -> 1.51.  512 keeps three radix-8 passes on pairs of lines (16 x 32 line
-// by line: z 0.291 -> 0.303 ms, half the threads idle in the radix-32 pass).
+// 1.07G cells): 1.88 -> 1.51.  The y passes of 512 keep three radix-8 passes on pairs of lines (16 x 32
+// line by line: y 0.182 -> 0.192 ms); the z passes of the larger grids have plans of their own
+// (TurnPlan), at thread counts of their own (pm_spectral.cuh: turn_nt).
 // ---------------------------------------------------------------------------------
 // Lengths whose blocked transforms run on pairs of lines: the plans of radix 8 or less, and
 // 128 (8 x 16).  The radix-12/16/24 plans hold too many values per pair of lines and run

@@ -28,7 +28,7 @@
 // and held as float32 pairs (48 bits and more), and products and sums with them are carried as
 // pairs (Dekker's and Knuth's error-free transformations), rounded to float32 once at the end.
 // 128^3: spectra of the displacements 170 -> 18 us, particles 227 -> 44, field 59 -> 19; the whole
-// call 772 -> 282, with 18 launches instead of 30.
+// call 772 -> 268, with 18 launches instead of 30.
 #include "pm_host.cuh"
 #include "pm_pair.cuh"
 

@@ -395,12 +395,12 @@ __global__ void __launch_bounds__(SP_NT) k_z_green(const Sim* __restrict__ sims,
 // ---------------------------------------------------------------------------------
 // TMA-streamed line pass (y forward / y inverse / z Green) over one or many simulations.
 //
-// Persistent CTA with a 3-stage shared-memory ring.  A unit is BPC bundles of one
+// Persistent CTA with a shared-memory ring of STAGES stages (3; the turn on 384, 512 and 768: 2).  A unit is BPC bundles of one
 // simulation; a bundle is BW consecutive kx of one plane, loaded as N / BOX TMA boxes of
 // {2 BW floats, BOX rows} with the simulation's tensor map (maps[2 s] for y, maps[2 s + 1]
 // for z, in device memory).  One elected thread issues the loads of unit i+1 while all
 // threads transform unit i; finished bundles leave by TMA bulk store, and a stage is
-// refilled only once the store issued from it two iterations earlier has finished
+// refilled only once the store issued from it STAGES - 1 iterations earlier has finished
 // reading it.  Stages hold the bundles blocked (Blocked layout of pm_fft.cuh).
 // ---------------------------------------------------------------------------------
 // Green function of potential.py:15 / fourier_utils.py:15-16 (k = 0 -> 0; the 1/n^3 of the
