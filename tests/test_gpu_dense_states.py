@@ -137,3 +137,30 @@ def test_a_million_particles_in_a_cell(cuda, n, count):
     ctx.check_device()
     assert torch.equal(out, want) and torch.equal(p1, p2) and torch.equal(v1, v2)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [768, 1024])
+def test_dense_slab(cuda, n):
+    """The largest grids with dense tiles in a slab of 64 planes, more than there are CTAs: whole tiles of
+    768 cells, halves of 1024 (gates as test_dense_tiles; 0.3 particles per cell: 5e-8)."""
+    torch = cuda
+    from oracle import torch64
+    from pmgpu.config import Config
+    from pmgpu.context import PMContext
+    g = torch.Generator(device="cuda").manual_seed(n)
+    pos = torch.rand((3, int(0.3 * 64 * n * n)), generator=g, device="cuda")
+    pos[:2] *= n * (1 - 2 ** -20)
+    pos[2] *= 64
+    assert int((tile_entries(torch, pos, n) >= TWO_WORDS).sum()) > 1000
+    ctx = PMContext(Config(n_parts=n // 2, n_cells=n, box_size=100.0))
+    rho = ctx.density(pos, 1.0)
+    ref = torch64.density(pos.double(), 1.0, n)
+    assert float((rho.double() - ref).norm() / ref.norm()) < 7e-8
+    del ref
+    p1, p2, out = pos.clone(), pos.clone(), ctx.grid()
+    v1, v2 = torch.zeros_like(pos), torch.zeros_like(pos)
+    ctx.step(p1, v1, 1.0, 0.02, 0.00098)
+    ctx.step(p2, v2, 1.0, 0.02, 0.00098, rho_out=out)
+    ctx.check_device()
+    assert torch.equal(out, rho) and torch.equal(p1, p2) and torch.equal(v1, v2)
+    ctx.close()
